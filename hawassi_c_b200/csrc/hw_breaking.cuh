@@ -241,24 +241,26 @@ __device__ __forceinline__ void breaking_reset(Ctx<M>& X) {
   }
 }
 
-// criterion scan over this CTA's physical points (1d/breaking.c:36-61,72)
+// criterion scan (1d/breaking.c:36-61,72) over the listed points of the window
+// [xbstart, xbstart + lenIF) that are not below the threshold (the threads that formed
+// eta listed them): a few in a hundred, so one sweep of the CTA takes them, where a
+// thread that walked its own eight points waited for each crest in turn
+// (21 against 7 thousand cycles an RHS in the 256-member ensemble)
 template <int M>
 __device__ __forceinline__ void breaking_scan(Ctx<M>& X, const double2* PE, const double* Heta, int hs) {
   const DevMember& d = X.d;
   BrkDev* bk = d.bk;
-  const int N = d.N;
-  const int w0 = d.xbstart, w1 = d.xbstart + d.lenIF;   // window [w0, w1)
+  const int N = d.N, n = *X.ncand;
+  const int w0 = d.xbstart, w1 = d.xbstart + d.lenIF;
   bool above = false;
-  HW_FOREACH(X) {
-    (void)idx;
-    if (p >= w0 && p < w1) {
-      const double e = PE[p].x;
-      if (e > d.MaxEtaInit) above = true;
-      if (p >= w0 + 1 && p <= w1 - 2 && !(e < d.MaxEtaInit) && e > PE[p + 1].x && e > PE[p - 1].x &&
-          crest_breaks(d, PE, Heta, hs, p)) {
-        const int slot = atomicAdd(&bk->npk, 1);
-        if (slot < N) bk->pk[slot] = p;
-      }
+  for (int q = X.tid; q < n; q += Ctx<M>::T) {
+    const int p = X.cand[q];
+    const bool inner = p >= w0 + 1 && p <= w1 - 2;
+    const double e = PE[p].x, el = inner ? PE[p - 1].x : 0.0, er = inner ? PE[p + 1].x : 0.0;
+    if (e > d.MaxEtaInit) above = true;
+    if (inner && e > er && e > el && crest_breaks(d, PE, Heta, hs, p)) {
+      const int slot = atomicAdd(&bk->npk, 1);
+      if (slot < N) bk->pk[slot] = p;
     }
   }
   // one flag update per warp
@@ -269,8 +271,16 @@ template <int M>
 __device__ __forceinline__ void breaking_lead(Ctx<M>& X, double t, const double2* PE, const double* Heta, int hs) {
   if (X.c == 0 && X.tid == 0) {
     BrkDev* bk = X.d.bk;
-    if (bk->npk > X.d.N) bk->npk = X.d.N;
-    breaking_leader(X.d, bk, t, PE, Heta, hs);
+    const int npk = bk->npk, flag = bk->flag, touched = bk->n_touched, it = bk->ITERbdt;
+    const int dirty = bk->dirty_cb | bk->dirty_cbn;
+    if (npk == 0 && flag == 0 && touched == 0 && dirty == 0) {
+      // no crest passes and none is tracked: every record is clear, and all that
+      // breaking_leader would change is the output interval's counter
+      if (t > (it * X.d.dt_in)) bk->ITERbdt = it + 1;
+    } else {
+      if (npk > X.d.N) bk->npk = X.d.N;
+      breaking_leader(X.d, bk, t, PE, Heta, hs);
+    }
     __threadfence();
   }
 }
@@ -326,6 +336,13 @@ template <int M>
 __device__ __noinline__ bool breaking_rhs(Ctx<M>& X, double t, const double2* PE, const double* Heta, int hs,
                                           const double2* AEadj, double2* Rb) {
   breaking_reset(X);
+  if (X.tid == 0) *X.ncand = 0;
+  __syncthreads();
+  HW_FOREACH(X) {
+    (void)idx;
+    if (p >= X.d.xbstart && p < X.d.xbstart + X.d.lenIF && !(PE[p].x < X.d.MaxEtaInit))
+      X.cand[atomicAdd(X.ncand, 1)] = (unsigned short)p;
+  }
   member_sync(X.d.C);
   breaking_scan(X, PE, Heta, hs);
   member_sync(X.d.C);

@@ -45,6 +45,7 @@ struct DevMember {
   // geometry / model
   int N, C, M, logC;
   int model, flat, nref, brk, has_influx, prop_mode, n_in, exact;
+  int act;              // alias band: pairs {k, N-k} of a slice with first index >= act have aal == 0
   double invN, dx, eps_abs, eps_rel;
   // spectral tables, permuted "cyclic" order (position c*M + i holds wavenumber c + C*i)
   const double* k;
@@ -59,10 +60,12 @@ struct DevMember {
   // physical tables, natural order
   const double* dcoef;
   const double* dchar;
+  const double* damp;   // dcoef dchar
   const double* chi;
   const double* depth;
   const double* gam;    // [nref][N]
   // influx splines over ttrace
+  double tt0, tth, ttl; // first, second minus first and last influx time
   const double* tt;
   const double* ins;
   const double* insc;

@@ -235,7 +235,7 @@ bool hw_ctx::upload_member(HostMember& h) {
   // size the arena
   size_t bytes = 0;
   auto add = [&](size_t b) { bytes += ((b + 255) / 256) * 256; };
-  for (int i = 0; i < 10 + 2; ++i) add(sizeof(double) * N);                 // real tables
+  for (int i = 0; i < 10 + 3; ++i) add(sizeof(double) * N);                 // real tables
   add(sizeof(double2) * N * 2);                                              // gamX, gamXs
   add(sizeof(double) * size_t(N) * std::max(K, 1) * 2);                      // Csq, gam
   for (int i = 0; i < 5; ++i) add(sizeof(double) * std::max(n, 2));          // splines
@@ -281,6 +281,14 @@ bool hw_ctx::upload_member(HostMember& h) {
   d.aal = up(permute(m.aal, N, C, M), N);
   d.c1 = up(permute(c1, N, C, M), N);
   d.gk = up(permute(gk, N, C, M), N);
+  // first pair index outside the alias band (pair_at's ownership: partners count as
+  // their pair's first index; position M / 2 of CTA 0 goes with position 0)
+  for (int q = 0; q < N; ++q) {
+    const int c = q % C, i = q / C;
+    if (m.aal[q] == 0.0) continue;
+    const int first = i < M / 2 ? i : (c == 0 ? (M - i) % (M / 2) : M - 1 - i);
+    d.act = std::max(d.act, first + 1);
+  }
   d.M0im = up(permute(m.M0im, N, C, M), N);
   d.L = up(permute(m.L, N, C, M), N);
   {
@@ -303,9 +311,15 @@ bool hw_ctx::upload_member(HostMember& h) {
   }
   d.dcoef = up(m.dampcoef, N);
   d.dchar = up(m.dampchar, N);
+  std::vector<double> damp(N);
+  for (int i = 0; i < N; ++i) damp[i] = m.dampcoef[i] * m.dampchar[i];
+  d.damp = up(damp, N);
   d.chi = up(m.ChiAdj, N);
   d.depth = up(m.depth, N);
   const size_t ns = size_t(std::max(n, 2));
+  d.tt0 = m.ttrace[0];
+  d.tth = n > 1 ? m.ttrace[1] - m.ttrace[0] : 1.0;
+  d.ttl = m.ttrace[size_t(n - 1)];
   d.tt = up(m.ttrace, ns);
   d.ins = up(m.insig, ns);
   d.insc = up(m.sp_c_in.empty() ? std::vector<double>(ns, 0.0) : m.sp_c_in, ns);

@@ -19,17 +19,18 @@ namespace hwdev {
 // its stop index (clipping steps at each sample like the reference), mode 1 takes one
 // evolve_apply to sd.t1.  The member's descriptor is in shared memory (sd).
 template <int M>
-__device__ __forceinline__ void evolve_member(DevMember* mems, int mi, int mode, DevMember& sd, double* red,
+__device__ __forceinline__ void evolve_member(DevMember* mems, int mi, int mode, DevMember& sd, Scratch<M>& sc,
                                               double2* smem_buf, int C, int rank) {
   if (threadIdx.x == 0) sd = mems[mi];
   // a cluster barrier, not only the CTA's: the RHS's first phase writes into the
   // partner CTA's shared memory, which must be running
   member_sync(C);
-  Ctx<M> X = make_ctx<M>(sd, smem_buf, red, rank);
+  Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);
   Bufs B;
   B.y = sd.y;
   B.yn = sd.ynew;
   for (int i = 0; i < 7; ++i) B.k[i] = sd.kb[i];
+  spread_unmoved(X);
   StepState S{sd.t, sd.h, sd.status, sd.k1_valid, 0, 0, 0};
   int iout = sd.i_out;
   if (S.status == kOk) {
@@ -77,13 +78,13 @@ __global__ void __launch_bounds__(M / kPts, HW_EVOLVE_MIN_BLOCKS(M))
     k_evolve(DevMember* mems, const int* list, int mode, int* queue, int nlist) {
   extern __shared__ double2 smem_buf[];
   __shared__ DevMember sd;
-  __shared__ double red[48];
+  __shared__ Scratch<M> sc;
   __shared__ int s_next;
   cg::cluster_group cl = cg::this_cluster();
   const int C = int(cl.num_blocks());
   const int rank = int(cl.block_rank());
   if (!queue) {
-    evolve_member<M>(mems, list[blockIdx.x / C], mode, sd, red, smem_buf, C, rank);
+    evolve_member<M>(mems, list[blockIdx.x / C], mode, sd, sc, smem_buf, C, rank);
     return;
   }
   for (;;) {
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(M / kPts, HW_EVOLVE_MIN_BLOCKS(M))
     // member's work below passes through cluster barriers first
     const int w = C > 1 ? *cl.map_shared_rank(&s_next, 0) : s_next;
     if (w >= nlist) break;
-    evolve_member<M>(mems, list[w], mode, sd, red, smem_buf, C, rank);
+    evolve_member<M>(mems, list[w], mode, sd, sc, smem_buf, C, rank);
   }
   // no CTA leaves while a peer may still read its shared memory
   member_sync(C);
@@ -104,14 +105,15 @@ template <int M>
 __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs(DevMember* mems, const int* list, double t) {
   extern __shared__ double2 smem_buf[];
   __shared__ DevMember sd;
-  __shared__ double red[48];
+  __shared__ Scratch<M> sc;
   cg::cluster_group cl = cg::this_cluster();
   const int C = int(cl.num_blocks());
   const int rank = int(cl.block_rank());
   const int mi = list[blockIdx.x / C];
   if (threadIdx.x == 0) sd = mems[mi];
   __syncthreads();
-  Ctx<M> X = make_ctx<M>(sd, smem_buf, red, rank);
+  Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);
+  X.full = true;
   rhs_eval<M>(X, t, sd.kb[6]);
   member_sync(C);
   if (rank == 0 && threadIdx.x == 0) mems[mi].rhs_calls += 1;

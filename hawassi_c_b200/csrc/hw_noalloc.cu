@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs_noalloc(DevMember*
                                                                       double2* scratch) {
   extern __shared__ double2 smem_buf[];
   __shared__ DevMember sd;
-  __shared__ double red[48];
+  __shared__ Scratch<M> sc;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = int(cl.block_rank());
   if (threadIdx.x == 0) {
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs_noalloc(DevMember*
     for (int i = 0; i < kScratch; ++i) sd.sc[i] = scratch + size_t(4 + i) * N;
   }
   __syncthreads();
-  Ctx<M> X = make_ctx<M>(sd, smem_buf, red, rank);
+  Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);
   const int N = sd.N;
   // reference layout -> this CTA's spectral slice of the stage input
   HW_FOREACH(X) {
@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs_noalloc(DevMember*
     sd.zs[p] = make_double2(y_ref[kk], y_ref[N + kk]);
     sd.zs[N + p] = make_double2(y_ref[2 * N + kk], y_ref[3 * N + kk]);
   }
+  X.full = true;
   rhs_eval<M>(X, t, sd.kb[6]);
   HW_FOREACH(X) {
     const int kk = X.c + (idx << sd.logC);

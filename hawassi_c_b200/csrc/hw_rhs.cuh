@@ -43,39 +43,58 @@ struct StageSrc {
 __device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 
-// one element of the stage input, in GSL rkf45's expression forms
-__device__ __forceinline__ double2 stage_val(const StageSrc& st, int q) {
-  if (st.s == 1) return st.y[q];
-  const double2 y = st.y[q], a = st.k[0][q];
-  const double h = st.h;
-  if (st.s == 2) {
-    const double f = rmul(RK_ah[0], h);
-    return make_double2(radd(y.x, rmul(f, a.x)), radd(y.y, rmul(f, a.y)));
+// one element of the stage input of stage S (1: the state itself), in GSL rkf45's
+// expression forms, from values already loaded: k[j] is k_(j+1)
+template <int S>
+__device__ __forceinline__ double stage_comb(double y, double h, const double* k) {
+  if constexpr (S == 1) return y;
+  else if constexpr (S == 2) return radd(y, rmul(rmul(RK_ah[0], h), k[0]));
+  else if constexpr (S == 3) return radd(y, rmul(h, radd(rmul(RK_b3[0], k[0]), rmul(RK_b3[1], k[1]))));
+  else {
+    auto b = [](int j) { return S == 4 ? RK_b4[j] : (S == 5 ? RK_b5[j] : RK_b6[j]); };
+    double v = radd(rmul(b(0), k[0]), rmul(b(1), k[1]));
+#pragma unroll
+    for (int j = 2; j < S - 1; ++j) v = radd(v, rmul(b(j), k[j]));
+    return radd(y, rmul(h, v));
   }
-  const double2 b = st.k[1][q];
-  if (st.s == 3)
-    return make_double2(radd(y.x, rmul(h, radd(rmul(RK_b3[0], a.x), rmul(RK_b3[1], b.x)))),
-                        radd(y.y, rmul(h, radd(rmul(RK_b3[0], a.y), rmul(RK_b3[1], b.y)))));
-  const double2 c3 = st.k[2][q];
-  if (st.s == 4)
-    return make_double2(
-        radd(y.x, rmul(h, radd(radd(rmul(RK_b4[0], a.x), rmul(RK_b4[1], b.x)), rmul(RK_b4[2], c3.x)))),
-        radd(y.y, rmul(h, radd(radd(rmul(RK_b4[0], a.y), rmul(RK_b4[1], b.y)), rmul(RK_b4[2], c3.y)))));
-  const double2 c4 = st.k[3][q];
-  if (st.s == 5)
-    return make_double2(
-        radd(y.x, rmul(h, radd(radd(radd(rmul(RK_b5[0], a.x), rmul(RK_b5[1], b.x)), rmul(RK_b5[2], c3.x)),
-                               rmul(RK_b5[3], c4.x)))),
-        radd(y.y, rmul(h, radd(radd(radd(rmul(RK_b5[0], a.y), rmul(RK_b5[1], b.y)), rmul(RK_b5[2], c3.y)),
-                               rmul(RK_b5[3], c4.y)))));
-  const double2 c5 = st.k[4][q];
-  return make_double2(
-      radd(y.x, rmul(h, radd(radd(radd(radd(rmul(RK_b6[0], a.x), rmul(RK_b6[1], b.x)), rmul(RK_b6[2], c3.x)),
-                                  rmul(RK_b6[3], c4.x)),
-                             rmul(RK_b6[4], c5.x)))),
-      radd(y.y, rmul(h, radd(radd(radd(radd(rmul(RK_b6[0], a.y), rmul(RK_b6[1], b.y)), rmul(RK_b6[2], c3.y)),
-                                  rmul(RK_b6[3], c4.y)),
-                             rmul(RK_b6[4], c5.y)))));
+}
+
+// the operands of stage value q: loaded apart from their use, so that a thread has
+// those of several values in flight
+template <int S>
+struct StageOps {
+  double2 y, k[S > 1 ? S - 1 : 1];
+  __device__ __forceinline__ void load(const double2* __restrict__ ys, const double2* const* ks, int q) {
+    y = ys[q];
+#pragma unroll
+    for (int j = 0; j < S - 1; ++j) k[j] = ks[j][q];
+  }
+  __device__ __forceinline__ double2 value(double h) const {
+    double kx[S > 1 ? S - 1 : 1], ky[S > 1 ? S - 1 : 1];
+#pragma unroll
+    for (int j = 0; j < S - 1; ++j) {
+      kx[j] = k[j].x;
+      ky[j] = k[j].y;
+    }
+    return make_double2(stage_comb<S>(y.x, h, kx), stage_comb<S>(y.y, h, ky));
+  }
+};
+
+template <int S>
+__device__ __forceinline__ double2 stage_one(const StageSrc& st, int q) {
+  StageOps<S> o;
+  o.load(st.y, st.k, q);
+  return o.value(st.h);
+}
+__device__ __forceinline__ double2 stage_val(const StageSrc& st, int q) {
+  switch (st.s) {
+    case 1: return stage_one<1>(st, q);
+    case 2: return stage_one<2>(st, q);
+    case 3: return stage_one<3>(st, q);
+    case 4: return stage_one<4>(st, q);
+    case 5: return stage_one<5>(st, q);
+    default: return stage_one<6>(st, q);
+  }
 }
 
 template <int M>
@@ -84,19 +103,53 @@ struct Ctx {
   const DevMember& d;
   double2* buf;   // M-point FFT slice (padded) in shared memory
   double2* buf2;  // second slice for the dual transforms
-  double* red;    // reduction scratch in shared memory
+  double* red;    // reduction scratch in shared memory (kRed doubles)
+  unsigned short* cand;   // grid points of this CTA's threads above the breaking threshold
+  int* ncand;
   int c;          // rank of this CTA in the member's cluster
   int tid;
   const StageSrc* stg = nullptr;   // set: zs is to be formed from y and the k's first
+  bool full = false;               // dz is written outside the alias band too (as zeros)
 };
+
+// scratch of one CTA in static shared memory, beside the transform slices
+constexpr int kRed = 48;
+constexpr int kRedPv = 40, kRedPs = 41;   // influx signals at the stage time
+template <int M>
+struct Scratch {
+  double red[kRed];
+  int ncand;
+  unsigned short cand[M];
+};
+
+// The Hermitian pairs {k, N-k} of the member, each owned by one thread wherever spectral
+// values are formed: CTA c takes the first half of its slice, i < M / 2, with the
+// partners, which lie in the second half of CTA (C - c) mod C.  Positions 0 and M / 2
+// of CTA 0 are their own partners; they go as one "pair" of two such points (self).
+// The owner is the same in every phase, so the RK vectors need no barrier between the
+// phase that writes them and the ones that read them.
+struct PairAt {
+  int i, j, p, pp;   // slice indices and positions of the two points
+  bool self;
+};
+template <int M>
+__device__ __forceinline__ PairAt pair_at(int c, int cq, int i) {
+  PairAt r;
+  r.i = i;
+  r.self = c == 0 && i == 0;
+  r.j = r.self ? M / 2 : (c == 0 ? M - i : M - 1 - i);
+  r.p = c * M + r.i;
+  r.pp = cq * M + r.j;
+  return r;
+}
 
 // dynamic shared memory of the 1D kernels of slice M: two padded FFT slices (no more:
 // what the SM does not give to shared memory serves as L1 cache)
 __host__ __device__ constexpr size_t slice_smem_bytes(int m) { return 2 * size_t(padded(m)) * sizeof(double2); }
 
 template <int M>
-__device__ __forceinline__ Ctx<M> make_ctx(const DevMember& d, double2* smem, double* red, int rank) {
-  return Ctx<M>{d, smem, smem + padded(M), red, rank, int(threadIdx.x)};
+__device__ __forceinline__ Ctx<M> make_ctx(const DevMember& d, double2* smem, Scratch<M>& sc, int rank) {
+  return Ctx<M>{d, smem, smem + padded(M), sc.red, sc.cand, &sc.ncand, rank, int(threadIdx.x)};
 }
 
 #define HW_FOREACH(X)                            \
@@ -164,20 +217,32 @@ __device__ __forceinline__ void fft_inverse_then(Ctx<M>& X, G&& g) {
   HW_FOREACH(X) { g(u, idx, p, X.buf[pidx(idx)]); }
 }
 
-// natural cubic spline evaluation (GSL cspline + bsearch index rule)
-__device__ __forceinline__ double spline_eval(const double* __restrict__ x, const double* __restrict__ y,
-                                              const double* __restrict__ c, int n, double t) {
-  if (!(t >= x[0] && t <= x[n - 1])) return __longlong_as_double(0x7ff8000000000000ULL);
-  const double h0 = x[1] - x[0];
-  int lo = int((t - x[0]) / h0);
+// natural cubic spline evaluation (GSL cspline + bsearch index rule) of the influx
+// signal and its running integral at t.  Both need the same interval: every value of a
+// guessed one is loaded at once, and the guess moves on if the samples' times ask for it.
+__device__ __forceinline__ double2 influx_at(const DevMember& d, double t) {
+  const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+  if (!(t >= d.tt0 && t <= d.ttl)) return make_double2(nan, nan);
+  const int n = d.n_in;
+  int lo = int((t - d.tt0) / d.tth);
   lo = lo < 0 ? 0 : (lo > n - 2 ? n - 2 : lo);
-  while (lo > 0 && x[lo] > t) --lo;
-  while (lo < n - 2 && x[lo + 1] <= t) ++lo;
-  const double xl = x[lo], h = x[lo + 1] - xl, dy = y[lo + 1] - y[lo], delx = t - xl;
-  const double ci = c[lo], cp = c[lo + 1];
-  const double b = dy / h - h * (cp + 2.0 * ci) / 3.0;
-  const double dd = (cp - ci) / (3.0 * h);
-  return y[lo] + delx * (b + delx * (ci + delx * dd));
+  double xl, xh, y0, y1, c0, c1, s0, s1, e0, e1;
+  for (;;) {
+    xl = d.tt[lo]; xh = d.tt[lo + 1];
+    y0 = d.ins[lo]; y1 = d.ins[lo + 1]; c0 = d.insc[lo]; c1 = d.insc[lo + 1];
+    s0 = d.skw[lo]; s1 = d.skw[lo + 1]; e0 = d.skwc[lo]; e1 = d.skwc[lo + 1];
+    if (lo > 0 && xl > t) --lo;
+    else if (lo < n - 2 && xh <= t) ++lo;
+    else break;
+  }
+  const double h = xh - xl, delx = t - xl;
+  auto cubic = [&](double a, double b, double ci, double cp) {
+    const double dy = b - a;
+    const double bb = dy / h - h * (cp + 2.0 * ci) / 3.0;
+    const double dd = (cp - ci) / (3.0 * h);
+    return a + delx * (bb + delx * (ci + delx * dd));
+  };
+  return make_double2(cubic(y0, y1, c0, c1), cubic(s0, s1, e0, e1));
 }
 
 // HSS (1d/functions.c:2861): out = 1/2 sum_j [ F(gam_j Re F^-1(Csq_j A)) + Csq_j F(gam_j a) ]
@@ -461,8 +526,9 @@ __device__ __noinline__ void rhs_eval(Ctx<M>& X, double t, double2* __restrict__
   // (11) assembly (1d/rhs.c:217-228, 373-385, 73-83) with the source term (1d/rhs.c:659)
   double pv = 0.0, ps = 0.0;
   if (d.has_influx) {
-    pv = spline_eval(d.tt, d.ins, d.insc, d.n_in, t);
-    ps = spline_eval(d.tt, d.skw, d.skwc, d.n_in, t);
+    const double2 s = influx_at(d, t);
+    pv = s.x;
+    ps = s.y;
   }
   member_sync(d.C);
   HW_FOREACH(X) {

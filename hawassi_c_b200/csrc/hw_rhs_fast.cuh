@@ -1,55 +1,137 @@
 // hw_rhs_fast.cuh -- HS2 on a flat bottom (rhs_HsF2 with ifft_fft_Hsf2,
 // 1d/rhs.c:96-241, 1d/functions.c:1458-1526), the hot path of the plain and the
 // batched runs, with the fields kept in two shared-memory slices:
-//   * stage input -> Hermitian packing through shared memory / DSMEM partners;
+//   * stage input -> Hermitian packing, pair by pair;
 //   * eta, u and M0 u, Hilbert(eta) from one dual inverse transform;
-//   * the five real products from one dual forward transform;
+//   * the three real products from one dual forward transform;
 //   * the nonlinear adjustment: one inverse transform, ChiAdj, and a dual forward
-//     transform that also carries the damping of u.
-// Global memory sees the stage input, the per-point tables and five spectral
-// results per point (d^ eta, d^ u, adjusted nonlinear terms, damping), instead
-// of a round trip per transform.
+//     transform that also carries the damping of eta and u.
+// What bounds it: the latency of the loads between the transforms.  Each phase names
+// its loads before its stores, the pair's owner forms both of its points (half the
+// table loads), and outside the alias band, where aal = 0 and every k_j is zero (half
+// the pairs under HS2), nothing but y is read.  Against loads taken point by point
+// (B200, 256 ragged members, thousand cycles a CTA and RHS): stage input 57 -> 16,
+// assembly 32 -> 10, H2 terms 14 -> 5, criterion 21 -> 7, the transforms 38 as before;
+// three output samples of the ensemble 111 -> 69 ms, ten of one 4096-point tank (512-point
+// slices) 27.6 -> 17.1 ms.
 #pragma once
 
 #include "hw_rhs.cuh"
 
 namespace hwdev {
 
-// Hilbert-transform multiplier of the breaking criterion (1d/breaking.c:133-143)
-__device__ __forceinline__ double2 hilbert_hat(double k, double2 e) {
-  if (k == 0) return make_double2(0.0, 0.0);
-  const double s = k / fabs(k);
-  return make_double2(s * e.y, -s * e.x);
+// (A + i B) s of a pair's first point, and of its partner, from the Hermitian parts
+// A, B at the first (the partner's are their conjugates)
+__device__ __forceinline__ double2 pack_conj(double2 a, double2 b, double s) {
+  return make_double2((a.x + b.y) * s, (b.x - a.y) * s);
 }
 
-// the influx source term of the assembly (1d/rhs.c:659-693): force = (fr, fi)
-__device__ __forceinline__ void source_term(const DevMember& d, int p, double pv, double ps, double& fr, double& fi) {
-  fr = 0.0;
-  fi = 0.0;
-  if (d.has_influx) {
-    const double2 gx = d.gamX[p], gs = d.gamXs[p];
-    if (d.prop_mode == 0) { fr = 0.5 * (pv * gx.x - ps * gs.x); fi = 0.5 * (pv * gx.y - ps * gs.y); }
-    else if (d.prop_mode == 1) { fr = 0.5 * (pv * gx.x + ps * gs.x); fi = 0.5 * (pv * gx.y + ps * gs.y); }
-    else if (d.prop_mode == 2) { fr = pv * gx.x; fi = pv * gx.y; }
+// shared-memory slices of the CTA that holds the partners
+template <int M>
+struct PairBufs {
+  double2 *Aq, *Bq;
+  int cq;
+  __device__ __forceinline__ PairBufs(Ctx<M>& X) {
+    cq = (X.d.C - X.c) & (X.d.C - 1);
+    Aq = X.buf;
+    Bq = X.buf2;
+    if (cq != X.c) {
+      cg::cluster_group cl = cg::this_cluster();
+      Aq = cl.map_shared_rank(X.buf, cq);
+      Bq = cl.map_shared_rank(X.buf2, cq);
+    }
+  }
+};
+
+// Stage input of stage S (y + h sum_j b_sj k_j, kept in zs for the assembly) and its
+// Hermitian packing for the first dual inverse transform: A <- eta^ + i u^,
+// B <- M0 u^ + i H(eta)^ (real parts only, as the reference).  M0 u^ = -i c1 u^ and the
+// Hilbert multiplier (1d/breaking.c:133-143) takes the sign of c1 = (C^2/g) k.
+// The stage is a template argument so that a pair's loads (up to 24) are independent
+// of any branch and in flight together.
+template <int M, int S>
+__device__ __noinline__ void stage_pack(Ctx<M>& X) {
+  const DevMember& d = X.d;
+  constexpr int T = Ctx<M>::T;
+  const double2* y = X.stg->y;
+  const double2* ks[S > 1 ? S - 1 : 1];
+#pragma unroll
+  for (int j = 0; j < S - 1; ++j) ks[j] = X.stg->k[j];
+  const double h = X.stg->h, invN = d.invN;
+  const double* __restrict__ c1 = d.c1;
+  double2* zw = d.zs;
+  const int N = d.N, c = X.c, act = d.act;
+  const bool brk = d.brk != 0;
+  const PairBufs<M> pb(X);
+  double2 *A = X.buf, *B = X.buf2, *Aq = pb.Aq, *Bq = pb.Bq;
+  auto emit = [&](const PairAt& r, double ca, double cb, double2 e, double2 ep, double2 w, double2 wp) {
+    auto point = [&](double k, double kq, double2 f, double2 fp, double2 g, double2 gp, double2& H, double2& S2) {
+      H = herm(make_double2(k * g.y, -k * g.x), make_double2(kq * gp.y, -kq * gp.x));
+      S2 = make_double2(0.0, 0.0);
+      if (brk) {
+        const double s = k == 0 ? 0.0 : copysign(1.0, k), sq = kq == 0 ? 0.0 : copysign(1.0, kq);
+        S2 = herm(make_double2(s * f.y, -s * f.x), make_double2(sq * fp.y, -sq * fp.x));
+      }
+    };
+    double2 H, S2;
+    if (r.self) {
+      point(ca, ca, e, e, w, w, H, S2);
+      A[pidx(r.i)] = pack(herm(e, e), herm(w, w), invN);
+      B[pidx(r.i)] = pack(H, S2, invN);
+      point(cb, cb, ep, ep, wp, wp, H, S2);
+      A[pidx(r.j)] = pack(herm(ep, ep), herm(wp, wp), invN);
+      B[pidx(r.j)] = pack(H, S2, invN);
+      return;
+    }
+    const double2 E = herm(e, ep), W = herm(w, wp);
+    point(ca, cb, e, ep, w, wp, H, S2);
+    A[pidx(r.i)] = pack(E, W, invN);
+    Aq[pidx(r.j)] = pack_conj(E, W, invN);
+    B[pidx(r.i)] = pack(H, S2, invN);
+    Bq[pidx(r.j)] = pack_conj(H, S2, invN);
+  };
+#pragma unroll 1
+  for (int u = 0; u < kPts / 2; ++u) {
+    const PairAt r = pair_at<M>(c, pb.cq, X.tid + u * T);
+    const double ca = c1[r.p], cb = c1[r.pp];
+    if (r.i < act) {
+      StageOps<S> oe, oep, ow, owp;
+      oe.load(y, ks, r.p);
+      oep.load(y, ks, r.pp);
+      ow.load(y, ks, N + r.p);
+      owp.load(y, ks, N + r.pp);
+      const double2 e = oe.value(h), ep = oep.value(h), w = ow.value(h), wp = owp.value(h);
+      if (S > 1 || zw != y) {   // (a direct RHS's state is zs itself)
+        zw[r.p] = e;
+        zw[r.pp] = ep;
+        zw[N + r.p] = w;
+        zw[N + r.pp] = wp;
+      }
+      emit(r, ca, cb, e, ep, w, wp);
+    } else {
+      emit(r, ca, cb, y[r.p], y[r.pp], y[N + r.p], y[N + r.pp]);
+    }
   }
 }
 
-// assembly of dz at spectral position p (1d/rhs.c:217-228): delta H1 + adjusted
-// nonlinear terms (ae, au) + breaking force (rb) + 2 force - damping (de, du), times aal
-__device__ __forceinline__ void assemble_flat(const DevMember& d, int p, double2 ae, double2 au, double2 rb, double2 de,
-                                              double2 du, double pv, double ps, double2* __restrict__ dz) {
-  const int N = d.N;
-  const double2 ze = d.zs[p], zu = d.zs[N + p];
-  const double c1 = d.c1[p], gk = d.gk[p];
-  double2 te = make_double2(c1 * zu.y, -c1 * zu.x);
-  double2 tu = make_double2(gk * ze.y, -gk * ze.x);
-  double fr, fi;
-  source_term(d, p, pv, ps, fr, fi);
-  const double al = d.aal[p];
-  te = cadd(te, ae);
-  tu = cadd(cadd(tu, au), rb);
-  dz[p] = make_double2((te.x + 2 * fr - de.x) * al, (te.y + 2 * fi - de.y) * al);
-  dz[N + p] = make_double2((tu.x - du.x) * al, (tu.y - du.y) * al);
+template <int M>
+__device__ __forceinline__ void stage_pack_any(Ctx<M>& X) {
+  switch (X.stg->s) {
+    case 1: stage_pack<M, 1>(X); break;
+    case 2: stage_pack<M, 2>(X); break;
+    case 3: stage_pack<M, 3>(X); break;
+    case 4: stage_pack<M, 4>(X); break;
+    case 5: stage_pack<M, 5>(X); break;
+    default: stage_pack<M, 6>(X); break;
+  }
+}
+
+// the influx source term of the assembly (1d/rhs.c:659-693) from the loaded kernels
+__device__ __forceinline__ double2 source_term(int mode, double2 gx, double2 gs, double pv, double ps) {
+  if (mode == 0) return make_double2(0.5 * (pv * gx.x - ps * gs.x), 0.5 * (pv * gx.y - ps * gs.y));
+  if (mode == 1) return make_double2(0.5 * (pv * gx.x + ps * gs.x), 0.5 * (pv * gx.y + ps * gs.y));
+  if (mode == 2) return make_double2(pv * gx.x, pv * gx.y);
+  return make_double2(0.0, 0.0);
 }
 
 // Cluster members: the inverse transform's cross-CTA step, the pointwise work in
@@ -59,32 +141,55 @@ __device__ __forceinline__ void assemble_flat(const DevMember& d, int p, double2
 // all three in registers: gather, twiddle, inverse C-point DFT, pointwise step,
 // forward C-point DFT, twiddle, scatter.  Two cluster barriers replace four and the
 // physical fields never pass through shared memory.
-//
-// First meeting (1d/functions.c:1486-1498): A = eta + i u, B = M0 u + i H(eta) in;
-// out A = (eta u) + i (eta M0 u), B = (u^2 - (M0 u)^2) + i (damping of eta); the
-// damping of u waits in the member's scratch (damp_u_field) for the second meeting;
-// eta, u and H(eta) go to global memory for the breaking criterion.
-// the physical damping of u between the products and the adjustment, one double per
-// grid point in the member's scratch field 5 (used for the spectral damping of u only
-// after that); kept out of shared memory, which leaves the SM more L1 cache
-__device__ __forceinline__ double* damp_u_field(const DevMember& d) { return reinterpret_cast<double*>(d.sc[5]); }
+
+// What the first meeting does at physical point n (1d/functions.c:1486-1498), given
+// e = (eta, u), m = (M0 u, H(eta)): a <- (eta u) + i (eta M0 u), b <- u^2 - (M0 u)^2.
+// (eta, u) goes to global memory where the damping zones read it back, and with
+// breaking everywhere, beside H(eta) and a list of the points above the threshold.
+template <int M>
+__device__ __forceinline__ void product_point(Ctx<M>& X, int n, double2 e, double2 m, double damp, double2* PE,
+                                              double2* PM, double2& a, double2& b) {
+  const DevMember& d = X.d;
+  if (d.brk) {
+    PE[n] = e;
+    PM[n].y = m.y;
+    if (n >= d.xbstart && n < d.xbstart + d.lenIF && !(e.x < d.MaxEtaInit))
+      X.cand[atomicAdd(X.ncand, 1)] = (unsigned short)n;
+  } else if (damp != 0.0) {
+    PE[n] = e;
+  }
+  a = make_double2(e.x * e.y, e.x * m.x);
+  b = make_double2(e.y * e.y - m.x * m.x, 0.0);
+}
+
+// What the second meeting does (1d/rhs.c:695-715): the nonlinear terms times ChiAdj,
+// paired with the damping of eta and u
+__device__ __forceinline__ void adjust_point(const double2* PE, int n, double chi, double damp, double2& a, double2& b) {
+  a = make_double2(a.x * chi, a.y * chi);
+  b = make_double2(0.0, 0.0);
+  if (damp != 0.0) {
+    const double2 e = PE[n];
+    b = make_double2(damp * e.x, damp * e.y);
+  }
+}
 
 template <int M, int C>
-__device__ __forceinline__ void cross_products(Ctx<M>& X, double2* A, double2* B, bool brk, double2* PE, double2* PM) {
+__device__ __forceinline__ void cross_products(Ctx<M>& X, double2* A, double2* B, double2* PE, double2* PM) {
   constexpr int T = M / kPts;
   constexpr int PER = kPts / C;
   const DevMember& d = X.d;
-  double* du = damp_u_field(d);
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
     const int i = X.c * T + X.tid + q * (C * T);
     double2 va[C], vb[C], w[C > 1 ? C : 2];
+    double dm[C];
 #pragma unroll
     for (int r = 0; r < C; ++r) {
       va[r] = cl.map_shared_rank(A, r)[pidx(i)];
       vb[r] = cl.map_shared_rank(B, r)[pidx(i)];
+      dm[r] = __ldg(d.damp + r * M + i);
     }
     twiddle_powers<C>(twd(d.tw, i, +1), w);
 #pragma unroll
@@ -95,25 +200,13 @@ __device__ __forceinline__ void cross_products(Ctx<M>& X, double2* A, double2* B
     dft_small<C>(va, +1);
     dft_small<C>(vb, +1);
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      const int n = r * M + i;
-      const double2 e = va[r], m = vb[r];
-      if (brk) {
-        PE[n] = e;
-        PM[n].y = m.y;
-      }
-      const double dc = d.dcoef[n], ch = d.dchar[n];
-      du[n] = (dc * e.y) * ch;
-      va[r] = make_double2(e.x * e.y, e.x * m.x);
-      vb[r] = make_double2(e.y * e.y - m.x * m.x, (dc * e.x) * ch);
-    }
+    for (int r = 0; r < C; ++r) product_point<M>(X, r * M + i, va[r], vb[r], dm[r], PE, PM, va[r], vb[r]);
     dft_small<C>(va, -1);
     dft_small<C>(vb, -1);
-    twiddle_powers<C>(twd(d.tw, i, -1), w);
 #pragma unroll
     for (int r = 1; r < C; ++r) {
-      va[r] = cmul(va[r], w[r]);
-      vb[r] = cmul(vb[r], w[r]);
+      va[r] = cmul(va[r], cconj(w[r]));
+      vb[r] = cmul(vb[r], cconj(w[r]));
     }
 #pragma unroll
     for (int r = 0; r < C; ++r) {
@@ -124,40 +217,36 @@ __device__ __forceinline__ void cross_products(Ctx<M>& X, double2* A, double2* B
   cl.sync();
 }
 
-// Second meeting (1d/rhs.c:695-715): the nonlinear terms' inverse transform times
-// ChiAdj, paired with the damping of u kept by the first meeting, into the forward
-// dual transform: A in (one transform), out A = ChiAdj-adjusted terms, B = damping of u.
 template <int M, int C>
-__device__ __forceinline__ void cross_adjust(Ctx<M>& X, double2* A, double2* B) {
+__device__ __forceinline__ void cross_adjust(Ctx<M>& X, double2* A, double2* B, const double2* PE) {
   constexpr int T = M / kPts;
   constexpr int PER = kPts / C;
   const DevMember& d = X.d;
-  const double* du = damp_u_field(d);
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
     const int i = X.c * T + X.tid + q * (C * T);
     double2 va[C], vb[C], w[C > 1 ? C : 2];
+    double dm[C], ch[C];
 #pragma unroll
-    for (int r = 0; r < C; ++r) va[r] = cl.map_shared_rank(A, r)[pidx(i)];
+    for (int r = 0; r < C; ++r) {
+      va[r] = cl.map_shared_rank(A, r)[pidx(i)];
+      dm[r] = __ldg(d.damp + r * M + i);
+      ch[r] = __ldg(d.chi + r * M + i);
+    }
     twiddle_powers<C>(twd(d.tw, i, +1), w);
 #pragma unroll
     for (int r = 1; r < C; ++r) va[r] = cmul(va[r], w[r]);
     dft_small<C>(va, +1);
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      const double ch = d.chi[r * M + i];
-      va[r] = make_double2(va[r].x * ch, va[r].y * ch);
-      vb[r] = make_double2(du[r * M + i], 0.0);
-    }
+    for (int r = 0; r < C; ++r) adjust_point(PE, r * M + i, ch[r], dm[r], va[r], vb[r]);
     dft_small<C>(va, -1);
     dft_small<C>(vb, -1);
-    twiddle_powers<C>(twd(d.tw, i, -1), w);
 #pragma unroll
     for (int r = 1; r < C; ++r) {
-      va[r] = cmul(va[r], w[r]);
-      vb[r] = cmul(vb[r], w[r]);
+      va[r] = cmul(va[r], cconj(w[r]));
+      vb[r] = cmul(vb[r], cconj(w[r]));
     }
 #pragma unroll
     for (int r = 0; r < C; ++r) {
@@ -169,228 +258,235 @@ __device__ __forceinline__ void cross_adjust(Ctx<M>& X, double2* A, double2* B) 
 }
 
 template <int M>
-__device__ __forceinline__ void cross_products_any(Ctx<M>& X, double2* A, double2* B, bool brk, double2* PE, double2* PM) {
-  if (X.d.C == 2) cross_products<M, 2>(X, A, B, brk, PE, PM);
-  else if (X.d.C == 4) cross_products<M, 4>(X, A, B, brk, PE, PM);
-  else cross_products<M, 8>(X, A, B, brk, PE, PM);
+__device__ __forceinline__ void cross_products_any(Ctx<M>& X, double2* A, double2* B, double2* PE, double2* PM) {
+  if (X.d.C == 2) cross_products<M, 2>(X, A, B, PE, PM);
+  else if (X.d.C == 4) cross_products<M, 4>(X, A, B, PE, PM);
+  else cross_products<M, 8>(X, A, B, PE, PM);
 }
 template <int M>
-__device__ __forceinline__ void cross_adjust_any(Ctx<M>& X, double2* A, double2* B) {
-  if (X.d.C == 2) cross_adjust<M, 2>(X, A, B);
-  else if (X.d.C == 4) cross_adjust<M, 4>(X, A, B);
-  else cross_adjust<M, 8>(X, A, B);
+__device__ __forceinline__ void cross_adjust_any(Ctx<M>& X, double2* A, double2* B, const double2* PE) {
+  if (X.d.C == 2) cross_adjust<M, 2>(X, A, B, PE);
+  else if (X.d.C == 4) cross_adjust<M, 4>(X, A, B, PE);
+  else cross_adjust<M, 8>(X, A, B, PE);
+}
+
+// Assembly of dz (1d/rhs.c:217-228): delta H1 + adjusted nonlinear terms + breaking
+// force + 2 force - damping, times aal, for the pairs inside the alias band; outside it
+// dz is zero, and was when the buffer was made.  LIVE: the adjusted terms and the force
+// come from the scratch fields (some node breaks), else from the slices.
+template <int M, bool LIVE>
+__device__ __noinline__ void assemble_flat(Ctx<M>& X, double2* __restrict__ dz, const double2* AE, const double2* AU,
+                                           const double2* RB) {
+  const DevMember& d = X.d;
+  constexpr int T = Ctx<M>::T;
+  const int N = d.N, c = X.c, act = d.act, mode = d.has_influx ? d.prop_mode : 3;
+  const PairBufs<M> pb(X);
+  const double2 *A = X.buf, *B = X.buf2, *Aq = pb.Aq, *Bq = pb.Bq;
+  const double2* zs = d.zs;
+  const double* __restrict__ kt = d.k;
+  const double* __restrict__ c1t = d.c1;
+  const double* __restrict__ aalt = d.aal;
+  const double2* __restrict__ gxt = d.gamX;
+  const double2* __restrict__ gst = d.gamXs;
+  const double pv = X.red[kRedPv], ps = X.red[kRedPs];
+#pragma unroll 1
+  for (int u = 0; u < kPts / 2; ++u) {
+    const PairAt r = pair_at<M>(c, pb.cq, X.tid + u * T);
+    if (r.i >= act) {
+      if (X.full) dz[r.p] = dz[r.pp] = dz[N + r.p] = dz[N + r.pp] = make_double2(0.0, 0.0);
+      continue;
+    }
+    const int pos[2] = {r.p, r.pp};
+    double2 ze[2], zu[2], gx[2], gs[2], ae[2], au[2];
+    double kk[2], c1[2], al[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      ze[s] = zs[pos[s]];
+      zu[s] = zs[N + pos[s]];
+      kk[s] = kt[pos[s]];
+      c1[s] = c1t[pos[s]];
+      al[s] = aalt[pos[s]];
+      gx[s] = gs[s] = make_double2(0.0, 0.0);
+      if (mode != 3) {
+        gx[s] = gxt[pos[s]];
+        gs[s] = gst[pos[s]];
+      }
+      if constexpr (LIVE) {
+        const double2 f = RB[pos[s]];
+        ae[s] = AE[pos[s]];
+        au[s] = cadd(AU[pos[s]], f);
+      }
+    }
+    const double2 z = A[pidx(r.i)], zp = Aq[pidx(r.j)], zb = B[pidx(r.i)], zbp = Bq[pidx(r.j)];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const double2 a = s ? zp : z, b = s ? zbp : zb;
+      const double2 aq = r.self ? a : (s ? z : zp), bq = r.self ? b : (s ? zb : zbp);
+      if constexpr (!LIVE) {
+        ae[s] = split_re(a, aq);
+        au[s] = split_im(a, aq);
+      }
+      const double2 de = split_re(b, bq), du = split_im(b, bq);
+      const double gk = kG * kk[s];
+      const double2 f = source_term(mode, gx[s], gs[s], pv, ps);
+      const double2 te = make_double2(c1[s] * zu[s].y + ae[s].x, -c1[s] * zu[s].x + ae[s].y);
+      const double2 tu = make_double2(gk * ze[s].y + au[s].x, -gk * ze[s].x + au[s].y);
+      dz[pos[s]] = make_double2((te.x + 2 * f.x - de.x) * al[s], (te.y + 2 * f.y - de.y) * al[s]);
+      dz[N + pos[s]] = make_double2((tu.x - du.x) * al[s], (tu.y - du.y) * al[s]);
+    }
+  }
 }
 
 template <int M>
 __device__ __noinline__ void rhs_hs2_flat(Ctx<M>& X, double t, double2* __restrict__ dz) {
   const DevMember& d = X.d;
-  const int N = d.N, C = d.C;
+  constexpr int T = Ctx<M>::T;
+  const int C = d.C;
   double2* A = X.buf;
   double2* Bf = X.buf2;
-  const double2* ZE = d.zs;
-  const double2* ZU = d.zs + N;
-  double2* PE = d.sc[0];   // physical (eta, u)           [breaking only]
+  double2* PE = d.sc[0];   // physical (eta, u)           [breaking, and in the damping zones]
   double2* PM = d.sc[1];   // physical (., Hilbert eta)   [breaking only]
   double2* AE = d.sc[2];   // adjusted nonlinear eta term [breaking force live only]
   double2* AU = d.sc[3];   // adjusted nonlinear u term   [breaking force live only]
-  double2* DE = d.sc[4];   // FFT(damping eta)
-  double2* DU = d.sc[5];   // FFT(damping u)              [breaking force live only]
   double2* RB = d.sc[11];  // FFT(breaking force)
   const bool brk = d.brk != 0;
-  const double2* Ap = A;
-  const double2* Bp = Bf;
-  if (C > 1) {
-    cg::cluster_group cl = cg::this_cluster();
-    const int cp = (C - X.c) & (C - 1);
-    Ap = cl.map_shared_rank(A, cp);
-    Bp = cl.map_shared_rank(Bf, cp);
-  }
-  auto jpart = [&](int idx) { return X.c == 0 ? ((M - idx) & (M - 1)) : (M - 1 - idx); };
-  double2 va[kPts], vb[kPts];
+  const PairBufs<M> pb(X);
 
-  // (0)-(1) stage input (spectral, cyclic) and its Hermitian packing for the first
-  // dual inverse transform: A <- eta^ + i u^, B <- M0 u^ + i H(eta)^ (real parts
-  // only, as the reference).  Every exit of this function leaves the slices unread
-  // by the other CTAs (a barrier follows the last partner reads), so they can be
-  // written at once.
+  // (0)-(1) stage input and its packing.  Every exit of this function leaves the slices
+  // unread by the other CTAs (a barrier follows the last partner reads), so they can be
+  // written at once; with zs written by the caller, other threads' writes of it and the
+  // start of the partner CTA come first.
   if (brk) breaking_reset(X);
-  auto packed = [&](int p, int pp, double2 e, double2 ep, double2 w, double2 wp, double2& a, double2& b) {
-    a = pack(herm(e, ep), herm(w, wp), d.invN);
-    const double2 m0 = mul_ik(d.M0im[p], w), m0p = mul_ik(d.M0im[pp], wp);
-    const double2 s2 = brk ? herm(hilbert_hat(d.k[p], e), hilbert_hat(d.k[pp], ep)) : make_double2(0.0, 0.0);
-    b = pack(herm(m0, m0p), s2, d.invN);
-  };
+  if (X.tid == 0) *X.ncand = 0;
   if (X.stg) {
-    // during a step the stage input is formed here from y and the k's (and kept in
-    // zs for the assembly).  Each Hermitian pair {k, N - k} is formed once, by one
-    // thread: CTA c takes the first half of its slice, i < M / 2, with the partners
-    // (CTA (C - c) mod C, index M - 1 - i, or (M - i) mod M in CTA 0), which lie in the
-    // partner CTA's second half; CTA 0's positions 0 and M / 2 are their own partners.
-    // The thread writes both packed values, the partner's into the partner CTA's slices
-    // (its shared memory through the cluster when that is another CTA).
-    double2* zw = d.zs;
-    constexpr int T = Ctx<M>::T;
-    const int c = X.c, cq = (C - c) & (C - 1);
-    double2* Aq = A;
-    double2* Bq = Bf;
-    if (cq != c) {
-      cg::cluster_group cl = cg::this_cluster();
-      Aq = cl.map_shared_rank(A, cq);
-      Bq = cl.map_shared_rank(Bf, cq);
-    }
-    const StageSrc& st = *X.stg;
-    auto pair = [&](int i, int j) {
-      const int p = c * M + i, pp = cq * M + j;
-      const double2 e = stage_val(st, p), w = stage_val(st, N + p);
-      if (p == pp) {
-        zw[p] = e;
-        zw[N + p] = w;
-        double2 a, b;
-        packed(p, p, e, e, w, w, a, b);
-        A[pidx(i)] = a;
-        Bf[pidx(i)] = b;
-        return;
-      }
-      const double2 ep = stage_val(st, pp), wp = stage_val(st, N + pp);
-      zw[p] = e;
-      zw[N + p] = w;
-      zw[pp] = ep;
-      zw[N + pp] = wp;
-      double2 a, b;
-      packed(p, pp, e, ep, w, wp, a, b);
-      A[pidx(i)] = a;
-      Bf[pidx(i)] = b;
-      packed(pp, p, ep, e, wp, w, a, b);
-      Aq[pidx(j)] = a;
-      Bq[pidx(j)] = b;
-    };
-#pragma unroll
-    for (int u = 0; u < kPts / 2; ++u) {
-      const int i = X.tid + u * T;
-      pair(i, c == 0 ? ((M - i) & (M - 1)) : (M - 1 - i));
-    }
-    if (c == 0 && X.tid == 0) pair(M / 2, M / 2);
-    if (C > 1) cg::this_cluster().sync();   // the partners' slices are written
+    stage_pack_any(X);
   } else {
-    // zs written by the caller: the partner values come through the slices
-    HW_FOREACH(X) {
-      A[pidx(idx)] = ZE[p];
-      Bf[pidx(idx)] = ZU[p];
-    }
     member_sync(C);
-    HW_FOREACH(X) {
-      const int jp = jpart(idx), pp = partner_pos(X, idx);
-      packed(p, pp, A[pidx(idx)], Ap[pidx(jp)], Bf[pidx(idx)], Bp[pidx(jp)], va[u], vb[u]);
-    }
-    member_sync(C);
-    HW_FOREACH(X) {
-      (void)p;
-      A[pidx(idx)] = va[u];
-      Bf[pidx(idx)] = vb[u];
-    }
+    const StageSrc own{d.zs, {nullptr, nullptr, nullptr, nullptr, nullptr}, 1, 0.0};
+    X.stg = &own;
+    stage_pack<M, 1>(X);
+    X.stg = nullptr;
   }
-  // (2) products in physical space (1d/functions.c:1486-1498); the damping of u
-  // waits in the member's scratch for the adjustment's transform
+  if (C > 1) cg::this_cluster().sync();   // the partners' slices are written
+  // (2) products in physical space (1d/functions.c:1486-1498)
   const bool fused = C == 2 || C == 4 || C == 8;
-  double* du = damp_u_field(d);
   if (fused) {
     fft_local2<M>(A, Bf, d.tw, C, +1);
-    cross_products_any<M>(X, A, Bf, brk, PE, PM);
+    cross_products_any<M>(X, A, Bf, PE, PM);
     fft_local2<M>(A, Bf, d.tw, C, -1);
   } else {
-    fft_inverse2<M>(A, Bf, d.tw, N, C, X.c);
+    double dm[kPts];
     HW_FOREACH(X) {
-      const double2 e = A[pidx(idx)], m = Bf[pidx(idx)];
-      if (brk) {
-        PE[p] = e;
-        PM[p].y = m.y;
-      }
-      du[p] = (d.dcoef[p] * e.y) * d.dchar[p];
-      A[pidx(idx)] = make_double2(e.x * e.y, e.x * m.x);
-      Bf[pidx(idx)] = make_double2(e.y * e.y - m.x * m.x, (d.dcoef[p] * e.x) * d.dchar[p]);
+      (void)idx;
+      dm[u] = __ldg(d.damp + p);
     }
-    fft_forward2<M>(A, Bf, d.tw, N, C, X.c);
+    fft_inverse2<M>(A, Bf, d.tw, d.N, C, X.c);
+    HW_FOREACH(X) {
+      double2 a, b;
+      product_point<M>(X, p, A[pidx(idx)], Bf[pidx(idx)], dm[u], PE, PM, a, b);
+      A[pidx(idx)] = a;
+      Bf[pidx(idx)] = b;
+    }
+    fft_forward2<M>(A, Bf, d.tw, d.N, C, X.c);
   }
   // breaking criterion (1d/breaking.c:36-95) on eta, u, H(eta): the transform's
   // barriers made PE / PM complete member-wide
   if (brk) breaking_scan(X, PE, &PM[0].y, 2);
   // (3) spectra of the products, H2 terms (1d/rhs.c:141-147) and, in the same
-  // pass, the Hermitian packing of the nonlinear adjustment (1d/rhs.c:695-715):
-  // each thread forms the terms at its wavenumber k and at N - k from the pair of
-  // transformed values it holds, so no exchange separates the two steps
+  // pass, the Hermitian packing of the nonlinear adjustment (1d/rhs.c:695-715): the
+  // pair's owner reads both transformed values and rewrites them in place
   member_sync(C);
-  HW_FOREACH(X) {
-    const int jp = jpart(idx), pp = partner_pos(X, idx);
-    const double2 z1 = A[pidx(idx)], z1p = Ap[pidx(jp)], z2 = Bf[pidx(idx)], z2p = Bp[pidx(jp)];
-    DE[p] = split_im(z2, z2p);
-    const double kp = d.k[p], kq = d.k[pp];
-    // at k
-    const double2 ah = split_re(z1, z1p), bh = split_im(z1, z1p), ch = split_re(z2, z2p);
-    const double2 lem = cscale(bh, d.L[p]), ik = mul_ik(kp, ah), ikc = mul_ik(kp, ch);
-    const double2 te = make_double2(-lem.x - ik.x, -lem.y - ik.y);
-    const double2 tu = make_double2(-ikc.x / 2, -ikc.y / 2);
-    // at N - k (the partner's pair is (z1p, z1))
-    const double2 ahq = split_re(z1p, z1), bhq = split_im(z1p, z1), chq = split_re(z2p, z2);
-    const double2 lemq = cscale(bhq, d.L[pp]), ikq = mul_ik(kq, ahq), ikcq = mul_ik(kq, chq);
-    const double2 teq = make_double2(-lemq.x - ikq.x, -lemq.y - ikq.y);
-    const double2 tuq = make_double2(-ikcq.x / 2, -ikcq.y / 2);
-    va[u] = pack(herm(te, teq), herm(tu, tuq), d.invN);
+  {
+    const double* __restrict__ kt = d.k;
+    const double* __restrict__ c1t = d.c1;
+    const double invN = d.invN;
+    double kk[kPts], cc[kPts];
+#pragma unroll
+    for (int u = 0; u < kPts / 2; ++u) {
+      const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
+      kk[2 * u] = kt[r.p];
+      kk[2 * u + 1] = kt[r.pp];
+      cc[2 * u] = c1t[r.p];
+      cc[2 * u + 1] = c1t[r.pp];
+    }
+#pragma unroll
+    for (int u = 0; u < kPts / 2; ++u) {
+      const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
+      const double2 z1 = A[pidx(r.i)], z1p = pb.Aq[pidx(r.j)], z2 = Bf[pidx(r.i)], z2p = pb.Bq[pidx(r.j)];
+      // -L (eta M0u)^ - i k (eta u)^ and -i k (u^2 - (M0u)^2)^ / 2 at one point
+      auto terms = [&](double k, double c1, double2 a, double2 ap, double2 b, double2 bp, double2& te, double2& tu) {
+        const double2 ah = split_re(a, ap), bh = split_im(a, ap), ch = split_re(b, bp);
+        const double L = k * c1;
+        te = make_double2(-L * bh.x + k * ah.y, -L * bh.y - k * ah.x);
+        tu = make_double2(0.5 * k * ch.y, -0.5 * k * ch.x);
+      };
+      double2 te, tu, teq, tuq;
+      if (r.self) {
+        terms(kk[2 * u], cc[2 * u], z1, z1, z2, z2, te, tu);
+        terms(kk[2 * u + 1], cc[2 * u + 1], z1p, z1p, z2p, z2p, teq, tuq);
+        A[pidx(r.i)] = pack(herm(te, te), herm(tu, tu), invN);
+        A[pidx(r.j)] = pack(herm(teq, teq), herm(tuq, tuq), invN);
+      } else {
+        terms(kk[2 * u], cc[2 * u], z1, z1p, z2, z2p, te, tu);
+        terms(kk[2 * u + 1], cc[2 * u + 1], z1p, z1, z2p, z2, teq, tuq);
+        const double2 E = herm(te, teq), U = herm(tu, tuq);
+        A[pidx(r.i)] = pack(E, U, invN);
+        pb.Aq[pidx(r.j)] = pack_conj(E, U, invN);
+      }
+    }
   }
   if (brk) breaking_lead(X, t, PE, &PM[0].y, 2);
-  member_sync(C);
-  HW_FOREACH(X) {
-    (void)p;
-    A[pidx(idx)] = va[u];
+  if (d.has_influx && X.tid == T - 1) {   // beside the leader of the breaking machine
+    const double2 s = influx_at(d, t);
+    X.red[kRedPv] = s.x;
+    X.red[kRedPs] = s.y;
   }
+  member_sync(C);
+  // (4) nonlinear adjustment and damping
   if (fused) {
     fft_local<M>(A, d.tw, C, +1);
-    cross_adjust_any<M>(X, A, Bf);
+    cross_adjust_any<M>(X, A, Bf, PE);
     fft_local2<M>(A, Bf, d.tw, C, -1);
   } else {
-    fft_inverse<M>(A, d.tw, N, C, X.c);
+    double dm[kPts], ch[kPts];
     HW_FOREACH(X) {
-      const double2 v = A[pidx(idx)];
-      const double ch = d.chi[p];
-      A[pidx(idx)] = make_double2(v.x * ch, v.y * ch);
-      Bf[pidx(idx)] = make_double2(du[p], 0.0);
+      (void)idx;
+      dm[u] = __ldg(d.damp + p);
+      ch[u] = __ldg(d.chi + p);
     }
-    fft_forward2<M>(A, Bf, d.tw, N, C, X.c);
-  }
-  double pv = 0.0, ps = 0.0;
-  if (d.has_influx) {
-    pv = spline_eval(d.tt, d.ins, d.insc, d.n_in, t);
-    ps = spline_eval(d.tt, d.skw, d.skwc, d.n_in, t);
+    fft_inverse<M>(A, d.tw, d.N, C, X.c);
+    HW_FOREACH(X) {
+      double2 a = A[pidx(idx)], b;
+      adjust_point(PE, p, ch[u], dm[u], a, b);
+      A[pidx(idx)] = a;
+      Bf[pidx(idx)] = b;
+    }
+    fft_forward2<M>(A, Bf, d.tw, d.N, C, X.c);
   }
   member_sync(C);
   // the leader's node count is visible member-wide after the transforms' barriers
   const bool rb_live = brk && d.bk->npk > 0;
   if (!rb_live) {
-    // (6) assembly (1d/rhs.c:217-228) straight from the adjusted spectra
-    HW_FOREACH(X) {
-      const int jp = jpart(idx);
-      const double2 z = A[pidx(idx)], zp = Ap[pidx(jp)], zb = Bf[pidx(idx)], zbp = Bp[pidx(jp)];
-      assemble_flat(d, p, split_re(z, zp), split_im(z, zp), make_double2(0.0, 0.0), DE[p], split_re(zb, zbp), pv, ps,
-                    dz);
-    }
+    assemble_flat<M, false>(X, dz, nullptr, nullptr, nullptr);
     member_sync(C);   // the partner reads of the slices are done
     return;
   }
-  HW_FOREACH(X) {
-    const int jp = jpart(idx);
-    const double2 z = A[pidx(idx)], zp = Ap[pidx(jp)], zb = Bf[pidx(idx)], zbp = Bp[pidx(jp)];
-    AE[p] = split_re(z, zp);
-    AU[p] = split_im(z, zp);
-    DU[p] = split_re(zb, zbp);
+  // (5) kinematic breaking: the eddy-viscosity force on the u-equation takes slice A,
+  // so the adjusted terms move to global memory; the damping stays in slice B
+#pragma unroll 1
+  for (int u = 0; u < kPts / 2; ++u) {
+    const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
+    const double2 z = A[pidx(r.i)], zp = pb.Aq[pidx(r.j)];
+    AE[r.p] = split_re(z, r.self ? z : zp);
+    AU[r.p] = split_im(z, r.self ? z : zp);
+    AE[r.pp] = split_re(zp, r.self ? zp : z);
+    AU[r.pp] = split_im(zp, r.self ? zp : z);
   }
   member_sync(C);
-  // (5) kinematic breaking: eddy-viscosity force on the u-equation
   breaking_force<M>(X, PE, AE, RB);
-  // (6) assembly with the force
   member_sync(C);
-  HW_FOREACH(X) {
-    (void)idx;
-    assemble_flat(d, p, AE[p], AU[p], RB[p], DE[p], DU[p], pv, ps, dz);
-  }
+  assemble_flat<M, true>(X, dz, AE, AU, RB);
+  member_sync(C);
 }
 
 }  // namespace hwdev

@@ -17,20 +17,6 @@ struct Bufs {
   double2* k[7];   // k1..k6, kout
 };
 
-// stage input zs = y + h sum_j b_sj k_j for stage s = 2..6 (GSL's expression forms)
-template <int M>
-__device__ __forceinline__ void stage_input(Ctx<M>& X, const Bufs& B, int s, double h) {
-  const DevMember& d = X.d;
-  const StageSrc st{B.y, {B.k[0], B.k[1], B.k[2], B.k[3], B.k[4]}, s, h};
-  for (int part = 0; part < 2; ++part) {
-    const int off = part * d.N;
-    HW_FOREACH(X) {
-      (void)idx;
-      d.zs[p + off] = stage_val(st, p + off);
-    }
-  }
-}
-
 // max over the member (all CTAs of the cluster); identical result in every thread
 template <int M>
 __device__ __forceinline__ double member_max(Ctx<M>& X, double v) {
@@ -54,36 +40,71 @@ __device__ __forceinline__ double member_max(Ctx<M>& X, double v) {
   return m;
 }
 
-// ynew = y + h sum c_i k_i ; yerr = h sum ec_i k_i ; returns max |yerr| / D0
+// ynew = y + h sum c_i k_i ; yerr = h sum ec_i k_i ; returns max |yerr| / D0, with D0 =
+// eps_rel |ynew| + eps_abs.  Pairs outside the alias band are left out: their k_i are
+// zero, so ynew = y there (both buffers hold it since the launch began) and yerr = 0.
+// A thread keeps the numerator and denominator of its largest ratio and divides once.
 template <int M>
-__device__ __forceinline__ double final_combine(Ctx<M>& X, const Bufs& B, double h) {
+__device__ __noinline__ double final_combine(Ctx<M>& X, const Bufs& B, double h) {
   const DevMember& d = X.d;
-  double rm = 2.2250738585072014e-308;   // DBL_MIN
+  constexpr int T = Ctx<M>::T;
+  const double2* __restrict__ ys = B.y;
+  const double2* __restrict__ k1 = B.k[0];
+  const double2* __restrict__ k3 = B.k[2];
+  const double2* __restrict__ k4 = B.k[3];
+  const double2* __restrict__ k5 = B.k[4];
+  const double2* __restrict__ k6 = B.k[5];
+  double2* __restrict__ yn = B.yn;
+  const double er = d.eps_rel, ea = d.eps_abs;
+  const int N = d.N, act = d.act, cq = (d.C - X.c) & (d.C - 1);
+  double num = 0.0, den = 1.0;
   bool bad = false;
-  for (int part = 0; part < 2; ++part) {
-    const int off = part * d.N;
-    HW_FOREACH(X) {
-      (void)idx;
-      const int q = p + off;
-      const double2 y = B.y[q], a = B.k[0][q], c = B.k[2][q], e = B.k[3][q], f = B.k[4][q], g = B.k[5][q];
-      const double dix = radd(radd(radd(radd(rmul(RK_c1, a.x), rmul(RK_c3, c.x)), rmul(RK_c4, e.x)), rmul(RK_c5, f.x)),
-                              rmul(RK_c6, g.x));
-      const double diy = radd(radd(radd(radd(rmul(RK_c1, a.y), rmul(RK_c3, c.y)), rmul(RK_c4, e.y)), rmul(RK_c5, f.y)),
-                              rmul(RK_c6, g.y));
-      const double2 yn = make_double2(radd(y.x, rmul(h, dix)), radd(y.y, rmul(h, diy)));
-      B.yn[q] = yn;
-      const double ex = rmul(h, radd(radd(radd(radd(rmul(RK_ec1, a.x), rmul(RK_ec3, c.x)), rmul(RK_ec4, e.x)),
-                                           rmul(RK_ec5, f.x)), rmul(RK_ec6, g.x)));
-      const double ey = rmul(h, radd(radd(radd(radd(rmul(RK_ec1, a.y), rmul(RK_ec3, c.y)), rmul(RK_ec4, e.y)),
-                                           rmul(RK_ec5, f.y)), rmul(RK_ec6, g.y)));
-      const double rx = fabs(ex) / fabs(radd(rmul(d.eps_rel, fabs(yn.x)), d.eps_abs));
-      const double ry = fabs(ey) / fabs(radd(rmul(d.eps_rel, fabs(yn.y)), d.eps_abs));
-      bad = bad || !(rx == rx) || !(ry == ry) || isinf(yn.x) || isinf(yn.y);
-      rm = fmax(rm, fmax(rx, ry));
+  auto one = [&](double y, double a, double c, double e, double f, double g) {
+    const double di = radd(radd(radd(radd(rmul(RK_c1, a), rmul(RK_c3, c)), rmul(RK_c4, e)), rmul(RK_c5, f)),
+                           rmul(RK_c6, g));
+    const double v = radd(y, rmul(h, di));
+    const double ex = fabs(rmul(h, radd(radd(radd(radd(rmul(RK_ec1, a), rmul(RK_ec3, c)), rmul(RK_ec4, e)),
+                                             rmul(RK_ec5, f)), rmul(RK_ec6, g))));
+    const double D = fabs(radd(rmul(er, fabs(v)), ea));
+    bad = bad || !(ex <= 1.7976931348623157e308) || !(fabs(v) <= 1.7976931348623157e308);
+    if (ex * den > num * D) {
+      num = ex;
+      den = D;
+    }
+    return v;
+  };
+#pragma unroll 1
+  for (int u = 0; u < kPts / 2; ++u) {
+    const PairAt r = pair_at<M>(X.c, cq, X.tid + u * T);
+    if (r.i >= act) continue;
+#pragma unroll 1
+    for (int off = 0; off <= N; off += N) {
+      const int q0 = r.p + off, q1 = r.pp + off;
+      const double2 y0 = ys[q0], a0 = k1[q0], c0 = k3[q0], e0 = k4[q0], f0 = k5[q0], g0 = k6[q0];
+      const double2 y1 = ys[q1], a1 = k1[q1], c1 = k3[q1], e1 = k4[q1], f1 = k5[q1], g1 = k6[q1];
+      yn[q0] = make_double2(one(y0.x, a0.x, c0.x, e0.x, f0.x, g0.x), one(y0.y, a0.y, c0.y, e0.y, f0.y, g0.y));
+      yn[q1] = make_double2(one(y1.x, a1.x, c1.x, e1.x, f1.x, g1.x), one(y1.y, a1.y, c1.y, e1.y, f1.y, g1.y));
     }
   }
+  double rm = fmax(num / den, 2.2250738585072014e-308);   // DBL_MIN
   if (bad) rm = __longlong_as_double(0x7ff0000000000000ULL);   // +inf: forces a failure path
   return member_max(X, rm);
+}
+
+// Outside the alias band every k_i is zero and the state stays what it is: the second
+// state buffer and the stage input take those points once, when a launch begins.
+template <int M>
+__device__ __forceinline__ void spread_unmoved(Ctx<M>& X) {
+  const DevMember& d = X.d;
+  const int cq = (d.C - X.c) & (d.C - 1);
+  for (int u = 0; u < kPts / 2; ++u) {
+    const PairAt r = pair_at<M>(X.c, cq, X.tid + u * Ctx<M>::T);
+    if (r.i < d.act) continue;
+    for (int off = 0; off <= d.N; off += d.N) {
+      d.ynew[r.p + off] = d.zs[r.p + off] = d.y[r.p + off];
+      d.ynew[r.pp + off] = d.zs[r.pp + off] = d.y[r.pp + off];
+    }
+  }
 }
 
 struct StepState {
@@ -107,19 +128,6 @@ __device__ __forceinline__ void rhs_at(Ctx<M>& X, StepState& S, double t, const 
   X.stg = &st;
   rhs_into(X, S, t, out);
   X.stg = nullptr;
-}
-
-// copy a state buffer into the stage-input buffer
-template <int M>
-__device__ __forceinline__ void load_stage(Ctx<M>& X, const double2* src) {
-  const DevMember& d = X.d;
-  for (int part = 0; part < 2; ++part) {
-    const int off = part * d.N;
-    HW_FOREACH(X) {
-      (void)idx;
-      d.zs[p + off] = src[p + off];
-    }
-  }
 }
 
 // gsl_odeiv_evolve_apply with rkf45 and control_y, one member
