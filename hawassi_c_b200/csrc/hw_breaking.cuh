@@ -293,15 +293,14 @@ __device__ __noinline__ void breaking_force(Ctx<M>& X, const double2* PE, const 
   BrkDev* bk = d.bk;
   const int N = d.N;
   const double2* ZU = d.zs + N;
-  const double2* HS = d.sc[6];
+  const double2* M0h = d.sc[6];   // M0 u^ on a varying bottom
   auto teta = [&](int q) -> double2 {
     double2 h1;
     if (d.flat) {
       const double c1 = d.c1[q];
       h1 = make_double2(c1 * ZU[q].y, -c1 * ZU[q].x);
     } else {
-      const double kq = d.k[q];
-      h1 = make_double2((HS[q].y / kG) * kq, -(HS[q].x / kG) * kq);
+      h1 = M0h[q];
     }
     return cadd(h1, AEadj[q]);
   };
@@ -327,30 +326,6 @@ __device__ __noinline__ void breaking_force(Ctx<M>& X, const double2* PE, const 
     X.buf[pidx(idx)] = make_double2(rb, 0.0);
   }
   fft_forward_split(X, [&](int, int, int p, double2 z, double2 zp) { Rb[p] = split_re(z, zp); });
-}
-
-// The whole breaking step of one RHS, after the adjusted nonlinear terms: returns
-// false (Rb untouched) when no node breaks: the force is then identically zero, as
-// the reference's FFT of a zero flux gives, and the assembly skips it
-template <int M>
-__device__ __noinline__ bool breaking_rhs(Ctx<M>& X, double t, const double2* PE, const double* Heta, int hs,
-                                          const double2* AEadj, double2* Rb) {
-  breaking_reset(X);
-  if (X.tid == 0) *X.ncand = 0;
-  __syncthreads();
-  HW_FOREACH(X) {
-    (void)idx;
-    if (p >= X.d.xbstart && p < X.d.xbstart + X.d.lenIF && !(PE[p].x < X.d.MaxEtaInit))
-      X.cand[atomicAdd(X.ncand, 1)] = (unsigned short)p;
-  }
-  member_sync(X.d.C);
-  breaking_scan(X, PE, Heta, hs);
-  member_sync(X.d.C);
-  breaking_lead(X, t, PE, Heta, hs);
-  member_sync(X.d.C);
-  if (X.d.bk->npk == 0) return false;   // B identically zero: FFT(0) = 0, as the reference computes it
-  breaking_force(X, PE, AEadj, Rb);
-  return true;
 }
 
 }  // namespace hwdev

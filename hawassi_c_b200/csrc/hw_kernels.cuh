@@ -4,6 +4,7 @@
 
 #include "hw_breaking.cuh"
 #include "hw_rhs_fast.cuh"
+#include "hw_rhs_gen.cuh"
 #include "hw_kernels.h"
 #include "hw_stepper.cuh"
 #include "hw_output.cuh"

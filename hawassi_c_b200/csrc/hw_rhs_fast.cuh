@@ -43,14 +43,38 @@ struct PairBufs {
   }
 };
 
+// one complex transform's input at a pair from two spectra x, y (given at both points,
+// not necessarily Hermitian): (herm x + i herm y) / N, real parts only as the reference
+__device__ __forceinline__ void emit_pair(double2* A, double2* Aq, const PairAt& r, double2 x, double2 xp, double2 y,
+                                          double2 yp, double invN) {
+  if (r.self) {
+    A[pidx(r.i)] = pack(herm(x, x), herm(y, y), invN);
+    A[pidx(r.j)] = pack(herm(xp, xp), herm(yp, yp), invN);
+  } else {
+    const double2 E = herm(x, xp), F = herm(y, yp);
+    A[pidx(r.i)] = pack(E, F, invN);
+    Aq[pidx(r.j)] = pack_conj(E, F, invN);
+  }
+}
+__device__ __forceinline__ double2 cmi(double s, double2 a) { return make_double2(s * a.y, -s * a.x); }   // -i s a
+__device__ __forceinline__ double2 czero() { return make_double2(0.0, 0.0); }
+// Hilbert transform's multiplier (1d/breaking.c:133-143): -i sign(k)
+__device__ __forceinline__ double2 hilbert_hat(double k, double2 e) {
+  return k == 0 ? czero() : cmi(copysign(1.0, k), e);
+}
+
+// what the first inverse transform carries beside eta and u
+enum : int { kWithM0Hilbert = 0, kWithM0Dx = 1, kWithRefs = 2, kWithNone = 3 };
+
 // Stage input of stage S (y + h sum_j b_sj k_j, kept in zs for the assembly) and its
-// Hermitian packing for the first dual inverse transform: A <- eta^ + i u^,
-// B <- M0 u^ + i H(eta)^ (real parts only, as the reference).  M0 u^ = -i c1 u^ and the
-// Hilbert multiplier (1d/breaking.c:133-143) takes the sign of c1 = (C^2/g) k.
+// Hermitian packing for the first inverse transform: A <- eta^ + i u^ and, by `with`,
+// B <- M0 u^ + i H(eta)^ (flat HS2), M0 u^ + i (d_x u)^ (flat HS3), the images of u^
+// under the first two reference depths (varying bottom) or nothing (HS1).  On a flat
+// bottom M0 u^ = -i c1 u^, and the Hilbert multiplier takes the sign of c1 = (C^2/g) k.
 // The stage is a template argument so that a pair's loads (up to 24) are independent
 // of any branch and in flight together.
 template <int M, int S>
-__device__ __noinline__ void stage_pack(Ctx<M>& X) {
+__device__ __noinline__ void stage_pack(Ctx<M>& X, int with) {
   const DevMember& d = X.d;
   constexpr int T = Ctx<M>::T;
   const double2* y = X.stg->y;
@@ -58,42 +82,33 @@ __device__ __noinline__ void stage_pack(Ctx<M>& X) {
 #pragma unroll
   for (int j = 0; j < S - 1; ++j) ks[j] = X.stg->k[j];
   const double h = X.stg->h, invN = d.invN;
-  const double* __restrict__ c1 = d.c1;
-  double2* zw = d.zs;
   const int N = d.N, c = X.c, act = d.act;
+  const double* __restrict__ t1 = with == kWithRefs ? d.Csq : d.c1;
+  const double* __restrict__ t2 = with == kWithRefs ? d.Csq + N : d.k;
+  double2* zw = d.zs;
   const bool brk = d.brk != 0;
   const PairBufs<M> pb(X);
   double2 *A = X.buf, *B = X.buf2, *Aq = pb.Aq, *Bq = pb.Bq;
-  auto emit = [&](const PairAt& r, double ca, double cb, double2 e, double2 ep, double2 w, double2 wp) {
-    auto point = [&](double k, double kq, double2 f, double2 fp, double2 g, double2 gp, double2& H, double2& S2) {
-      H = herm(make_double2(k * g.y, -k * g.x), make_double2(kq * gp.y, -kq * gp.x));
-      S2 = make_double2(0.0, 0.0);
-      if (brk) {
-        const double s = k == 0 ? 0.0 : copysign(1.0, k), sq = kq == 0 ? 0.0 : copysign(1.0, kq);
-        S2 = herm(make_double2(s * f.y, -s * f.x), make_double2(sq * fp.y, -sq * fp.x));
-      }
-    };
-    double2 H, S2;
-    if (r.self) {
-      point(ca, ca, e, e, w, w, H, S2);
-      A[pidx(r.i)] = pack(herm(e, e), herm(w, w), invN);
-      B[pidx(r.i)] = pack(H, S2, invN);
-      point(cb, cb, ep, ep, wp, wp, H, S2);
-      A[pidx(r.j)] = pack(herm(ep, ep), herm(wp, wp), invN);
-      B[pidx(r.j)] = pack(H, S2, invN);
-      return;
+  auto emit = [&](const PairAt& r, double a, double aq, double b, double bq, double2 e, double2 ep, double2 w, double2 wp) {
+    emit_pair(A, Aq, r, e, ep, w, wp, invN);
+    if (with == kWithM0Hilbert) {
+      emit_pair(B, Bq, r, cmi(a, w), cmi(aq, wp), brk ? hilbert_hat(a, e) : czero(), brk ? hilbert_hat(aq, ep) : czero(),
+                invN);
+    } else if (with == kWithM0Dx) {
+      emit_pair(B, Bq, r, cmi(a, w), cmi(aq, wp), cmi(-b, w), cmi(-bq, wp), invN);
+    } else if (with == kWithRefs) {
+      emit_pair(B, Bq, r, cscale(w, a), cscale(wp, aq), cscale(w, b), cscale(wp, bq), invN);
     }
-    const double2 E = herm(e, ep), W = herm(w, wp);
-    point(ca, cb, e, ep, w, wp, H, S2);
-    A[pidx(r.i)] = pack(E, W, invN);
-    Aq[pidx(r.j)] = pack_conj(E, W, invN);
-    B[pidx(r.i)] = pack(H, S2, invN);
-    Bq[pidx(r.j)] = pack_conj(H, S2, invN);
   };
 #pragma unroll 1
   for (int u = 0; u < kPts / 2; ++u) {
     const PairAt r = pair_at<M>(c, pb.cq, X.tid + u * T);
-    const double ca = c1[r.p], cb = c1[r.pp];
+    const double a = t1[r.p], aq = t1[r.pp];
+    double b = 0.0, bq = 0.0;
+    if (with != kWithM0Hilbert) {
+      b = t2[r.p];
+      bq = t2[r.pp];
+    }
     if (r.i < act) {
       StageOps<S> oe, oep, ow, owp;
       oe.load(y, ks, r.p);
@@ -107,23 +122,36 @@ __device__ __noinline__ void stage_pack(Ctx<M>& X) {
         zw[N + r.p] = w;
         zw[N + r.pp] = wp;
       }
-      emit(r, ca, cb, e, ep, w, wp);
+      emit(r, a, aq, b, bq, e, ep, w, wp);
     } else {
-      emit(r, ca, cb, y[r.p], y[r.pp], y[N + r.p], y[N + r.pp]);
+      emit(r, a, aq, b, bq, y[r.p], y[r.pp], y[N + r.p], y[N + r.pp]);
     }
   }
 }
 
+// the stage phase with its barriers.  Every RHS leaves the slices unread by the other
+// CTAs (a barrier follows its last partner reads), so they can be written at once; with
+// zs written by the caller, other threads' writes of it and the start of the partner
+// CTA come first.
 template <int M>
-__device__ __forceinline__ void stage_pack_any(Ctx<M>& X) {
-  switch (X.stg->s) {
-    case 1: stage_pack<M, 1>(X); break;
-    case 2: stage_pack<M, 2>(X); break;
-    case 3: stage_pack<M, 3>(X); break;
-    case 4: stage_pack<M, 4>(X); break;
-    case 5: stage_pack<M, 5>(X); break;
-    default: stage_pack<M, 6>(X); break;
+__device__ __forceinline__ void stage_phase(Ctx<M>& X, int with) {
+  if (X.stg) {
+    switch (X.stg->s) {
+      case 1: stage_pack<M, 1>(X, with); break;
+      case 2: stage_pack<M, 2>(X, with); break;
+      case 3: stage_pack<M, 3>(X, with); break;
+      case 4: stage_pack<M, 4>(X, with); break;
+      case 5: stage_pack<M, 5>(X, with); break;
+      default: stage_pack<M, 6>(X, with); break;
+    }
+  } else {
+    member_sync(X.d.C);
+    const StageSrc own{X.d.zs, {nullptr, nullptr, nullptr, nullptr, nullptr}, 1, 0.0};
+    X.stg = &own;
+    stage_pack<M, 1>(X, with);
+    X.stg = nullptr;
   }
+  if (X.d.C > 1) cg::this_cluster().sync();   // the partners' slices are written
 }
 
 // the influx source term of the assembly (1d/rhs.c:659-693) from the loaded kernels
@@ -270,18 +298,22 @@ __device__ __forceinline__ void cross_adjust_any(Ctx<M>& X, double2* A, double2*
   else cross_adjust<M, 8>(X, A, B, PE);
 }
 
-// Assembly of dz (1d/rhs.c:217-228): delta H1 + adjusted nonlinear terms + breaking
-// force + 2 force - damping, times aal, for the pairs inside the alias band; outside it
-// dz is zero, and was when the buffer was made.  LIVE: the adjusted terms and the force
-// come from the scratch fields (some node breaks), else from the slices.
-template <int M, bool LIVE>
-__device__ __noinline__ void assemble_flat(Ctx<M>& X, double2* __restrict__ dz, const double2* AE, const double2* AU,
-                                           const double2* RB) {
+// Assembly of dz (1d/rhs.c:217-228, 373-385, 73-83): delta H1 + adjusted nonlinear terms
+// + breaking force + 2 force - damping, times aal, for the pairs inside the alias band;
+// outside it dz is zero, and was when the buffer was made.  delta H1 of eta is M0h on a varying
+// bottom (VAR), else -i c1 u^.  MODE: the adjusted terms come from slice A
+// (damping from B), from scratch with the force (some node breaks; damping from B), or
+// there are none (HS1; damping from A).
+enum : int { kAsmSlices = 0, kAsmLive = 1, kAsmLinear = 2 };
+template <int M, int MODE, bool VAR>
+__device__ __noinline__ void assemble(Ctx<M>& X, double2* __restrict__ dz, const double2* M0h, const double2* AE,
+                                      const double2* AU, const double2* RB) {
   const DevMember& d = X.d;
   constexpr int T = Ctx<M>::T;
   const int N = d.N, c = X.c, act = d.act, mode = d.has_influx ? d.prop_mode : 3;
   const PairBufs<M> pb(X);
-  const double2 *A = X.buf, *B = X.buf2, *Aq = pb.Aq, *Bq = pb.Bq;
+  const double2 *A = X.buf, *Aq = pb.Aq;
+  const double2 *B = MODE == kAsmLinear ? X.buf : X.buf2, *Bq = MODE == kAsmLinear ? pb.Aq : pb.Bq;
   const double2* zs = d.zs;
   const double* __restrict__ kt = d.k;
   const double* __restrict__ c1t = d.c1;
@@ -293,25 +325,25 @@ __device__ __noinline__ void assemble_flat(Ctx<M>& X, double2* __restrict__ dz, 
   for (int u = 0; u < kPts / 2; ++u) {
     const PairAt r = pair_at<M>(c, pb.cq, X.tid + u * T);
     if (r.i >= act) {
-      if (X.full) dz[r.p] = dz[r.pp] = dz[N + r.p] = dz[N + r.pp] = make_double2(0.0, 0.0);
+      if (X.full) dz[r.p] = dz[r.pp] = dz[N + r.p] = dz[N + r.pp] = czero();
       continue;
     }
     const int pos[2] = {r.p, r.pp};
-    double2 ze[2], zu[2], gx[2], gs[2], ae[2], au[2];
+    double2 ze[2], h1[2], gx[2], gs[2], ae[2], au[2];
     double kk[2], c1[2], al[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       ze[s] = zs[pos[s]];
-      zu[s] = zs[N + pos[s]];
+      h1[s] = VAR ? M0h[pos[s]] : zs[N + pos[s]];
+      c1[s] = VAR ? 0.0 : c1t[pos[s]];
       kk[s] = kt[pos[s]];
-      c1[s] = c1t[pos[s]];
       al[s] = aalt[pos[s]];
-      gx[s] = gs[s] = make_double2(0.0, 0.0);
+      gx[s] = gs[s] = ae[s] = au[s] = czero();
       if (mode != 3) {
         gx[s] = gxt[pos[s]];
         gs[s] = gst[pos[s]];
       }
-      if constexpr (LIVE) {
+      if constexpr (MODE == kAsmLive) {
         const double2 f = RB[pos[s]];
         ae[s] = AE[pos[s]];
         au[s] = cadd(AU[pos[s]], f);
@@ -322,19 +354,91 @@ __device__ __noinline__ void assemble_flat(Ctx<M>& X, double2* __restrict__ dz, 
     for (int s = 0; s < 2; ++s) {
       const double2 a = s ? zp : z, b = s ? zbp : zb;
       const double2 aq = r.self ? a : (s ? z : zp), bq = r.self ? b : (s ? zb : zbp);
-      if constexpr (!LIVE) {
+      if constexpr (MODE == kAsmSlices) {
         ae[s] = split_re(a, aq);
         au[s] = split_im(a, aq);
       }
       const double2 de = split_re(b, bq), du = split_im(b, bq);
       const double gk = kG * kk[s];
       const double2 f = source_term(mode, gx[s], gs[s], pv, ps);
-      const double2 te = make_double2(c1[s] * zu[s].y + ae[s].x, -c1[s] * zu[s].x + ae[s].y);
+      const double2 te = cadd(VAR ? h1[s] : cmi(c1[s], h1[s]), ae[s]);
       const double2 tu = make_double2(gk * ze[s].y + au[s].x, -gk * ze[s].x + au[s].y);
       dz[pos[s]] = make_double2((te.x + 2 * f.x - de.x) * al[s], (te.y + 2 * f.y - de.y) * al[s]);
       dz[N + pos[s]] = make_double2((tu.x - du.x) * al[s], (tu.y - du.y) * al[s]);
     }
   }
+}
+
+// beside the last spectral phase: the breaking machine's leader and, by another thread,
+// the influx signals at the stage time (read after the phase's barrier)
+template <int M>
+__device__ __forceinline__ void lead_and_influx(Ctx<M>& X, double t, const double2* PE, const double* Heta) {
+  if (X.d.brk) breaking_lead(X, t, PE, Heta, 2);
+  if (X.d.has_influx && X.tid == Ctx<M>::T - 1) {
+    const double2 s = influx_at(X.d, t);
+    X.red[kRedPv] = s.x;
+    X.red[kRedPs] = s.y;
+  }
+}
+
+// From the packed nonlinear terms in slice A to dz: the nonlinear adjustment with the
+// damping, the breaking force where some node breaks, the assembly.
+template <int M>
+__device__ __noinline__ void finish_rhs(Ctx<M>& X, double2* __restrict__ dz, const double2* M0h) {
+  const DevMember& d = X.d;
+  constexpr int T = Ctx<M>::T;
+  const int C = d.C;
+  double2* A = X.buf;
+  double2* Bf = X.buf2;
+  const double2* PE = d.sc[0];
+  if (C == 2 || C == 4 || C == 8) {
+    fft_local<M>(A, d.tw, C, +1);
+    cross_adjust_any<M>(X, A, Bf, PE);
+    fft_local2<M>(A, Bf, d.tw, C, -1);
+  } else {
+    double dm[kPts], ch[kPts];
+    HW_FOREACH(X) {
+      (void)idx;
+      dm[u] = __ldg(d.damp + p);
+      ch[u] = __ldg(d.chi + p);
+    }
+    fft_inverse<M>(A, d.tw, d.N, C, X.c);
+    HW_FOREACH(X) {
+      double2 a = A[pidx(idx)], b;
+      adjust_point(PE, p, ch[u], dm[u], a, b);
+      A[pidx(idx)] = a;
+      Bf[pidx(idx)] = b;
+    }
+    fft_forward2<M>(A, Bf, d.tw, d.N, C, X.c);
+  }
+  member_sync(C);
+  // the leader's node count is visible member-wide after the transforms' barriers
+  const bool rb_live = d.brk != 0 && d.bk->npk > 0;
+  if (!rb_live) {
+    if (M0h) assemble<M, kAsmSlices, true>(X, dz, M0h, nullptr, nullptr, nullptr);
+    else assemble<M, kAsmSlices, false>(X, dz, nullptr, nullptr, nullptr, nullptr);
+    member_sync(C);   // the partner reads of the slices are done
+    return;
+  }
+  // kinematic breaking: the eddy-viscosity force on the u-equation takes slice A, so
+  // the adjusted terms move to global memory; the damping stays in slice B
+  double2 *AE = d.sc[2], *AU = d.sc[3], *RB = d.sc[11];
+  const PairBufs<M> pb(X);
+#pragma unroll 1
+  for (int u = 0; u < kPts / 2; ++u) {
+    const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
+    const double2 z = A[pidx(r.i)], zp = pb.Aq[pidx(r.j)];
+    AE[r.p] = split_re(z, r.self ? z : zp);
+    AU[r.p] = split_im(z, r.self ? z : zp);
+    AE[r.pp] = split_re(zp, r.self ? zp : z);
+    AU[r.pp] = split_im(zp, r.self ? zp : z);
+  }
+  member_sync(C);
+  breaking_force<M>(X, PE, AE, RB);
+  member_sync(C);
+  if (M0h) assemble<M, kAsmLive, true>(X, dz, M0h, AE, AU, RB);
+  else assemble<M, kAsmLive, false>(X, dz, nullptr, AE, AU, RB);
+  member_sync(C);
 }
 
 template <int M>
@@ -346,28 +450,13 @@ __device__ __noinline__ void rhs_hs2_flat(Ctx<M>& X, double t, double2* __restri
   double2* Bf = X.buf2;
   double2* PE = d.sc[0];   // physical (eta, u)           [breaking, and in the damping zones]
   double2* PM = d.sc[1];   // physical (., Hilbert eta)   [breaking only]
-  double2* AE = d.sc[2];   // adjusted nonlinear eta term [breaking force live only]
-  double2* AU = d.sc[3];   // adjusted nonlinear u term   [breaking force live only]
-  double2* RB = d.sc[11];  // FFT(breaking force)
   const bool brk = d.brk != 0;
   const PairBufs<M> pb(X);
 
-  // (0)-(1) stage input and its packing.  Every exit of this function leaves the slices
-  // unread by the other CTAs (a barrier follows the last partner reads), so they can be
-  // written at once; with zs written by the caller, other threads' writes of it and the
-  // start of the partner CTA come first.
+  // (0)-(1) stage input and its packing
   if (brk) breaking_reset(X);
   if (X.tid == 0) *X.ncand = 0;
-  if (X.stg) {
-    stage_pack_any(X);
-  } else {
-    member_sync(C);
-    const StageSrc own{d.zs, {nullptr, nullptr, nullptr, nullptr, nullptr}, 1, 0.0};
-    X.stg = &own;
-    stage_pack<M, 1>(X);
-    X.stg = nullptr;
-  }
-  if (C > 1) cg::this_cluster().sync();   // the partners' slices are written
+  stage_phase(X, kWithM0Hilbert);
   // (2) products in physical space (1d/functions.c:1486-1498)
   const bool fused = C == 2 || C == 4 || C == 8;
   if (fused) {
@@ -421,72 +510,15 @@ __device__ __noinline__ void rhs_hs2_flat(Ctx<M>& X, double t, double2* __restri
         tu = make_double2(0.5 * k * ch.y, -0.5 * k * ch.x);
       };
       double2 te, tu, teq, tuq;
-      if (r.self) {
-        terms(kk[2 * u], cc[2 * u], z1, z1, z2, z2, te, tu);
-        terms(kk[2 * u + 1], cc[2 * u + 1], z1p, z1p, z2p, z2p, teq, tuq);
-        A[pidx(r.i)] = pack(herm(te, te), herm(tu, tu), invN);
-        A[pidx(r.j)] = pack(herm(teq, teq), herm(tuq, tuq), invN);
-      } else {
-        terms(kk[2 * u], cc[2 * u], z1, z1p, z2, z2p, te, tu);
-        terms(kk[2 * u + 1], cc[2 * u + 1], z1p, z1, z2p, z2, teq, tuq);
-        const double2 E = herm(te, teq), U = herm(tu, tuq);
-        A[pidx(r.i)] = pack(E, U, invN);
-        pb.Aq[pidx(r.j)] = pack_conj(E, U, invN);
-      }
+      terms(kk[2 * u], cc[2 * u], z1, r.self ? z1 : z1p, z2, r.self ? z2 : z2p, te, tu);
+      terms(kk[2 * u + 1], cc[2 * u + 1], z1p, r.self ? z1p : z1, z2p, r.self ? z2p : z2, teq, tuq);
+      emit_pair(A, pb.Aq, r, te, teq, tu, tuq, invN);
     }
   }
-  if (brk) breaking_lead(X, t, PE, &PM[0].y, 2);
-  if (d.has_influx && X.tid == T - 1) {   // beside the leader of the breaking machine
-    const double2 s = influx_at(d, t);
-    X.red[kRedPv] = s.x;
-    X.red[kRedPs] = s.y;
-  }
+  lead_and_influx(X, t, PE, &PM[0].y);
   member_sync(C);
-  // (4) nonlinear adjustment and damping
-  if (fused) {
-    fft_local<M>(A, d.tw, C, +1);
-    cross_adjust_any<M>(X, A, Bf, PE);
-    fft_local2<M>(A, Bf, d.tw, C, -1);
-  } else {
-    double dm[kPts], ch[kPts];
-    HW_FOREACH(X) {
-      (void)idx;
-      dm[u] = __ldg(d.damp + p);
-      ch[u] = __ldg(d.chi + p);
-    }
-    fft_inverse<M>(A, d.tw, d.N, C, X.c);
-    HW_FOREACH(X) {
-      double2 a = A[pidx(idx)], b;
-      adjust_point(PE, p, ch[u], dm[u], a, b);
-      A[pidx(idx)] = a;
-      Bf[pidx(idx)] = b;
-    }
-    fft_forward2<M>(A, Bf, d.tw, d.N, C, X.c);
-  }
-  member_sync(C);
-  // the leader's node count is visible member-wide after the transforms' barriers
-  const bool rb_live = brk && d.bk->npk > 0;
-  if (!rb_live) {
-    assemble_flat<M, false>(X, dz, nullptr, nullptr, nullptr);
-    member_sync(C);   // the partner reads of the slices are done
-    return;
-  }
-  // (5) kinematic breaking: the eddy-viscosity force on the u-equation takes slice A,
-  // so the adjusted terms move to global memory; the damping stays in slice B
-#pragma unroll 1
-  for (int u = 0; u < kPts / 2; ++u) {
-    const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
-    const double2 z = A[pidx(r.i)], zp = pb.Aq[pidx(r.j)];
-    AE[r.p] = split_re(z, r.self ? z : zp);
-    AU[r.p] = split_im(z, r.self ? z : zp);
-    AE[r.pp] = split_re(zp, r.self ? zp : z);
-    AU[r.pp] = split_im(zp, r.self ? zp : z);
-  }
-  member_sync(C);
-  breaking_force<M>(X, PE, AE, RB);
-  member_sync(C);
-  assemble_flat<M, true>(X, dz, AE, AU, RB);
-  member_sync(C);
+  // (4) nonlinear adjustment, damping, breaking force, assembly
+  finish_rhs(X, dz, nullptr);
 }
 
 }  // namespace hwdev
