@@ -1,25 +1,30 @@
-// hw2d.cuh -- HAWASSI 2D flat-bottom RHS (rhs_AB2_2DF_uv, 2d/fun_odesolver.c:4458)
-// and its rkf45 attempt as five fused FFT passes plus stepper kernels.
+// hw2d.cuh -- HAWASSI 2D right-hand sides: what every bottom and order shares, the
+// passes of a flat bottom (rhs_AB1/AB2/AB3_2DF_uv, 2d/fun_odesolver.c:4404-4734), and
+// the rkf45 attempt's stepper kernels.
 //
 // A 2D transform is a row pass and a column pass.  Row passes run one CTA per row
 // pair {r, Ny-r} (with {0, Ny/2} sharing a CTA): that pair holds every point's
 // conjugate mirror (-ky, -kx), so the Hermitian operations the reference
 // performs on whole arrays (fftwcomplex_2d_sym before an inverse transform, real
 // parts after it, the split of two real fields packed into one complex transform)
-// are CTA-local.  Column passes run one CTA per column pair {2c, 2c+1} and do the
-// physical-space products.  A CTA holds S slices (rows or columns) of M points in
-// shared memory and transforms them with G groups of M/8 threads, one slice per
-// group, in rounds.
+// are CTA-local.  Column passes run one CTA per column pair {2c, 2c+1}.  A CTA holds
+// slices (rows or columns) of M points in shared memory, each transformed by M/16
+// threads.
 //
-// One RHS (HS2) = 5 kernels:
-//   A row pass:    stage input z, E(eta)+iE(L phi), E(u)+iE(M0 u), E(v)+iE(M0 v), inverse row FFT
-//   B column pass: inverse column FFT -> eta, Lphi, u, M0u, v, M0v -> 8 products
-//                  packed into 4 complex fields -> forward column FFT
-//   C row pass:    forward row FFT, split, damping spectra out, the four H2 terms
-//                  symmetrised (fun_adjust's input), inverse row FFT
-//   D column pass: inverse column FFT, x ChiAdj, forward column FFT; the source's
-//                  column transform (its row transform is a set-up table)
-//   E row pass:    forward row FFT of the adjusted terms, assembly of dt Z (x aal)
+// What an RHS cannot do without is fewer transforms than its terms name, because
+// they are linear: delu H2^ and delv H2^ (and the cubic ones) enter only as their sum,
+// whose operator part is L (eta L phi)^ of one real field; L phi is the sum of M0u
+// and M0v in physical space; the damping of u, v, and of eta less the source, are added
+// where the adjusted terms are in physical space.  HS2 on a flat bottom:
+//   A row   (eta, u), (v, L phi)                                      -> inverse rows
+//   B col   inverse -> eta u, eta v, eta L phi, deletaH2, two to a field -> forward
+//   C row   forward, split -> S(i kx deletaH2^), S(i ky deletaH2^), S(delu + delv) -> inverse
+//   D col   inverse, x ChiAdj, with the damping and the source        -> forward
+//   E row   forward -> dt Z (x aal)
+// is 13 field passes (a field: two slices in one direction) where one of the terms each
+// takes 24.  HS3 adds one round trip between C and D, HS1 leaves C and D out.
+// Passes whose fields are independent (A, D, E) run a CTA per field, so that several
+// share an SM.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -41,7 +46,6 @@ using hwdev::twiddle_powers;
 using hwdev::twd;
 
 constexpr double kGrav = 9.80665;
-constexpr int kGroups = 4;
 
 struct Tab2 {
   int nx, ny, n, model, nt, chi_one, has_src;
@@ -53,8 +57,9 @@ struct Tab2 {
   const double* aal;
   const double* damp;           // 7 Cpeak fbdy.charac
   const double* chi;            // ChiAdj
-  const double2* gx;            // row transform of newGam
-  const double2* sx;            // row transform of +-SkewGam (sign of the propagation)
+  const double* gsrc;           // newGam
+  const double* ssrc;           // +-SkewGam (sign of the propagation)
+  double t0, tl, dts;           // first, last line-signal time, second minus first
   const double* tsig;           // [nt]
   const double* sig;            // [ny][nt] line signals and their spline coefficients
   const double* sigc;
@@ -62,25 +67,15 @@ struct Tab2 {
   const double* sigsc;
   const double2* twx;           // exp(-2 pi i q / nx)
   const double2* twy;           // exp(-2 pi i q / ny)
-  // varying bottom, two reference depths (rhs_AB2_2DB_uv); var = 0 on a flat bottom
   int var;
-  const double* gmin;           // Gam_min, Gam_plus (physical)
-  const double* gplus;
-  const double* cmin;           // Csqr2d_min, Csqr2d_plus (spectral)
-  const double* cplus;
-  const double* omin;           // Om2dSq_min, Om2dSq_plus (spectral)
-  const double* oplus;
   const double* wallchar;       // dominfo.wallchar (harbour walls), nullptr: none
   const double* c2d;            // Oprt.C2d (flat bottom with walls only)
   int refl_one;                 // flat bottom, refl_coef == 1: fun_delphiH1hat's flux branch
   const double* gwx;            // fun_gradient(wallchar) (refl_one only)
   const double* gwy;
-  // three reference depths (HSSgen_3depth): the middle depth's tables, nullptr: two
-  const double* gmid;
-  const double* cmid;
-  const double* omid;
-  // K reference depths (the plain K-reference and the learned operators): [K][N] weights,
-  // C^2 and Omega^2 of each depth; nk = 0 when the min / plus (/ mid) tables serve
+  // varying bottom: K reference depths (HSSgen_2depth, HSSgen_3depth, and the same sum over
+  // K depths of the plain K-reference and the learned operators), rows [K][N] of the
+  // weights (physical), C^2 and Omega^2 (spectral); var = nk = 0 on a flat bottom
   int nk;
   const double* gk;
   const double* ck;
@@ -89,28 +84,22 @@ struct Tab2 {
 
 struct Work2 {
   double2* z;                   // stage input, 3 fields
-  double2* R;                   // A -> B, 3 fields
-  double2* Q;                   // B -> C, 4 fields
-  double2* D;                   // damping spectra, 3 fields
-  double2* W;                   // C -> D, 4 fields
-  double2* V;                   // D -> E, 4 fields
-  double2* src;                 // source spectrum
+  double2* R;                   // row pass -> column pass
+  double2* Q;                   // column pass -> row pass
+  double2* D;                   // spectrum of damping of eta less the source (breaking, ChiAdj = 1);
+                                // of damping of u and v (ChiAdj = 1)
+  double2* W;                   // C -> D, 3 fields
+  double2* V;                   // -> E, 3 fields
+  double2* T;                   // left half of every row: delu + delv (0), deletaH (1), L of the
+                                // operand's kept part (2)
   double* insig;                // [ny] line signal at the stage time
   double* insigs;
   double* part;                 // per-block maxima of the error ratio
-  // varying bottom only
   double* phys;                 // eta, u, v in physical space (3 real fields)
-  double* pe;                   // eta M0u, eta M0v in physical space (2 real fields)
-  double2* H1;                  // delu H1^, delv H1^ (2 fields)
-  double2* EU;                  // (eta u)^, (eta v)^, deletaH2^ (3 fields)
-  // kinematic breaking only: delphiH^ as the assembly forms it (nullptr: off)
-  double2* dph;
-  // flat bottom with walls: the round trip of (C u^, C v^) (delphiH1^ lands in H1)
-  double2* WP;
-  // HS3 on the flat bottom: eta, L phi in physical space (2 real fields) and the
-  // HS2 terms with (eta^2 M0u)^, (eta^2 M0v)^ between passes C3 and I3 (6 fields)
-  double* p3;
-  double2* T3;
+  double* op;                   // operand of an HSS, L phi in physical space (2 real fields)
+  double2* H1;                  // delphiH1^ (varying bottom; flat bottom with walls)
+  double2* WP;                  // flat bottom with walls: the round trip of (C u^, C v^)
+  double2* dph;                 // breaking: delphiH^ as the assembly forms it (nullptr: off)
 };
 
 // device control block of the stepper (one per engine)
@@ -153,150 +142,286 @@ __device__ __forceinline__ bool rhs_active(const Ctl2* c, int cond) {
 }
 
 // ---------------------------------------------------------------------------
-// one M-point slice in shared memory, transformed by one group of M/8 threads.
-// Groups of at least a warp synchronise on their own named barrier (id 1 + g), so
-// the groups of a CTA run their transforms independently; smaller groups fall
-// back to the CTA barrier and keep step with each other.
+// M-point transforms of slices in shared memory
 // ---------------------------------------------------------------------------
-template <int T>
-__device__ __forceinline__ void group_sync(int g) {
-  if constexpr (T >= 32) asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(T) : "memory");
-  else __syncthreads();
+// Position i of slice s: the swizzle of the 1D slices, odd slices turned by half a
+// 128-byte group, so that the two columns of a pair, which lie side by side in memory
+// and go to neighbouring slices, meet no bank conflict.
+__device__ __forceinline__ int sidx(int M, int s, int i) { return s * M + (pidx(i) ^ ((s & 1) << 2)); }
+__device__ __forceinline__ double2 slot(const double2* sm, int M, int s, int i) { return sm[sidx(M, s, i)]; }
+__device__ __forceinline__ void put(double2* sm, int M, int s, int i, double2 v) { sm[sidx(M, s, i)] = v; }
+
+// threads of a CTA that transforms two slices at a time, or four (1024 points; on
+// shorter slices the threads that no transform needs share the pointwise work: at
+// 256 x 128, M/16 threads a slice and no more took 65 us an RHS against 39), and the
+// CTAs that an SM's registers hold at 128 a thread (16 points and their twiddles).
+// 256 and 512 threads at 1024 points, one CTA less an SM, took 764 us an RHS against 665.
+__host__ __device__ constexpr int ctas(int threads) { return 512 / threads; }
+__host__ __device__ constexpr int thr2(int) { return 128; }
+__host__ __device__ constexpr int thr4(int) { return 256; }
+
+// 16-point DFT as 4 x 4
+__device__ __forceinline__ void dft16(double2* v, int sign) {
+  constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173, r = 0.70710678118654752440;
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    double2 t[4] = {v[n], v[n + 4], v[n + 8], v[n + 12]};
+    dft_small<4>(t, sign);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[n + 4 * k] = t[k];
+  }
+  // x W16^(n k), n the column, k the row of the 4 x 4 block
+  const double sg = double(sign);
+  auto rot = [&](double2 a, double c, double s) { return make_double2(c * a.x - sg * s * a.y, c * a.y + sg * s * a.x); };
+  v[5] = rot(v[5], c1, s1);
+  v[6] = rot(v[6], r, r);
+  v[7] = rot(v[7], s1, c1);
+  v[9] = rot(v[9], r, r);
+  v[10] = hwdev::mul_pm_i(v[10], sign);
+  v[11] = rot(v[11], -r, r);
+  v[13] = rot(v[13], s1, c1);
+  v[14] = rot(v[14], -r, r);
+  v[15] = rot(v[15], -c1, -s1);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) dft_small<4>(v + 4 * k, sign);
+  // v[4 k2 + k1] holds X[4 k1 + k2]
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = a + 1; b < 4; ++b) {
+      const double2 t = v[4 * a + b];
+      v[4 * a + b] = v[4 * b + a];
+      v[4 * b + a] = t;
+    }
 }
 
+// the threads of one slice: within a warp up to 512 points, two warps for 1024
+template <int TP>
+__device__ __forceinline__ void slice_sync(int g) {
+  if constexpr (TP > 32) asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(TP) : "memory");
+  else __syncwarp();
+}
+
+// one in-place Stockham radix-R pass of a slice by M/16 threads, 16 points each
 template <int M, int R>
-__device__ __forceinline__ void gpass(double2* buf, int Ns, const double2* __restrict__ tw, int sign, int tid,
-                                      int g, bool act) {
-  constexpr int T = M / 8;
-  constexpr int NB = M / R;
-  constexpr int BPT = 8 / R;
+__device__ __forceinline__ void spass(double2* sm, int s, int Ns, const double2* __restrict__ tw, int sign, int tid, int g,
+                                      bool act) {
+  constexpr int TP = M / 16, NB = M / R, BPT = 16 / R;
   double2 v[BPT][R];
   if (act) {
 #pragma unroll
-    for (int u = 0; u < BPT; ++u) {
-      const int j = tid + u * T;
+    for (int u = 0; u < BPT; ++u)
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[u][r] = buf[pidx(j + r * NB)];
-    }
+      for (int r = 0; r < R; ++r) v[u][r] = sm[sidx(M, s, tid + u * TP + r * NB)];
   }
-  group_sync<T>(g);
+  slice_sync<TP>(g);
   if (act) {
 #pragma unroll
     for (int u = 0; u < BPT; ++u) {
-      const int j = tid + u * T;
-      const int jm = j & (Ns - 1);
+      const int j = tid + u * TP, jm = j & (Ns - 1);
       if (Ns > 1) {
         const int qb = jm * (M / (Ns * R));
-        double2 w[R];
-        twiddle_powers<R>(twd(tw, qb, sign), w);
+        if constexpr (R == 16) {
+          // powers from w, w^2, w^4, w^8: at most three factors each
+          const double2 w1 = twd(tw, qb, sign), w2 = twd(tw, 2 * qb, sign), w4 = twd(tw, 4 * qb, sign),
+                        w8 = twd(tw, 8 * qb, sign), w3 = cmul(w2, w1);
+          const double2 lo[4] = {make_double2(1.0, 0.0), w1, w2, w3};
 #pragma unroll
-        for (int r = 1; r < R; ++r) v[u][r] = cmul(v[u][r], w[r]);
+          for (int r = 1; r < 4; ++r) v[u][r] = cmul(v[u][r], lo[r]);
+#pragma unroll
+          for (int h = 1; h < 4; ++h) {
+            const double2 wh = h == 1 ? w4 : (h == 2 ? w8 : cmul(w8, w4));
+            v[u][4 * h] = cmul(v[u][4 * h], wh);
+#pragma unroll
+            for (int r = 1; r < 4; ++r) v[u][4 * h + r] = cmul(v[u][4 * h + r], cmul(wh, lo[r]));
+          }
+        } else {
+          double2 w[R];
+          twiddle_powers<R>(twd(tw, qb, sign), w);
+#pragma unroll
+          for (int r = 1; r < R; ++r) v[u][r] = cmul(v[u][r], w[r]);
+        }
       }
-      dft_small<R>(v[u], sign);
-      const int idxD = (j - jm) * R + jm;
+      if constexpr (R == 16) dft16(v[u], sign);
+      else dft_small<R>(v[u], sign);
+      const int d = (j - jm) * R + jm;
 #pragma unroll
-      for (int r = 0; r < R; ++r) buf[pidx(idxD + r * Ns)] = v[u][r];
+      for (int r = 0; r < R; ++r) sm[sidx(M, s, d + r * Ns)] = v[u][r];
     }
   }
-  group_sync<T>(g);
+  slice_sync<TP>(g);
 }
 
-template <int M>
-__device__ __forceinline__ void gfft(double2* buf, const double2* __restrict__ tw, int sign, int tid, int g,
-                                     bool act) {
-  constexpr int L8 = (M >= 512) ? 3 : (M >= 64 ? 2 : 1);
-  constexpr int rem = M / (1 << (3 * L8));
-  int Ns = 1;
-#pragma unroll
-  for (int p = 0; p < L8; ++p) {
-    gpass<M, 8>(buf, Ns, tw, sign, tid, g, act);
-    Ns *= 8;
-  }
-  if constexpr (rem == 8) gpass<M, 8>(buf, Ns, tw, sign, tid, g, act);
-  else if constexpr (rem == 4) gpass<M, 4>(buf, Ns, tw, sign, tid, g, act);
-  else if constexpr (rem == 2) gpass<M, 2>(buf, Ns, tw, sign, tid, g, act);
-}
-
-// transform slices [0, ns) of the CTA's smem, kGroups at a time; CTA-wide barriers
-// on entry and exit (the phases around read and write every slice)
-template <int M>
-__device__ __forceinline__ void fft_slices(double2* sm, int ns, const double2* __restrict__ tw, int sign) {
-  constexpr int T = M / 8;
-  const int g = threadIdx.x / T, tid = threadIdx.x % T;
+// slices [s0, s0 + ns) by a CTA of NT threads, NT / (M/16) at a time; CTA-wide
+// barriers on entry and exit (the phases around read and write every slice).  Sixteen
+// points a thread: two passes of radix 16 for 256 points, three for 512 and 1024 where
+// eight points a thread took three and four, and no barrier wider than two warps.
+template <int M, int NT>
+__device__ __forceinline__ void fft_slices(double2* sm, int s0, int ns, const double2* __restrict__ tw, int sign) {
+  constexpr int TP = M / 16, G = NT / TP;
+  const int g = threadIdx.x / TP, tid = threadIdx.x % TP;
   __syncthreads();
-  for (int base = 0; base < ns; base += kGroups) {
-    const int s = base + g;
-    if constexpr (T >= 32) {
-      if (s < ns) gfft<M>(sm + (size_t)s * padded(M), tw, sign, tid, g, true);
+  for (int base = 0; base < ns; base += G) {
+    const int s = s0 + base + g;
+    const bool act = base + g < ns;
+    if (TP > 32 && !act) break;
+    if constexpr (M == 1024) {
+      spass<M, 8>(sm, s, 1, tw, sign, tid, g, act);
+      spass<M, 8>(sm, s, 8, tw, sign, tid, g, act);
+      spass<M, 16>(sm, s, 64, tw, sign, tid, g, act);
+    } else if constexpr (M == 512) {
+      spass<M, 8>(sm, s, 1, tw, sign, tid, g, act);
+      spass<M, 8>(sm, s, 8, tw, sign, tid, g, act);
+      spass<M, 8>(sm, s, 64, tw, sign, tid, g, act);
+    } else if constexpr (M == 256) {
+      spass<M, 16>(sm, s, 1, tw, sign, tid, g, act);
+      spass<M, 16>(sm, s, 16, tw, sign, tid, g, act);
+    } else if constexpr (M == 128) {
+      spass<M, 8>(sm, s, 1, tw, sign, tid, g, act);
+      spass<M, 16>(sm, s, 8, tw, sign, tid, g, act);
     } else {
-      gfft<M>(sm + (size_t)s * padded(M), tw, sign, tid, g, s < ns);
+      static_assert(M == 64, "slices of 64 to 1024 points");
+      spass<M, 8>(sm, s, 1, tw, sign, tid, g, act);
+      spass<M, 8>(sm, s, 8, tw, sign, tid, g, act);
     }
   }
   __syncthreads();
 }
 
-__device__ __forceinline__ double2 slot(double2* sm, int M, int s, int i) { return sm[(size_t)s * padded(M) + pidx(i)]; }
-__device__ __forceinline__ void put(double2* sm, int M, int s, int i, double2 v) { sm[(size_t)s * padded(M) + pidx(i)] = v; }
+// global -> shared copies without registers: every copy of a phase is in flight at once
+__device__ __forceinline__ void copy16(double2* dst, const double2* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // row-pair geometry and the Hermitian operators
 // ---------------------------------------------------------------------------
 struct Pair {
   int r[2];      // rows held (slice 2f + k holds row r[k] of field f)
-  int mr[2];     // index (0/1) of the mirror row of r[k]
+  int flip;      // the mirror of row r[k] is r[k ^ flip]
+  __device__ __forceinline__ int row(int k) const { return k ? r[1] : r[0]; }
 };
 
 __device__ __forceinline__ Pair row_pair(int b, int Ny) {
   Pair p;
-  if (b == 0) { p.r[0] = 0; p.r[1] = Ny / 2; p.mr[0] = 0; p.mr[1] = 1; }
-  else { p.r[0] = b; p.r[1] = Ny - b; p.mr[0] = 1; p.mr[1] = 0; }
+  p.flip = b != 0;
+  p.r[0] = b;
+  p.r[1] = b == 0 ? Ny / 2 : Ny - b;
   return p;
 }
 
-// value of E(A) (herm) or S(A) (!herm) at (row k, column c) where S is the
-// reference's fftwcomplex_2d_sym and E the Hermitian part of S(A) (what the real
-// part of the inverse transform sees).  v[k][s]: A at row r[k], column (s ? cm : c)
-// with cm = (Nx - c) % Nx.
-__device__ __forceinline__ double2 sym_at(const double2 v[2][2], const Pair& P, int k, int s, int c, int Nx, int Ny,
-                                          bool herm) {
-  const int r = P.r[k];
-  const double2 a = v[k][s];
-  const double2 m = v[P.mr[k]][s ^ 1];
-  if (c >= 1 && c < Nx / 2) return a;
-  if (c > Nx / 2) return cconj(m);
-  const bool selfrow = (r == 0) || (r == Ny / 2);
-  if (selfrow) return make_double2(a.x, 0.0);
-  if (c == 0) return (r < Ny / 2) ? a : cconj(m);
+// columns j and Nx - j of both rows: four points, each other's mirrors.  The
+// reference's symmetrisation takes the right half of a row from the left one, so what
+// is formed spectrally is formed at s = 0 alone and conjugated; columns 0 and Nx / 2,
+// their own mirrors, go as one quad (self) of which both are formed.
+struct Quad {
+  int r[2], cc[2], flip;
+  bool self;
+  __device__ __forceinline__ Quad(const Pair& P, int j, int Nx) {
+    r[0] = P.r[0];
+    r[1] = P.r[1];
+    flip = P.flip;
+    self = j == 0;
+    cc[0] = j;
+    cc[1] = self ? Nx / 2 : Nx - j;
+  }
+  __device__ __forceinline__ bool has(int s) const { return s == 0 || self; }
+  __device__ __forceinline__ size_t at(int k, int s, int Nx) const { return (size_t)r[k] * Nx + cc[s]; }
+};
+
+// spectra of the two real fields packed in slices s0, s0 + 1, at point (k, s)
+__device__ __forceinline__ void split_at(const double2* sm, int M, int s0, const Quad& Q, int k, int s, double2& A,
+                                         double2& B) {
+  const double2 z = slot(sm, M, s0 + k, Q.cc[s]);
+  const double2 m = slot(sm, M, s0 + (k ^ Q.flip), Q.cc[Q.self ? s : s ^ 1]);
+  A = make_double2(0.5 * (z.x + m.x), 0.5 * (z.y - m.y));
+  B = make_double2(0.5 * (z.y + m.y), -0.5 * (z.x - m.x));
+}
+
+// the reference's fftwcomplex_2d_sym (S) at a point of column 0 (s = 0) or Nx / 2, or
+// (herm) the Hermitian part of it, which the real part of the inverse transform sees
+__device__ __forceinline__ double2 self_sym(double2 a, double2 m, int r, int s, int Ny, bool herm) {
+  if (r == 0 || r == Ny / 2) return make_double2(a.x, 0.0);
+  if (s == 0) return r < Ny / 2 ? a : cconj(m);
   return herm ? make_double2(0.5 * (a.x + m.x), 0.5 * (a.y - m.y)) : a;
+}
+
+// E(S(x)) + i E(S(y)) into slices s0, s0 + 1 at the quad's points; x[k][s] for s = 0
+// (and 1 in a self quad)
+__device__ __forceinline__ void emit_pack(double2* sm, int M, int s0, const Quad& Q, int Ny, const double2 x[2][2],
+                                          const double2 y[2][2]) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (!Q.self) {
+      const double2 a = x[k][0], b = y[k][0], c = Q.flip ? x[k ^ 1][0] : x[k][0], d = Q.flip ? y[k ^ 1][0] : y[k][0];
+      put(sm, M, s0 + k, Q.cc[0], make_double2(a.x - b.y, a.y + b.x));
+      put(sm, M, s0 + k, Q.cc[1], make_double2(c.x + d.y, d.x - c.y));
+    } else {
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const double2 a = self_sym(x[k][s], Q.flip ? x[k ^ 1][s] : x[k][s], Q.r[k], s, Ny, true);
+        const double2 b = self_sym(y[k][s], Q.flip ? y[k ^ 1][s] : y[k][s], Q.r[k], s, Ny, true);
+        put(sm, M, s0 + k, Q.cc[s], make_double2(a.x - b.y, a.y + b.x));
+      }
+    }
+  }
+}
+// S(x) (not its Hermitian part) into slices s0, s0 + 1
+__device__ __forceinline__ void emit_sym(double2* sm, int M, int s0, const Quad& Q, int Ny, const double2 x[2][2]) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (!Q.self) {
+      put(sm, M, s0 + k, Q.cc[0], x[k][0]);
+      put(sm, M, s0 + k, Q.cc[1], cconj(Q.flip ? x[k ^ 1][0] : x[k][0]));
+    } else {
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+        put(sm, M, s0 + k, Q.cc[s], self_sym(x[k][s], Q.flip ? x[k ^ 1][s] : x[k][s], Q.r[k], s, Ny, false));
+    }
+  }
 }
 
 // split Z = FFT(a + i b) at a point given Z there (z) and at its mirror (zm)
 __device__ __forceinline__ void split2(double2 z, double2 zm, double2& A, double2& B) {
   A = make_double2(0.5 * (z.x + zm.x), 0.5 * (z.y - zm.y));
-  const double2 w = make_double2(z.x - zm.x, z.y + zm.y);   // z - conj(zm)
-  B = make_double2(0.5 * w.y, -0.5 * w.x);                  // w / (2i)
+  B = make_double2(0.5 * (z.y + zm.y), -0.5 * (z.x - zm.x));
 }
 
+__device__ __forceinline__ double2 zero2() { return make_double2(0.0, 0.0); }
 // mul by -i s: (x, y) -> (s y, -s x)
 __device__ __forceinline__ double2 mul_mi(double2 a, double s) { return make_double2(s * a.y, -s * a.x); }
 // mul by +i s
 __device__ __forceinline__ double2 mul_pi(double2 a, double s) { return make_double2(-s * a.y, s * a.x); }
 
-// GSL natural cubic spline evaluation with a plain binary search
-__device__ __forceinline__ double spline2(const double* __restrict__ xs, const double* __restrict__ ys,
-                                          const double* __restrict__ cs, int n, double x) {
-  if (x < xs[0] || x > xs[n - 1]) return __longlong_as_double(0x7ff8000000000000ULL);
-  int lo = 0, hi = n - 1;
-  while (hi > lo + 1) {
-    const int i = (hi + lo) / 2;
-    if (xs[i] > x) hi = i; else lo = i;
+// GSL natural cubic spline evaluation of a row's line signal and its quadrature at x
+// (the bsearch's interval: a guess from the even spacing of the samples, moved on where
+// their times ask for it)
+__device__ __forceinline__ double2 line_signal(const Tab2& tb, int r, double x) {
+  const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+  if (x < tb.t0 || x > tb.tl || x != x) return make_double2(nan, nan);
+  const int n = tb.nt;
+  const size_t o = (size_t)r * n;
+  int lo = (int)((x - tb.t0) / tb.dts);
+  lo = lo < 0 ? 0 : (lo > n - 2 ? n - 2 : lo);
+  double xl, xh, y0, y1, c0, c1, s0, s1, e0, e1;
+  for (;;) {
+    xl = tb.tsig[lo]; xh = tb.tsig[lo + 1];
+    y0 = tb.sig[o + lo]; y1 = tb.sig[o + lo + 1]; c0 = tb.sigc[o + lo]; c1 = tb.sigc[o + lo + 1];
+    s0 = tb.sigs[o + lo]; s1 = tb.sigs[o + lo + 1]; e0 = tb.sigsc[o + lo]; e1 = tb.sigsc[o + lo + 1];
+    if (lo > 0 && xl > x) --lo;
+    else if (lo < n - 2 && xh <= x) ++lo;
+    else break;
   }
-  const double xl = xs[lo], xh = xs[lo + 1], yl = ys[lo], yh = ys[lo + 1];
-  const double h = xh - xl, dy = yh - yl, dx = x - xl;
-  const double ci = cs[lo], cip = cs[lo + 1];
-  const double bi = dy / h - h * (cip + 2.0 * ci) / 3.0;
-  const double di = (cip - ci) / (3.0 * h);
-  return yl + dx * (bi + dx * (ci + dx * di));
+  const double h = xh - xl, dx = x - xl;
+  auto cubic = [&](double a, double b, double ci, double cip) {
+    const double dy = b - a;
+    const double bi = dy / h - h * (cip + 2.0 * ci) / 3.0;
+    const double di = (cip - ci) / (3.0 * h);
+    return a + dx * (bi + dx * (ci + dx * di));
+  };
+  return make_double2(cubic(y0, y1, c0, c1), cubic(s0, s1, e0, e1));
 }
 
 // modes: 0 direct RHS, 1 k1 (dydt_in), 2..6 the rkf45 stages, 7 k_out after an
@@ -370,365 +495,489 @@ k2_stage(RK2 rk, Work2 w, const Ctl2* __restrict__ ctl, int mode, int cond, size
 }
 
 // ---------------------------------------------------------------------------
-// A: row pass, stage input -> symmetrised spectra -> inverse row FFT
-// smem slices: 2f + k = field f (0: eta|Lphi, 1: u|M0u, 2: v|M0v), row r[k]
+// what the passes share
 // ---------------------------------------------------------------------------
-template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
-k2_rowA(Tab2 tb, Work2 w, RK2 rk, const Ctl2* __restrict__ ctl, Ctl2* ctlw, int mode, int cond) {
-  if (!rhs_active(ctl, cond)) return;
-  extern __shared__ double2 sm[];
-  const int Nx = tb.nx, Ny = tb.ny;
-  const size_t n = (size_t)tb.n;
-  const Pair P = row_pair(blockIdx.x, Ny);
-  const double ts = stage_time(ctl, mode);
-  if (blockIdx.x == 0 && threadIdx.x == 0 && ctlw) ctlw->rhs += 1;
-  // line signals of the two rows at the stage time
-  if (tb.has_src && threadIdx.x < 2) {
-    const int r = P.r[threadIdx.x];
-    const size_t o = (size_t)r * tb.nt;
-    w.insig[r] = spline2(tb.tsig, tb.sig + o, tb.sigc + o, tb.nt, ts);
-    w.insigs[r] = spline2(tb.tsig, tb.sigs + o, tb.sigsc + o, tb.nt, ts);
+// nf fields (two rows each) into / out of slices s0...
+template <int M, int NT>
+__device__ __forceinline__ void row_load(double2* sm, int s0, int nf, const double2* __restrict__ F, const Pair& P, size_t n) {
+  for (int s = 0; s < 2 * nf; ++s) {
+    const double2* src = F + (s >> 1) * n + (size_t)P.row(s & 1) * M;
+    for (int j = threadIdx.x; j < M; j += NT) copy16(sm + sidx(M, s0 + s, j), src + j);
   }
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
-    double2 e[2][2], u[2][2], v[2][2], t1[2][2], t2[2][2];
+  copies_done();
+}
+template <int M, int NT>
+__device__ __forceinline__ void row_store(const double2* sm, int s0, int nf, double2* __restrict__ F, const Pair& P, size_t n) {
+  for (int s = 0; s < 2 * nf; ++s) {
+    double2* dst = F + (s >> 1) * n + (size_t)P.row(s & 1) * M;
+#pragma unroll 4
+    for (int j = threadIdx.x; j < M; j += NT) dst[j] = slot(sm, M, s0 + s, j);
+  }
+}
+// the same for column pairs (slice 2f + k = field f, column 2c + k): neighbouring lanes
+// take the two columns, 32 contiguous bytes of a row
+template <int M, int NT>
+__device__ __forceinline__ void col_load(double2* sm, int s0, int nf, const double2* __restrict__ F, int Nx, int c, size_t n) {
+  for (int f = 0; f < nf; ++f) {
+    const double2* src = F + f * n + 2 * c;
+    for (int t = threadIdx.x; t < 2 * M; t += NT)
+      copy16(sm + sidx(M, s0 + 2 * f + (t & 1), t >> 1), src + (size_t)(t >> 1) * Nx + (t & 1));
+  }
+  copies_done();
+}
+template <int M, int NT>
+__device__ __forceinline__ void col_store(const double2* sm, int s0, int nf, double2* __restrict__ F, int Nx, int c, size_t n) {
+  for (int f = 0; f < nf; ++f) {
+    double2* dst = F + f * n + 2 * c;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < 2 * M; t += NT)
+      dst[(size_t)(t >> 1) * Nx + (t & 1)] = slot(sm, M, s0 + 2 * f + (t & 1), t >> 1);
+  }
+}
+// physical point t of a column pair
+struct ColPt {
+  int y, k;
+  size_t q;
+  __device__ __forceinline__ ColPt(int t, int c, int Nx) : y(t >> 1), k(t & 1), q((size_t)(t >> 1) * Nx + 2 * c + (t & 1)) {}
+};
+
+// damping of eta less the source in physical space; D0's field
+__device__ __forceinline__ double eta_loss(const Tab2& tb, const Work2& w, size_t q, int y, double damp, double eta) {
+  double d = damp * eta;
+  if (tb.has_src) d -= tb.fac_src * w.insig[y] * tb.gsrc[q] + w.insigs[y] * tb.ssrc[q];
+  return d;
+}
+
+// how the damping travels: 0 in pass D's physical space; with breaking, whose update
+// rewrites dt eta^, that of eta by itself as a spectrum (1); with ChiAdj = 1, where no
+// pass D runs, all three as spectra (2)
+__device__ __forceinline__ int damp_fields(const Tab2& tb, const Work2& w) { return tb.chi_one ? 2 : (w.dph ? 1 : 0); }
+
+// the loss fields of a physical point into slices s0 + 2 f + k
+__device__ __forceinline__ void emit_loss(double2* sm, int M, int s0, int nd, const ColPt& p, const Tab2& tb, const Work2& w,
+                                          double eta, double u, double v) {
+  if (nd == 0) return;
+  const double dm = tb.damp[p.q];
+  put(sm, M, s0 + p.k, p.y, make_double2(eta_loss(tb, w, p.q, p.y, dm, eta), nd == 2 ? dm * u : 0.0));
+  if (nd == 2) put(sm, M, s0 + 2 + p.k, p.y, make_double2(dm * v, 0.0));
+}
+// and their spectra, at all of a quad's points, into w.D
+__device__ __forceinline__ void store_loss(const double2* sm, int M, int s0, int nd, const Quad& Q, int Nx, const Work2& w,
+                                           size_t n) {
+  if (nd == 0) return;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int r = P.r[k];
+  for (int k = 0; k < 2; ++k)
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const size_t q = (size_t)r * Nx + cc[s];
-        const double2 ze = w.z[q], zu = w.z[n + q], zv = w.z[2 * n + q];
-        e[k][s] = ze; u[k][s] = zu; v[k][s] = zv;
-        // M0 u^ = -i (C^2/g) kx u^ ; M0 v^ = -i (C^2/g) ky v^
-        const double cg = tb.c2g[q];
-        const double kxv = tb.kx[cc[s]], kyv = tb.ky[r];
-        t1[k][s] = make_double2(cg * kxv * zu.y, -cg * kxv * zu.x);
-        t2[k][s] = make_double2(cg * kyv * zv.y, -cg * kyv * zv.x);
+    for (int s = 0; s < 2; ++s) {
+      double2 a, b;
+      split_at(sm, M, s0, Q, k, s, a, b);
+      w.D[Q.at(k, s, Nx)] = a;
+      if (nd == 2) {
+        w.D[n + Q.at(k, s, Nx)] = b;
+        split_at(sm, M, s0 + 2, Q, k, s, a, b);
+        w.D[2 * n + Q.at(k, s, Nx)] = a;
       }
     }
-    // slices 2..5: E(u^) + i E(M0u^), E(v^) + i E(M0v^)
+}
+
+// the adjustment's input at a quad: S(i kx dH), S(i ky dH), S(a) into slices 0..5
+__device__ __forceinline__ void emit_adjust(double2* sm, int M, const Quad& Q, const Tab2& tb, const double2 dH[2][2],
+                                            const double2 a[2][2]) {
+  double2 x[2][2];
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+  for (int k = 0; k < 2; ++k)
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        const double2 U1 = sym_at(u, P, k, s, c, Nx, Ny, true), U2 = sym_at(t1, P, k, s, c, Nx, Ny, true);
-        const double2 V1 = sym_at(v, P, k, s, c, Nx, Ny, true), V2 = sym_at(t2, P, k, s, c, Nx, Ny, true);
-        put(sm, M, 2 + k, c, make_double2(U1.x - U2.y, U1.y + U2.x));
-        put(sm, M, 4 + k, c, make_double2(V1.x - V2.y, V1.y + V2.x));
-      }
-    // L phi^ = M0u^ + M0v^ ; slices 0, 1: E(eta^) + i E(L phi^)
+    for (int s = 0; s < 2; ++s)
+      if (Q.has(s)) x[k][s] = mul_pi(dH[k][s], tb.kx[Q.cc[s]]);
+  emit_sym(sm, M, 0, Q, tb.ny, x);
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+  for (int k = 0; k < 2; ++k)
 #pragma unroll
-      for (int s = 0; s < 2; ++s) t1[k][s] = make_double2(t1[k][s].x + t2[k][s].x, t1[k][s].y + t2[k][s].y);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        const double2 E1 = sym_at(e, P, k, s, c, Nx, Ny, true), E2 = sym_at(t1, P, k, s, c, Nx, Ny, true);
-        put(sm, M, 0 + k, c, make_double2(E1.x - E2.y, E1.y + E2.x));
-      }
+    for (int s = 0; s < 2; ++s)
+      if (Q.has(s)) x[k][s] = mul_pi(dH[k][s], tb.ky[Q.r[k]]);
+  emit_sym(sm, M, 2, Q, tb.ny, x);
+  emit_sym(sm, M, 4, Q, tb.ny, a);
+}
+// and on its way: inverse rows into w.W, or with ChiAdj = 1, which leaves S(A) as it is,
+// the terms with the damping of u and v straight into w.V
+template <int M, int NT>
+__device__ __forceinline__ void send_adjust(double2* sm, const Pair& P, const Tab2& tb, const Work2& w, size_t n) {
+  if (!tb.chi_one) {
+    fft_slices<M, NT>(sm, 0, 6, tb.twx, +1);
+    row_store<M, NT>(sm, 0, 3, w.W, P, n);
+    return;
   }
-  fft_slices<M>(sm, 6, tb.twx, +1);
+  __syncthreads();
   for (int s = 0; s < 6; ++s) {
-    const int f = s >> 1, k = s & 1;
-    double2* dst = w.R + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) dst[j] = slot(sm, M, s, j);
+    const size_t row = (size_t)P.row(s & 1) * M;
+    for (int j = threadIdx.x; j < M; j += NT) {
+      double2 v = slot(sm, M, s, j);
+      if (s < 4) v = cadd(v, w.D[(1 + (s >> 1)) * n + row + j]);
+      w.V[(s >> 1) * n + row + j] = v;
+    }
   }
 }
 
-// column-pair load / store helpers (slice 2f + k = field f, column 2c + k)
-template <int M>
-__device__ __forceinline__ void col_load(double2* sm, int s0, const double2* __restrict__ F, int Nx, int c) {
-  for (int y = threadIdx.x; y < M; y += blockDim.x) {
-    const double2* p = F + (size_t)y * Nx + 2 * c;
-    put(sm, M, s0, y, p[0]);
-    put(sm, M, s0 + 1, y, p[1]);
-  }
-}
-template <int M>
-__device__ __forceinline__ void col_store(const double2* sm, int s0, double2* __restrict__ F, int Nx, int c) {
-  for (int y = threadIdx.x; y < M; y += blockDim.x) {
-    double2* p = F + (size_t)y * Nx + 2 * c;
-    p[0] = sm[(size_t)s0 * padded(M) + pidx(y)];
-    p[1] = sm[(size_t)(s0 + 1) * padded(M) + pidx(y)];
+// the first row pass's extras: the RHS counter and the two rows' line signals at the
+// stage time, by the last warp's lanes
+__device__ __forceinline__ void stage_extras(const Tab2& tb, const Work2& w, const Pair& P, const Ctl2* ctl, Ctl2* ctlw, int mode,
+                                             int NT) {
+  if (blockIdx.y != 0) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && ctlw) ctlw->rhs += 1;
+  const int l = NT - 1 - (int)threadIdx.x;
+  if (tb.has_src && l < 2) {
+    const double2 s = line_signal(tb, P.r[l], stage_time(ctl, mode));
+    w.insig[P.r[l]] = s.x;
+    w.insigs[P.r[l]] = s.y;
   }
 }
 
 // ---------------------------------------------------------------------------
-// B: column pass, inverse column FFT -> physical products -> forward column FFT
+// A: row pass of the flat bottom, one CTA per row pair and field:
+//    0 (eta, u); 1 (v, L phi) under HS2, (v, M0u) under HS3, (v, -) under HS1; 2 (M0v, -)
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+k2_rowA(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, Ctl2* ctlw, int mode, int cond) {
+  if (!rhs_active(ctl, cond)) return;
+  extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
+  const int Nx = M, Ny = tb.ny, f = blockIdx.y;
+  const size_t n = (size_t)tb.n;
+  const Pair P = row_pair(blockIdx.x, Ny);
+  stage_extras(tb, w, P, ctl, ctlw, mode, NT);
+#pragma unroll 2
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
+    double2 x[2][2], y[2][2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
+        if (f == 0) {
+          x[k][s] = w.z[q];
+          y[k][s] = w.z[n + q];
+        } else {
+          const double2 zu = w.z[n + q], zv = w.z[2 * n + q];
+          // M0 u^ = -i (C^2/g) kx u^, M0 v^ = -i (C^2/g) ky v^
+          const double cg = tb.c2g[q];
+          const double2 mu = mul_mi(zu, cg * tb.kx[Q.cc[s]]), mv = mul_mi(zv, cg * tb.ky[Q.r[k]]);
+          x[k][s] = f == 1 ? zv : mv;
+          y[k][s] = f == 2 || tb.model == 1 ? zero2() : (tb.model == 3 ? mu : cadd(mu, mv));
+        }
+      }
+    emit_pack(sm, M, 0, Q, Ny, x, y);
+  }
+  fft_slices<M, NT>(sm, 0, 2, tb.twx, +1);
+  row_store<M, NT>(sm, 0, 1, w.R + f * n, P, n);
+}
+
+// ---------------------------------------------------------------------------
+// B: column pass of the flat bottom, inverse -> products (each x wallchar,
+//    2d/fun_odesolver.c:3239-3249) -> forward.  Fields: 0 (eta L phi, eta u),
+//    1 (eta v, deletaH2), under HS3 2 (eta^2 M0u, eta^2 M0v), then the loss fields.
+// ---------------------------------------------------------------------------
+template <int M>
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
 k2_colB(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  const int Nx = tb.nx;
+  constexpr int NT = thr4(M);
+  const int Nx = tb.nx, c = blockIdx.x, nd = damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
-  const int c = blockIdx.x;
-  for (int f = 0; f < 3; ++f) col_load<M>(sm, 2 * f, w.R + f * n, Nx, c);
-  fft_slices<M>(sm, 6, tb.twy, +1);
+  const bool hs3 = tb.model == 3;
+  const int nin = hs3 ? 3 : 2, np = hs3 ? 3 : 2;
+  col_load<M, NT>(sm, 0, nin, w.R, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 2 * nin, tb.twy, +1);
   const double invN = 1.0 / ((double)tb.n);
-  for (int y = threadIdx.x; y < M; y += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const size_t q = (size_t)y * Nx + 2 * c + k;
-      const double2 P1 = slot(sm, M, 0 + k, y), P2 = slot(sm, M, 2 + k, y), P3 = slot(sm, M, 4 + k, y);
-      const double eta = P1.x * invN, lphi = P1.y * invN;
-      const double u = P2.x * invN, m0u = P2.y * invN;
-      const double v = P3.x * invN, m0v = P3.y * invN;
-      if (w.phys) {   // kept for the breaking kernels
-        w.phys[q] = eta;
-        w.phys[n + q] = u;
-        w.phys[2 * n + q] = v;
-      }
-      const double dmp = tb.damp[q];
-      // Q1 = dampeta + i dampu, Q2 = dampv + i deletaH2, Q3 = etaM0u + i eta u, Q4 = etaM0v + i eta v
-      put(sm, M, 0 + k, y, make_double2(dmp * eta, dmp * u));
-      put(sm, M, 2 + k, y, make_double2(dmp * v, 0.5 * ((u * u + v * v) - lphi * lphi)));
-      if (tb.wallchar) {   // the H2 products carry wallchar (2d/fun_odesolver.c:3239-3249)
-        const double wc = tb.wallchar[q];
-        put(sm, M, 2 + k, y, make_double2(dmp * v, 0.5 * ((u * u + v * v) - lphi * lphi) * wc));
-        put(sm, M, 4 + k, y, make_double2(eta * m0u * wc, eta * u * wc));
-        put(sm, M, 6 + k, y, make_double2(eta * m0v * wc, eta * v * wc));
-      } else {
-        put(sm, M, 4 + k, y, make_double2(eta * m0u, eta * u));
-        put(sm, M, 6 + k, y, make_double2(eta * m0v, eta * v));
-      }
+#pragma unroll 2
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+    const ColPt p(t, c, Nx);
+    const double wc = tb.wallchar ? tb.wallchar[p.q] : 1.0;
+    const double2 P1 = slot(sm, M, p.k, p.y), P2 = slot(sm, M, 2 + p.k, p.y);
+    const double eta = P1.x * invN, u = P1.y * invN, v = P2.x * invN;
+    double lphi = P2.y * invN;
+    if (hs3) {
+      const double m0u = lphi, m0v = slot(sm, M, 4 + p.k, p.y).x * invN;
+      lphi = m0u + m0v;
+      put(sm, M, 4 + p.k, p.y, make_double2(eta * eta * m0u * wc, eta * eta * m0v * wc));
+      w.op[n + p.q] = lphi;
     }
+    w.phys[p.q] = eta;
+    w.phys[n + p.q] = u;
+    w.phys[2 * n + p.q] = v;
+    put(sm, M, p.k, p.y, make_double2(eta * lphi * wc, eta * u * wc));
+    put(sm, M, 2 + p.k, p.y, make_double2(eta * v * wc, 0.5 * ((u * u + v * v) - lphi * lphi) * wc));
+    emit_loss(sm, M, 2 * np, nd, p, tb, w, eta, u, v);
   }
-  fft_slices<M>(sm, 8, tb.twy, -1);
-  for (int f = 0; f < 4; ++f) col_store<M>(sm, 2 * f, w.Q + f * n, Nx, c);
+  fft_slices<M, NT>(sm, 0, 2 * (np + nd), tb.twy, -1);
+  col_store<M, NT>(sm, 0, np + nd, w.Q, Nx, c, n);
 }
 
 // ---------------------------------------------------------------------------
-// C: row pass, forward row FFT -> split -> damping spectra, symmetrised H2 terms
-//    -> inverse row FFT (or, with ChiAdj = 1, the adjusted terms themselves)
+// C: row pass of the flat bottom, forward, split.  HS2: the adjustment's input -> inverse
+//    rows.  HS3 (fun_termshat_AB3_2DF_uv, :3512-3897): the second-order terms less
+//    (kx^2 (eta^2 M0u)^ + ky^2 (eta^2 M0v)^) / 2 are kept, and (L (eta L phi), div(grad phi))
+//    goes to physical space.
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
 k2_rowC(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  const int Nx = tb.nx, Ny = tb.ny;
+  constexpr int NT = thr4(M);
+  const int Nx = M, Ny = tb.ny, nd = damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
+  const bool hs3 = tb.model == 3;
+  const int np = hs3 ? 3 : 2;
   const Pair P = row_pair(blockIdx.x, Ny);
-  for (int s = 0; s < 8; ++s) {
-    const int f = s >> 1, k = s & 1;
-    const double2* src = w.Q + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) put(sm, M, s, j, src[j]);
+  row_load<M, NT>(sm, 0, np + nd, w.Q, P, n);
+  fft_slices<M, NT>(sm, 0, 2 * (np + nd), tb.twx, -1);
+#pragma unroll 1
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
+    double2 dH[2][2], a[2][2], lq[2][2], dv[2][2];
+    store_loss(sm, M, 2 * np, nd, Q, Nx, w, n);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
+        const double L = tb.l2d[q], kx = tb.kx[Q.cc[s]], ky = tb.ky[Q.r[k]];
+        double2 qh, eu, ev;
+        split_at(sm, M, 0, Q, k, s, qh, eu);
+        split_at(sm, M, 2, Q, k, s, ev, dH[k][s]);
+        // delu H2^ + delv H2^ = -L (eta L phi)^ - i kx (eta u)^ - i ky (eta v)^
+        lq[k][s] = cscale(qh, L);
+        a[k][s] = csub(cadd(mul_mi(eu, kx), mul_mi(ev, ky)), lq[k][s]);
+        if (hs3) {
+          double2 cu, cv;
+          split_at(sm, M, 4, Q, k, s, cu, cv);
+          a[k][s] = csub(a[k][s], cadd(cscale(cu, 0.5 * (kx * kx)), cscale(cv, 0.5 * (ky * ky))));
+          dv[k][s] = cadd(mul_pi(w.z[n + q], kx), mul_pi(w.z[2 * n + q], ky));
+          w.T[q] = a[k][s];
+          w.T[n + q] = dH[k][s];
+        }
+      }
+    if (hs3) emit_pack(sm, M, 0, Q, Ny, lq, dv);
+    else emit_adjust(sm, M, Q, tb, dH, a);
   }
-  fft_slices<M>(sm, 8, tb.twx, -1);
-  // Each quad (columns j and Nx - j of both rows) is read and rewritten by one
-  // thread at its own positions only, so no barrier separates the reads from the
-  // writes.  Output slices: 0,1 S(ikx deletaH2^), 2,3 S(iky deletaH2^),
-  // 4,5 S(deluH2^), 6,7 S(delvH2^); each pair of slices is written after the
-  // quad's values of the field held there have been read.
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
-    double2 z[2][2], a1[2][2], a2[2][2];
-    // Q1 -> damping spectra of eta and u
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) z[k][s] = slot(sm, M, 0 + k, cc[s]);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        double2 de, du;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], de, du);
-        const size_t q = (size_t)P.r[k] * Nx + cc[s];
-        w.D[q] = de;
-        w.D[n + q] = du;
-      }
-    // Q2 -> damping spectrum of v, deletaH2^ -> i kx deletaH2^, i ky deletaH2^
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) z[k][s] = slot(sm, M, 2 + k, cc[s]);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 dv, dH;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], dv, dH);
-        const int r = P.r[k], c = cc[s];
-        if (s == 0 || cm != j) w.D[2 * n + (size_t)r * Nx + c] = dv;
-        a1[k][s] = mul_pi(dH, tb.kx[c]);
-        a2[k][s] = mul_pi(dH, tb.ky[r]);
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        put(sm, M, 0 + k, c, sym_at(a1, P, k, s, c, Nx, Ny, false));
-        put(sm, M, 2 + k, c, sym_at(a2, P, k, s, c, Nx, Ny, false));
-      }
-    // Q3 -> deluH2^ = -L (eta M0u)^ - i kx (eta u)^
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) z[k][s] = slot(sm, M, 4 + k, cc[s]);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 em, eu;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], em, eu);
-        const int r = P.r[k], c = cc[s];
-        const double L = tb.l2d[(size_t)r * Nx + c], kxv = tb.kx[c];
-        a1[k][s] = make_double2(-L * em.x + kxv * eu.y, -L * em.y - kxv * eu.x);
-      }
-    // Q4 -> delvH2^ = -L (eta M0v)^ - i ky (eta v)^
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) z[k][s] = slot(sm, M, 6 + k, cc[s]);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 em, ev;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], em, ev);
-        const int r = P.r[k], c = cc[s];
-        const double L = tb.l2d[(size_t)r * Nx + c], kyv = tb.ky[r];
-        a2[k][s] = make_double2(-L * em.x + kyv * ev.y, -L * em.y - kyv * ev.x);
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        put(sm, M, 4 + k, c, sym_at(a1, P, k, s, c, Nx, Ny, false));
-        put(sm, M, 6 + k, c, sym_at(a2, P, k, s, c, Nx, Ny, false));
-      }
-  }
-  __syncthreads();
-  double2* dst = tb.chi_one ? w.V : w.W;
-  if (!tb.chi_one) fft_slices<M>(sm, 8, tb.twx, +1);
-  for (int s = 0; s < 8; ++s) {
-    const int f = s >> 1, k = s & 1;
-    double2* d = dst + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) d[j] = slot(sm, M, s, j);
+  if (hs3) {
+    fft_slices<M, NT>(sm, 0, 2, tb.twx, +1);
+    row_store<M, NT>(sm, 0, 1, w.R, P, n);
+  } else {
+    send_adjust<M, NT>(sm, P, tb, w, n);
   }
 }
 
 // ---------------------------------------------------------------------------
-// D: column pass, inverse column FFT -> x ChiAdj / N -> forward column FFT;
-//    slices 8, 9: column transform of the source (row transform tabulated)
+// HS3: the cubic products from L (eta L phi), div(grad phi) in physical space:
+//   p  = eta L(eta L phi) + eta^2 div(grad phi) / 2, whose L^ adds to delu + delv,
+//   h3 = L phi (eta div(grad phi) + L(eta L phi)) = deletaH3
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double2 cubic_products(const Tab2& tb, const Work2& w, size_t q, size_t n, double lel, double divg) {
+  const double eta = w.phys[q], lphi = w.op[n + q];
+  const double wc = tb.wallchar ? tb.wallchar[q] : 1.0;
+  return make_double2(eta * lel + 0.5 * (eta * eta * divg * wc), lphi * eta * divg + lphi * lel);
+}
+template <int M>
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+k2_colH3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
+  if (!rhs_active(ctl, cond)) return;
+  extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
+  const int Nx = tb.nx, c = blockIdx.x;
+  const size_t n = (size_t)tb.n;
+  col_load<M, NT>(sm, 0, 1, w.R, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, +1);
+  const double invN = 1.0 / ((double)tb.n);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+    const ColPt p(t, c, Nx);
+    const double2 a = slot(sm, M, p.k, p.y);
+    put(sm, M, p.k, p.y, cubic_products(tb, w, p.q, n, a.x * invN, a.y * invN));
+  }
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, -1);
+  col_store<M, NT>(sm, 0, 1, w.Q, Nx, c, n);
+}
+template <int M>
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2_rowI3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
+  if (!rhs_active(ctl, cond)) return;
+  extern __shared__ double2 sm[];
+  constexpr int NT = thr4(M);
+  const int Nx = M;
+  const size_t n = (size_t)tb.n;
+  const Pair P = row_pair(blockIdx.x, tb.ny);
+  row_load<M, NT>(sm, 0, 1, w.Q, P, n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twx, -1);
+#pragma unroll 1
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
+    double2 dH[2][2], a[2][2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
+        double2 ph, h3;
+        split_at(sm, M, 0, Q, k, s, ph, h3);
+        a[k][s] = cadd(w.T[q], cscale(ph, tb.l2d[q]));
+        dH[k][s] = cadd(w.T[n + q], h3);
+      }
+    emit_adjust(sm, M, Q, tb, dH, a);
+  }
+  send_adjust<M, NT>(sm, P, tb, w, n);
+}
+
+// ---------------------------------------------------------------------------
+// D: column pass, one CTA per column pair and field f: inverse -> x ChiAdj / N, with the
+//    damping (and source) that no spectrum carries -> forward.  The adjustment's complex
+//    intermediate is kept (the Nyquist column of S(A) is not Hermitian).
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2_colD(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  const int Nx = tb.nx;
+  constexpr int NT = thr2(M);
+  const int Nx = tb.nx, c = blockIdx.x, f = blockIdx.y;
   const size_t n = (size_t)tb.n;
-  const int c = blockIdx.x;
-  const int nadj = tb.chi_one ? 0 : 8;
-  if (!tb.chi_one) {
-    for (int f = 0; f < 4; ++f) col_load<M>(sm, 2 * f, w.W + f * n, Nx, c);
-    __syncthreads();
-    fft_slices<M>(sm, 8, tb.twy, +1);
-    const double invN = 1.0 / ((double)tb.n);
-    for (int y = threadIdx.x; y < M; y += blockDim.x) {
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const double ch = tb.chi[(size_t)y * Nx + 2 * c + k];
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          const double2 a = slot(sm, M, 2 * f + k, y);
-          put(sm, M, 2 * f + k, y, make_double2(a.x * invN * ch, a.y * invN * ch));
-        }
-      }
+  const bool loss = f < 2 || !w.dph;
+  const double* __restrict__ src = w.phys + (f == 2 ? 0 : f + 1) * n;
+  col_load<M, NT>(sm, 0, 1, w.W + f * n, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, +1);
+  const double invN = 1.0 / ((double)tb.n);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+    const ColPt p(t, c, Nx);
+    const double ch = tb.chi[p.q] * invN;
+    double d = 0.0;
+    if (loss) {
+      const double dm = tb.damp[p.q], v = src[p.q];
+      d = f == 2 ? -eta_loss(tb, w, p.q, p.y, dm, v) : dm * v;
     }
+    const double2 a = slot(sm, M, p.k, p.y);
+    put(sm, M, p.k, p.y, make_double2(a.x * ch + d, a.y * ch));
   }
-  if (tb.has_src) {
-    for (int y = threadIdx.x; y < M; y += blockDim.x) {
-      const double a = tb.fac_src * w.insig[y], b = w.insigs[y];
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const size_t q = (size_t)y * Nx + 2 * c + k;
-        const double2 g = tb.gx[q], s = tb.sx[q];
-        put(sm, M, nadj + k, y, make_double2(a * g.x + b * s.x, a * g.y + b * s.y));
-      }
-    }
-  }
-  __syncthreads();
-  const int ns = nadj + (tb.has_src ? 2 : 0);
-  fft_slices<M>(sm, ns, tb.twy, -1);
-  if (!tb.chi_one)
-    for (int f = 0; f < 4; ++f) col_store<M>(sm, 2 * f, w.V + f * n, Nx, c);
-  if (tb.has_src) col_store<M>(sm, nadj, w.src, Nx, c);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, -1);
+  col_store<M, NT>(sm, 0, 1, w.V + f * n, Nx, c, n);
 }
 
 // ---------------------------------------------------------------------------
-// E: row pass, forward row FFT of the adjusted terms -> dt Z
+// E: row pass, one CTA per row pair and component (0 u, 1 v, 2 eta): forward -> dt Z
 // ---------------------------------------------------------------------------
+// delphiH1^ at a point: the operator's on a varying bottom, the wall branch's on a flat
+// one with walls, else -i (kx C^2/g u^ + ky C^2/g v^)
+__device__ __forceinline__ double2 delphi_h1(const Tab2& tb, const Work2& w, size_t q, size_t n, double kx, double ky) {
+  if (tb.var || tb.wallchar) return w.H1[q];
+  const double cg = tb.c2g[q];
+  return cadd(mul_mi(w.z[n + q], cg * kx), mul_mi(w.z[2 * n + q], cg * ky));
+}
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2_rowE(Tab2 tb, Work2 w, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int cond, double2* __restrict__ direct_out) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  const int Nx = tb.nx, Ny = tb.ny;
+  constexpr int NT = thr2(M);
+  const int Nx = M, f = blockIdx.y;
   const size_t n = (size_t)tb.n;
-  const Pair P = row_pair(blockIdx.x, Ny);
-  for (int s = 0; s < 8; ++s) {
-    const int f = s >> 1, k = s & 1;
-    const double2* src = w.V + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) put(sm, M, s, j, src[j]);
+  const Pair P = row_pair(blockIdx.x, tb.ny);
+  const bool dspec = tb.chi_one || w.dph;   // the damping of eta comes as a spectrum
+  row_load<M, NT>(sm, 0, 1, w.V + f * n, P, n);
+  if (tb.chi_one) __syncthreads();
+  else fft_slices<M, NT>(sm, 0, 2, tb.twx, -1);
+  double2* out = rhs_out(rk, ctl, mode, direct_out) + (f == 2 ? 0 : f + 1) * n;
+  for (int k = 0; k < 2; ++k) {
+    const int r = P.row(k);
+    const double ky = tb.ky[r];
+#pragma unroll 4
+    for (int j = threadIdx.x; j < Nx; j += NT) {
+      const size_t q = (size_t)r * Nx + j;
+      const double kx = tb.kx[j], a = tb.aal[q];
+      const double2 v = slot(sm, M, k, j);
+      if (f == 2) {
+        const double2 dphi = cadd(delphi_h1(tb, w, q, n, kx, ky), v);
+        const double2 d = dspec ? w.D[q] : zero2();
+        if (w.dph) w.dph[q] = dphi;
+        out[q] = make_double2((dphi.x - d.x) * a, (dphi.y - d.y) * a);
+      } else {
+        const double2 h = mul_mi(w.z[q], kGrav * (f == 0 ? kx : ky));
+        out[q] = make_double2((h.x - v.x) * a, (h.y - v.y) * a);
+      }
+    }
   }
-  __syncthreads();
-  if (!tb.chi_one) fft_slices<M>(sm, 8, tb.twx, -1);
+}
+
+// ---------------------------------------------------------------------------
+// HS1 (rhs_AB1_2DF_uv / rhs_AB1_2DB_uv, 2d/fun_odesolver.c:4350-4456): no H2 terms.  Column
+// pass: eta, u, v (inverse transforms of pass A's fields; on a varying bottom already in
+// physical space) -> their damping; row pass: dt Z.
+// ---------------------------------------------------------------------------
+template <int M>
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2_colH1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
+  if (!rhs_active(ctl, cond)) return;
+  extern __shared__ double2 sm[];
+  constexpr int NT = thr4(M);
+  const int Nx = tb.nx, c = blockIdx.x;
+  const size_t n = (size_t)tb.n;
+  if (!tb.var) {
+    col_load<M, NT>(sm, 0, 2, w.R, Nx, c, n);
+    fft_slices<M, NT>(sm, 0, 4, tb.twy, +1);
+  }
+  const double invN = 1.0 / ((double)tb.n);
+#pragma unroll 2
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+    const ColPt p(t, c, Nx);
+    double eta, u, v;
+    if (tb.var) {
+      eta = w.phys[p.q];
+      u = w.phys[n + p.q];
+      v = w.phys[2 * n + p.q];
+    } else {
+      const double2 a = slot(sm, M, p.k, p.y), b = slot(sm, M, 2 + p.k, p.y);
+      eta = a.x * invN;
+      u = a.y * invN;
+      v = b.x * invN;
+    }
+    emit_loss(sm, M, 0, 2, p, tb, w, eta, u, v);
+  }
+  fft_slices<M, NT>(sm, 0, 4, tb.twy, -1);
+  col_store<M, NT>(sm, 0, 2, w.Q, Nx, c, n);
+}
+template <int M>
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2_rowH1(Tab2 tb, Work2 w, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int cond, double2* __restrict__ direct_out) {
+  if (!rhs_active(ctl, cond)) return;
+  extern __shared__ double2 sm[];
+  constexpr int NT = thr4(M);
+  const int Nx = M;
+  const size_t n = (size_t)tb.n;
+  const Pair P = row_pair(blockIdx.x, tb.ny);
+  row_load<M, NT>(sm, 0, 2, w.Q, P, n);
+  fft_slices<M, NT>(sm, 0, 4, tb.twx, -1);
   double2* out = rhs_out(rk, ctl, mode, direct_out);
   for (int k = 0; k < 2; ++k) {
-    const int r = P.r[k];
-    const double kyv = tb.ky[r];
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) {
+    const int r = P.row(k);
+    const double ky = tb.ky[r];
+#pragma unroll 2
+    for (int j = threadIdx.x; j < Nx; j += NT) {
       const size_t q = (size_t)r * Nx + j;
-      const double kxv = tb.kx[j];
-      const double a = tb.aal[q], cg = tb.var ? 0.0 : tb.c2g[q];
-      const double2 ze = w.z[q], zu = w.z[n + q], zv = w.z[2 * n + q];
-      double2 dphi;
-      if (tb.var) {
-        // delu H1^ + delv H1^ from the two-depth operator (2d/fun_odesolver.c:4560-4563)
-        const double2 h1u = w.H1[q], h1v = w.H1[n + q];
-        dphi = make_double2(h1u.x + h1v.x, h1u.y + h1v.y);
-      } else if (tb.wallchar) {
-        dphi = w.H1[q];   // the wall branch's delphiH1^ (k2w_row3)
-      } else {
-        // delphiH1^ = -i (kx C^2/g u^ + ky C^2/g v^)
-        const double2 du1 = make_double2(cg * zu.x, cg * zu.y), dv1 = make_double2(cg * zv.x, cg * zv.y);
-        dphi = make_double2(kxv * du1.y + kyv * dv1.y, -kxv * du1.x - kyv * dv1.x);
-      }
-      double2 ix = slot(sm, M, 0 + k, j), iy = slot(sm, M, 2 + k, j);
-      if (tb.model != 1) {   // HS2, HS3 (the cubic terms are summed into the same slices)
-        const double2 au = slot(sm, M, 4 + k, j), av = slot(sm, M, 6 + k, j);
-        dphi = make_double2(dphi.x + au.x + av.x, dphi.y + au.y + av.y);
-      } else {
-        // HS1 (rhs_AB1_2DF_uv / rhs_AB1_2DB_uv, 2d/fun_odesolver.c:4350-4456): no H2 terms
-        ix = make_double2(0.0, 0.0);
-        iy = make_double2(0.0, 0.0);
-      }
-      if (w.dph) w.dph[q] = dphi;
-      const double2 S = tb.has_src ? w.src[q] : make_double2(0.0, 0.0);
-      const double2 de = w.D[q], du = w.D[n + q], dv = w.D[2 * n + q];
-      out[q] = make_double2((S.x + dphi.x - de.x) * a, (S.y + dphi.y - de.y) * a);
-      out[n + q] = make_double2((kGrav * kxv * ze.y - ix.x - du.x) * a, (-kGrav * kxv * ze.x - ix.y - du.y) * a);
-      out[2 * n + q] = make_double2((kGrav * kyv * ze.y - iy.x - dv.x) * a, (-kGrav * kyv * ze.x - iy.y - dv.y) * a);
+      const double kx = tb.kx[j], a = tb.aal[q];
+      const int jm = (Nx - j) & (Nx - 1), km = k ^ P.flip;
+      double2 de, du, dv, none;
+      split2(slot(sm, M, k, j), slot(sm, M, km, jm), de, du);
+      split2(slot(sm, M, 2 + k, j), slot(sm, M, 2 + km, jm), dv, none);
+      const double2 ze = w.z[q], dphi = delphi_h1(tb, w, q, n, kx, ky);
+      const double2 hu = mul_mi(ze, kGrav * kx), hv = mul_mi(ze, kGrav * ky);
+      out[q] = make_double2((dphi.x - de.x) * a, (dphi.y - de.y) * a);
+      out[n + q] = make_double2((hu.x - du.x) * a, (hu.y - du.y) * a);
+      out[2 * n + q] = make_double2((hv.x - dv.x) * a, (hv.y - dv.y) * a);
     }
   }
 }

@@ -170,70 +170,69 @@ __device__ __forceinline__ double gyat(const double* a, int st, int Nx, int Ny, 
 // rowI: S(delphiH^) into dt eta^, and E(S(delphiH^)) + i E(S(HilbEta^)) -> inverse rows
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2b_rowI(Tab2 tb, Work2 w, Brk2 b, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int cond,
          double2* __restrict__ direct_out) {
   if (!rhs_active(ctl, cond) || !brk_update(ctl, mode)) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx, Ny = tb.ny;
   const Pair P = row_pair(blockIdx.x, Ny);
   double2* out = rhs_out(rk, ctl, mode, direct_out);
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
+#pragma unroll 1
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
     double2 D[2][2], H[2][2];
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int r = P.r[k];
-        const size_t q = (size_t)r * Nx + cc[s];
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
         D[k][s] = w.dph[q];
         const double2 e = w.z[q];
-        const double sg = (double)fsign(tb.kx[cc[s]] + tb.ky[r]);
+        const double sg = (double)fsign(tb.kx[Q.cc[s]] + tb.ky[Q.r[k]]);
         H[k][s] = make_double2(e.y * sg, -e.x * sg);   // HilbEta^ (2d/breaking.c:252-259)
       }
+    emit_pack(sm, M, 0, Q, Ny, D, H);
+    // S(delphiH^) at all four points
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        const size_t q = (size_t)P.r[k] * Nx + c;
-        const double2 Sd = sym_at(D, P, k, s, c, Nx, Ny, false);
+        const size_t q = Q.at(k, s, Nx);
+        double2 Sd;
+        if (Q.self) Sd = self_sym(D[k][s], Q.flip ? D[k ^ 1][s] : D[k][s], Q.r[k], s, Ny, false);
+        else if (s == 0) Sd = D[k][0];
+        else Sd = cconj(Q.flip ? D[k ^ 1][0] : D[k][0]);
         const double a = tb.aal[q];
-        const double2 S = tb.has_src ? w.src[q] : make_double2(0.0, 0.0);
-        const double2 de = w.D[q];
-        out[q] = make_double2((S.x + Sd.x - de.x) * a, (S.y + Sd.y - de.y) * a);
-        const double2 Ed = sym_at(D, P, k, s, c, Nx, Ny, true), Eh = sym_at(H, P, k, s, c, Nx, Ny, true);
-        put(sm, M, k, c, make_double2(Ed.x - Eh.y, Ed.y + Eh.x));
+        const double2 d = w.D[q];   // damping of eta less the source
+        out[q] = make_double2((Sd.x - d.x) * a, (Sd.y - d.y) * a);
       }
   }
-  fft_slices<M>(sm, 2, tb.twx, +1);
-  for (int k = 0; k < 2; ++k) {
-    double2* dst = b.P + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) dst[j] = slot(sm, M, k, j);
-  }
+  fft_slices<M, NT>(sm, 0, 2, tb.twx, +1);
+  row_store<M, NT>(sm, 0, 1, b.P, P, (size_t)tb.n);
 }
 
 // colI: inverse column FFT -> delphi (real part) and HilbEta (imaginary part) / N
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2b_colI(Tab2 tb, Brk2 b, const Ctl2* __restrict__ ctl, int mode, int cond) {
   if (!rhs_active(ctl, cond) || !brk_update(ctl, mode)) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx;
   const int c = blockIdx.x;
   if (c == 0 && threadIdx.x == 0) b.st->npeaks = 0;
-  col_load<M>(sm, 0, b.P, Nx, c);
-  fft_slices<M>(sm, 2, tb.twy, +1);
+  col_load<M, NT>(sm, 0, 1, b.P, Nx, c, (size_t)tb.n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, +1);
   const double invN = 1.0 / ((double)tb.n);
-  for (int y = threadIdx.x; y < M; y += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const double2 v = slot(sm, M, k, y);
-      b.dh[(size_t)y * Nx + 2 * c + k] = make_double2(v.x * invN, v.y * invN);
-    }
+#pragma unroll 4
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+    const ColPt p(t, c, Nx);
+    const double2 v = slot(sm, M, p.k, p.y);
+    b.dh[p.q] = make_double2(v.x * invN, v.y * invN);
+  }
 }
 
 // peaks: B = 0 and fun_peaks' test on EtaChecked = eta pb.Char at every point
@@ -566,18 +565,18 @@ __global__ void k2b_flux(Tab2 tb, Work2 w, Brk2 b, const Ctl2* __restrict__ ctl,
 // sbcol: fun_gradient (periodic forward / backward differences, clipped), Sb = grad
 // Flux / (eta - bathy), Sb_x + i Sb_y -> forward column FFT
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2b_sbcol(Tab2 tb, Work2 w, Brk2 b, const Ctl2* __restrict__ ctl, int mode, int cond) {
   if (!rhs_active(ctl, cond) || !brk_update(ctl, mode) || b.st->sb_zero) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx, Ny = tb.ny;
   const int c = blockIdx.x;
   const double* f = b.flux;
-  for (int y = threadIdx.x; y < M; y += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int x = 2 * c + k;
-      const size_t q = (size_t)y * Nx + x;
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+      const ColPt p(t, c, Nx);
+      const int x = 2 * c + p.k, y = p.y;
+      const size_t q = p.q;
       const size_t r = (size_t)y * Nx;
       double Fx = (x < Nx - 1) ? rs2(f[q + 1], f[q]) / b.dx : rs2(f[r], f[q]) / b.dx;
       double Fy = (y < Ny - 1) ? rs2(f[q + Nx], f[q]) / b.dy : rs2(f[x], f[q]) / b.dy;
@@ -588,38 +587,36 @@ k2b_sbcol(Tab2 tb, Work2 w, Brk2 b, const Ctl2* __restrict__ ctl, int mode, int 
       if (Bx < 0) Bx = 0;
       if (By < 0) By = 0;
       const double hq = rs2(w.phys[q], b.bathy[q]);
-      put(sm, M, k, y, make_double2(ra2(Fx, Bx) / hq, ra2(Fy, By) / hq));
+      put(sm, M, p.k, p.y, make_double2(ra2(Fx, Bx) / hq, ra2(Fy, By) / hq));
     }
-  fft_slices<M>(sm, 2, tb.twy, -1);
-  col_store<M>(sm, 0, b.P, Nx, c);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, -1);
+  col_store<M, NT>(sm, 0, 1, b.P, Nx, c, (size_t)tb.n);
 }
 
 // sbrow: forward row FFT and split -> Sb_xhat, Sb_yhat (on an update with B > 0),
 // then dt u^ += Sb_xhat aal, dt v^ += Sb_yhat aal whenever Sb is not zero
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2b_sbrow(Tab2 tb, Brk2 b, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int cond, double2* __restrict__ direct_out) {
   if (!rhs_active(ctl, cond) || b.st->sb_zero) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx, Ny = tb.ny;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, Ny);
   const bool upd = brk_update(ctl, mode);
   if (upd) {
-    for (int k = 0; k < 2; ++k) {
-      const double2* src = b.P + (size_t)P.r[k] * Nx;
-      for (int j = threadIdx.x; j < Nx; j += blockDim.x) put(sm, M, k, j, src[j]);
-    }
-    fft_slices<M>(sm, 2, tb.twx, -1);
+    row_load<M, NT>(sm, 0, 1, b.P, P, n);
+    fft_slices<M, NT>(sm, 0, 2, tb.twx, -1);
   }
   double2* out = rhs_out(rk, ctl, mode, direct_out);
   for (int k = 0; k < 2; ++k) {
-    const int r = P.r[k];
+    const int r = P.row(k);
     for (int j = threadIdx.x; j < Nx; j += blockDim.x) {
       const size_t q = (size_t)r * Nx + j;
       double2 A, Bv;
       if (upd) {
-        split2(slot(sm, M, k, j), slot(sm, M, P.mr[k], (Nx - j) % Nx), A, Bv);
+        split2(slot(sm, M, k, j), slot(sm, M, k ^ P.flip, (Nx - j) % Nx), A, Bv);
         b.sb[q] = A;
         b.sb[n + q] = Bv;
       } else {

@@ -1,4 +1,4 @@
-// hw2d_engine.cu -- C ABI of the 2D flat-bottom engine: tables upload, the
+// hw2d_engine.cu -- C ABI of the 2D engine: tables upload, the
 // RHS entry points and the device-resident rkf45 loop.
 //
 // One step attempt is a fixed launch sequence captured once as a CUDA graph:
@@ -18,8 +18,6 @@
 #include "../../include/hawassi_b200.h"
 #include "hw2d.cuh"
 #include "hw2d_brk.cuh"
-#include "hw2d_gen.cuh"
-#include "hw2d_hs3.cuh"
 #include "hw2d_out.cuh"
 #include "hw2d_var.cuh"
 #include "hw2d_wall.cuh"
@@ -35,77 +33,54 @@ namespace {
 std::string g_err2d;
 
 constexpr int kMinM = 64, kMaxM = 1024;
+constexpr int kMaxRef2 = 16;   // reference depths
 constexpr long long kMaxAttemptsPerRun = 2000000;
 
 template <int M>
 size_t smem_bytes(int slices) { return (size_t)slices * hwdev::padded(M) * sizeof(double2); }
 
+template <class Kernel>
+void allow(Kernel* k, size_t bytes) {
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+// the most slices that each pass takes
 template <int M>
 void set_attrs() {
-  cudaFuncSetAttribute(hw2d::k2_rowA<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
-  cudaFuncSetAttribute(hw2d::k2_colB<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(8));
-  cudaFuncSetAttribute(hw2d::k2_rowC<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(8));
-  cudaFuncSetAttribute(hw2d::k2_colD<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(10));
-  cudaFuncSetAttribute(hw2d::k2_rowE<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(8));
-  cudaFuncSetAttribute(hw2d::k2v_rowA<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(8));
-  cudaFuncSetAttribute(hw2d::k2v_colB<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(12));
-  cudaFuncSetAttribute(hw2d::k2v_rowC<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(12));
-  cudaFuncSetAttribute(hw2d::k2v_colD<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
-  cudaFuncSetAttribute(hw2d::k2v_rowE<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
-  cudaFuncSetAttribute(hw2d::k2v_colF<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(8));
-  cudaFuncSetAttribute(hw2d::k2v_rowG<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(8));
-  cudaFuncSetAttribute(hw2d::k2b_rowI<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
-  cudaFuncSetAttribute(hw2d::k2b_colI<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
-  cudaFuncSetAttribute(hw2d::k2b_sbcol<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
-  cudaFuncSetAttribute(hw2d::k2b_sbrow<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
-  cudaFuncSetAttribute(hw2d::k2w_row1<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
-  cudaFuncSetAttribute(hw2d::k2w_col2<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
-  cudaFuncSetAttribute(hw2d::k2w_row3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
-  cudaFuncSetAttribute(hw2d::k2w_rowV1<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
-  cudaFuncSetAttribute(hw2d::k2w_colV2<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
-  cudaFuncSetAttribute(hw2d::k2w_rowV3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
-  cudaFuncSetAttribute(hw2d::k2_colB3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(10));
-  cudaFuncSetAttribute(hw2d::k2_rowC3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(10));
-  cudaFuncSetAttribute(hw2d::k2_colH3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
-  cudaFuncSetAttribute(hw2d::k2_rowI3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(8));
-  cudaFuncSetAttribute(hw2d::k2o_row<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
-  cudaFuncSetAttribute(hw2d::k2o_col<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
-  cudaFuncSetAttribute(hw2d::k2g_rows<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
-  cudaFuncSetAttribute(hw2d::k2g_cols<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
-}
-
-// the general path's transform passes over nf consecutive fields (rows: M = nx,
-// four rows per CTA; columns: M = ny, four columns per CTA)
-template <int M>
-void launch_gen(int cols, double2* f, int nf, int nx, int ny, const double2* tw, int sign, cudaStream_t s,
-                const Ctl2* ctl, int cond) {
-  const int blk = hw2d::kGroups * (M / 8);
-  if (!cols)
-    hw2d::k2g_rows<M><<<dim3(ny / hw2d::kGroups, nf), blk, smem_bytes<M>(4), s>>>(f, nx, ny, tw, sign, ctl, cond);
-  else
-    hw2d::k2g_cols<M><<<dim3(nx / 4, nf), blk, smem_bytes<M>(4), s>>>(f, nx, ny, tw, sign, ctl, cond);
-}
-void gen_pass(int M, int cols, double2* f, int nf, int nx, int ny, const double2* tw, int sign, cudaStream_t s,
-              const Ctl2* ctl, int cond) {
-  switch (M) {
-    case 64: launch_gen<64>(cols, f, nf, nx, ny, tw, sign, s, ctl, cond); break;
-    case 128: launch_gen<128>(cols, f, nf, nx, ny, tw, sign, s, ctl, cond); break;
-    case 256: launch_gen<256>(cols, f, nf, nx, ny, tw, sign, s, ctl, cond); break;
-    case 512: launch_gen<512>(cols, f, nf, nx, ny, tw, sign, s, ctl, cond); break;
-    default: launch_gen<1024>(cols, f, nf, nx, ny, tw, sign, s, ctl, cond); break;
-  }
-}
-
-// the first kernel of a general-path RHS: counts the call when it runs
-__global__ void k2g_count(hw2d::Ctl2* ctl, int cond) {
-  if (hw2d::rhs_active(ctl, cond)) ctl->rhs += 1;
+  allow(hw2d::k2_rowA<M>, smem_bytes<M>(2));
+  allow(hw2d::k2_colB<M>, smem_bytes<M>(10));
+  allow(hw2d::k2_rowC<M>, smem_bytes<M>(10));
+  allow(hw2d::k2_colD<M>, smem_bytes<M>(2));
+  allow(hw2d::k2_rowE<M>, smem_bytes<M>(2));
+  allow(hw2d::k2_colH3<M>, smem_bytes<M>(2));
+  allow(hw2d::k2_rowI3<M>, smem_bytes<M>(6));
+  allow(hw2d::k2_colH1<M>, smem_bytes<M>(4));
+  allow(hw2d::k2_rowH1<M>, smem_bytes<M>(4));
+  allow(hw2d::k2v_row1<M>, smem_bytes<M>(2));
+  allow(hw2d::k2v_col2<M>, smem_bytes<M>(6));
+  allow(hw2d::k2v_row3<M>, smem_bytes<M>(8));
+  allow(hw2d::k2v_col4<M>, smem_bytes<M>(10));
+  allow(hw2d::k2v_row5<M>, smem_bytes<M>(10));
+  allow(hw2d::k2v_col6<M>, smem_bytes<M>(6));
+  allow(hw2d::k2v_row7<M>, smem_bytes<M>(6));
+  allow(hw2d::k2b_rowI<M>, smem_bytes<M>(2));
+  allow(hw2d::k2b_colI<M>, smem_bytes<M>(2));
+  allow(hw2d::k2b_sbcol<M>, smem_bytes<M>(2));
+  allow(hw2d::k2b_sbrow<M>, smem_bytes<M>(2));
+  allow(hw2d::k2w_row1<M>, smem_bytes<M>(2));
+  allow(hw2d::k2w_col2<M>, smem_bytes<M>(2));
+  allow(hw2d::k2w_row3<M>, smem_bytes<M>(2));
+  allow(hw2d::k2w_rowV1<M>, smem_bytes<M>(4));
+  allow(hw2d::k2w_colV2<M>, smem_bytes<M>(4));
+  allow(hw2d::k2w_rowV3<M>, smem_bytes<M>(2));
+  allow(hw2d::k2o_row<M>, smem_bytes<M>(4));
+  allow(hw2d::k2o_col<M>, smem_bytes<M>(4));
 }
 
 // the output stage's two passes (row M = nx, column M = ny)
 template <int M>
 void launch_out(int which, int nblocks, cudaStream_t s, const Tab2& tb, const double2* z, double2* P, double* phys,
                 float* f32) {
-  const int blk = hw2d::kGroups * (M / 8);
+  const int blk = hw2d::thr2(M);
   if (which == 0) hw2d::k2o_row<M><<<nblocks, blk, smem_bytes<M>(4), s>>>(tb, z, P);
   else hw2d::k2o_col<M><<<nblocks, blk, smem_bytes<M>(4), s>>>(tb, P, phys, f32);
 }
@@ -123,7 +98,7 @@ void out_pass(int M, int which, int nb, cudaStream_t s, const Tab2& tb, const do
 // the flat bottom's wall round trip (row M = nx, column M = ny)
 template <int M>
 void launch_wall(int which, int nblocks, cudaStream_t s, const Tab2& tb, const Work2& w, const Ctl2* ctl, int cond) {
-  const int blk = hw2d::kGroups * (M / 8);
+  const int blk = hw2d::thr2(M);
   if (which == 0) hw2d::k2w_row1<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, ctl, cond);
   else if (which == 1) hw2d::k2w_col2<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, ctl, cond);
   else if (which == 2) hw2d::k2w_row3<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, ctl, cond);
@@ -145,14 +120,14 @@ void wall_pass(int M, int which, int nb, cudaStream_t s, const Tab2& tb, const W
 template <int M>
 void launch_brk_row(int which, int nblocks, cudaStream_t s, const Tab2& tb, const Work2& w, const hw2d::Brk2& b,
                     const RK2& rk, const Ctl2* ctl, int mode, int cond, double2* out) {
-  const int blk = hw2d::kGroups * (M / 8);
+  const int blk = hw2d::thr2(M);
   if (which == 0) hw2d::k2b_rowI<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, b, rk, ctl, mode, cond, out);
   else hw2d::k2b_sbrow<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, b, rk, ctl, mode, cond, out);
 }
 template <int M>
 void launch_brk_col(int which, int nblocks, cudaStream_t s, const Tab2& tb, const Work2& w, const hw2d::Brk2& b,
                     const Ctl2* ctl, int mode, int cond) {
-  const int blk = hw2d::kGroups * (M / 8);
+  const int blk = hw2d::thr2(M);
   if (which == 0) hw2d::k2b_colI<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, b, ctl, mode, cond);
   else hw2d::k2b_sbcol<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, b, ctl, mode, cond);
 }
@@ -177,51 +152,72 @@ void brk_col(int M, int which, int nb, cudaStream_t s, const Tab2& tb, const Wor
   }
 }
 
-// the five kernels of one RHS for a row length Mx and a column length My
-template <int M>
-void launch_row(int which, int nblocks, cudaStream_t s, const Tab2& tb, const Work2& w, const RK2& rk,
-                const Ctl2* ctl, Ctl2* ctlw, int mode, int cond, double2* out) {
-  const dim3 blk(hw2d::kGroups * (M / 8));
-  if (which == 0) hw2d::k2_rowA<M><<<nblocks, blk, smem_bytes<M>(6), s>>>(tb, w, rk, ctl, ctlw, mode, cond);
-  else if (which == 2) hw2d::k2_rowC<M><<<nblocks, blk, smem_bytes<M>(8), s>>>(tb, w, ctl, cond);
-  else if (which == 10) hw2d::k2v_rowA<M><<<nblocks, blk, smem_bytes<M>(8), s>>>(tb, w, rk, ctl, ctlw, mode, cond);
-  else if (which == 12) hw2d::k2v_rowC<M><<<nblocks, blk, smem_bytes<M>(12), s>>>(tb, w, ctl, cond);
-  else if (which == 14) hw2d::k2v_rowE<M><<<nblocks, blk, smem_bytes<M>(6), s>>>(tb, w, ctl, cond);
-  else if (which == 16) hw2d::k2v_rowG<M><<<nblocks, blk, smem_bytes<M>(8), s>>>(tb, w, ctl, cond);
-  else if (which == 20) hw2d::k2_rowC3<M><<<nblocks, blk, smem_bytes<M>(10), s>>>(tb, w, ctl, cond);
-  else if (which == 22) hw2d::k2_rowI3<M><<<nblocks, blk, smem_bytes<M>(8), s>>>(tb, w, ctl, cond);
-  else hw2d::k2_rowE<M><<<nblocks, blk, smem_bytes<M>(8), s>>>(tb, w, rk, ctl, mode, cond, out);
-}
-template <int M>
-void launch_col(int which, int nblocks, cudaStream_t s, const Tab2& tb, const Work2& w, const Ctl2* ctl, int cond) {
-  const dim3 blk(hw2d::kGroups * (M / 8));
-  if (which == 1) hw2d::k2_colB<M><<<nblocks, blk, smem_bytes<M>(8), s>>>(tb, w, ctl, cond);
-  else if (which == 11) hw2d::k2v_colB<M><<<nblocks, blk, smem_bytes<M>(12), s>>>(tb, w, ctl, cond);
-  else if (which == 13) hw2d::k2v_colD<M><<<nblocks, blk, smem_bytes<M>(6), s>>>(tb, w, ctl, cond);
-  else if (which == 15) hw2d::k2v_colF<M><<<nblocks, blk, smem_bytes<M>(8), s>>>(tb, w, ctl, cond);
-  else if (which == 21) hw2d::k2_colB3<M><<<nblocks, blk, smem_bytes<M>(10), s>>>(tb, w, ctl, cond);
-  else if (which == 23) hw2d::k2_colH3<M><<<nblocks, blk, smem_bytes<M>(6), s>>>(tb, w, ctl, cond);
-  else hw2d::k2_colD<M><<<nblocks, blk, smem_bytes<M>(10), s>>>(tb, w, ctl, cond);
-}
+// the passes of one RHS: rows (row length M = nx) and columns (M = ny)
+enum RowPass { kRowA, kRowC, kRowE, kRowI3, kRowH1, kRowV1, kRowV3, kRowV5, kRowV7 };
+enum ColPass { kColB, kColD, kColH3, kColH1, kColV2, kColV4, kColV6 };
 
-void row_dispatch(int M, int which, int nb, cudaStream_t s, const Tab2& tb, const Work2& w, const RK2& rk,
-                  const Ctl2* ctl, Ctl2* ctlw, int mode, int cond, double2* out) {
-  switch (M) {
-    case 64: launch_row<64>(which, nb, s, tb, w, rk, ctl, ctlw, mode, cond, out); break;
-    case 128: launch_row<128>(which, nb, s, tb, w, rk, ctl, ctlw, mode, cond, out); break;
-    case 256: launch_row<256>(which, nb, s, tb, w, rk, ctl, ctlw, mode, cond, out); break;
-    case 512: launch_row<512>(which, nb, s, tb, w, rk, ctl, ctlw, mode, cond, out); break;
-    default: launch_row<1024>(which, nb, s, tb, w, rk, ctl, ctlw, mode, cond, out); break;
+struct PassArgs {
+  cudaStream_t s;
+  const Tab2& tb;
+  const Work2& w;
+  const RK2& rk;
+  Ctl2* ctl;
+  int mode, cond;
+  double2* out;
+};
+
+template <int M>
+void launch_row(RowPass which, int cubic, const PassArgs& a) {
+  const Tab2& tb = a.tb;
+  const int nb = tb.ny / 2, nd = tb.chi_one ? 2 : (a.w.dph ? 1 : 0), np = (tb.model == 3 ? 3 : 2) + nd;
+  const int t2 = hw2d::thr2(M), t4 = hw2d::thr4(M);
+  switch (which) {
+    case kRowA:
+      hw2d::k2_rowA<M><<<dim3(nb, tb.model == 3 ? 3 : 2), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.ctl, a.mode, a.cond);
+      break;
+    case kRowC: hw2d::k2_rowC<M><<<nb, t4, smem_bytes<M>(std::max(6, 2 * np)), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kRowE: hw2d::k2_rowE<M><<<dim3(nb, 3), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.rk, a.ctl, a.mode, a.cond, a.out); break;
+    case kRowI3: hw2d::k2_rowI3<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kRowH1: hw2d::k2_rowH1<M><<<nb, t4, smem_bytes<M>(4), a.s>>>(tb, a.w, a.rk, a.ctl, a.mode, a.cond, a.out); break;
+    case kRowV1:
+      hw2d::k2v_row1<M><<<dim3(nb, 2 + tb.nk), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.ctl, a.mode, a.cond);
+      break;
+    case kRowV3: hw2d::k2v_row3<M><<<nb, t4, smem_bytes<M>(tb.model == 3 ? 8 : 6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kRowV5: hw2d::k2v_row5<M><<<nb, t4, smem_bytes<M>(std::max(6, cubic ? 2 : 2 * np)), a.s>>>(tb, a.w, a.ctl, a.cond, cubic); break;
+    case kRowV7: hw2d::k2v_row7<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond, cubic); break;
   }
 }
-void col_dispatch(int M, int which, int nb, cudaStream_t s, const Tab2& tb, const Work2& w, const Ctl2* ctl,
-                  int cond) {
-  switch (M) {
-    case 64: launch_col<64>(which, nb, s, tb, w, ctl, cond); break;
-    case 128: launch_col<128>(which, nb, s, tb, w, ctl, cond); break;
-    case 256: launch_col<256>(which, nb, s, tb, w, ctl, cond); break;
-    case 512: launch_col<512>(which, nb, s, tb, w, ctl, cond); break;
-    default: launch_col<1024>(which, nb, s, tb, w, ctl, cond); break;
+template <int M>
+void launch_col(ColPass which, int cubic, const PassArgs& a) {
+  const Tab2& tb = a.tb;
+  const int nb = tb.nx / 2, nd = tb.chi_one ? 2 : (a.w.dph ? 1 : 0), np = (tb.model == 3 ? 3 : 2) + nd;
+  const int t2 = hw2d::thr2(M), t4 = hw2d::thr4(M);
+  switch (which) {
+    case kColB: hw2d::k2_colB<M><<<nb, t4, smem_bytes<M>(std::max(tb.model == 3 ? 6 : 4, 2 * np)), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kColD: hw2d::k2_colD<M><<<dim3(nb, 3), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kColH3: hw2d::k2_colH3<M><<<nb, t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kColH1: hw2d::k2_colH1<M><<<nb, t4, smem_bytes<M>(4), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kColV2: hw2d::k2v_col2<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kColV4: hw2d::k2v_col4<M><<<nb, t4, smem_bytes<M>(std::max(4, cubic ? 2 : 2 * np)), a.s>>>(tb, a.w, a.ctl, a.cond, cubic); break;
+    case kColV6: hw2d::k2v_col6<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+  }
+}
+void row_pass(RowPass which, const PassArgs& a, int cubic = 0) {
+  switch (a.tb.nx) {
+    case 64: launch_row<64>(which, cubic, a); break;
+    case 128: launch_row<128>(which, cubic, a); break;
+    case 256: launch_row<256>(which, cubic, a); break;
+    case 512: launch_row<512>(which, cubic, a); break;
+    default: launch_row<1024>(which, cubic, a); break;
+  }
+}
+void col_pass(ColPass which, const PassArgs& a, int cubic = 0) {
+  switch (a.tb.ny) {
+    case 64: launch_col<64>(which, cubic, a); break;
+    case 128: launch_col<128>(which, cubic, a); break;
+    case 256: launch_col<256>(which, cubic, a); break;
+    case 512: launch_col<512>(which, cubic, a); break;
+    default: launch_col<1024>(which, cubic, a); break;
   }
 }
 
@@ -306,246 +302,49 @@ struct hw2d_ctx {
     }
     return true;
   }
-  // ---- the general varying-bottom path (hw2d_gen.cuh) ----
-  // pool of complex N-point fields; the numbered slots below
-  enum GenSlot {
-    gEH = 0, gP = 3, gCU = 6, gCV = 7, gD = 8, gH1 = 11, gM = 13, gEM0U = 16, gEU = 17, gEM0V = 18, gEV = 19,
-    gDH2 = 20, gEM0UH = 21, gEM0VH = 22, gLU = 23, gLV = 24, gADJIN = 25, gADJ = 29, gSRC = 33, gHSS = 34,
-    // HS3
-    gLMU = 43, gLMV = 44, gDIVG = 45, gLELP = 46, gDXU = 47, gDYV = 48, gE2U = 49, gE2V = 50, gPK = 51, gPH = 55,
-    gDH3 = 59, gLP = 60, gADJ3IN = 64, gADJ3 = 68, gSlotsHS2 = 43, gSlotsHS3 = 72
-  };
-  int gen = 0;              // 1: the general path serves this bottom / model
-  double2* gpool = nullptr;
-  int gcount = 0;           // kernels of the RHS being issued
-  double2* G(int i) const { return gpool + (size_t)i * n; }
-  void g_fft(double2* f, int nf, int sign, cudaStream_t s, int cond) {
-    gen_pass(nx, 0, f, nf, nx, ny, tb.twx, sign, s, ctl, cond);
-    gen_pass(ny, 1, f, nf, nx, ny, tb.twy, sign, s, ctl, cond);
-    gcount += 2;
-  }
-  void g_sym(double2* f, int nf, cudaStream_t s, int cond) {
-    hw2d::k2g_sym<<<hw2d::kGenBlocks, hw2d::kGenThreads, 0, s>>>(f, nf, nx, ny, ctl, cond);
-    ++gcount;
-  }
-  template <class Op>
-  void g_map(const Op& op, cudaStream_t s, int cond) {
-    hw2d::k2g_map<Op><<<hw2d::kGenBlocks, hw2d::kGenThreads, 0, s>>>(op, n, nx, ctl, cond);
-    ++gcount;
-  }
-  // HSSgen_2depth / HSSgen_3depth (2d/fun_odesolver.c:500-697): res from phi (the
-  // unnormalised physical field, real part used) and its spectrum phihat, with the
-  // spectral tables O of the reference depths (min, [mid,] plus)
-  // With K reference depths (tb.nk > 0) the same sum runs over the K depths' tables
-  // (O = the C^2 or the Omega^2 rows of ck / ok, as omega selects), in the same order.
-  int hss_base = gHSS;      // first pool slot of the operator's 3K scratch fields
-  void g_hss(const double2* phi, const double2* phihat, const double* omin, const double* omid, const double* oplus,
-             double2* res, cudaStream_t s, int cond, bool omega = false) {
-    const int K = tb.nk ? tb.nk : (tb.gmid ? 3 : 2);
-    const double* O[hw2d::kMaxRef2];
-    const double* Gm[hw2d::kMaxRef2];
-    if (tb.nk) {
-      for (int d = 0; d < K; ++d) {
-        O[d] = (omega ? tb.ok : tb.ck) + (size_t)d * n;
-        Gm[d] = tb.gk + (size_t)d * n;
-      }
-    } else {
-      O[0] = omin;
-      O[1] = tb.gmid ? omid : oplus;
-      O[2] = oplus;
-      Gm[0] = tb.gmin;
-      Gm[1] = tb.gmid ? tb.gmid : tb.gplus;
-      Gm[2] = tb.gplus;
-    }
-    const double N = double(nx) * double(ny);
-    double2* L0 = G(hss_base);
-    double2* g = G(hss_base + K);
-    double2* gl = G(hss_base + 2 * K);
-    for (int d = 0; d < K; ++d) g_map(hw2d::OpScaleTable{L0 + d * n, phihat, O[d]}, s, cond);
-    g_sym(L0, K, s, cond);
-    g_fft(L0, K, +1, s, cond);
-    for (int d = 0; d < K; ++d) {
-      g_map(hw2d::OpGam{g + d * n, phi, Gm[d], N}, s, cond);
-      g_map(hw2d::OpGam{gl + d * n, L0 + d * n, Gm[d], N}, s, cond);
-    }
-    g_fft(g, 2 * K, -1, s, cond);
-    hw2d::OpHssSum sum{};
-    sum.res = res;
-    for (int d = 0; d < K; ++d) {
-      sum.g[d] = g + (size_t)d * n;
-      sum.gl[d] = gl + (size_t)d * n;
-      sum.o[d] = O[d];
-    }
-    sum.K = K;
-    g_map(sum, s, cond);
-  }
-  // fun_adjust (2d/fun_odesolver.c:810-884) of nf consecutive fields A into AChi:
-  // S(A) in place, AChi = F(ChiAdj F^-1(S(A)) / N)
-  void g_adjust(double2* A, double2* AChi, int nf, cudaStream_t s, int cond) {
-    const double N = double(nx) * double(ny);
-    g_sym(A, nf, s, cond);
-    for (int f = 0; f < nf; ++f) g_map(hw2d::OpCopy{AChi + f * n, A + f * n}, s, cond);
-    g_fft(AChi, nf, +1, s, cond);
-    for (int f = 0; f < nf; ++f) g_map(hw2d::OpChi{AChi + f * n, tb.chi, N}, s, cond);
-    g_fft(AChi, nf, -1, s, cond);
-  }
-  // one RHS of rhs_AB1/AB2/AB3_2DB_uv from the stage input w.z into out
-  void gen_rhs(int mode, int cond, cudaStream_t s, double2* out) {
-    gcount = 0;
-    k2g_count<<<1, 1, 0, s>>>(ctl, cond);
-    ++gcount;
-    const double N = double(nx) * double(ny), f2 = N * N, f3 = N * N * N, g = hw2d::kGrav;
-    const int model = tb.model;
-    // AB1: symmetrised spectra, physical fields, HSS of u^ and v^ with Csqr
-    for (int f = 0; f < 3; ++f) g_map(hw2d::OpCopy{G(gEH + f), w.z + f * n}, s, cond);
-    g_sym(G(gEH), 3, s, cond);
-    for (int f = 0; f < 3; ++f) g_map(hw2d::OpCopy{G(gP + f), G(gEH + f)}, s, cond);
-    g_fft(G(gP), 3, +1, s, cond);
-    g_hss(G(gP + 1), G(gEH + 1), tb.cmin, tb.cmid, tb.cplus, G(gCU), s, cond);
-    g_hss(G(gP + 2), G(gEH + 2), tb.cmin, tb.cmid, tb.cplus, G(gCV), s, cond);
-    // the damping spectra and the source spectrum go where the breaking kernels read
-    // them when they rewrite dt eta^ (w.D, w.src)
-    g_map(hw2d::OpDampH1{w.D, w.D + n, w.D + 2 * n, G(gH1), G(gH1 + 1), G(gP), G(gP + 1), G(gP + 2), G(gCU),
-                         G(gCV), tb.damp, tb.kx, tb.ky, N, g},
-          s, cond);
-    g_fft(w.D, 3, -1, s, cond);
-    const double2* src = nullptr;
-    if (tb.has_src) {
-      hw2d::k2g_signal<<<(ny + 127) / 128, 128, 0, s>>>(tb, w, ctl, mode, cond);
-      ++gcount;
-      g_map(hw2d::OpSource{w.src, tb.gx, tb.sx, w.insig, w.insigs, tb.fac_src}, s, cond);
-      gen_pass(ny, 1, w.src, 1, nx, ny, tb.twy, -1, s, ctl, cond);   // its row transform is a set-up table
-      ++gcount;
-      src = w.src;
-    }
-    hw2d::OpAssemble as{};
-    as.out = out;
-    as.rk = rk;
-    as.ctl = ctl;
-    as.mode = mode;
-    as.dph = w.dph;
-    as.z = w.z;
-    as.src = src;
-    as.h1u = G(gH1);
-    as.h1v = G(gH1 + 1);
-    as.de = w.D;
-    as.du = w.D + n;
-    as.dv = w.D + 2 * n;
-    as.aal = tb.aal;
-    as.kx = tb.kx;
-    as.ky = tb.ky;
-    as.g = g;
-    as.model = model;
-    as.n = n;
-    if (model >= 2) {
-      // AB2: M0u, M0v, L phi in physical space; the H2 products
-      g_map(hw2d::OpM0{G(gM), G(gM + 1), G(gM + 2), G(gH1), G(gH1 + 1)}, s, cond);
-      g_sym(G(gM), 3, s, cond);
-      g_fft(G(gM), 3, +1, s, cond);
-      g_map(hw2d::OpH2Products{G(gEM0U), G(gEU), G(gEM0V), G(gEV), G(gDH2), G(gEM0UH), G(gEM0VH), w.phys, G(gP),
-                               G(gP + 1), G(gP + 2), G(gM), G(gM + 1), G(gM + 2), tb.wallchar, N, f2, n},
-            s, cond);
-      g_fft(G(gEU), 1, -1, s, cond);
-      g_fft(G(gEV), 4, -1, s, cond);   // eta v, deletaH2, (eta M0u)^, (eta M0v)^
-      g_map(hw2d::OpScaleRe{G(gEM0U), N}, s, cond);
-      g_map(hw2d::OpScaleRe{G(gEM0V), N}, s, cond);
-      g_hss(G(gEM0U), G(gEM0UH), tb.omin, tb.omid, tb.oplus, G(gLU), s, cond, true);
-      g_hss(G(gEM0V), G(gEM0VH), tb.omin, tb.omid, tb.oplus, G(gLV), s, cond, true);
-      // adjust inputs: ikx, iky, delu, delv
-      g_map(hw2d::OpDelH2{G(gADJIN), G(gADJIN + 1), G(gADJIN + 2), G(gADJIN + 3), G(gDH2), G(gEU), G(gEV), G(gLU),
-                          G(gLV), tb.kx, tb.ky, g},
-            s, cond);
-      g_adjust(G(gADJIN), G(gADJ), 4, s, cond);
-      as.ikx = G(gADJ);
-      as.iky = G(gADJ + 1);
-      as.au = G(gADJ + 2);
-      as.av = G(gADJ + 3);
-    }
-    if (model == 3) {
-      // the cubic terms (fun_termshat_AB3_2DB_uv), L applied as HSS(.; Om2dSq) / g
-      g_map(hw2d::OpH3Pre{G(gLMU), G(gLMV), G(gLELP), G(gDIVG), G(gE2U), G(gE2V), G(gDXU), G(gDYV), G(gLU),
-                          G(gLV), w.z, G(gP), G(gM), G(gM + 1), tb.kx, tb.ky, tb.wallchar, g, f3, n},
-            s, cond);
-      g_sym(G(gLMU), 6, s, cond);           // LMu, LMv, divgradphi, LetaLphi, dxu, dyv
-      g_fft(G(gLMU), 6, +1, s, cond);
-      g_fft(G(gE2U), 2, -1, s, cond);
-      hw2d::OpH3Products pr{};
-      for (int k = 0; k < 4; ++k) {
-        pr.p[k] = G(gPK + k);
-        pr.ph[k] = G(gPH + k);
-      }
-      pr.dh3 = G(gDH3);
-      pr.eta = G(gP);
-      pr.lmu = G(gLMU);
-      pr.lmv = G(gLMV);
-      pr.dxu = G(gDXU);
-      pr.dyv = G(gDYV);
-      pr.lphi = G(gM + 2);
-      pr.divg = G(gDIVG);
-      pr.lelp = G(gLELP);
-      pr.wall = tb.wallchar;
-      pr.N = N;
-      pr.f3 = f3;
-      g_map(pr, s, cond);
-      g_fft(G(gPH), 5, -1, s, cond);        // the four products' spectra and deletaH3^
-      for (int k = 0; k < 4; ++k) g_map(hw2d::OpScaleRe{G(gPK + k), N}, s, cond);
-      for (int k = 0; k < 4; ++k)
-        g_hss(G(gPK + k), G(gPH + k), tb.omin, tb.omid, tb.oplus, G(gLP + k), s, cond, true);
-      g_map(hw2d::OpDelH3{G(gADJ3IN), G(gADJ3IN + 1), G(gADJ3IN + 2), G(gADJ3IN + 3), G(gDH3), G(gLP), G(gLP + 1),
-                          G(gLP + 2), G(gLP + 3), G(gE2U), G(gE2V), tb.kx, tb.ky, g},
-            s, cond);
-      g_adjust(G(gADJ3IN), G(gADJ3), 4, s, cond);
-      as.ikx3 = G(gADJ3);
-      as.iky3 = G(gADJ3 + 1);
-      as.au3 = G(gADJ3 + 2);
-      as.av3 = G(gADJ3 + 3);
-    }
-    g_map(as, s, cond);
-    per_rhs = gcount;
-  }
-
   void rhs_launch(int mode, int cond, cudaStream_t s, double2* out) {
     const int rows = ny / 2, cols = nx / 2;
     if (mode != 0) hw2d::k2_stage<<<hw2d::kCombBlocks, 256, 0, s>>>(rk, w, ctl, mode, cond, 3 * n);
-    if (gen) {
-      gen_rhs(mode, cond, s, out);
-      per_rhs += 1;
-      if (brk.on) brk_launch(mode, cond, s, out);
+    per_rhs = 1;
+    const PassArgs a{s, tb, w, rk, ctl, mode, cond, out};
+    auto row = [&](RowPass p, int cubic = 0) { row_pass(p, a, cubic); ++per_rhs; };
+    auto col = [&](ColPass p, int cubic = 0) { col_pass(p, a, cubic); ++per_rhs; };
+    if (tb.var) {
+      row(kRowV1);
+      col(kColV2);
+      row(kRowV3);
+    } else {
+      if (tb.wallchar) {
+        const int base = tb.refl_one ? 3 : 0;
+        wall_pass(nx, base + 0, rows, s, tb, w, ctl, cond);
+        wall_pass(ny, base + 1, cols, s, tb, w, ctl, cond);
+        wall_pass(nx, base + 2, rows, s, tb, w, ctl, cond);
+        per_rhs += 3;
+      }
+      row(kRowA);
+    }
+    if (tb.model == 1) {
+      col(kColH1);
+      row(kRowH1);
       return;
     }
     if (tb.var) {
-      row_dispatch(nx, 10, rows, s, tb, w, rk, ctl, ctl, mode, cond, nullptr);
-      col_dispatch(ny, 11, cols, s, tb, w, ctl, cond);
-      row_dispatch(nx, 12, rows, s, tb, w, rk, ctl, ctl, mode, cond, nullptr);
-      col_dispatch(ny, 13, cols, s, tb, w, ctl, cond);
-      row_dispatch(nx, 14, rows, s, tb, w, rk, ctl, ctl, mode, cond, nullptr);
-      col_dispatch(ny, 15, cols, s, tb, w, ctl, cond);
-      row_dispatch(nx, 16, rows, s, tb, w, rk, ctl, ctl, mode, cond, nullptr);
-      if (!tb.chi_one || tb.has_src) col_dispatch(ny, 3, cols, s, tb, w, ctl, cond);
-      row_dispatch(nx, 4, rows, s, tb, w, rk, ctl, ctl, mode, cond, out);
-      per_rhs = ((!tb.chi_one || tb.has_src) ? 9 : 8) + 1;
-      if (brk.on) brk_launch(mode, cond, s, out);
-      return;
-    }
-    if (tb.wallchar) {
-      const int base = tb.refl_one ? 3 : 0;
-      wall_pass(nx, base + 0, rows, s, tb, w, ctl, cond);
-      wall_pass(ny, base + 1, cols, s, tb, w, ctl, cond);
-      wall_pass(nx, base + 2, rows, s, tb, w, ctl, cond);
-    }
-    row_dispatch(nx, 0, rows, s, tb, w, rk, ctl, ctl, mode, cond, nullptr);
-    if (tb.model == 3) {   // HS3: B3, C3, H3, I3 in place of B, C
-      col_dispatch(ny, 21, cols, s, tb, w, ctl, cond);
-      row_dispatch(nx, 20, rows, s, tb, w, rk, ctl, ctl, mode, cond, nullptr);
-      col_dispatch(ny, 23, cols, s, tb, w, ctl, cond);
-      row_dispatch(nx, 22, rows, s, tb, w, rk, ctl, ctl, mode, cond, nullptr);
+      for (int cubic = 0; cubic <= (tb.model == 3 ? 1 : 0); ++cubic) {
+        col(kColV4, cubic);
+        row(kRowV5, cubic);
+        col(kColV6, cubic);
+        row(kRowV7, cubic);
+      }
     } else {
-      col_dispatch(ny, 1, cols, s, tb, w, ctl, cond);
-      row_dispatch(nx, 2, rows, s, tb, w, rk, ctl, ctl, mode, cond, nullptr);
+      col(kColB);
+      row(kRowC);
+      if (tb.model == 3) {
+        col(kColH3);
+        row(kRowI3);
+      }
     }
-    if (!tb.chi_one || tb.has_src) col_dispatch(ny, 3, cols, s, tb, w, ctl, cond);
-    row_dispatch(nx, 4, rows, s, tb, w, rk, ctl, ctl, mode, cond, out);
-    per_rhs = ((!tb.chi_one || tb.has_src) ? 5 : 4) + 1 + (tb.wallchar ? 3 : 0) + (tb.model == 3 ? 2 : 0);
+    if (!tb.chi_one) col(kColD);
+    row(kRowE);
     if (brk.on) brk_launch(mode, cond, s, out);
   }
   // the breaking kernels after the assembly pass (both bottoms)
@@ -705,7 +504,7 @@ hw2d_ctx* hw2d_create(const hw2d_tables* t, const hw_opts* o) {
     return nullptr;
   }
   const bool kref = t->nrefk != 0;
-  if (kref && (t->nrefk < 2 || t->nrefk > hw2d::kMaxRef2 || !t->gam_k || !t->csq_k || !t->om2_k)) {
+  if (kref && (t->nrefk < 2 || t->nrefk > kMaxRef2 || !t->gam_k || !t->csq_k || !t->om2_k)) {
     g_err2d = "hw2d_create: K reference depths need 2 <= nrefk <= 16 and gam_k, csq_k, om2_k";
     return nullptr;
   }
@@ -759,26 +558,18 @@ hw2d_ctx* hw2d_create(const hw2d_tables* t, const hw_opts* o) {
   tb.twx = c->upload(twiddles(nx));
   tb.twy = c->upload(twiddles(ny));
   if (has_src) {
-    // row transforms of the area kernels (the source's row pass is done once here)
     const double sk = t->propagation == 0 ? -1.0 : (t->propagation == 1 ? 1.0 : 0.0);
-    std::vector<double2> gx(n), sx(n);
-    std::vector<double> re(nx), im(nx);
-    for (int i = 0; i < ny; ++i) {
-      for (int j = 0; j < nx; ++j) { re[j] = t->newgam[(size_t)i * nx + j]; im[j] = 0.0; }
-      hw::host_dft(re, im, -1);
-      for (int j = 0; j < nx; ++j) gx[(size_t)i * nx + j] = make_double2(re[j], im[j]);
-      for (int j = 0; j < nx; ++j) {
-        re[j] = t->skewgam ? sk * t->skewgam[(size_t)i * nx + j] : 0.0;
-        im[j] = 0.0;
-      }
-      hw::host_dft(re, im, -1);
-      for (int j = 0; j < nx; ++j) sx[(size_t)i * nx + j] = make_double2(re[j], im[j]);
-    }
-    tb.gx = c->upload(gx);
-    tb.sx = c->upload(sx);
+    std::vector<double> ss(n, 0.0);
+    if (t->skewgam)
+      for (size_t q = 0; q < n; ++q) ss[q] = sk * t->skewgam[q];
+    tb.gsrc = c->upload(std::vector<double>(t->newgam, t->newgam + n));
+    tb.ssrc = c->upload(ss);
     const int nt = t->nt;
     tb.nt = nt;
     std::vector<double> ts(t->tsig, t->tsig + nt);
+    tb.t0 = ts[0];
+    tb.tl = ts[size_t(nt - 1)];
+    tb.dts = ts[1] - ts[0];
     std::vector<double> sig((size_t)ny * nt), sigc((size_t)ny * nt), sigs((size_t)ny * nt, 0.0),
         sigsc((size_t)ny * nt, 0.0);
     for (int i = 0; i < ny; ++i) {
@@ -805,28 +596,20 @@ hw2d_ctx* hw2d_create(const hw2d_tables* t, const hw_opts* o) {
   if (o && o->h0 > 0) c->h_first = o->h0;
   const bool var = kref || (t->gam_min && t->gam_plus && t->csq_min && t->csq_plus && t->om2_min && t->om2_plus);
   tb.var = var ? 1 : 0;
-  if (kref) {   // K reference depths: the general path with the K-depth sum
-    const size_t kn = (size_t)t->nrefk * n;
-    tb.nk = t->nrefk;
-    tb.gk = c->upload(std::vector<double>(t->gam_k, t->gam_k + kn));
-    tb.ck = c->upload(std::vector<double>(t->csq_k, t->csq_k + kn));
-    tb.ok = c->upload(std::vector<double>(t->om2_k, t->om2_k + kn));
-    c->gen = 1;
-  } else if (var) {
-    tb.gmin = c->upload(std::vector<double>(t->gam_min, t->gam_min + n));
-    tb.gplus = c->upload(std::vector<double>(t->gam_plus, t->gam_plus + n));
-    tb.cmin = c->upload(std::vector<double>(t->csq_min, t->csq_min + n));
-    tb.cplus = c->upload(std::vector<double>(t->csq_plus, t->csq_plus + n));
-    tb.omin = c->upload(std::vector<double>(t->om2_min, t->om2_min + n));
-    tb.oplus = c->upload(std::vector<double>(t->om2_plus, t->om2_plus + n));
-    if (t->gam_mid) {   // three reference depths: the general path
-      tb.gmid = c->upload(std::vector<double>(t->gam_mid, t->gam_mid + n));
-      tb.cmid = c->upload(std::vector<double>(t->csq_mid, t->csq_mid + n));
-      tb.omid = c->upload(std::vector<double>(t->om2_mid, t->om2_mid + n));
-    }
-    // the fused passes serve two reference depths under HS1 / HS2; three depths and
-    // HS3 on this bottom take the general path
-    c->gen = (t->gam_mid || t->model == 3) ? 1 : 0;
+  if (var) {
+    // rows of the reference depths: K given ones, or min, (mid,) plus in HSSgen's order
+    auto rows = [&](const double* all, const double* lo, const double* mid, const double* hi) {
+      std::vector<double> v;
+      if (kref) v.assign(all, all + (size_t)t->nrefk * n);
+      else
+        for (const double* r : {lo, mid, hi})
+          if (r) v.insert(v.end(), r, r + n);
+      return v;
+    };
+    tb.nk = kref ? t->nrefk : (t->gam_mid ? 3 : 2);
+    tb.gk = c->upload(rows(t->gam_k, t->gam_min, t->gam_mid, t->gam_plus));
+    tb.ck = c->upload(rows(t->csq_k, t->csq_min, t->csq_mid, t->csq_plus));
+    tb.ok = c->upload(rows(t->om2_k, t->om2_min, t->om2_mid, t->om2_plus));
   }
   if (t->wallchar) {
     tb.wallchar = c->upload(std::vector<double>(t->wallchar, t->wallchar + n));
@@ -913,36 +696,18 @@ hw2d_ctx* hw2d_create(const hw2d_tables* t, const hw_opts* o) {
 
   Work2& w = c->w;
   w.dph = bk.on ? c->dalloc<double2>(n) : nullptr;
+  const int K = tb.nk, nd = chi_one ? 2 : (bk.on ? 1 : 0);
   w.z = c->dalloc<double2>(3 * n);
-  w.R = c->dalloc<double2>(4 * n);
-  w.Q = c->dalloc<double2>((var ? 6 : (t->model == 3 ? 5 : 4)) * n);
-  if (t->model == 3) {
-    w.p3 = c->dalloc<double>(2 * n);
-    w.T3 = c->dalloc<double2>(6 * n);
-  }
-  if (!var && bk.on) w.phys = c->dalloc<double>(3 * n);   // eta, u, v for the breaking kernels
-  if (!var && t->wallchar) {   // the flat bottom's wall round trip
-    w.WP = c->dalloc<double2>((tb.refl_one ? 2 : 1) * n);
-    w.H1 = c->dalloc<double2>(n);
-  }
-  if (var) {
-    w.phys = c->dalloc<double>(3 * n);
-    w.pe = c->dalloc<double>(2 * n);
-    w.H1 = c->dalloc<double2>(2 * n);
-    w.EU = c->dalloc<double2>(3 * n);
-  }
-  if (c->gen) {
-    int slots = t->model == 3 ? hw2d_ctx::gSlotsHS3 : hw2d_ctx::gSlotsHS2;
-    if (kref && t->nrefk > 3) {   // the operator's 3K scratch fields after the model's own
-      c->hss_base = slots;
-      slots += 3 * t->nrefk;
-    }
-    c->gpool = c->dalloc<double2>((size_t)slots * n);
-  }
+  w.R = c->dalloc<double2>((size_t)(var ? 2 + K : 3) * n);
+  w.Q = c->dalloc<double2>((size_t)std::max(1 + K, 3 + nd + (K + 1) / 2) * n);
+  w.T = c->dalloc<double2>(3 * n);
   w.D = c->dalloc<double2>(3 * n);
-  w.W = chi_one ? nullptr : c->dalloc<double2>(4 * n);
-  w.V = c->dalloc<double2>(4 * n);
-  w.src = has_src ? c->dalloc<double2>(n) : nullptr;
+  w.W = chi_one ? nullptr : c->dalloc<double2>(3 * n);
+  w.V = c->dalloc<double2>(3 * n);
+  w.phys = c->dalloc<double>(3 * n);
+  w.op = c->dalloc<double>(2 * n);
+  if (var || t->wallchar) w.H1 = c->dalloc<double2>(n);
+  if (!var && t->wallchar) w.WP = c->dalloc<double2>((tb.refl_one ? 2 : 1) * n);   // the wall's round trip
   w.insig = c->dalloc<double>(ny);
   w.insigs = c->dalloc<double>(ny);
   w.part = c->dalloc<double>(hw2d::kCombBlocks);
@@ -954,14 +719,11 @@ hw2d_ctx* hw2d_create(const hw2d_tables* t, const hw_opts* o) {
   c->dout = c->dalloc<double2>(3 * n);
   c->ctl = c->dalloc<Ctl2>(1);
   bool ok = tb.kx && tb.ky && tb.c2g && tb.l2d && tb.aal && tb.damp && tb.chi && tb.twx && tb.twy && w.z && w.R &&
-            w.Q && w.D && w.V && w.insig && w.insigs && w.part && c->dref && c->dout && c->ctl &&
-            (chi_one || w.W) && (!has_src || (tb.gx && tb.sx && tb.sig && w.src)) && (!bk.on || (w.dph && w.phys)) &&
-            (var || !t->wallchar || (w.WP && w.H1 && tb.c2d && (!tb.refl_one || (tb.gwx && tb.gwy)))) &&
-            (!var || ((kref ? (tb.gk && tb.ck && tb.ok) : (tb.gmin && tb.gplus && tb.cmin && tb.cplus && tb.omin &&
-                                                             tb.oplus)) &&
-                      w.phys && w.pe && w.H1 && w.EU)) &&
-            (!t->wallchar || tb.wallchar) && (t->model != 3 || (w.p3 && w.T3)) &&
-            (!c->gen || (c->gpool && (!t->gam_mid || (tb.gmid && tb.cmid && tb.omid))));
+            w.Q && w.T && w.D && w.V && w.phys && w.op && w.insig && w.insigs && w.part && c->dref && c->dout && c->ctl &&
+            (chi_one || w.W) && (!has_src || (tb.gsrc && tb.ssrc && tb.sig && tb.sigc && tb.sigs && tb.sigsc)) &&
+            (!bk.on || w.dph) && (!var || (tb.gk && tb.ck && tb.ok && w.H1)) &&
+            (!t->wallchar || (tb.wallchar && w.H1 &&
+                              (var || (w.WP && tb.c2d && (!tb.refl_one || (tb.gwx && tb.gwy))))));
   for (int i = 0; i < 2; ++i) ok = ok && rk.y[i] && rk.kk[i];
   for (int i = 0; i < 5; ++i) ok = ok && rk.ks[i];
   if (!ok || cudaMallocHost(&c->hctl, sizeof(Ctl2)) != cudaSuccess) {

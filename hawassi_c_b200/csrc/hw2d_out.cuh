@@ -17,61 +17,52 @@
 namespace hw2d {
 
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2o_row(Tab2 tb, const double2* __restrict__ z, double2* __restrict__ P) {
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx, Ny = tb.ny;
   const size_t n = (size_t)tb.n;
   const Pair pr = row_pair(blockIdx.x, Ny);
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
-    double2 A[2][2], B[2][2], C[2][2];
+#pragma unroll 2
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(pr, j, Nx);
+    double2 A[2][2], B[2][2], C[2][2], Z[2][2];
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const size_t q = (size_t)pr.r[k] * Nx + cc[s];
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
         A[k][s] = z[q];
         B[k][s] = z[n + q];
         C[k][s] = z[2 * n + q];
+        Z[k][s] = zero2();
       }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        const double2 ea = sym_at(A, pr, k, s, c, Nx, Ny, true), eb = sym_at(B, pr, k, s, c, Nx, Ny, true);
-        put(sm, M, k, c, make_double2(ea.x - eb.y, ea.y + eb.x));
-        put(sm, M, 2 + k, c, sym_at(C, pr, k, s, c, Nx, Ny, true));
-      }
+    emit_pack(sm, M, 0, Q, Ny, A, B);
+    emit_pack(sm, M, 2, Q, Ny, C, Z);
   }
-  fft_slices<M>(sm, 4, tb.twx, +1);
-  for (int f = 0; f < 2; ++f)
-    for (int k = 0; k < 2; ++k) {
-      double2* dst = P + f * n + (size_t)pr.r[k] * Nx;
-      for (int j = threadIdx.x; j < Nx; j += blockDim.x) dst[j] = slot(sm, M, 2 * f + k, j);
-    }
+  fft_slices<M, NT>(sm, 0, 4, tb.twx, +1);
+  row_store<M, NT>(sm, 0, 2, P, pr, n);
 }
 
 // phys: eta, u, v (3 n doubles); f32: the same as floats (nullptr: not kept)
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2o_col(Tab2 tb, const double2* __restrict__ P, double* __restrict__ phys, float* __restrict__ f32) {
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx;
   const size_t n = (size_t)tb.n;
   const int c = blockIdx.x;
-  col_load<M>(sm, 0, P, Nx, c);
-  col_load<M>(sm, 2, P + n, Nx, c);
-  fft_slices<M>(sm, 4, tb.twy, +1);
+  col_load<M, NT>(sm, 0, 2, P, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 4, tb.twy, +1);
   const double invN = 1.0 / ((double)tb.n);
-  for (int y = threadIdx.x; y < M; y += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const size_t q = (size_t)y * Nx + 2 * c + k;
-      const double2 a = slot(sm, M, k, y), b = slot(sm, M, 2 + k, y);
+#pragma unroll 2
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+      const ColPt p(t, c, Nx);
+      const size_t q = p.q;
+      const double2 a = slot(sm, M, p.k, p.y), b = slot(sm, M, 2 + p.k, p.y);
       const double eta = a.x * invN, u = a.y * invN, v = b.x * invN;
       phys[q] = eta;
       phys[n + q] = u;

@@ -1,536 +1,424 @@
-// hw2d_var.cuh -- HAWASSI 2D RHS on a varying bottom with two reference depths
-// (rhs_AB2_2DB_uv, 2d/fun_odesolver.c:4542-4626; fun_termshat_AB1_2DB_uv :2874,
-// fun_termshat_AB2_2DB_uv :3327; HSSgen_2depth :500).  The two-depth operator
-//   HSS(phi; O) = [F(gam_min Re F^-1 S(O_min phi^)) + O_min F(gam_min phi)
-//                 + F(gam_plus Re F^-1 S(O_plus phi^)) + O_plus F(gam_plus phi)] / 2
-// needs a round trip through physical space per application, so one RHS is nine
-// fused passes (the last two, adjust + source and assembly, are the flat path's
-// k2_colD and k2_rowE):
-//   A row:  stage input -> E(eta^)+iE(u^), E(v^)+iE(Cm S u^), E(Cp S u^)+iE(Cm S v^), E(Cp S v^) -> inverse rows
-//   B col:  inverse cols -> eta, u, v (kept), Cm/Cp applied u, v -> damping and gam products -> forward cols
-//   C row:  forward rows -> split -> damping spectra, Csqr u^, Csqr v^ -> delu H1^, delv H1^ (kept)
-//           -> E(M0u^)+iE(M0v^), E(L phi^) -> inverse rows
-//   D col:  inverse cols -> M0u, M0v, L phi -> eta M0u, eta u, eta M0v, eta v, deletaH2 -> forward cols
-//   E row:  forward rows -> split -> (eta u)^, (eta v)^, deletaH2^ (kept), E(Om (eta M0u)^)... -> inverse rows
-//   F col:  inverse cols -> gam products of eta M0u, eta M0v and their Om images -> forward cols
-//   G row:  forward rows -> split -> L(eta M0u)^, L(eta M0v)^ -> H2 terms -> S -> inverse rows (adjust)
+// hw2d_var.cuh -- HAWASSI 2D right-hand sides on a varying bottom with K reference
+// depths (rhs_AB1/AB2/AB3_2DB_uv, 2d/fun_odesolver.c:4350-4402, 4542-4626, 4735-4844;
+// fun_termshat_AB1/AB2/AB3_2DB_uv :2874-2960, 3327-3510, 4104-4296; HSSgen_2depth /
+// HSSgen_3depth :500-697; K = 2 and 3 in the reference, up to 16 for the plain
+// K-reference operator and the learned blend).  The operator of a real field a,
+//   HSS(a; O) = 1/2 [ F( sum_j gam_j Re F^-1 S(O_j a^) ) + sum_j O_j F(gam_j a) ],
+// takes K real inverse transforms, K real forward ones and one more: the weighted images
+// are summed in physical space and go back once.  It is linear, so
+//   C^2 u, C^2 v are needed only as kx C^2 u^ + ky C^2 v^ (delphiH1^, and L phi = its
+//     image), the second-order operator term only as L (eta L phi)^ of one real field,
+//     the third-order ones as L p^ of one (hw2d.cuh, cubic_products).
+// Passes:
+//   V1 row   (eta, u), (v, -), (C_j u, C_j v) for every j               -> inverse rows
+//   V2 col   inverse -> eta, u, v; sum gam_j (C_j u, C_j v), (gam_j u, gam_j v) -> forward
+//   V3 row   forward -> delphiH1^ (kept), L phi (HS3: M0u, M0v)         -> inverse rows
+//   V4 col   inverse -> the products and gam_j (eta L phi), two to a field -> forward
+//   V5 row   forward -> the terms kept, Omega_j (eta L phi)^            -> inverse rows
+//   V6 col   inverse -> sum gam_j Omega_j (.)                           -> forward
+//   V7 row   forward -> the adjustment's input                          -> inverse rows
+// and D, E as on a flat bottom.  HS3: V7 sends (L (eta L phi), div(grad phi)) instead, and
+// V4, V5, V6, V7 run once more on the cubic products.  HS1 ends after V3.
+// Fields beyond the first few go through the column and row passes two or four slices
+// at a time, so a CTA's shared memory does not grow with K and two CTAs share an SM.
 #pragma once
 
 #include "hw2d.cuh"
 
 namespace hw2d {
 
-// E or S of (table o) * S(a) at every point of a quad
-__device__ __forceinline__ void op_sym(const double2 a[2][2], const Pair& P, const int cc[2], int r0, int r1, int Nx,
-                                       int Ny, const double* __restrict__ o, double2 out[2][2]) {
-  double2 sa[2][2];
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-#pragma unroll
-    for (int s = 0; s < 2; ++s) sa[k][s] = sym_at(a, P, k, s, cc[s], Nx, Ny, false);
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const double t = o[(size_t)(k ? r1 : r0) * Nx + cc[s]];
-      out[k][s] = make_double2(t * sa[k][s].x, t * sa[k][s].y);
-    }
-}
-
-__device__ __forceinline__ double2 packc(double2 X, double2 Y) { return make_double2(X.x - Y.y, X.y + Y.x); }
-
-// load a quad (columns j, cm of both rows) of slices s0 (row 0), s0 + 1 (row 1)
+// V1: one CTA per row pair and field (blockIdx.y): 0 (eta, u), 1 (v, -), 2 + j
 template <int M>
-__device__ __forceinline__ void quad_load(double2* sm, int s0, const int cc[2], double2 z[2][2]) {
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-#pragma unroll
-    for (int s = 0; s < 2; ++s) z[k][s] = slot(sm, M, s0 + k, cc[s]);
-}
-
-// ---------------------------------------------------------------------------
-template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
-k2v_rowA(Tab2 tb, Work2 w, RK2 rk, const Ctl2* __restrict__ ctl, Ctl2* ctlw, int mode, int cond) {
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+k2v_row1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, Ctl2* ctlw, int mode, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  const int Nx = tb.nx, Ny = tb.ny;
+  constexpr int NT = thr2(M);
+  const int Nx = M, f = blockIdx.y;
   const size_t n = (size_t)tb.n;
-  const Pair P = row_pair(blockIdx.x, Ny);
-  const int r0 = P.r[0], r1 = P.r[1];
-  const double ts = stage_time(ctl, mode);
-  if (blockIdx.x == 0 && threadIdx.x == 0 && ctlw) ctlw->rhs += 1;
-  if (tb.has_src && threadIdx.x < 2) {
-    const int r = P.r[threadIdx.x];
-    const size_t o = (size_t)r * tb.nt;
-    w.insig[r] = spline2(tb.tsig, tb.sig + o, tb.sigc + o, tb.nt, ts);
-    w.insigs[r] = spline2(tb.tsig, tb.sigs + o, tb.sigsc + o, tb.nt, ts);
-  }
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
-    // one pair of output slices at a time keeps the quad's live values few
-    double2 a[2][2], b[2][2];
+  const Pair P = row_pair(blockIdx.x, tb.ny);
+  stage_extras(tb, w, P, ctl, ctlw, mode, NT);
+  const double* __restrict__ O = tb.ck + (f > 1 ? f - 2 : 0) * n;
+#pragma unroll 2
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
+    double2 x[2][2], y[2][2];
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const size_t q = (size_t)P.r[k] * Nx + cc[s];
-        a[k][s] = w.z[q];
-        b[k][s] = w.z[n + q];
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        put(sm, M, 0 + k, c, packc(sym_at(a, P, k, s, c, Nx, Ny, true), sym_at(b, P, k, s, c, Nx, Ny, true)));
-      }
-    double2 t[2][2];
-    op_sym(b, P, cc, r0, r1, Nx, Ny, tb.cmin, t);        // Cm S(u^)
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) a[k][s] = w.z[2 * n + (size_t)P.r[k] * Nx + cc[s]];   // v^
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        put(sm, M, 2 + k, c, packc(sym_at(a, P, k, s, c, Nx, Ny, true), sym_at(t, P, k, s, c, Nx, Ny, true)));
-      }
-    op_sym(b, P, cc, r0, r1, Nx, Ny, tb.cplus, t);       // Cp S(u^)
-    op_sym(a, P, cc, r0, r1, Nx, Ny, tb.cmin, b);        // Cm S(v^)
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        put(sm, M, 4 + k, c, packc(sym_at(t, P, k, s, c, Nx, Ny, true), sym_at(b, P, k, s, c, Nx, Ny, true)));
-      }
-    op_sym(a, P, cc, r0, r1, Nx, Ny, tb.cplus, t);       // Cp S(v^)
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        put(sm, M, 6 + k, c, packc(sym_at(t, P, k, s, c, Nx, Ny, true), make_double2(0.0, 0.0)));
-      }
-  }
-  fft_slices<M>(sm, 8, tb.twx, +1);
-  for (int s = 0; s < 8; ++s) {
-    const int f = s >> 1, k = s & 1;
-    double2* dst = w.R + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) dst[j] = slot(sm, M, s, j);
-  }
-}
-
-// ---------------------------------------------------------------------------
-template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
-k2v_colB(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
-  if (!rhs_active(ctl, cond)) return;
-  extern __shared__ double2 sm[];
-  const int Nx = tb.nx;
-  const size_t n = (size_t)tb.n;
-  const int c = blockIdx.x;
-  for (int f = 0; f < 4; ++f) col_load<M>(sm, 2 * f, w.R + f * n, Nx, c);
-  fft_slices<M>(sm, 8, tb.twy, +1);
-  const double invN = 1.0 / ((double)tb.n);
-  for (int y = threadIdx.x; y < M; y += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const size_t q = (size_t)y * Nx + 2 * c + k;
-      const double2 P1 = slot(sm, M, 0 + k, y), P2 = slot(sm, M, 2 + k, y);
-      const double2 P3 = slot(sm, M, 4 + k, y), P4 = slot(sm, M, 6 + k, y);
-      const double eta = P1.x * invN, u = P1.y * invN, v = P2.x * invN;
-      const double lmu = P2.y * invN, lpu = P3.x * invN, lmv = P3.y * invN, lpv = P4.x * invN;
-      w.phys[q] = eta;
-      w.phys[n + q] = u;
-      w.phys[2 * n + q] = v;
-      const double dmp = tb.damp[q], gm = tb.gmin[q], gp = tb.gplus[q];
-      put(sm, M, 0 + k, y, make_double2(dmp * eta, dmp * u));
-      put(sm, M, 2 + k, y, make_double2(dmp * v, gm * u));
-      put(sm, M, 4 + k, y, make_double2(gp * u, gm * lmu));
-      put(sm, M, 6 + k, y, make_double2(gp * lpu, gm * v));
-      put(sm, M, 8 + k, y, make_double2(gp * v, gm * lmv));
-      put(sm, M, 10 + k, y, make_double2(gp * lpv, 0.0));
-    }
-  }
-  fft_slices<M>(sm, 12, tb.twy, -1);
-  for (int f = 0; f < 6; ++f) col_store<M>(sm, 2 * f, w.Q + f * n, Nx, c);
-}
-
-// ---------------------------------------------------------------------------
-template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
-k2v_rowC(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
-  if (!rhs_active(ctl, cond)) return;
-  extern __shared__ double2 sm[];
-  const int Nx = tb.nx, Ny = tb.ny;
-  const size_t n = (size_t)tb.n;
-  const Pair P = row_pair(blockIdx.x, Ny);
-  for (int s = 0; s < 12; ++s) {
-    const int f = s >> 1, k = s & 1;
-    const double2* src = w.Q + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) put(sm, M, s, j, src[j]);
-  }
-  fft_slices<M>(sm, 12, tb.twx, -1);
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
-    double2 z[2][2], au[2][2], tu[2][2], av[2][2], tv[2][2];
-    auto q_of = [&](int k, int s) { return (size_t)P.r[k] * Nx + cc[s]; };
-    // Q1: damping of eta, u
-    quad_load<M>(sm, 0, cc, z);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        w.D[q_of(k, s)] = a;
-        w.D[n + q_of(k, s)] = b;
-      }
-    // Q2: damping of v, F(gm u)
-    quad_load<M>(sm, 2, cc, z);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        if (s == 0 || cm != j) w.D[2 * n + q_of(k, s)] = a;
-        const double cmn = tb.cmin[q_of(k, s)];
-        tu[k][s] = make_double2(cmn * b.x, cmn * b.y);   // Cm F(gm u)
-      }
-    // Q3: F(gp u), F(gm Lm u)
-    quad_load<M>(sm, 4, cc, z);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        au[k][s] = make_double2(b.x + tu[k][s].x, b.y + tu[k][s].y);   // F(gm Lm u) + Cm F(gm u)
-        const double cpl = tb.cplus[q_of(k, s)];
-        tu[k][s] = make_double2(cpl * a.x, cpl * a.y);                   // Cp F(gp u)
-      }
-    // Q4: F(gp Lp u), F(gm v)
-    quad_load<M>(sm, 6, cc, z);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        au[k][s] = make_double2((au[k][s].x + a.x + tu[k][s].x) / 2, (au[k][s].y + a.y + tu[k][s].y) / 2);
-        const double cmn = tb.cmin[q_of(k, s)];
-        tv[k][s] = make_double2(cmn * b.x, cmn * b.y);
-      }
-    // Q5: F(gp v), F(gm Lm v)
-    quad_load<M>(sm, 8, cc, z);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        av[k][s] = make_double2(b.x + tv[k][s].x, b.y + tv[k][s].y);
-        const double cpl = tb.cplus[q_of(k, s)];
-        tv[k][s] = make_double2(cpl * a.x, cpl * a.y);
-      }
-    // Q6: F(gp Lp v)
-    quad_load<M>(sm, 10, cc, z);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        av[k][s] = make_double2((av[k][s].x + a.x + tv[k][s].x) / 2, (av[k][s].y + a.y + tv[k][s].y) / 2);
-      }
-    // delu H1^ = -i kx Csqr u^ / g, delv H1^ = -i ky Csqr v^ / g (2d/fun_odesolver.c:2943-2946)
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const double kxv = tb.kx[cc[s]], kyv = tb.ky[P.r[k]];
-        const double2 cu = au[k][s], cv = av[k][s];
-        au[k][s] = make_double2(cu.y / kGrav * kxv, -cu.x / kGrav * kxv);
-        av[k][s] = make_double2(cv.y / kGrav * kyv, -cv.x / kGrav * kyv);
-        tu[k][s] = make_double2(au[k][s].x + av[k][s].x, au[k][s].y + av[k][s].y);   // L phi^
-        if (s == 0 || cm != j) {
-          w.H1[q_of(k, s)] = au[k][s];
-          w.H1[n + q_of(k, s)] = av[k][s];
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
+        if (f == 0) {
+          x[k][s] = w.z[q];
+          y[k][s] = w.z[n + q];
+        } else if (f == 1) {
+          x[k][s] = w.z[2 * n + q];
+          y[k][s] = zero2();
+        } else {
+          const double o = O[q];
+          x[k][s] = cscale(w.z[n + q], o);
+          y[k][s] = cscale(w.z[2 * n + q], o);
         }
       }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        put(sm, M, 0 + k, c, packc(sym_at(au, P, k, s, c, Nx, Ny, true), sym_at(av, P, k, s, c, Nx, Ny, true)));
-        put(sm, M, 2 + k, c, packc(sym_at(tu, P, k, s, c, Nx, Ny, true), make_double2(0.0, 0.0)));
-      }
+    emit_pack(sm, M, 0, Q, tb.ny, x, y);
   }
-  fft_slices<M>(sm, 4, tb.twx, +1);
-  for (int s = 0; s < 4; ++s) {
-    const int f = s >> 1, k = s & 1;
-    double2* dst = w.R + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) dst[j] = slot(sm, M, s, j);
-  }
+  fft_slices<M, NT>(sm, 0, 2, tb.twx, +1);
+  row_store<M, NT>(sm, 0, 1, w.R + f * n, P, n);
 }
 
-// ---------------------------------------------------------------------------
+// V2: slices 0, 1 the sum, 2..5 two references at a time.  Fields out: 0 the sum
+// (u in the real, v in the imaginary part), 1 + j (gam_j u, gam_j v).
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
-k2v_colD(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2v_col2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  const int Nx = tb.nx;
+  constexpr int NT = thr4(M);
+  const int Nx = tb.nx, c = blockIdx.x, K = tb.nk;
   const size_t n = (size_t)tb.n;
-  const int c = blockIdx.x;
-  for (int f = 0; f < 2; ++f) col_load<M>(sm, 2 * f, w.R + f * n, Nx, c);
-  fft_slices<M>(sm, 4, tb.twy, +1);
   const double invN = 1.0 / ((double)tb.n);
-  for (int y = threadIdx.x; y < M; y += blockDim.x) {
+  col_load<M, NT>(sm, 2, 2, w.R, Nx, c, n);
+  fft_slices<M, NT>(sm, 2, 4, tb.twy, +1);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+    const ColPt p(t, c, Nx);
+    const double2 a = slot(sm, M, 2 + p.k, p.y), b = slot(sm, M, 4 + p.k, p.y);
+    w.phys[p.q] = a.x * invN;
+    w.phys[n + p.q] = a.y * invN;
+    w.phys[2 * n + p.q] = b.x * invN;
+    put(sm, M, p.k, p.y, zero2());
+  }
+  for (int j = 0; j < K; j += 2) {
+    const int nj = K - j > 1 ? 2 : 1;
+    __syncthreads();   // the slices' last readers are done
+    col_load<M, NT>(sm, 2, nj, w.R + (2 + j) * n, Nx, c, n);
+    fft_slices<M, NT>(sm, 2, 2 * nj, tb.twy, +1);
+#pragma unroll 2
+    for (int t = threadIdx.x; t < 2 * M; t += NT) {
+      const ColPt p(t, c, Nx);
+      const double u = w.phys[n + p.q], v = w.phys[2 * n + p.q];
+      double2 s = slot(sm, M, p.k, p.y);
+      for (int i = 0; i < nj; ++i) {
+        const double g = tb.gk[(j + i) * n + p.q], gn = g * invN;
+        const double2 a = slot(sm, M, 2 + 2 * i + p.k, p.y);
+        s = cadd(s, cscale(a, gn));
+        put(sm, M, 2 + 2 * i + p.k, p.y, make_double2(g * u, g * v));
+      }
+      put(sm, M, p.k, p.y, s);
+    }
+    fft_slices<M, NT>(sm, 2, 2 * nj, tb.twy, -1);
+    col_store<M, NT>(sm, 2, nj, w.Q + (1 + j) * n, Nx, c, n);
+  }
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, -1);
+  col_store<M, NT>(sm, 0, 1, w.Q, Nx, c, n);
+}
+
+// V3: slices 0..3 two fields at a time, 4, 5 the sum kx (.) + ky (.), under HS3 6, 7 its
+// kx part at the points that the symmetrisation keeps (columns up to Nx / 2)
+template <int M>
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2v_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
+  if (!rhs_active(ctl, cond)) return;
+  extern __shared__ double2 sm[];
+  constexpr int NT = thr4(M);
+  const int Nx = M, K = tb.nk;
+  const size_t n = (size_t)tb.n;
+  const bool hs3 = tb.model == 3;
+  const Pair P = row_pair(blockIdx.x, tb.ny);
+  for (int f = 0; f <= K; f += 2) {
+    const int nf = K + 1 - f > 1 ? 2 : 1;
+    __syncthreads();
+    row_load<M, NT>(sm, 0, nf, w.Q + f * n, P, n);
+    fft_slices<M, NT>(sm, 0, 2 * nf, tb.twx, -1);
+#pragma unroll 1
+    for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+      const Quad Q(P, j, Nx);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const size_t q = (size_t)y * Nx + 2 * c + k;
-      const double2 P1 = slot(sm, M, 0 + k, y), P2 = slot(sm, M, 2 + k, y);
-      const double m0u = P1.x * invN, m0v = P1.y * invN, lphi = P2.x * invN;
-      const double eta = w.phys[q], u = w.phys[n + q], v = w.phys[2 * n + q];
-      const double wc = tb.wallchar ? tb.wallchar[q] : 1.0;   // H2 products x wallchar (:3416-3430)
-      const double em = eta * m0u * wc, evm = eta * m0v * wc;
-      w.pe[q] = em;
-      w.pe[n + q] = evm;
-      put(sm, M, 0 + k, y, make_double2(em, eta * u * wc));
-      put(sm, M, 2 + k, y, make_double2(evm, eta * v * wc));
-      put(sm, M, 4 + k, y, make_double2(0.5 * ((u * u + v * v) - lphi * lphi) * wc, 0.0));
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          const size_t q = Q.at(k, s, Nx);
+          const double kx = tb.kx[Q.cc[s]], ky = tb.ky[Q.r[k]];
+          // field 0 is the summed images (coefficient 1), field 1 + j reference j's
+          const double o0 = f == 0 ? 1.0 : tb.ck[(f - 1) * n + q], o1 = nf == 2 ? tb.ck[f * n + q] : 0.0;
+          double2 a, b;
+          split_at(sm, M, 0, Q, k, s, a, b);
+          double2 pu = cscale(a, o0), pv = cscale(b, o0);
+          if (nf == 2) {
+            split_at(sm, M, 2, Q, k, s, a, b);
+            pu = cadd(pu, cscale(a, o1));
+            pv = cadd(pv, cscale(b, o1));
+          }
+          double2 t = cadd(cscale(pu, kx), cscale(pv, ky));
+          if (f > 0) t = cadd(t, slot(sm, M, 4 + k, Q.cc[s]));
+          put(sm, M, 4 + k, Q.cc[s], t);
+          if (hs3 && Q.has(s)) {
+            double2 tu = cscale(pu, kx);
+            if (f > 0) tu = cadd(tu, slot(sm, M, 6 + k, Q.cc[s]));
+            put(sm, M, 6 + k, Q.cc[s], tu);
+          }
+        }
     }
   }
-  fft_slices<M>(sm, 6, tb.twy, -1);
-  for (int f = 0; f < 3; ++f) col_store<M>(sm, 2 * f, w.Q + f * n, Nx, c);
-}
-
-// ---------------------------------------------------------------------------
-template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
-k2v_rowE(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
-  if (!rhs_active(ctl, cond)) return;
-  extern __shared__ double2 sm[];
-  const int Nx = tb.nx, Ny = tb.ny;
-  const size_t n = (size_t)tb.n;
-  const Pair P = row_pair(blockIdx.x, Ny);
-  const int r0 = P.r[0], r1 = P.r[1];
-  for (int s = 0; s < 6; ++s) {
-    const int f = s >> 1, k = s & 1;
-    const double2* src = w.Q + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) put(sm, M, s, j, src[j]);
-  }
-  fft_slices<M>(sm, 6, tb.twx, -1);
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
-    double2 z1[2][2], z2[2][2], z3[2][2], em[2][2], ev[2][2];
-    quad_load<M>(sm, 0, cc, z1);
-    quad_load<M>(sm, 2, cc, z2);
-    quad_load<M>(sm, 4, cc, z3);
+  // delphiH1^ = -i (kx C^2 u^ + ky C^2 v^) / g (2d/fun_odesolver.c:2943-2946, 4560-4563)
+  const double h = 0.5 / kGrav;
+#pragma unroll 1
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
+    double2 x[2][2], y[2][2];
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        double2 a, b, c2, d2, dh, zero;
-        split2(z1[k][s], z1[P.mr[k]][s ^ 1], a, b);
-        split2(z2[k][s], z2[P.mr[k]][s ^ 1], c2, d2);
-        split2(z3[k][s], z3[P.mr[k]][s ^ 1], dh, zero);
-        em[k][s] = a;
-        ev[k][s] = c2;
-        if (s == 0 || cm != j) {
-          const size_t q = (size_t)P.r[k] * Nx + cc[s];
-          w.EU[q] = b;
-          w.EU[n + q] = d2;
-          w.EU[2 * n + q] = dh;
+        const double2 t = mul_mi(slot(sm, M, 4 + k, Q.cc[s]), h);
+        w.H1[Q.at(k, s, Nx)] = t;
+        if (!Q.has(s)) continue;
+        x[k][s] = t;
+        y[k][s] = zero2();
+        if (hs3) {
+          x[k][s] = mul_mi(slot(sm, M, 6 + k, Q.cc[s]), h);
+          y[k][s] = csub(t, x[k][s]);
         }
       }
-    // E(Om_min (eta M0u)^) + i E(Om_plus (eta M0u)^); the same for v.  The spectra are
-    // products of the tables with unsymmetrised transforms (HSSgen_2depth :516-526).
-    double2 xm[2][2], xp[2][2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const size_t q = (size_t)(k ? r1 : r0) * Nx + cc[s];
-        xm[k][s] = make_double2(tb.omin[q] * em[k][s].x, tb.omin[q] * em[k][s].y);
-        xp[k][s] = make_double2(tb.oplus[q] * em[k][s].x, tb.oplus[q] * em[k][s].y);
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        put(sm, M, 0 + k, cc[s], packc(sym_at(xm, P, k, s, cc[s], Nx, Ny, true), sym_at(xp, P, k, s, cc[s], Nx, Ny, true)));
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const size_t q = (size_t)(k ? r1 : r0) * Nx + cc[s];
-        xm[k][s] = make_double2(tb.omin[q] * ev[k][s].x, tb.omin[q] * ev[k][s].y);
-        xp[k][s] = make_double2(tb.oplus[q] * ev[k][s].x, tb.oplus[q] * ev[k][s].y);
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        put(sm, M, 2 + k, cc[s], packc(sym_at(xm, P, k, s, cc[s], Nx, Ny, true), sym_at(xp, P, k, s, cc[s], Nx, Ny, true)));
-      }
+    if (tb.model != 1) emit_pack(sm, M, 4, Q, tb.ny, x, y);
   }
-  fft_slices<M>(sm, 4, tb.twx, +1);
-  for (int s = 0; s < 4; ++s) {
-    const int f = s >> 1, k = s & 1;
-    double2* dst = w.R + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) dst[j] = slot(sm, M, s, j);
-  }
+  if (tb.model == 1) return;
+  fft_slices<M, NT>(sm, 4, 2, tb.twx, +1);
+  row_store<M, NT>(sm, 4, 1, w.R, P, n);
 }
 
-// ---------------------------------------------------------------------------
+// where pass V4 puts its fields in w.Q: the products, the loss fields, then the gam_j pairs
+__device__ __forceinline__ int first_pair(const Tab2& tb, int nd, int cubic) { return cubic ? 1 : (tb.model == 3 ? 3 : 2) + nd; }
+
+// V4: column pass, inverse -> products -> forward; then gam_j q, four references at a time.
+// cubic = 0: L phi (HS3: M0u, M0v) in; fields 0 (q, eta u), 1 (eta v, deletaH2), under HS3
+// 2 (eta^2 M0u, eta^2 M0v), the loss fields; q = eta L phi.  cubic = 1: L q, div(grad phi) in;
+// field 0 (p, h3); q = p.
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
-k2v_colF(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2v_col4(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  const int Nx = tb.nx;
+  constexpr int NT = thr4(M);
+  const int Nx = tb.nx, c = blockIdx.x, K = tb.nk, nd = cubic ? 0 : damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
-  const int c = blockIdx.x;
-  for (int f = 0; f < 2; ++f) col_load<M>(sm, 2 * f, w.R + f * n, Nx, c);
-  fft_slices<M>(sm, 4, tb.twy, +1);
+  const bool hs3 = tb.model == 3;
+  const int f0 = first_pair(tb, nd, cubic);
   const double invN = 1.0 / ((double)tb.n);
-  for (int y = threadIdx.x; y < M; y += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const size_t q = (size_t)y * Nx + 2 * c + k;
-      const double2 P1 = slot(sm, M, 0 + k, y), P2 = slot(sm, M, 2 + k, y);
-      const double lmu = P1.x * invN, lpu = P1.y * invN, lmv = P2.x * invN, lpv = P2.y * invN;
-      const double em = w.pe[q], ev = w.pe[n + q];
-      const double gm = tb.gmin[q], gp = tb.gplus[q];
-      put(sm, M, 0 + k, y, make_double2(gm * em, gp * em));
-      put(sm, M, 2 + k, y, make_double2(gm * lmu, gp * lpu));
-      put(sm, M, 4 + k, y, make_double2(gm * ev, gp * ev));
-      put(sm, M, 6 + k, y, make_double2(gm * lmv, gp * lpv));
+  col_load<M, NT>(sm, 0, 1, w.R, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, +1);
+#pragma unroll 2
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+    const ColPt p(t, c, Nx);
+    const double2 a = cscale(slot(sm, M, p.k, p.y), invN);
+    if (cubic) {
+      const double2 r = cubic_products(tb, w, p.q, n, a.x, a.y);
+      put(sm, M, p.k, p.y, r);
+      w.op[p.q] = r.x;
+    } else {
+      const double wc = tb.wallchar ? tb.wallchar[p.q] : 1.0;
+      const double eta = w.phys[p.q], u = w.phys[n + p.q], v = w.phys[2 * n + p.q];
+      const double lphi = hs3 ? a.x + a.y : a.x, q = eta * lphi * wc;
+      put(sm, M, p.k, p.y, make_double2(q, eta * u * wc));
+      put(sm, M, 2 + p.k, p.y, make_double2(eta * v * wc, 0.5 * ((u * u + v * v) - lphi * lphi) * wc));
+      w.op[p.q] = q;
+      if (hs3) {
+        put(sm, M, 4 + p.k, p.y, make_double2(eta * eta * a.x * wc, eta * eta * a.y * wc));
+        w.op[n + p.q] = lphi;
+      }
+      emit_loss(sm, M, 2 * (hs3 ? 3 : 2), nd, p, tb, w, eta, u, v);
     }
   }
-  fft_slices<M>(sm, 8, tb.twy, -1);
-  for (int f = 0; f < 4; ++f) col_store<M>(sm, 2 * f, w.Q + f * n, Nx, c);
+  fft_slices<M, NT>(sm, 0, 2 * f0, tb.twy, -1);
+  col_store<M, NT>(sm, 0, f0, w.Q, Nx, c, n);
+  for (int j = 0; j < K; j += 4) {
+    const int nf = K - j > 2 ? 2 : 1;
+    __syncthreads();
+#pragma unroll 2
+    for (int t = threadIdx.x; t < 2 * M; t += NT) {
+      const ColPt p(t, c, Nx);
+      const double q = w.op[p.q];
+      double g[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[i] = j + i < K ? tb.gk[(j + i) * n + p.q] : 0.0;
+      put(sm, M, p.k, p.y, make_double2(g[0] * q, g[1] * q));
+      if (nf == 2) put(sm, M, 2 + p.k, p.y, make_double2(g[2] * q, g[3] * q));
+    }
+    fft_slices<M, NT>(sm, 0, 2 * nf, tb.twy, -1);
+    col_store<M, NT>(sm, 0, nf, w.Q + (f0 + j / 2) * n, Nx, c, n);
+  }
 }
 
-// ---------------------------------------------------------------------------
+// V5: row pass, forward, split; what the images still to come do not change is kept in w.T
+// (delu + delv, deletaH, and 1/2 sum_j Omega_j F(gam_j q) / g), and Omega_j q^ goes to
+// physical space, two references to a field
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
-k2v_rowG(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2v_row5(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  const int Nx = tb.nx, Ny = tb.ny;
+  constexpr int NT = thr4(M);
+  const int Nx = M, K = tb.nk, nd = cubic ? 0 : damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
-  const Pair P = row_pair(blockIdx.x, Ny);
-  for (int s = 0; s < 8; ++s) {
-    const int f = s >> 1, k = s & 1;
-    const double2* src = w.Q + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) put(sm, M, s, j, src[j]);
+  const bool hs3 = tb.model == 3;
+  const int f0 = first_pair(tb, nd, cubic), np = cubic ? 1 : (hs3 ? 3 : 2);
+  const Pair P = row_pair(blockIdx.x, tb.ny);
+  row_load<M, NT>(sm, 0, f0, w.Q, P, n);
+  fft_slices<M, NT>(sm, 0, 2 * f0, tb.twx, -1);
+#pragma unroll 1
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
+    if (!cubic) store_loss(sm, M, 2 * np, nd, Q, Nx, w, n);
+    double2 keep[2][2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
+        double2 qh, b;
+        split_at(sm, M, 0, Q, k, s, qh, b);
+        keep[k][s] = qh;
+        if (cubic) {
+          w.T[n + q] = cadd(w.T[n + q], b);   // deletaH3
+        } else {
+          const double kx = tb.kx[Q.cc[s]], ky = tb.ky[Q.r[k]];
+          double2 ev, dH;
+          split_at(sm, M, 2, Q, k, s, ev, dH);
+          double2 a = cadd(mul_mi(b, kx), mul_mi(ev, ky));   // -i kx (eta u)^ - i ky (eta v)^
+          if (hs3) {
+            double2 cu, cv;
+            split_at(sm, M, 4, Q, k, s, cu, cv);
+            a = csub(a, cadd(cscale(cu, 0.5 * (kx * kx)), cscale(cv, 0.5 * (ky * ky))));
+          }
+          w.T[q] = a;
+          w.T[n + q] = dH;
+        }
+      }
+    // q^ stays in slices 0, 1 at the points that the symmetrisation keeps
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+        if (Q.has(s)) put(sm, M, k, Q.cc[s], keep[k][s]);
   }
-  fft_slices<M>(sm, 8, tb.twx, -1);
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
-    auto q_of = [&](int k, int s) { return (size_t)P.r[k] * Nx + cc[s]; };
-    double2 z[2][2], acc[2][2], t2[2][2], a1[2][2], a2[2][2];
-    // L (eta M0u)^ = [F(gm Lm) + Om_min F(gm .) + F(gp Lp) + Om_plus F(gp .)] / 2
-    quad_load<M>(sm, 0, cc, z);
+  const double h = 0.5 / kGrav;
+  for (int j0 = 0; j0 < K; j0 += 4) {
+    const int nf = K - j0 > 2 ? 2 : 1;
+    __syncthreads();
+    row_load<M, NT>(sm, 2, nf, w.Q + (f0 + j0 / 2) * n, P, n);
+    fft_slices<M, NT>(sm, 2, 2 * nf, tb.twx, -1);
+#pragma unroll 1
+    for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+      const Quad Q(P, j, Nx);
+      double2 x[4][2][2];
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+      for (int k = 0; k < 2; ++k)
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        const size_t q = q_of(k, s);
-        acc[k][s] = make_double2(tb.omin[q] * a.x, tb.omin[q] * a.y);
-        t2[k][s] = make_double2(tb.oplus[q] * b.x, tb.oplus[q] * b.y);
-      }
-    quad_load<M>(sm, 2, cc, z);
+        for (int s = 0; s < 2; ++s) {
+          if (!Q.has(s)) continue;
+          const size_t q = Q.at(k, s, Nx);
+          double o[4];
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
+          for (int i = 0; i < 4; ++i) o[i] = j0 + i < K ? tb.ok[(j0 + i) * n + q] : 0.0;
+          double2 acc = j0 > 0 ? w.T[2 * n + q] : zero2();
+          double2 a, b;
+          split_at(sm, M, 2, Q, k, s, a, b);
+          acc = cadd(acc, cadd(cscale(a, h * o[0]), cscale(b, h * o[1])));
+          if (nf == 2) {
+            split_at(sm, M, 4, Q, k, s, a, b);
+            acc = cadd(acc, cadd(cscale(a, h * o[2]), cscale(b, h * o[3])));
+          }
+          w.T[2 * n + q] = acc;
+          const double2 qh = slot(sm, M, k, Q.cc[s]);
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        const double2 L = make_double2((a.x + acc[k][s].x + b.x + t2[k][s].x) / 2,
-                                       (a.y + acc[k][s].y + b.y + t2[k][s].y) / 2);
-        const size_t q = q_of(k, s);
-        const double2 eu = w.EU[q];
-        const double kxv = tb.kx[cc[s]];
-        a1[k][s] = make_double2(kxv * eu.y - L.x / kGrav, -kxv * eu.x - L.y / kGrav);   // delu H2^
-      }
-    quad_load<M>(sm, 4, cc, z);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        const size_t q = q_of(k, s);
-        acc[k][s] = make_double2(tb.omin[q] * a.x, tb.omin[q] * a.y);
-        t2[k][s] = make_double2(tb.oplus[q] * b.x, tb.oplus[q] * b.y);
-      }
-    quad_load<M>(sm, 6, cc, z);
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        double2 a, b;
-        split2(z[k][s], z[P.mr[k]][s ^ 1], a, b);
-        const double2 L = make_double2((a.x + acc[k][s].x + b.x + t2[k][s].x) / 2,
-                                       (a.y + acc[k][s].y + b.y + t2[k][s].y) / 2);
-        const size_t q = q_of(k, s);
-        const double2 ev = w.EU[n + q];
-        const double kyv = tb.ky[P.r[k]];
-        a2[k][s] = make_double2(kyv * ev.y - L.x / kGrav, -kyv * ev.x - L.y / kGrav);   // delv H2^
-      }
-    // i kx deletaH2^, i ky deletaH2^
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const double2 dh = w.EU[2 * n + q_of(k, s)];
-        acc[k][s] = mul_pi(dh, tb.kx[cc[s]]);
-        t2[k][s] = mul_pi(dh, tb.ky[P.r[k]]);
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        put(sm, M, 0 + k, c, sym_at(acc, P, k, s, c, Nx, Ny, false));
-        put(sm, M, 2 + k, c, sym_at(t2, P, k, s, c, Nx, Ny, false));
-        put(sm, M, 4 + k, c, sym_at(a1, P, k, s, c, Nx, Ny, false));
-        put(sm, M, 6 + k, c, sym_at(a2, P, k, s, c, Nx, Ny, false));
-      }
+          for (int i = 0; i < 4; ++i) x[i][k][s] = cscale(qh, o[i]);
+        }
+      emit_pack(sm, M, 2, Q, tb.ny, x[0], x[1]);
+      if (nf == 2) emit_pack(sm, M, 4, Q, tb.ny, x[2], x[3]);
+    }
+    fft_slices<M, NT>(sm, 2, 2 * nf, tb.twx, +1);
+    row_store<M, NT>(sm, 2, nf, w.R + (j0 / 2) * n, P, n);
   }
-  __syncthreads();
-  double2* dst = tb.chi_one ? w.V : w.W;
-  if (!tb.chi_one) fft_slices<M>(sm, 8, tb.twx, +1);
-  for (int s = 0; s < 8; ++s) {
-    const int f = s >> 1, k = s & 1;
-    double2* d = dst + f * n + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) d[j] = slot(sm, M, s, j);
+}
+
+// V6: slices 0, 1 the sum of the weighted images (real), 2..5 four references at a time
+template <int M>
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2v_col6(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
+  if (!rhs_active(ctl, cond)) return;
+  extern __shared__ double2 sm[];
+  constexpr int NT = thr4(M);
+  const int Nx = tb.nx, c = blockIdx.x, K = tb.nk;
+  const size_t n = (size_t)tb.n;
+  const double invN = 1.0 / ((double)tb.n);
+  for (int j = 0; j < K; j += 4) {
+    const int nf = K - j > 2 ? 2 : 1;
+    __syncthreads();
+    col_load<M, NT>(sm, 2, nf, w.R + (j / 2) * n, Nx, c, n);
+    fft_slices<M, NT>(sm, 2, 2 * nf, tb.twy, +1);
+#pragma unroll 2
+    for (int t = threadIdx.x; t < 2 * M; t += NT) {
+      const ColPt p(t, c, Nx);
+      double g[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[i] = j + i < K ? tb.gk[(j + i) * n + p.q] : 0.0;
+      const double2 a = slot(sm, M, 2 + p.k, p.y), b = nf == 2 ? slot(sm, M, 4 + p.k, p.y) : zero2();
+      double s = (g[0] * a.x + g[1] * a.y + (g[2] * b.x + g[3] * b.y)) * invN;
+      if (j > 0) s += slot(sm, M, p.k, p.y).x;
+      put(sm, M, p.k, p.y, make_double2(s, 0.0));
+    }
+  }
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, -1);
+  col_store<M, NT>(sm, 0, 1, w.Q, Nx, c, n);
+}
+
+// V7: row pass, forward: L q^ = (sum_j Omega_j F(gam_j q) + F(sum)) / (2 g).  The second-order
+// operand's enters delu + delv with a minus, the cubic one's with a plus; under HS3 the
+// former, with div(grad phi), goes to physical space for the cubic products.
+template <int M>
+__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+k2v_row7(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
+  if (!rhs_active(ctl, cond)) return;
+  extern __shared__ double2 sm[];
+  constexpr int NT = thr4(M);
+  const int Nx = M;
+  const size_t n = (size_t)tb.n;
+  const bool more = tb.model == 3 && !cubic;
+  const double h = 0.5 / kGrav;
+  const Pair P = row_pair(blockIdx.x, tb.ny);
+  row_load<M, NT>(sm, 0, 1, w.Q, P, n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twx, -1);
+#pragma unroll 1
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
+    double2 dH[2][2], a[2][2], lq[2][2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
+        double2 x, none;
+        split_at(sm, M, 0, Q, k, s, x, none);
+        lq[k][s] = cadd(w.T[2 * n + q], cscale(x, h));
+        a[k][s] = cubic ? cadd(w.T[q], lq[k][s]) : csub(w.T[q], lq[k][s]);
+        if (more) {
+          w.T[q] = a[k][s];
+          dH[k][s] = cadd(mul_pi(w.z[n + q], tb.kx[Q.cc[s]]), mul_pi(w.z[2 * n + q], tb.ky[Q.r[k]]));
+        } else {
+          dH[k][s] = w.T[n + q];
+        }
+      }
+    if (more) emit_pack(sm, M, 0, Q, tb.ny, lq, dH);
+    else emit_adjust(sm, M, Q, tb, dH, a);
+  }
+  if (more) {
+    fft_slices<M, NT>(sm, 0, 2, tb.twx, +1);
+    row_store<M, NT>(sm, 0, 1, w.R, P, n);
+  } else {
+    send_adjust<M, NT>(sm, P, tb, w, n);
   }
 }
 

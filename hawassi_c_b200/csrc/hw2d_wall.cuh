@@ -23,85 +23,76 @@
 namespace hw2d {
 
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2w_row1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx, Ny = tb.ny;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, Ny);
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
+#pragma unroll 2
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
     double2 A[2][2], B[2][2];
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const size_t q = (size_t)P.r[k] * Nx + cc[s];
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
         const double C = tb.c2d[q];
         const double2 zu = w.z[n + q], zv = w.z[2 * n + q];
         A[k][s] = make_double2(C * zu.x, C * zu.y);
         B[k][s] = make_double2(C * zv.x, C * zv.y);
       }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        const double2 ea = sym_at(A, P, k, s, c, Nx, Ny, true), eb = sym_at(B, P, k, s, c, Nx, Ny, true);
-        put(sm, M, k, c, make_double2(ea.x - eb.y, ea.y + eb.x));
-      }
+    emit_pack(sm, M, 0, Q, Ny, A, B);
   }
-  fft_slices<M>(sm, 2, tb.twx, +1);
-  for (int k = 0; k < 2; ++k) {
-    double2* dst = w.WP + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) dst[j] = slot(sm, M, k, j);
-  }
+  fft_slices<M, NT>(sm, 0, 2, tb.twx, +1);
+  row_store<M, NT>(sm, 0, 1, w.WP, P, n);
 }
 
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2w_col2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx;
   const int c = blockIdx.x;
-  col_load<M>(sm, 0, w.WP, Nx, c);
-  fft_slices<M>(sm, 2, tb.twy, +1);
+  const size_t n = (size_t)tb.n;
+  col_load<M, NT>(sm, 0, 1, w.WP, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, +1);
   const double invN = 1.0 / ((double)tb.n);
-  for (int y = threadIdx.x; y < M; y += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const size_t q = (size_t)y * Nx + 2 * c + k;
-      const double2 v = slot(sm, M, k, y);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+      const ColPt p(t, c, Nx);
+      const size_t q = p.q;
+      const double2 v = slot(sm, M, p.k, p.y);
       const double wc = tb.wallchar[q];
-      put(sm, M, k, y, make_double2(v.x * invN * wc, v.y * invN * wc));
+      put(sm, M, p.k, p.y, make_double2(v.x * invN * wc, v.y * invN * wc));
     }
-  fft_slices<M>(sm, 2, tb.twy, -1);
-  col_store<M>(sm, 0, w.WP, Nx, c);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, -1);
+  col_store<M, NT>(sm, 0, 1, w.WP, Nx, c, n);
 }
 
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2w_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx, Ny = tb.ny;
   const Pair P = row_pair(blockIdx.x, Ny);
+  row_load<M, NT>(sm, 0, 1, w.WP, P, (size_t)tb.n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twx, -1);
   for (int k = 0; k < 2; ++k) {
-    const double2* src = w.WP + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) put(sm, M, k, j, src[j]);
-  }
-  fft_slices<M>(sm, 2, tb.twx, -1);
-  for (int k = 0; k < 2; ++k) {
-    const int r = P.r[k];
+    const int r = P.row(k);
     const double kyv = tb.ky[r];
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) {
+    for (int j = threadIdx.x; j < Nx; j += NT) {
       const size_t q = (size_t)r * Nx + j;
       double2 X, Y;   // F(wallchar C u), F(wallchar C v)
-      split2(slot(sm, M, k, j), slot(sm, M, P.mr[k], (Nx - j) % Nx), X, Y);
+      split2(slot(sm, M, k, j), slot(sm, M, k ^ P.flip, (Nx - j) % Nx), X, Y);
       const double cg = tb.c2d[q] / kGrav;
       const double2 du = make_double2(cg * X.x, cg * X.y), dv = make_double2(cg * Y.x, cg * Y.y);
       const double kxv = tb.kx[j];
@@ -111,97 +102,89 @@ k2w_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 }
 
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2w_rowV1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx, Ny = tb.ny;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, Ny);
-  for (int j = threadIdx.x; j <= Nx / 2; j += blockDim.x) {
-    const int cm = (Nx - j) % Nx;
-    const int cc[2] = {j, cm};
-    double2 A[2][2], B[2][2], D[2][2];
+#pragma unroll 2
+  for (int j = threadIdx.x; j < Nx / 2; j += NT) {
+    const Quad Q(P, j, Nx);
+    double2 A[2][2], B[2][2], D[2][2], Z[2][2];
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const size_t q = (size_t)P.r[k] * Nx + cc[s];
+        if (!Q.has(s)) continue;
+        const size_t q = Q.at(k, s, Nx);
         const double cg = tb.c2g[q];
         const double2 zu = w.z[n + q], zv = w.z[2 * n + q];
         A[k][s] = make_double2(cg * zu.x, cg * zu.y);
         B[k][s] = make_double2(cg * zv.x, cg * zv.y);
       }
-    // divC2u^ from the symmetrised spectra at every point of the quad
+    // divC2u^ = -i (kx S(.) + ky S(.)) from the symmetrised spectra
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        const int c = cc[s];
-        const double2 sa = sym_at(A, P, k, s, c, Nx, Ny, false), sb = sym_at(B, P, k, s, c, Nx, Ny, false);
-        const double kxv = tb.kx[c], kyv = tb.ky[P.r[k]];
-        D[k][s] = make_double2(-(-kxv * sa.y - kyv * sb.y), -(kxv * sa.x + kyv * sb.x));
+        if (!Q.has(s)) continue;
+        double2 sa = A[k][s], sb = B[k][s];
+        if (Q.self) {
+          sa = self_sym(sa, Q.flip ? A[k ^ 1][s] : sa, Q.r[k], s, Ny, false);
+          sb = self_sym(sb, Q.flip ? B[k ^ 1][s] : sb, Q.r[k], s, Ny, false);
+        }
+        D[k][s] = cadd(mul_mi(sa, tb.kx[Q.cc[s]]), mul_mi(sb, tb.ky[Q.r[k]]));
+        Z[k][s] = zero2();
       }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        if (s == 1 && cm == j) continue;
-        const int c = cc[s];
-        const double2 ea = sym_at(A, P, k, s, c, Nx, Ny, true), eb = sym_at(B, P, k, s, c, Nx, Ny, true);
-        put(sm, M, k, c, make_double2(ea.x - eb.y, ea.y + eb.x));
-        put(sm, M, 2 + k, c, sym_at(D, P, k, s, c, Nx, Ny, true));
-      }
+    emit_pack(sm, M, 0, Q, Ny, A, B);
+    emit_pack(sm, M, 2, Q, Ny, D, Z);
   }
-  fft_slices<M>(sm, 4, tb.twx, +1);
-  for (int f = 0; f < 2; ++f)
-    for (int k = 0; k < 2; ++k) {
-      double2* dst = w.WP + f * n + (size_t)P.r[k] * Nx;
-      for (int j = threadIdx.x; j < Nx; j += blockDim.x) dst[j] = slot(sm, M, 2 * f + k, j);
-    }
+  fft_slices<M, NT>(sm, 0, 4, tb.twx, +1);
+  row_store<M, NT>(sm, 0, 2, w.WP, P, n);
 }
 
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2w_colV2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx;
   const size_t n = (size_t)tb.n;
   const int c = blockIdx.x;
-  col_load<M>(sm, 0, w.WP, Nx, c);
-  col_load<M>(sm, 2, w.WP + n, Nx, c);
-  fft_slices<M>(sm, 4, tb.twy, +1);
+  col_load<M, NT>(sm, 0, 2, w.WP, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 4, tb.twy, +1);
   const double invN = 1.0 / ((double)tb.n);
-  for (int y = threadIdx.x; y < M; y += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const size_t q = (size_t)y * Nx + 2 * c + k;
-      const double2 fl = slot(sm, M, k, y), dv = slot(sm, M, 2 + k, y);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+      const ColPt p(t, c, Nx);
+      const size_t q = p.q;
+      const double2 fl = slot(sm, M, p.k, p.y), dv = slot(sm, M, 2 + p.k, p.y);
       const double fx = fl.x * invN, fy = fl.y * invN, div = dv.x * invN;
-      put(sm, M, k, y, make_double2(div * tb.wallchar[q], fx * tb.gwx[q] + fy * tb.gwy[q]));
+      put(sm, M, p.k, p.y, make_double2(div * tb.wallchar[q], fx * tb.gwx[q] + fy * tb.gwy[q]));
     }
-  fft_slices<M>(sm, 2, tb.twy, -1);
-  col_store<M>(sm, 0, w.WP, Nx, c);
+  fft_slices<M, NT>(sm, 0, 2, tb.twy, -1);
+  col_store<M, NT>(sm, 0, 1, w.WP, Nx, c, n);
 }
 
 template <int M>
-__global__ void __launch_bounds__(kGroups * (M / 8), 1)
+__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
 k2w_rowV3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
+  constexpr int NT = thr2(M);
   const int Nx = tb.nx, Ny = tb.ny;
   const Pair P = row_pair(blockIdx.x, Ny);
+  row_load<M, NT>(sm, 0, 1, w.WP, P, (size_t)tb.n);
+  fft_slices<M, NT>(sm, 0, 2, tb.twx, -1);
   for (int k = 0; k < 2; ++k) {
-    const double2* src = w.WP + (size_t)P.r[k] * Nx;
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) put(sm, M, k, j, src[j]);
-  }
-  fft_slices<M>(sm, 2, tb.twx, -1);
-  for (int k = 0; k < 2; ++k) {
-    const int r = P.r[k];
-    for (int j = threadIdx.x; j < Nx; j += blockDim.x) {
+    const int r = P.row(k);
+    for (int j = threadIdx.x; j < Nx; j += NT) {
       double2 X, Y;   // F(divC2u wallchar), F(Flux . grad wallchar)
-      split2(slot(sm, M, k, j), slot(sm, M, P.mr[k], (Nx - j) % Nx), X, Y);
+      split2(slot(sm, M, k, j), slot(sm, M, k ^ P.flip, (Nx - j) % Nx), X, Y);
       w.H1[(size_t)r * Nx + j] = make_double2(X.x - Y.x, X.y - Y.y);
     }
   }
