@@ -39,11 +39,8 @@ using hwdev::cconj;
 using hwdev::cmul;
 using hwdev::cscale;
 using hwdev::csub;
-using hwdev::dft_small;
 using hwdev::padded;
 using hwdev::pidx;
-using hwdev::twiddle_powers;
-using hwdev::twd;
 
 constexpr double kGrav = 9.80665;
 
@@ -160,98 +157,6 @@ __host__ __device__ constexpr int ctas(int threads) { return 512 / threads; }
 __host__ __device__ constexpr int thr2(int) { return 128; }
 __host__ __device__ constexpr int thr4(int) { return 256; }
 
-// 16-point DFT as 4 x 4
-__device__ __forceinline__ void dft16(double2* v, int sign) {
-  constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173, r = 0.70710678118654752440;
-#pragma unroll
-  for (int n = 0; n < 4; ++n) {
-    double2 t[4] = {v[n], v[n + 4], v[n + 8], v[n + 12]};
-    dft_small<4>(t, sign);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[n + 4 * k] = t[k];
-  }
-  // x W16^(n k), n the column, k the row of the 4 x 4 block
-  const double sg = double(sign);
-  auto rot = [&](double2 a, double c, double s) { return make_double2(c * a.x - sg * s * a.y, c * a.y + sg * s * a.x); };
-  v[5] = rot(v[5], c1, s1);
-  v[6] = rot(v[6], r, r);
-  v[7] = rot(v[7], s1, c1);
-  v[9] = rot(v[9], r, r);
-  v[10] = hwdev::mul_pm_i(v[10], sign);
-  v[11] = rot(v[11], -r, r);
-  v[13] = rot(v[13], s1, c1);
-  v[14] = rot(v[14], -r, r);
-  v[15] = rot(v[15], -c1, -s1);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) dft_small<4>(v + 4 * k, sign);
-  // v[4 k2 + k1] holds X[4 k1 + k2]
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = a + 1; b < 4; ++b) {
-      const double2 t = v[4 * a + b];
-      v[4 * a + b] = v[4 * b + a];
-      v[4 * b + a] = t;
-    }
-}
-
-// the threads of one slice: within a warp up to 512 points, two warps for 1024
-template <int TP>
-__device__ __forceinline__ void slice_sync(int g) {
-  if constexpr (TP > 32) asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(TP) : "memory");
-  else __syncwarp();
-}
-
-// one in-place Stockham radix-R pass of a slice by M/16 threads, 16 points each
-template <int M, int R>
-__device__ __forceinline__ void spass(double2* sm, int s, int Ns, const double2* __restrict__ tw, int sign, int tid, int g,
-                                      bool act) {
-  constexpr int TP = M / 16, NB = M / R, BPT = 16 / R;
-  double2 v[BPT][R];
-  if (act) {
-#pragma unroll
-    for (int u = 0; u < BPT; ++u)
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[u][r] = sm[sidx(M, s, tid + u * TP + r * NB)];
-  }
-  slice_sync<TP>(g);
-  if (act) {
-#pragma unroll
-    for (int u = 0; u < BPT; ++u) {
-      const int j = tid + u * TP, jm = j & (Ns - 1);
-      if (Ns > 1) {
-        const int qb = jm * (M / (Ns * R));
-        if constexpr (R == 16) {
-          // powers from w, w^2, w^4, w^8: at most three factors each
-          const double2 w1 = twd(tw, qb, sign), w2 = twd(tw, 2 * qb, sign), w4 = twd(tw, 4 * qb, sign),
-                        w8 = twd(tw, 8 * qb, sign), w3 = cmul(w2, w1);
-          const double2 lo[4] = {make_double2(1.0, 0.0), w1, w2, w3};
-#pragma unroll
-          for (int r = 1; r < 4; ++r) v[u][r] = cmul(v[u][r], lo[r]);
-#pragma unroll
-          for (int h = 1; h < 4; ++h) {
-            const double2 wh = h == 1 ? w4 : (h == 2 ? w8 : cmul(w8, w4));
-            v[u][4 * h] = cmul(v[u][4 * h], wh);
-#pragma unroll
-            for (int r = 1; r < 4; ++r) v[u][4 * h + r] = cmul(v[u][4 * h + r], cmul(wh, lo[r]));
-          }
-        } else {
-          double2 w[R];
-          twiddle_powers<R>(twd(tw, qb, sign), w);
-#pragma unroll
-          for (int r = 1; r < R; ++r) v[u][r] = cmul(v[u][r], w[r]);
-        }
-      }
-      if constexpr (R == 16) dft16(v[u], sign);
-      else dft_small<R>(v[u], sign);
-      const int d = (j - jm) * R + jm;
-#pragma unroll
-      for (int r = 0; r < R; ++r) sm[sidx(M, s, d + r * Ns)] = v[u][r];
-    }
-  }
-  slice_sync<TP>(g);
-}
-
 // slices [s0, s0 + ns) by a CTA of NT threads, NT / (M/16) at a time; CTA-wide
 // barriers on entry and exit (the phases around read and write every slice).  Sixteen
 // points a thread: two passes of radix 16 for 256 points, three for 512 and 1024 where
@@ -265,25 +170,7 @@ __device__ __forceinline__ void fft_slices(double2* sm, int s0, int ns, const do
     const int s = s0 + base + g;
     const bool act = base + g < ns;
     if (TP > 32 && !act) break;
-    if constexpr (M == 1024) {
-      spass<M, 8>(sm, s, 1, tw, sign, tid, g, act);
-      spass<M, 8>(sm, s, 8, tw, sign, tid, g, act);
-      spass<M, 16>(sm, s, 64, tw, sign, tid, g, act);
-    } else if constexpr (M == 512) {
-      spass<M, 8>(sm, s, 1, tw, sign, tid, g, act);
-      spass<M, 8>(sm, s, 8, tw, sign, tid, g, act);
-      spass<M, 8>(sm, s, 64, tw, sign, tid, g, act);
-    } else if constexpr (M == 256) {
-      spass<M, 16>(sm, s, 1, tw, sign, tid, g, act);
-      spass<M, 16>(sm, s, 16, tw, sign, tid, g, act);
-    } else if constexpr (M == 128) {
-      spass<M, 8>(sm, s, 1, tw, sign, tid, g, act);
-      spass<M, 16>(sm, s, 8, tw, sign, tid, g, act);
-    } else {
-      static_assert(M == 64, "slices of 64 to 1024 points");
-      spass<M, 8>(sm, s, 1, tw, sign, tid, g, act);
-      spass<M, 8>(sm, s, 8, tw, sign, tid, g, act);
-    }
+    hwdev::slice_fft<M>(sm + s * M, (s & 1) << 2, tw, 1, sign, tid, g, act);
   }
   __syncthreads();
 }

@@ -234,8 +234,8 @@ static __device__ __noinline__ void breaking_leader(const DevMember& d, BrkDev* 
 //                   count of nodes with B != 0 in bk->npk (0: no force);
 //   breaking_force  (all threads) after a barrier that follows the leader.
 template <int M>
-__device__ __forceinline__ void breaking_reset(Ctx<M>& X) {
-  if (X.c == 0 && X.tid == 0) {
+__device__ __forceinline__ void breaking_reset(Ctx<M> X) {
+  if (X.c == 0 && int(threadIdx.x) == 0) {
     X.d.bk->npk = 0;
     X.d.bk->any_above = 0;
   }
@@ -247,14 +247,14 @@ __device__ __forceinline__ void breaking_reset(Ctx<M>& X) {
 // thread that walked its own eight points waited for each crest in turn
 // (21 against 7 thousand cycles an RHS in the 256-member ensemble)
 template <int M>
-__device__ __forceinline__ void breaking_scan(Ctx<M>& X, const double2* PE, const double* Heta, int hs) {
+__device__ __forceinline__ void breaking_scan(Ctx<M> X, const double2* PE, const double* Heta, int hs) {
   const DevMember& d = X.d;
   BrkDev* bk = d.bk;
-  const int N = d.N, n = *X.ncand;
+  const int N = d.N, n = X.sc->ncand;
   const int w0 = d.xbstart, w1 = d.xbstart + d.lenIF;
   bool above = false;
-  for (int q = X.tid; q < n; q += Ctx<M>::T) {
-    const int p = X.cand[q];
+  for (int q = int(threadIdx.x); q < n; q += Ctx<M>::T) {
+    const int p = X.sc->cand[q];
     const bool inner = p >= w0 + 1 && p <= w1 - 2;
     const double e = PE[p].x, el = inner ? PE[p - 1].x : 0.0, er = inner ? PE[p + 1].x : 0.0;
     if (e > d.MaxEtaInit) above = true;
@@ -264,12 +264,12 @@ __device__ __forceinline__ void breaking_scan(Ctx<M>& X, const double2* PE, cons
     }
   }
   // one flag update per warp
-  if (__any_sync(0xffffffffu, above) && (X.tid & 31) == 0) atomicOr(&bk->any_above, 1);
+  if (__any_sync(0xffffffffu, above) && (int(threadIdx.x) & 31) == 0) atomicOr(&bk->any_above, 1);
 }
 
 template <int M>
-__device__ __forceinline__ void breaking_lead(Ctx<M>& X, double t, const double2* PE, const double* Heta, int hs) {
-  if (X.c == 0 && X.tid == 0) {
+__device__ __forceinline__ void breaking_lead(Ctx<M> X, double t, const double2* PE, const double* Heta, int hs) {
+  if (X.c == 0 && int(threadIdx.x) == 0) {
     BrkDev* bk = X.d.bk;
     const int npk = bk->npk, flag = bk->flag, touched = bk->n_touched, it = bk->ITERbdt;
     const int dirty = bk->dirty_cb | bk->dirty_cbn;
@@ -288,7 +288,7 @@ __device__ __forceinline__ void breaking_lead(Ctx<M>& X, double t, const double2
 // eddy-viscosity force (rhs_breaking, 1d/rhs.c:617-657): Rb = F(d_x Flux / (h + eta)),
 // Flux = -B delb^2 (h + eta) (d_t eta)^2, d_t eta = Re F^-1(dH1_eta + AEadj)
 template <int M>
-__device__ __noinline__ void breaking_force(Ctx<M>& X, const double2* PE, const double2* AEadj, double2* Rb) {
+__device__ __noinline__ void breaking_force(Ctx<M> X, const double2* PE, const double2* AEadj, double2* Rb) {
   const DevMember& d = X.d;
   BrkDev* bk = d.bk;
   const int N = d.N;

@@ -115,8 +115,142 @@ __device__ __forceinline__ void twiddle_powers(double2 w1, double2* w) {
   }
 }
 
-// One in-place Stockham radix-R pass over the M-point slice in shared memory.
-// tw_stride converts an index in units of 1/M of a turn to the N-point table.
+// 16-point DFT as 4 x 4
+template <>
+__device__ __forceinline__ void dft_small<16>(double2* v, int sign) {
+  constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173, r = 0.70710678118654752440;
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    double2 t[4] = {v[n], v[n + 4], v[n + 8], v[n + 12]};
+    dft_small<4>(t, sign);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[n + 4 * k] = t[k];
+  }
+  // x W16^(n k), n the column, k the row of the 4 x 4 block
+  const double sg = double(sign);
+  auto rot = [&](double2 a, double c, double s) { return make_double2(c * a.x - sg * s * a.y, c * a.y + sg * s * a.x); };
+  v[5] = rot(v[5], c1, s1);
+  v[6] = rot(v[6], r, r);
+  v[7] = rot(v[7], s1, c1);
+  v[9] = rot(v[9], r, r);
+  v[10] = mul_pm_i(v[10], sign);
+  v[11] = rot(v[11], -r, r);
+  v[13] = rot(v[13], s1, c1);
+  v[14] = rot(v[14], -r, r);
+  v[15] = rot(v[15], -c1, -s1);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) dft_small<4>(v + 4 * k, sign);
+  // v[4 k2 + k1] holds X[4 k1 + k2]
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = a + 1; b < 4; ++b) {
+      const double2 t = v[4 * a + b];
+      v[4 * a + b] = v[4 * b + a];
+      v[4 * b + a] = t;
+    }
+}
+
+// the TP threads of one slice: within a warp, or the warps of group g by their own barrier
+template <int TP>
+__device__ __forceinline__ void slice_sync(int g) {
+  if constexpr (TP > 32) asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "r"(TP) : "memory");
+  else __syncwarp();
+}
+
+// One in-place Stockham radix-R pass of an M-point slice by M/16 threads (rank tid of group
+// g), 16 points each.  xo turns the slice's swizzle (pidx(i) ^ xo); tw_stride converts an
+// index in units of 1/M of a turn to the table's.  Lanes with act = false only keep step.
+template <int M, int R>
+__device__ __forceinline__ void slice_pass(double2* buf, int xo, int Ns, const double2* __restrict__ tw, int tw_stride,
+                                           int sign, int tid, int g, bool act) {
+  constexpr int TP = M / 16, NB = M / R, BPT = 16 / R;
+  double2 v[BPT][R];
+  if (act) {
+#pragma unroll
+    for (int u = 0; u < BPT; ++u)
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[u][r] = buf[pidx(tid + u * TP + r * NB) ^ xo];
+  }
+  slice_sync<TP>(g);
+  if (act) {
+#pragma unroll
+    for (int u = 0; u < BPT; ++u) {
+      const int j = tid + u * TP, jm = j & (Ns - 1);
+      if (Ns > 1) {
+        const int qb = jm * (M / (Ns * R)) * tw_stride;
+        if constexpr (R == 16) {
+          // powers from w, w^2, w^4, w^8: at most three factors each
+          const double2 w1 = twd(tw, qb, sign), w2 = twd(tw, 2 * qb, sign), w4 = twd(tw, 4 * qb, sign),
+                        w8 = twd(tw, 8 * qb, sign), w3 = cmul(w2, w1);
+          const double2 lo[4] = {make_double2(1.0, 0.0), w1, w2, w3};
+#pragma unroll
+          for (int r = 1; r < 4; ++r) v[u][r] = cmul(v[u][r], lo[r]);
+#pragma unroll
+          for (int h = 1; h < 4; ++h) {
+            const double2 wh = h == 1 ? w4 : (h == 2 ? w8 : cmul(w8, w4));
+            v[u][4 * h] = cmul(v[u][4 * h], wh);
+#pragma unroll
+            for (int r = 1; r < 4; ++r) v[u][4 * h + r] = cmul(v[u][4 * h + r], cmul(wh, lo[r]));
+          }
+        } else {
+          double2 w[R];
+          twiddle_powers<R>(twd(tw, qb, sign), w);
+#pragma unroll
+          for (int r = 1; r < R; ++r) v[u][r] = cmul(v[u][r], w[r]);
+        }
+      }
+      dft_small<R>(v[u], sign);
+      const int d = (j - jm) * R + jm;
+#pragma unroll
+      for (int r = 0; r < R; ++r) buf[pidx(d + r * Ns) ^ xo] = v[u][r];
+    }
+  }
+  slice_sync<TP>(g);
+}
+
+// M-point transform of a slice, natural order in and out
+template <int M>
+__device__ __forceinline__ void slice_fft(double2* buf, int xo, const double2* __restrict__ tw, int tw_stride, int sign,
+                                          int tid, int g, bool act) {
+  if constexpr (M == 2048) {
+    slice_pass<M, 8>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 16>(buf, xo, 8, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 16>(buf, xo, 128, tw, tw_stride, sign, tid, g, act);
+  } else if constexpr (M == 1024) {
+    slice_pass<M, 8>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 8>(buf, xo, 8, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 16>(buf, xo, 64, tw, tw_stride, sign, tid, g, act);
+  } else if constexpr (M == 512) {
+    slice_pass<M, 8>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 8>(buf, xo, 8, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 8>(buf, xo, 64, tw, tw_stride, sign, tid, g, act);
+  } else if constexpr (M == 256) {
+    slice_pass<M, 16>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 16>(buf, xo, 16, tw, tw_stride, sign, tid, g, act);
+  } else if constexpr (M == 128) {
+    slice_pass<M, 8>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 16>(buf, xo, 8, tw, tw_stride, sign, tid, g, act);
+  } else {
+    static_assert(M == 64, "slices of 64 to 2048 points");
+    slice_pass<M, 8>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 8>(buf, xo, 8, tw, tw_stride, sign, tid, g, act);
+  }
+}
+
+// A member's two slices, M/16 of the CTA's M/8 threads each.  Sixteen points a thread:
+// three passes for 2048 points where eight points took four, and a barrier of one
+// slice's warps only; a slice of up to 512 points is one warp's.
+template <int M>
+__device__ __forceinline__ void local_fft2(double2* A, double2* B, const double2* __restrict__ tw, int tw_stride, int sign) {
+  constexpr int TP = M / 16;
+  const int g = threadIdx.x / TP;
+  slice_fft<M>(g ? B : A, 0, tw, tw_stride, sign, threadIdx.x % TP, g, true);
+  __syncthreads();
+}
+
+// One in-place Stockham radix-R pass of a single slice by all M/8 threads, eight points
+// each (half the threads, as in the pair, would leave the CTA's other warps idle).
 template <int M, int R>
 __device__ __forceinline__ void stockham_pass(double2* buf, int Ns, const double2* __restrict__ tw,
                                               int tw_stride, int sign) {
@@ -151,27 +285,21 @@ __device__ __forceinline__ void stockham_pass(double2* buf, int Ns, const double
   __syncthreads();
 }
 
-// Local M-point FFT, natural order in and out.
+// Local M-point transform of a single slice, natural order in and out: radix-8 passes
+// while they divide, then one radix-4 or radix-2 pass
 template <int M>
 __device__ __forceinline__ void local_fft(double2* buf, const double2* __restrict__ tw, int tw_stride, int sign) {
   int Ns = 1;
   constexpr int L8 = (M >= 512) ? 3 : (M >= 64 ? 2 : 1);
-  // radix-8 passes while they divide, then one radix-4 or radix-2 pass
   constexpr int rem = M / (1 << (3 * L8));
 #pragma unroll
   for (int p = 0; p < L8; ++p) {
     stockham_pass<M, 8>(buf, Ns, tw, tw_stride, sign);
     Ns *= 8;
   }
-  if constexpr (rem == 8) {
-    stockham_pass<M, 8>(buf, Ns, tw, tw_stride, sign);
-  } else if constexpr (rem == 4) {
-    stockham_pass<M, 4>(buf, Ns, tw, tw_stride, sign);
-  } else if constexpr (rem == 2) {
-    stockham_pass<M, 2>(buf, Ns, tw, tw_stride, sign);
-  }
+  if constexpr (rem == 4) stockham_pass<M, 4>(buf, Ns, tw, tw_stride, sign);
+  else if constexpr (rem == 2) stockham_pass<M, 2>(buf, Ns, tw, tw_stride, sign);
 }
-
 
 // Cross-CTA step of the distributed transform, as gather / C-point DFT / scatter:
 // the M positions of the slice are shared out over the C*T threads of the cluster;
@@ -318,70 +446,6 @@ namespace hwdev {
 // Dual transforms: two M-point slices (A and B) in one sweep -- twice the
 // independent work per thread, one set of twiddle loads and barriers for both.
 // ---------------------------------------------------------------------------
-template <int M, int R>
-__device__ __forceinline__ void stockham_pass2(double2* A, double2* B, int Ns, const double2* __restrict__ tw,
-                                               int tw_stride, int sign) {
-  constexpr int T = M / kPts;
-  constexpr int NB = M / R;
-  constexpr int BPT = kPts / R;
-  double2 va[BPT][R], vb[BPT][R];
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int u = 0; u < BPT; ++u) {
-    const int j = tid + u * T;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      va[u][r] = A[pidx(j + r * NB)];
-      vb[u][r] = B[pidx(j + r * NB)];
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < BPT; ++u) {
-    const int j = tid + u * T;
-    const int jm = j & (Ns - 1);
-    if (Ns > 1) {
-      const int qb = jm * (M / (Ns * R));
-      double2 w[R];
-      twiddle_powers<R>(twd(tw, qb * tw_stride, sign), w);
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        va[u][r] = cmul(va[u][r], w[r]);
-        vb[u][r] = cmul(vb[u][r], w[r]);
-      }
-    }
-    dft_small<R>(va[u], sign);
-    dft_small<R>(vb[u], sign);
-    const int idxD = (j - jm) * R + jm;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      A[pidx(idxD + r * Ns)] = va[u][r];
-      B[pidx(idxD + r * Ns)] = vb[u][r];
-    }
-  }
-  __syncthreads();
-}
-
-template <int M>
-__device__ __forceinline__ void local_fft2(double2* A, double2* B, const double2* __restrict__ tw, int tw_stride,
-                                           int sign) {
-  int Ns = 1;
-  constexpr int L8 = (M >= 512) ? 3 : (M >= 64 ? 2 : 1);
-  constexpr int rem = M / (1 << (3 * L8));
-#pragma unroll
-  for (int p = 0; p < L8; ++p) {
-    stockham_pass2<M, 8>(A, B, Ns, tw, tw_stride, sign);
-    Ns *= 8;
-  }
-  if constexpr (rem == 8) {
-    stockham_pass2<M, 8>(A, B, Ns, tw, tw_stride, sign);
-  } else if constexpr (rem == 4) {
-    stockham_pass2<M, 4>(A, B, Ns, tw, tw_stride, sign);
-  } else if constexpr (rem == 2) {
-    stockham_pass2<M, 2>(A, B, Ns, tw, tw_stride, sign);
-  }
-}
-
 // cross-CTA step of the distributed transform for both slices (see fft_forward /
 // fft_inverse): forward = C-point DFT then twiddle, inverse = twiddle then DFT.
 template <int M>

@@ -22,30 +22,32 @@ namespace hwdev {
 template <int M>
 __device__ __forceinline__ void evolve_member(DevMember* mems, int mi, int mode, DevMember& sd, Scratch<M>& sc,
                                               double2* smem_buf, int C, int rank) {
-  if (threadIdx.x == 0) sd = mems[mi];
+  if (threadIdx.x == 0) {
+    sd = mems[mi];
+    sc.bufs.y = sd.y;
+    sc.bufs.yn = sd.ynew;
+    for (int i = 0; i < 7; ++i) sc.bufs.k[i] = sd.kb[i];
+    sc.full = 0;
+  }
   // a cluster barrier, not only the CTA's: the RHS's first phase writes into the
   // partner CTA's shared memory, which must be running
   member_sync(C);
   Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);
-  Bufs B;
-  B.y = sd.y;
-  B.yn = sd.ynew;
-  for (int i = 0; i < 7; ++i) B.k[i] = sd.kb[i];
   spread_unmoved(X);
   StepState S{sd.t, sd.h, sd.status, sd.k1_valid, 0, 0, 0};
   int iout = sd.i_out;
   if (S.status == kOk) {
     if (mode == 1) {
-      evolve_apply<M>(X, B, S, sd.t1);
+      evolve_apply<M>(X, S, sd.t1);
     } else {
       while (iout < sd.i_stop && S.status == kOk) {
         const double ti = sd.tt[iout];
         while (S.t < ti && S.status == kOk) {
-          evolve_apply<M>(X, B, S, ti);
+          evolve_apply<M>(X, S, ti);
           if (S.rhs >= sd.rhs_budget && S.status == kOk) S.status = kBudget;   // bounded launch
         }
         if (S.status == kOk) {
-          if (sd.ngauge > 0 || sd.fields) output_stage<M>(X, B, S, iout);
+          if (sd.ngauge > 0 || sd.fields) output_stage<M>(X, S, iout);
           ++iout;
         }
       }
@@ -62,9 +64,9 @@ __device__ __forceinline__ void evolve_member(DevMember* mems, int mi, int mode,
     g.rhs_calls += S.rhs;
     g.accepted += S.acc;
     g.rejected += S.rej;
-    g.y = B.y;
-    g.ynew = B.yn;
-    for (int i = 0; i < 7; ++i) g.kb[i] = B.k[i];
+    g.y = sc.bufs.y;
+    g.ynew = sc.bufs.yn;
+    for (int i = 0; i < 7; ++i) g.kb[i] = sc.bufs.k[i];
   }
 }
 
@@ -111,10 +113,13 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs(DevMember* mems, c
   const int C = int(cl.num_blocks());
   const int rank = int(cl.block_rank());
   const int mi = list[blockIdx.x / C];
-  if (threadIdx.x == 0) sd = mems[mi];
+  if (threadIdx.x == 0) {
+    sd = mems[mi];
+    sc.stg.s = 0;
+    sc.full = 1;
+  }
   __syncthreads();
   Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);
-  X.full = true;
   rhs_eval<M>(X, t, sd.kb[6]);
   member_sync(C);
   if (rank == 0 && threadIdx.x == 0) mems[mi].rhs_calls += 1;

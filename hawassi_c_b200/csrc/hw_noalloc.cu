@@ -55,6 +55,8 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs_noalloc(DevMember*
     sd.zs = scratch;
     sd.kb[6] = scratch + 2 * N;
     for (int i = 0; i < kScratch; ++i) sd.sc[i] = scratch + size_t(4 + i) * N;
+    sc.stg.s = 0;
+    sc.full = 1;
   }
   __syncthreads();
   Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);
@@ -65,7 +67,6 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs_noalloc(DevMember*
     sd.zs[p] = make_double2(y_ref[kk], y_ref[N + kk]);
     sd.zs[N + p] = make_double2(y_ref[2 * N + kk], y_ref[3 * N + kk]);
   }
-  X.full = true;
   rhs_eval<M>(X, t, sd.kb[6]);
   HW_FOREACH(X) {
     const int kk = X.c + (idx << sd.logC);

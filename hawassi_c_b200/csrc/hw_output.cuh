@@ -29,8 +29,9 @@ __device__ __forceinline__ double2 phys_at(double2* buf, int C, int m) {
 }
 
 template <int M>
-__device__ __noinline__ void output_stage(Ctx<M>& X, Bufs& B, StepState& S, int row) {
+__device__ __noinline__ void output_stage(Ctx<M> X, StepState& S, int row) {
   const DevMember& d = X.d;
+  const Bufs& B = X.sc->bufs;
   const int N = d.N, C = d.C;
   // the derivative the reference's dy holds at this sample: the RHS it evaluated
   // last (the accepted step's dydt_out), zero before any RHS call
@@ -44,7 +45,7 @@ __device__ __noinline__ void output_stage(Ctx<M>& X, Bufs& B, StepState& S, int 
     dy = B.k[0];
   }
   double2* A = X.buf;
-  double2* Bf = X.buf2;
+  double2* Bf = X.buf2();
   HW_FOREACH(X) {
     A[pidx(idx)] = B.y[p];
     Bf[pidx(idx)] = none ? make_double2(0.0, 0.0) : dy[p];
@@ -80,7 +81,7 @@ __device__ __noinline__ void output_stage(Ctx<M>& X, Bufs& B, StepState& S, int 
     }
   }
   if (X.c == 0 && d.ngauge > 0) {
-    for (int g = X.tid; g < d.ngauge; g += Ctx<M>::T) {
+    for (int g = int(threadIdx.x); g < d.ngauge; g += Ctx<M>::T) {
       const int i = d.gidx[g];
       double ve = __longlong_as_double(0x7ff8000000000000ULL), vd = ve;
       if (i >= 0) {
@@ -155,9 +156,9 @@ __device__ __noinline__ void output_stage(Ctx<M>& X, Bufs& B, StepState& S, int 
       d.gout[(size_t)row * 2 * d.ngauge + g] = ve;
       d.gout[(size_t)row * 2 * d.ngauge + d.ngauge + g] = vd;
     }
-    if (X.tid == 0) d.gtim[row] = S.t;
+    if (int(threadIdx.x) == 0) d.gtim[row] = S.t;
   }
-  if (X.c == 0 && X.tid == 0 && d.ngauge == 0) d.gtim[row] = S.t;
+  if (X.c == 0 && int(threadIdx.x) == 0 && d.ngauge == 0) d.gtim[row] = S.t;
   member_sync(C);
   if (!fr) return;
   // u and phi = Re F^-1(-i u^ / k) (1d/functions.c:571-590: the k == 0 mode is zero)

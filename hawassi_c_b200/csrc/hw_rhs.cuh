@@ -28,7 +28,7 @@ __device__ constexpr double RK_ec5 = 1.0 / 50.0;
 __device__ constexpr double RK_ec6 = 2.0 / 55.0;
 
 // the stage input of an RK stage: zs = y + h sum_j b_sj k_j (s = 2..6), or zs = y
-// itself (s = 1: the state a first or last derivative is evaluated at)
+// itself (s = 1: the state a first or last derivative is evaluated at; s = 0: zs holds it)
 struct StageSrc {
   const double2* y;
   const double2* k[5];
@@ -78,29 +78,38 @@ struct StageOps {
   }
 };
 
-template <int M>
-struct Ctx {
-  static constexpr int T = M / kPts;
-  const DevMember& d;
-  double2* buf;   // M-point FFT slice (padded) in shared memory
-  double2* buf2;  // second slice for the dual transforms
-  double* red;    // reduction scratch in shared memory (kRed doubles)
-  unsigned short* cand;   // grid points of this CTA's threads above the breaking threshold
-  int* ncand;
-  int c;          // rank of this CTA in the member's cluster
-  int tid;
-  const StageSrc* stg = nullptr;   // set: zs is to be formed from y and the k's first
-  bool full = false;               // dz is written outside the alias band too (as zeros)
+// the stepper's buffers: y, ynew, k1..k6, kout (accepted steps swap pointers)
+struct Bufs {
+  double2* y;
+  double2* yn;
+  double2* k[7];
 };
 
-// scratch of one CTA in static shared memory, beside the transform slices
+// Scratch of one CTA in static shared memory, beside the transform slices.  What every
+// thread needs alike (the stage description, the buffers) stands here once, and not in
+// each thread's local memory: with 256 threads and kilobyte frames that overflows the L1
+// cache, and every access to it waited for L2.
 constexpr int kRed = 48;
 constexpr int kRedPv = 40, kRedPs = 41;   // influx signals at the stage time
 template <int M>
 struct Scratch {
   double red[kRed];
+  StageSrc stg;         // stage input of the coming RHS (stg.s = 0: zs holds it)
+  Bufs bufs;
+  int full;             // dz is written outside the alias band too (as zeros)
   int ncand;
-  unsigned short cand[M];
+  unsigned short cand[M];   // grid points of this CTA's threads above the breaking threshold
+};
+
+// what a device function of the member is given, by value (a few registers)
+template <int M>
+struct Ctx {
+  static constexpr int T = M / kPts;
+  const DevMember& d;
+  double2* buf;   // M-point transform slice in shared memory; the second one follows it
+  Scratch<M>* sc;
+  int c;          // rank of this CTA in the member's cluster
+  __device__ __forceinline__ double2* buf2() const { return buf + padded(M); }
 };
 
 // The Hermitian pairs {k, N-k} of the member, each owned by one thread wherever spectral
@@ -130,16 +139,16 @@ __host__ __device__ constexpr size_t slice_smem_bytes(int m) { return 2 * size_t
 
 template <int M>
 __device__ __forceinline__ Ctx<M> make_ctx(const DevMember& d, double2* smem, Scratch<M>& sc, int rank) {
-  return Ctx<M>{d, smem, smem + padded(M), sc.red, sc.cand, &sc.ncand, rank, int(threadIdx.x)};
+  return Ctx<M>{d, smem, &sc, rank};
 }
 
 #define HW_FOREACH(X)                            \
   _Pragma("unroll") for (int u = 0; u < kPts; ++u)  \
-    if (const int idx = (X).tid + u * Ctx<M>::T, p = (X).c * M + idx; true)
+    if (const int idx = int(threadIdx.x) + u * Ctx<M>::T, p = (X).c * M + idx; true)
 
 // permuted position of the wavenumber N - kk, for the spectral entry at slice index idx
 template <int M>
-__device__ __forceinline__ int partner_pos(const Ctx<M>& X, int idx) {
+__device__ __forceinline__ int partner_pos(Ctx<M> X, int idx) {
   const DevMember& d = X.d;
   const int kk = X.c + (idx << d.logC);
   const int kp = (d.N - kk) & (d.N - 1);
@@ -170,7 +179,7 @@ __device__ __forceinline__ double2 mul_ik(double a, double2 b) {
 // forward FFT of the physical slice in buf, then f(u, idx, p, Z, Zpartner) for each
 // of this thread's spectral points (Zpartner read from the owning CTA by DSMEM)
 template <int M, class F>
-__device__ __forceinline__ void fft_forward_split(Ctx<M>& X, F&& f) {
+__device__ __forceinline__ void fft_forward_split(Ctx<M> X, F&& f) {
   const DevMember& d = X.d;
   fft_forward<M>(X.buf, d.tw, d.N, d.C, X.c);
   const double2* pb = X.buf;
@@ -192,7 +201,7 @@ __device__ __forceinline__ void fft_forward_split(Ctx<M>& X, F&& f) {
 
 // inverse FFT of the spectral slice in buf; g(u, idx, p, v) for each physical point
 template <int M, class G>
-__device__ __forceinline__ void fft_inverse_then(Ctx<M>& X, G&& g) {
+__device__ __forceinline__ void fft_inverse_then(Ctx<M> X, G&& g) {
   const DevMember& d = X.d;
   fft_inverse<M>(X.buf, d.tw, d.N, d.C, X.c);
   HW_FOREACH(X) { g(u, idx, p, X.buf[pidx(idx)]); }
@@ -228,22 +237,22 @@ __device__ __forceinline__ double2 influx_at(const DevMember& d, double t) {
 
 // breaking hooks (implemented in hw_breaking.cuh)
 template <int M>
-__device__ __forceinline__ void breaking_reset(Ctx<M>& X);
+__device__ __forceinline__ void breaking_reset(Ctx<M> X);
 template <int M>
-__device__ __forceinline__ void breaking_scan(Ctx<M>& X, const double2* PE, const double* Heta, int hs);
+__device__ __forceinline__ void breaking_scan(Ctx<M> X, const double2* PE, const double* Heta, int hs);
 template <int M>
-__device__ __forceinline__ void breaking_lead(Ctx<M>& X, double t, const double2* PE, const double* Heta, int hs);
+__device__ __forceinline__ void breaking_lead(Ctx<M> X, double t, const double2* PE, const double* Heta, int hs);
 template <int M>
-__device__ __noinline__ void breaking_force(Ctx<M>& X, const double2* PE, const double2* AEadj, double2* Rb);
+__device__ __noinline__ void breaking_force(Ctx<M> X, const double2* PE, const double2* AEadj, double2* Rb);
 // HS2 on a flat bottom (hw_rhs_fast.cuh) and every other right-hand side (hw_rhs_gen.cuh)
 template <int M>
-__device__ __noinline__ void rhs_hs2_flat(Ctx<M>& X, double t, double2* __restrict__ dz);
+__device__ __noinline__ void rhs_hs2_flat(Ctx<M> X, double t, double2* __restrict__ dz);
 template <int M>
-__device__ __noinline__ void rhs_gen(Ctx<M>& X, double t, double2* __restrict__ dz);
+__device__ __noinline__ void rhs_gen(Ctx<M> X, double t, double2* __restrict__ dz);
 
 // One RHS evaluation dz = f(t, zs), zs = [eta^ | u^] (permuted spectral, 2N).
 template <int M>
-__device__ __forceinline__ void rhs_eval(Ctx<M>& X, double t, double2* __restrict__ dz) {
+__device__ __forceinline__ void rhs_eval(Ctx<M> X, double t, double2* __restrict__ dz) {
   if (X.d.model == 2 && X.d.flat) rhs_hs2_flat<M>(X, t, dz);
   else rhs_gen<M>(X, t, dz);
 }

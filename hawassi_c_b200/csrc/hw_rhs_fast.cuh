@@ -31,14 +31,14 @@ template <int M>
 struct PairBufs {
   double2 *Aq, *Bq;
   int cq;
-  __device__ __forceinline__ PairBufs(Ctx<M>& X) {
+  __device__ __forceinline__ explicit PairBufs(Ctx<M> X) {
     cq = (X.d.C - X.c) & (X.d.C - 1);
     Aq = X.buf;
-    Bq = X.buf2;
+    Bq = X.buf2();
     if (cq != X.c) {
       cg::cluster_group cl = cg::this_cluster();
       Aq = cl.map_shared_rank(X.buf, cq);
-      Bq = cl.map_shared_rank(X.buf2, cq);
+      Bq = cl.map_shared_rank(X.buf2(), cq);
     }
   }
 };
@@ -47,7 +47,7 @@ struct PairBufs {
 // not necessarily Hermitian): (herm x + i herm y) / N, real parts only as the reference
 __device__ __forceinline__ void emit_pair(double2* A, double2* Aq, const PairAt& r, double2 x, double2 xp, double2 y,
                                           double2 yp, double invN) {
-  if (r.self) {
+  if (r.self) {   // (one thread of a member)
     A[pidx(r.i)] = pack(herm(x, x), herm(y, y), invN);
     A[pidx(r.j)] = pack(herm(xp, xp), herm(yp, yp), invN);
   } else {
@@ -73,39 +73,46 @@ enum : int { kWithM0Hilbert = 0, kWithM0Dx = 1, kWithRefs = 2, kWithNone = 3 };
 // bottom M0 u^ = -i c1 u^, and the Hilbert multiplier takes the sign of c1 = (C^2/g) k.
 // The stage is a template argument so that a pair's loads (up to 24) are independent
 // of any branch and in flight together.
-template <int M, int S>
-__device__ __noinline__ void stage_pack(Ctx<M>& X, int with) {
+template <int M, int S, int WITH>
+__device__ __noinline__ void stage_pack(Ctx<M> X) {
   const DevMember& d = X.d;
   constexpr int T = Ctx<M>::T;
-  const double2* y = X.stg->y;
+  const double2* y = X.sc->stg.y;
   const double2* ks[S > 1 ? S - 1 : 1];
 #pragma unroll
-  for (int j = 0; j < S - 1; ++j) ks[j] = X.stg->k[j];
-  const double h = X.stg->h, invN = d.invN;
+  for (int j = 0; j < S - 1; ++j) ks[j] = X.sc->stg.k[j];
+  const double h = X.sc->stg.h, invN = d.invN;
   const int N = d.N, c = X.c, act = d.act;
-  const double* __restrict__ t1 = with == kWithRefs ? d.Csq : d.c1;
-  const double* __restrict__ t2 = with == kWithRefs ? d.Csq + N : d.k;
+  const double* __restrict__ t1 = WITH == kWithRefs ? d.Csq : d.c1;
+  const double* __restrict__ t2 = WITH == kWithRefs ? d.Csq + N : d.k;
   double2* zw = d.zs;
   const bool brk = d.brk != 0;
   const PairBufs<M> pb(X);
-  double2 *A = X.buf, *B = X.buf2, *Aq = pb.Aq, *Bq = pb.Bq;
+  double2 *A = X.buf, *B = X.buf2(), *Aq = pb.Aq, *Bq = pb.Bq;
   auto emit = [&](const PairAt& r, double a, double aq, double b, double bq, double2 e, double2 ep, double2 w, double2 wp) {
     emit_pair(A, Aq, r, e, ep, w, wp, invN);
-    if (with == kWithM0Hilbert) {
-      emit_pair(B, Bq, r, cmi(a, w), cmi(aq, wp), brk ? hilbert_hat(a, e) : czero(), brk ? hilbert_hat(aq, ep) : czero(),
-                invN);
-    } else if (with == kWithM0Dx) {
+    if constexpr (WITH == kWithM0Hilbert) {
+      double2 s = czero(), sp = czero();
+      if (brk) {
+        s = hilbert_hat(a, e);
+        sp = hilbert_hat(aq, ep);
+      }
+      emit_pair(B, Bq, r, cmi(a, w), cmi(aq, wp), s, sp, invN);
+    } else if constexpr (WITH == kWithM0Dx) {
       emit_pair(B, Bq, r, cmi(a, w), cmi(aq, wp), cmi(-b, w), cmi(-bq, wp), invN);
-    } else if (with == kWithRefs) {
+    } else if constexpr (WITH == kWithRefs) {
       emit_pair(B, Bq, r, cscale(w, a), cscale(wp, aq), cscale(w, b), cscale(wp, bq), invN);
     }
   };
 #pragma unroll 1
   for (int u = 0; u < kPts / 2; ++u) {
-    const PairAt r = pair_at<M>(c, pb.cq, X.tid + u * T);
-    const double a = t1[r.p], aq = t1[r.pp];
-    double b = 0.0, bq = 0.0;
-    if (with != kWithM0Hilbert) {
+    const PairAt r = pair_at<M>(c, pb.cq, int(threadIdx.x) + u * T);
+    double a = 0.0, aq = 0.0, b = 0.0, bq = 0.0;
+    if constexpr (WITH != kWithNone) {
+      a = t1[r.p];
+      aq = t1[r.pp];
+    }
+    if constexpr (WITH == kWithM0Dx || WITH == kWithRefs) {
       b = t2[r.p];
       bq = t2[r.pp];
     }
@@ -131,25 +138,24 @@ __device__ __noinline__ void stage_pack(Ctx<M>& X, int with) {
 
 // the stage phase with its barriers.  Every RHS leaves the slices unread by the other
 // CTAs (a barrier follows its last partner reads), so they can be written at once; with
-// zs written by the caller, other threads' writes of it and the start of the partner
-// CTA come first.
-template <int M>
-__device__ __forceinline__ void stage_phase(Ctx<M>& X, int with) {
-  if (X.stg) {
-    switch (X.stg->s) {
-      case 1: stage_pack<M, 1>(X, with); break;
-      case 2: stage_pack<M, 2>(X, with); break;
-      case 3: stage_pack<M, 3>(X, with); break;
-      case 4: stage_pack<M, 4>(X, with); break;
-      case 5: stage_pack<M, 5>(X, with); break;
-      default: stage_pack<M, 6>(X, with); break;
-    }
-  } else {
+// zs written by the caller (stage 0), other threads' writes of it and the start of the
+// partner CTA come first.
+template <int M, int WITH>
+__device__ __forceinline__ void stage_phase(Ctx<M> X) {
+  __syncthreads();   // the stage description
+  const int stage = X.sc->stg.s;
+  if (stage == 0) {
     member_sync(X.d.C);
-    const StageSrc own{X.d.zs, {nullptr, nullptr, nullptr, nullptr, nullptr}, 1, 0.0};
-    X.stg = &own;
-    stage_pack<M, 1>(X, with);
-    X.stg = nullptr;
+    if (threadIdx.x == 0) X.sc->stg.y = X.d.zs;
+    __syncthreads();
+  }
+  switch (stage) {
+    case 2: stage_pack<M, 2, WITH>(X); break;
+    case 3: stage_pack<M, 3, WITH>(X); break;
+    case 4: stage_pack<M, 4, WITH>(X); break;
+    case 5: stage_pack<M, 5, WITH>(X); break;
+    case 6: stage_pack<M, 6, WITH>(X); break;
+    default: stage_pack<M, 1, WITH>(X); break;
   }
   if (X.d.C > 1) cg::this_cluster().sync();   // the partners' slices are written
 }
@@ -170,19 +176,38 @@ __device__ __forceinline__ double2 source_term(int mode, double2 gx, double2 gs,
 // forward C-point DFT, twiddle, scatter.  Two cluster barriers replace four and the
 // physical fields never pass through shared memory.
 
+// The twiddles are formed anew on each side: kept across the pointwise work they took
+// the registers that its loads need.
+template <int C>
+__device__ __forceinline__ void cross_in(double2* v, const double2* __restrict__ tw, int i) {
+  double2 w[C > 1 ? C : 2];
+  twiddle_powers<C>(twd(tw, i, +1), w);
+#pragma unroll
+  for (int r = 1; r < C; ++r) v[r] = cmul(v[r], w[r]);
+  dft_small<C>(v, +1);
+}
+template <int C>
+__device__ __forceinline__ void cross_out(double2* v, const double2* __restrict__ tw, int i) {
+  double2 w[C > 1 ? C : 2];
+  dft_small<C>(v, -1);
+  twiddle_powers<C>(twd(tw, i, -1), w);
+#pragma unroll
+  for (int r = 1; r < C; ++r) v[r] = cmul(v[r], w[r]);
+}
+
 // What the first meeting does at physical point n (1d/functions.c:1486-1498), given
 // e = (eta, u), m = (M0 u, H(eta)): a <- (eta u) + i (eta M0 u), b <- u^2 - (M0 u)^2.
 // (eta, u) goes to global memory where the damping zones read it back, and with
 // breaking everywhere, beside H(eta) and a list of the points above the threshold.
 template <int M>
-__device__ __forceinline__ void product_point(Ctx<M>& X, int n, double2 e, double2 m, double damp, double2* PE,
+__device__ __forceinline__ void product_point(Ctx<M> X, int n, double2 e, double2 m, double damp, double2* PE,
                                               double2* PM, double2& a, double2& b) {
   const DevMember& d = X.d;
   if (d.brk) {
     PE[n] = e;
     PM[n].y = m.y;
     if (n >= d.xbstart && n < d.xbstart + d.lenIF && !(e.x < d.MaxEtaInit))
-      X.cand[atomicAdd(X.ncand, 1)] = (unsigned short)n;
+      X.sc->cand[atomicAdd(&X.sc->ncand, 1)] = (unsigned short)n;
   } else if (damp != 0.0) {
     PE[n] = e;
   }
@@ -202,7 +227,7 @@ __device__ __forceinline__ void adjust_point(const double2* PE, int n, double ch
 }
 
 template <int M, int C>
-__device__ __forceinline__ void cross_products(Ctx<M>& X, double2* A, double2* B, double2* PE, double2* PM) {
+__device__ __forceinline__ void cross_products(Ctx<M> X, double2* A, double2* B, double2* PE, double2* PM) {
   constexpr int T = M / kPts;
   constexpr int PER = kPts / C;
   const DevMember& d = X.d;
@@ -210,8 +235,8 @@ __device__ __forceinline__ void cross_products(Ctx<M>& X, double2* A, double2* B
   cl.sync();
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
-    const int i = X.c * T + X.tid + q * (C * T);
-    double2 va[C], vb[C], w[C > 1 ? C : 2];
+    const int i = X.c * T + int(threadIdx.x) + q * (C * T);
+    double2 va[C], vb[C];
     double dm[C];
 #pragma unroll
     for (int r = 0; r < C; ++r) {
@@ -219,23 +244,12 @@ __device__ __forceinline__ void cross_products(Ctx<M>& X, double2* A, double2* B
       vb[r] = cl.map_shared_rank(B, r)[pidx(i)];
       dm[r] = __ldg(d.damp + r * M + i);
     }
-    twiddle_powers<C>(twd(d.tw, i, +1), w);
-#pragma unroll
-    for (int r = 1; r < C; ++r) {
-      va[r] = cmul(va[r], w[r]);
-      vb[r] = cmul(vb[r], w[r]);
-    }
-    dft_small<C>(va, +1);
-    dft_small<C>(vb, +1);
+    cross_in<C>(va, d.tw, i);
+    cross_in<C>(vb, d.tw, i);
 #pragma unroll
     for (int r = 0; r < C; ++r) product_point<M>(X, r * M + i, va[r], vb[r], dm[r], PE, PM, va[r], vb[r]);
-    dft_small<C>(va, -1);
-    dft_small<C>(vb, -1);
-#pragma unroll
-    for (int r = 1; r < C; ++r) {
-      va[r] = cmul(va[r], cconj(w[r]));
-      vb[r] = cmul(vb[r], cconj(w[r]));
-    }
+    cross_out<C>(va, d.tw, i);
+    cross_out<C>(vb, d.tw, i);
 #pragma unroll
     for (int r = 0; r < C; ++r) {
       cl.map_shared_rank(A, r)[pidx(i)] = va[r];
@@ -246,7 +260,7 @@ __device__ __forceinline__ void cross_products(Ctx<M>& X, double2* A, double2* B
 }
 
 template <int M, int C>
-__device__ __forceinline__ void cross_adjust(Ctx<M>& X, double2* A, double2* B, const double2* PE) {
+__device__ __forceinline__ void cross_adjust(Ctx<M> X, double2* A, double2* B, const double2* PE) {
   constexpr int T = M / kPts;
   constexpr int PER = kPts / C;
   const DevMember& d = X.d;
@@ -254,8 +268,8 @@ __device__ __forceinline__ void cross_adjust(Ctx<M>& X, double2* A, double2* B, 
   cl.sync();
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
-    const int i = X.c * T + X.tid + q * (C * T);
-    double2 va[C], vb[C], w[C > 1 ? C : 2];
+    const int i = X.c * T + int(threadIdx.x) + q * (C * T);
+    double2 va[C], vb[C];
     double dm[C], ch[C];
 #pragma unroll
     for (int r = 0; r < C; ++r) {
@@ -263,19 +277,11 @@ __device__ __forceinline__ void cross_adjust(Ctx<M>& X, double2* A, double2* B, 
       dm[r] = __ldg(d.damp + r * M + i);
       ch[r] = __ldg(d.chi + r * M + i);
     }
-    twiddle_powers<C>(twd(d.tw, i, +1), w);
-#pragma unroll
-    for (int r = 1; r < C; ++r) va[r] = cmul(va[r], w[r]);
-    dft_small<C>(va, +1);
+    cross_in<C>(va, d.tw, i);
 #pragma unroll
     for (int r = 0; r < C; ++r) adjust_point(PE, r * M + i, ch[r], dm[r], va[r], vb[r]);
-    dft_small<C>(va, -1);
-    dft_small<C>(vb, -1);
-#pragma unroll
-    for (int r = 1; r < C; ++r) {
-      va[r] = cmul(va[r], cconj(w[r]));
-      vb[r] = cmul(vb[r], cconj(w[r]));
-    }
+    cross_out<C>(va, d.tw, i);
+    cross_out<C>(vb, d.tw, i);
 #pragma unroll
     for (int r = 0; r < C; ++r) {
       cl.map_shared_rank(A, r)[pidx(i)] = va[r];
@@ -286,13 +292,13 @@ __device__ __forceinline__ void cross_adjust(Ctx<M>& X, double2* A, double2* B, 
 }
 
 template <int M>
-__device__ __forceinline__ void cross_products_any(Ctx<M>& X, double2* A, double2* B, double2* PE, double2* PM) {
+__device__ __forceinline__ void cross_products_any(Ctx<M> X, double2* A, double2* B, double2* PE, double2* PM) {
   if (X.d.C == 2) cross_products<M, 2>(X, A, B, PE, PM);
   else if (X.d.C == 4) cross_products<M, 4>(X, A, B, PE, PM);
   else cross_products<M, 8>(X, A, B, PE, PM);
 }
 template <int M>
-__device__ __forceinline__ void cross_adjust_any(Ctx<M>& X, double2* A, double2* B, const double2* PE) {
+__device__ __forceinline__ void cross_adjust_any(Ctx<M> X, double2* A, double2* B, const double2* PE) {
   if (X.d.C == 2) cross_adjust<M, 2>(X, A, B, PE);
   else if (X.d.C == 4) cross_adjust<M, 4>(X, A, B, PE);
   else cross_adjust<M, 8>(X, A, B, PE);
@@ -306,26 +312,26 @@ __device__ __forceinline__ void cross_adjust_any(Ctx<M>& X, double2* A, double2*
 // there are none (HS1; damping from A).
 enum : int { kAsmSlices = 0, kAsmLive = 1, kAsmLinear = 2 };
 template <int M, int MODE, bool VAR>
-__device__ __noinline__ void assemble(Ctx<M>& X, double2* __restrict__ dz, const double2* M0h, const double2* AE,
+__device__ __noinline__ void assemble(Ctx<M> X, double2* __restrict__ dz, const double2* M0h, const double2* AE,
                                       const double2* AU, const double2* RB) {
   const DevMember& d = X.d;
   constexpr int T = Ctx<M>::T;
   const int N = d.N, c = X.c, act = d.act, mode = d.has_influx ? d.prop_mode : 3;
   const PairBufs<M> pb(X);
   const double2 *A = X.buf, *Aq = pb.Aq;
-  const double2 *B = MODE == kAsmLinear ? X.buf : X.buf2, *Bq = MODE == kAsmLinear ? pb.Aq : pb.Bq;
+  const double2 *B = MODE == kAsmLinear ? X.buf : X.buf2(), *Bq = MODE == kAsmLinear ? pb.Aq : pb.Bq;
   const double2* zs = d.zs;
   const double* __restrict__ kt = d.k;
   const double* __restrict__ c1t = d.c1;
   const double* __restrict__ aalt = d.aal;
   const double2* __restrict__ gxt = d.gamX;
   const double2* __restrict__ gst = d.gamXs;
-  const double pv = X.red[kRedPv], ps = X.red[kRedPs];
+  const double pv = X.sc->red[kRedPv], ps = X.sc->red[kRedPs];
 #pragma unroll 1
   for (int u = 0; u < kPts / 2; ++u) {
-    const PairAt r = pair_at<M>(c, pb.cq, X.tid + u * T);
+    const PairAt r = pair_at<M>(c, pb.cq, int(threadIdx.x) + u * T);
     if (r.i >= act) {
-      if (X.full) dz[r.p] = dz[r.pp] = dz[N + r.p] = dz[N + r.pp] = czero();
+      if (X.sc->full) dz[r.p] = dz[r.pp] = dz[N + r.p] = dz[N + r.pp] = czero();
       continue;
     }
     const int pos[2] = {r.p, r.pp};
@@ -372,24 +378,24 @@ __device__ __noinline__ void assemble(Ctx<M>& X, double2* __restrict__ dz, const
 // beside the last spectral phase: the breaking machine's leader and, by another thread,
 // the influx signals at the stage time (read after the phase's barrier)
 template <int M>
-__device__ __forceinline__ void lead_and_influx(Ctx<M>& X, double t, const double2* PE, const double* Heta) {
+__device__ __forceinline__ void lead_and_influx(Ctx<M> X, double t, const double2* PE, const double* Heta) {
   if (X.d.brk) breaking_lead(X, t, PE, Heta, 2);
-  if (X.d.has_influx && X.tid == Ctx<M>::T - 1) {
+  if (X.d.has_influx && int(threadIdx.x) == Ctx<M>::T - 1) {
     const double2 s = influx_at(X.d, t);
-    X.red[kRedPv] = s.x;
-    X.red[kRedPs] = s.y;
+    X.sc->red[kRedPv] = s.x;
+    X.sc->red[kRedPs] = s.y;
   }
 }
 
 // From the packed nonlinear terms in slice A to dz: the nonlinear adjustment with the
 // damping, the breaking force where some node breaks, the assembly.
 template <int M>
-__device__ __noinline__ void finish_rhs(Ctx<M>& X, double2* __restrict__ dz, const double2* M0h) {
+__device__ __noinline__ void finish_rhs(Ctx<M> X, double2* __restrict__ dz, const double2* M0h) {
   const DevMember& d = X.d;
   constexpr int T = Ctx<M>::T;
   const int C = d.C;
   double2* A = X.buf;
-  double2* Bf = X.buf2;
+  double2* Bf = X.buf2();
   const double2* PE = d.sc[0];
   if (C == 2 || C == 4 || C == 8) {
     fft_local<M>(A, d.tw, C, +1);
@@ -426,7 +432,7 @@ __device__ __noinline__ void finish_rhs(Ctx<M>& X, double2* __restrict__ dz, con
   const PairBufs<M> pb(X);
 #pragma unroll 1
   for (int u = 0; u < kPts / 2; ++u) {
-    const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
+    const PairAt r = pair_at<M>(X.c, pb.cq, int(threadIdx.x) + u * T);
     const double2 z = A[pidx(r.i)], zp = pb.Aq[pidx(r.j)];
     AE[r.p] = split_re(z, r.self ? z : zp);
     AU[r.p] = split_im(z, r.self ? z : zp);
@@ -442,12 +448,12 @@ __device__ __noinline__ void finish_rhs(Ctx<M>& X, double2* __restrict__ dz, con
 }
 
 template <int M>
-__device__ __noinline__ void rhs_hs2_flat(Ctx<M>& X, double t, double2* __restrict__ dz) {
+__device__ __noinline__ void rhs_hs2_flat(Ctx<M> X, double t, double2* __restrict__ dz) {
   const DevMember& d = X.d;
   constexpr int T = Ctx<M>::T;
   const int C = d.C;
   double2* A = X.buf;
-  double2* Bf = X.buf2;
+  double2* Bf = X.buf2();
   double2* PE = d.sc[0];   // physical (eta, u)           [breaking, and in the damping zones]
   double2* PM = d.sc[1];   // physical (., Hilbert eta)   [breaking only]
   const bool brk = d.brk != 0;
@@ -455,8 +461,8 @@ __device__ __noinline__ void rhs_hs2_flat(Ctx<M>& X, double t, double2* __restri
 
   // (0)-(1) stage input and its packing
   if (brk) breaking_reset(X);
-  if (X.tid == 0) *X.ncand = 0;
-  stage_phase(X, kWithM0Hilbert);
+  if (int(threadIdx.x) == 0) X.sc->ncand = 0;
+  stage_phase<M, kWithM0Hilbert>(X);
   // (2) products in physical space (1d/functions.c:1486-1498)
   const bool fused = C == 2 || C == 4 || C == 8;
   if (fused) {
@@ -492,27 +498,36 @@ __device__ __noinline__ void rhs_hs2_flat(Ctx<M>& X, double t, double2* __restri
     double kk[kPts], cc[kPts];
 #pragma unroll
     for (int u = 0; u < kPts / 2; ++u) {
-      const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
+      const PairAt r = pair_at<M>(X.c, pb.cq, int(threadIdx.x) + u * T);
       kk[2 * u] = kt[r.p];
       kk[2 * u + 1] = kt[r.pp];
       cc[2 * u] = c1t[r.p];
       cc[2 * u + 1] = c1t[r.pp];
     }
+    // -L (eta M0u)^ - i k (eta u)^ and -i k (u^2 - (M0u)^2)^ / 2 at one point
+    auto terms = [&](double k, double c1, double2 a, double2 ap, double2 b, double2 bp, double2& te, double2& tu) {
+      const double2 ah = split_re(a, ap), bh = split_im(a, ap), ch = split_re(b, bp);
+      const double L = k * c1;
+      te = make_double2(-L * bh.x + k * ah.y, -L * bh.y - k * ah.x);
+      tu = make_double2(0.5 * k * ch.y, -0.5 * k * ch.x);
+    };
 #pragma unroll
     for (int u = 0; u < kPts / 2; ++u) {
-      const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
+      const PairAt r = pair_at<M>(X.c, pb.cq, int(threadIdx.x) + u * T);
       const double2 z1 = A[pidx(r.i)], z1p = pb.Aq[pidx(r.j)], z2 = Bf[pidx(r.i)], z2p = pb.Bq[pidx(r.j)];
-      // -L (eta M0u)^ - i k (eta u)^ and -i k (u^2 - (M0u)^2)^ / 2 at one point
-      auto terms = [&](double k, double c1, double2 a, double2 ap, double2 b, double2 bp, double2& te, double2& tu) {
-        const double2 ah = split_re(a, ap), bh = split_im(a, ap), ch = split_re(b, bp);
-        const double L = k * c1;
-        te = make_double2(-L * bh.x + k * ah.y, -L * bh.y - k * ah.x);
-        tu = make_double2(0.5 * k * ch.y, -0.5 * k * ch.x);
-      };
       double2 te, tu, teq, tuq;
-      terms(kk[2 * u], cc[2 * u], z1, r.self ? z1 : z1p, z2, r.self ? z2 : z2p, te, tu);
-      terms(kk[2 * u + 1], cc[2 * u + 1], z1p, r.self ? z1p : z1, z2p, r.self ? z2p : z2, teq, tuq);
-      emit_pair(A, pb.Aq, r, te, teq, tu, tuq, invN);
+      if (u == 0 && r.self) {
+        terms(kk[0], cc[0], z1, z1, z2, z2, te, tu);
+        terms(kk[1], cc[1], z1p, z1p, z2p, z2p, teq, tuq);
+        A[pidx(r.i)] = pack(herm(te, te), herm(tu, tu), invN);
+        A[pidx(r.j)] = pack(herm(teq, teq), herm(tuq, tuq), invN);
+        continue;
+      }
+      terms(kk[2 * u], cc[2 * u], z1, z1p, z2, z2p, te, tu);
+      terms(kk[2 * u + 1], cc[2 * u + 1], z1p, z1, z2p, z2, teq, tuq);
+      const double2 E = herm(te, teq), U = herm(tu, tuq);
+      A[pidx(r.i)] = pack(E, U, invN);
+      pb.Aq[pidx(r.j)] = pack_conj(E, U, invN);
     }
   }
   lead_and_influx(X, t, PE, &PM[0].y);

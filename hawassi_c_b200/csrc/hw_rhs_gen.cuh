@@ -21,8 +21,6 @@
 // global scratch, each read and written by the one thread that owns the point or pair.
 #pragma once
 
-#include <type_traits>
-
 #include "hw_rhs_fast.cuh"
 
 namespace hwdev {
@@ -32,45 +30,32 @@ namespace hwdev {
 // turns the transformed values into the next ones; two points' loads are in flight
 // together.  The meeting of cross-CTA steps is cross_products'.
 template <int M, int C, class Op>
-__device__ __forceinline__ void meet_cross(Ctx<M>& X, int nin, int nout, const Op& op) {
+__device__ __forceinline__ void meet_cross(Ctx<M> X, int nin, int nout, const Op& op) {
   constexpr int T = M / kPts;
   constexpr int PER = kPts / C;
   const DevMember& d = X.d;
-  double2 *A = X.buf, *B = X.buf2;
+  double2 *A = X.buf, *B = X.buf2();
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
 #pragma unroll 1
   for (int q = 0; q < PER; ++q) {
-    const int i = X.c * T + X.tid + q * (C * T);
-    double2 va[C], vb[C], w[C > 1 ? C : 2];
+    const int i = X.c * T + int(threadIdx.x) + q * (C * T);
+    double2 va[C], vb[C];
 #pragma unroll
     for (int r = 0; r < C; ++r) {
       va[r] = cl.map_shared_rank(A, r)[pidx(i)];
       vb[r] = nin == 2 ? cl.map_shared_rank(B, r)[pidx(i)] : czero();
     }
-    twiddle_powers<C>(twd(d.tw, i, +1), w);
-#pragma unroll
-    for (int r = 1; r < C; ++r) va[r] = cmul(va[r], w[r]);
-    dft_small<C>(va, +1);
-    if (nin == 2) {
-#pragma unroll
-      for (int r = 1; r < C; ++r) vb[r] = cmul(vb[r], w[r]);
-      dft_small<C>(vb, +1);
-    }
+    cross_in<C>(va, d.tw, i);
+    if (nin == 2) cross_in<C>(vb, d.tw, i);
 #pragma unroll
     for (int r = 0; r < C; r += 2) {
       const typename Op::L l0 = op.load(r * M + i), l1 = op.load((r + 1) * M + i);
       op(r * M + i, l0, va[r], vb[r]);
       op((r + 1) * M + i, l1, va[r + 1], vb[r + 1]);
     }
-    dft_small<C>(va, -1);
-#pragma unroll
-    for (int r = 1; r < C; ++r) va[r] = cmul(va[r], cconj(w[r]));
-    if (nout == 2) {
-      dft_small<C>(vb, -1);
-#pragma unroll
-      for (int r = 1; r < C; ++r) vb[r] = cmul(vb[r], cconj(w[r]));
-    }
+    cross_out<C>(va, d.tw, i);
+    if (nout == 2) cross_out<C>(vb, d.tw, i);
 #pragma unroll
     for (int r = 0; r < C; ++r) {
       cl.map_shared_rank(A, r)[pidx(i)] = va[r];
@@ -80,41 +65,63 @@ __device__ __forceinline__ void meet_cross(Ctx<M>& X, int nin, int nout, const O
   cl.sync();
 }
 
+// (op is made here, between the transforms' calls, from the member's description and the
+// iteration: its fields stay in registers)
 template <int M, class Op>
-__device__ __noinline__ void meet(Ctx<M>& X, int nin, int nout, const Op& op) {
+__device__ __noinline__ void meet(Ctx<M> X, int nin, int nout, int it) {
   const DevMember& d = X.d;
   const int C = d.C;
-  double2 *A = X.buf, *B = X.buf2;
   if (C == 2 || C == 4 || C == 8) {
-    if (nin == 2) fft_local2<M>(A, B, d.tw, C, +1);
-    else fft_local<M>(A, d.tw, C, +1);
-    if (C == 2) meet_cross<M, 2>(X, nin, nout, op);
-    else if (C == 4) meet_cross<M, 4>(X, nin, nout, op);
-    else meet_cross<M, 8>(X, nin, nout, op);
-    if (nout == 2) fft_local2<M>(A, B, d.tw, C, -1);
-    else fft_local<M>(A, d.tw, C, -1);
+    if (nin == 2) fft_local2<M>(X.buf, X.buf2(), d.tw, C, +1);
+    else fft_local<M>(X.buf, d.tw, C, +1);
+    if (C == 2) meet_cross<M, 2>(X, nin, nout, Op(X, it));
+    else if (C == 4) meet_cross<M, 4>(X, nin, nout, Op(X, it));
+    else meet_cross<M, 8>(X, nin, nout, Op(X, it));
+    if (nout == 2) fft_local2<M>(X.buf, X.buf2(), d.tw, C, -1);
+    else fft_local<M>(X.buf, d.tw, C, -1);
     return;
   }
-  if (nin == 2) fft_inverse2<M>(A, B, d.tw, d.N, C, X.c);
-  else fft_inverse<M>(A, d.tw, d.N, C, X.c);
+  if (nin == 2) fft_inverse2<M>(X.buf, X.buf2(), d.tw, d.N, C, X.c);
+  else fft_inverse<M>(X.buf, d.tw, d.N, C, X.c);
+  {
+    const Op op(X, it);
+    double2 *A = X.buf, *B = X.buf2();
 #pragma unroll 1
-  for (int u = 0; u < kPts; u += 2) {
-    const int i0 = X.tid + u * Ctx<M>::T, i1 = i0 + Ctx<M>::T, n0 = X.c * M + i0, n1 = X.c * M + i1;
-    const typename Op::L l0 = op.load(n0), l1 = op.load(n1);
-    double2 a0 = A[pidx(i0)], a1 = A[pidx(i1)];
-    double2 b0 = nin == 2 ? B[pidx(i0)] : czero(), b1 = nin == 2 ? B[pidx(i1)] : czero();
-    op(n0, l0, a0, b0);
-    op(n1, l1, a1, b1);
-    A[pidx(i0)] = a0;
-    A[pidx(i1)] = a1;
-    if (nout == 2) {
-      B[pidx(i0)] = b0;
-      B[pidx(i1)] = b1;
+    for (int u = 0; u < kPts; u += 2) {
+      const int i0 = int(threadIdx.x) + u * Ctx<M>::T, i1 = i0 + Ctx<M>::T, n0 = X.c * M + i0, n1 = X.c * M + i1;
+      const typename Op::L l0 = op.load(n0), l1 = op.load(n1);
+      double2 a0 = A[pidx(i0)], a1 = A[pidx(i1)];
+      double2 b0 = nin == 2 ? B[pidx(i0)] : czero(), b1 = nin == 2 ? B[pidx(i1)] : czero();
+      op(n0, l0, a0, b0);
+      op(n1, l1, a1, b1);
+      A[pidx(i0)] = a0;
+      A[pidx(i1)] = a1;
+      if (nout == 2) {
+        B[pidx(i0)] = b0;
+        B[pidx(i1)] = b1;
+      }
     }
   }
-  if (nout == 2) fft_forward2<M>(A, B, d.tw, d.N, C, X.c);
-  else fft_forward<M>(A, d.tw, d.N, C, X.c);
+  if (nout == 2) fft_forward2<M>(X.buf, X.buf2(), d.tw, d.N, C, X.c);
+  else fft_forward<M>(X.buf, d.tw, d.N, C, X.c);
 }
+
+// How K reference depths fill a sweep's iterations.  First sweep: fields in 0 eta, 1 u, then
+// the images; out gam_j u, and at index `at`, once the last image is in, the sum.  The others:
+// in one pair, then four images to an iteration; out three products, gam_j q, the sum.
+struct Plan {
+  int at, nit;
+};
+__device__ __forceinline__ Plan first_plan(int K) {
+  const int at = K % 4 == 3 ? K + 1 : K;
+  return Plan{at, at / 4 + 1};
+}
+__device__ __forceinline__ Plan rest_plan(int K) {
+  const int nimg = (K + 3) / 4, at = K > 0 ? (3 + K > 4 * nimg ? 3 + K : 4 * nimg) : 3;
+  return Plan{at, at / 4 + 1};
+}
+template <int M>
+__device__ __forceinline__ int refs(const Ctx<M>& X) { return X.d.flat ? 0 : X.d.nref; }
 
 // point n above the breaking threshold inside the window: listed for the criterion
 template <int M>
@@ -124,8 +131,8 @@ struct Listing {
   unsigned short* cand;
   int* ncand;
   __device__ __forceinline__ explicit Listing(const Ctx<M>& X)
-      : w0(X.d.xbstart), w1(X.d.brk ? X.d.xbstart + X.d.lenIF : X.d.xbstart), thr(X.d.MaxEtaInit), cand(X.cand),
-        ncand(X.ncand) {}
+      : w0(X.d.xbstart), w1(X.d.brk ? X.d.xbstart + X.d.lenIF : X.d.xbstart), thr(X.d.MaxEtaInit), cand(X.sc->cand),
+        ncand(&X.sc->ncand) {}
   __device__ __forceinline__ void operator()(int n, double e) const {
     if (n >= w0 && n < w1 && !(e < thr)) cand[atomicAdd(ncand, 1)] = (unsigned short)n;
   }
@@ -135,6 +142,7 @@ struct Listing {
 template <int M>
 struct OpLinear {
   const double* __restrict__ damp;
+  __device__ __forceinline__ OpLinear(Ctx<M> X, int) : damp(X.d.damp) {}
   struct L { double dm; };
   __device__ __forceinline__ L load(int n) const { return L{__ldg(damp + n)}; }
   __device__ __forceinline__ void operator()(int, const L& l, double2& a, double2&) const {
@@ -152,6 +160,9 @@ struct OpFirst {
   double* S;
   int N, K, it, at, more;
   Listing<M> list;
+  __device__ __forceinline__ OpFirst(Ctx<M> X, int it_)
+      : gam(X.d.gam), PE(X.d.sc[0]), S(reinterpret_cast<double*>(X.d.sc[5])), N(X.d.N), K(X.d.nref), it(it_),
+        at(first_plan(X.d.nref).at), more(it_ + 1 < first_plan(X.d.nref).nit), list(X) {}
   struct L { double u, s, g[6]; };   // g[m]: gam of reference 4 it - 2 + m
   __device__ __forceinline__ L load(int n) const {
     L l;
@@ -199,6 +210,10 @@ struct OpRest {
   double* S;
   int N, K, it, at, more, start;
   Listing<M> list;
+  __device__ __forceinline__ OpRest(Ctx<M> X, int it_)
+      : gam(X.d.gam), PE(X.d.sc[0]), PM(X.d.sc[1]), PA(X.d.sc[7]), S(reinterpret_cast<double*>(X.d.sc[5])), N(X.d.N),
+        K(refs(X)), it(it_), at(rest_plan(refs(X)).at), more(it_ + 1 < rest_plan(refs(X)).nit),
+        start(!CUBIC && refs(X) == 0 && it_ == 0), list(X) {}
   struct L { double2 e, m; double lm, s, g[5]; };   // g[m]: gam of reference 4 it - 4 + m
   __device__ __forceinline__ L load(int n) const {
     L l;
@@ -297,201 +312,221 @@ __device__ __forceinline__ void emit_refs(double2* A, double2* Aq, double2* B, d
   if (n == 2) emit_pair(B, Bq, r, cscale(a, t.c[2]), cscale(ap, t.cq[2]), cscale(a, t.c[3]), cscale(ap, t.cq[3]), invN);
 }
 
+// Spectral side of the first sweep's iteration `it`: the pair's owner adds its part of the
+// sum and forms the next input in place, at the end M0 u^ with H(eta) or d_x u.
 template <int M>
-__device__ __noinline__ void rhs_gen(Ctx<M>& X, double t, double2* __restrict__ dz) {
+__device__ __noinline__ void first_spectral(Ctx<M> X, int it, int nout) {
   const DevMember& d = X.d;
   constexpr int T = Ctx<M>::T;
-  const int N = d.N, C = d.C, K = d.flat ? 0 : d.nref;
+  const int N = d.N, K = d.nref, at = first_plan(K).at, last = it + 1 == first_plan(K).nit;
   const bool hs3 = d.model == 3, brk = d.brk != 0;
   const double invN = d.invN;
-  double2* PE = d.sc[0];    // physical (eta, u)
-  double2* PM = d.sc[1];    // physical (M0 u, Hilbert eta | d_x u)
-  double2* AE = d.sc[2];    // spectral eta-equation nonlinear terms
-  double2* AU = d.sc[3];    // spectral u-equation nonlinear terms
-  double2* acc = d.sc[4];   // spectral sum of an HSS
-  double* S = reinterpret_cast<double*>(d.sc[5]);   // physical sum of an HSS
-  double2* M0h = K > 0 ? d.sc[6] : nullptr;         // M0 u^ = delta H1 of eta (varying bottom)
-  double2* PA = d.sc[7];    // physical (L eta M0 u, Hilbert eta)
-  double2* Q = d.sc[10];    // spectrum of the HSS's operand
+  double2 *acc = d.sc[4], *M0h = d.sc[6];
   const double2 *ZE = d.zs, *ZU = d.zs + N;
+  const double* __restrict__ kt = d.k;
+  const PairBufs<M> pb(X);
+  double2 *A = X.buf, *B = X.buf2();
+  const int nnext = K + 2 - 4 * (it + 1) > 2 ? 2 : 1;
+#pragma unroll 1
+  for (int u = 0; u < kPts / 2; ++u) {
+    const PairAt r = pair_at<M>(X.c, pb.cq, int(threadIdx.x) + u * T);
+    RefRows back, next;
+    back.load(d.Csq, N, K, 4 * it, r);
+    back.add_sum(at - 4 * it);
+    double2 s = czero(), sq = czero();
+    if (it > 0) {
+      s = acc[r.p];
+      sq = acc[r.pp];
+    }
+    // the next input's operands: u^ again, or (last) eta^ and u^ with k
+    const double2 w = ZU[r.p], wp = ZU[r.pp], e = ZE[r.p], ep = ZE[r.pp];
+    const double k = kt[r.p], kq = kt[r.pp];
+    if (!last) next.load(d.Csq, N, K, 4 * it + 2, r);
+    const double2 y = nout == 2 ? B[pidx(r.i)] : czero(), yp = nout == 2 ? pb.Bq[pidx(r.j)] : czero();
+    const Four F(r, A[pidx(r.i)], pb.Aq[pidx(r.j)], y, yp);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      s = cadd(s, cscale(F.f[i], back.c[i]));
+      sq = cadd(sq, cscale(F.g[i], back.cq[i]));
+    }
+    if (!last) {
+      acc[r.p] = s;
+      acc[r.pp] = sq;
+      emit_refs(A, pb.Aq, B, pb.Bq, r, next, nnext, w, wp, invN);
+    } else {
+      // M0 u^ = -i k HSS / g
+      const double2 m = cmi(0.5 / kG * k, s), mq = cmi(0.5 / kG * kq, sq);
+      M0h[r.p] = m;
+      M0h[r.pp] = mq;
+      double2 h = czero(), hq = czero();
+      if (hs3) {
+        h = cmi(-k, w);
+        hq = cmi(-kq, wp);
+      } else if (brk) {
+        h = hilbert_hat(k, e);
+        hq = hilbert_hat(kq, ep);
+      }
+      emit_pair(A, pb.Aq, r, m, mq, h, hq, invN);
+    }
+  }
+}
+
+// Spectral side of a later sweep's iteration (see OpRest): the model's terms in iteration 0,
+// the sum, and at the end L q^ into the terms and the next input (the nonlinear adjustment's,
+// or, under HS3 after the second-order sweep, L (eta M0 u)^ with H(eta)).
+template <int M, bool CUBIC>
+__device__ __noinline__ void rest_spectral(Ctx<M> X, int it, int nout) {
+  const DevMember& d = X.d;
+  constexpr int T = Ctx<M>::T;
+  const int N = d.N, K = refs(X), at = rest_plan(K).at, last = it + 1 == rest_plan(K).nit;
+  const bool hs3 = d.model == 3, brk = d.brk != 0, final_sweep = CUBIC || !hs3;
+  const double invN = d.invN;
+  double2 *AE = d.sc[2], *AU = d.sc[3], *acc = d.sc[4], *Q = d.sc[10];
+  const double2* ZE = d.zs;
   const double* __restrict__ kt = d.k;
   const double* __restrict__ c1t = d.c1;
   const PairBufs<M> pb(X);
-  double2 *A = X.buf, *B = X.buf2;
+  double2 *A = X.buf, *B = X.buf2();
+  const int nnext = K - 4 * it > 2 ? 2 : 1;
+#pragma unroll 1
+  for (int u = 0; u < kPts / 2; ++u) {
+    const PairAt r = pair_at<M>(X.c, pb.cq, int(threadIdx.x) + u * T);
+    RefRows back, next;
+    back.load(d.Csq, N, K, 4 * it - 3, r);
+    if (K > 0) back.add_sum(at - 4 * it);
+    double2 s = czero(), sq = czero(), q = czero(), qq = czero(), ae = czero(), aeq = czero(), au = czero(),
+            auq = czero(), e = czero(), ep = czero();
+    if (it > 0) {
+      s = acc[r.p];
+      sq = acc[r.pp];
+      q = Q[r.p];
+      qq = Q[r.pp];
+    }
+    const double k = kt[r.p], kq = kt[r.pp];
+    const double L = K > 0 ? 0.5 / kG * (k * k) : k * c1t[r.p], Lq = K > 0 ? 0.5 / kG * (kq * kq) : kq * c1t[r.pp];
+    if (CUBIC || it > 0) {
+      ae = AE[r.p];
+      aeq = AE[r.pp];
+      au = AU[r.p];
+      auq = AU[r.pp];
+    }
+    if (!CUBIC && hs3 && brk && last) {
+      e = ZE[r.p];
+      ep = ZE[r.pp];
+    }
+    if (!last) next.load(d.Csq, N, K, 4 * it, r);
+    const double2 y = nout == 2 ? B[pidx(r.i)] : czero(), yp = nout == 2 ? pb.Bq[pidx(r.j)] : czero();
+    const Four F(r, A[pidx(r.i)], pb.Aq[pidx(r.j)], y, yp);
+    if (it == 0) {
+      if (CUBIC) {
+        // D3, F3: -k^2 D3^ / 2 and -i k F3^
+        ae = make_double2(ae.x - 0.5 * (k * k) * F.f[0].x, ae.y - 0.5 * (k * k) * F.f[0].y);
+        aeq = make_double2(aeq.x - 0.5 * (kq * kq) * F.g[0].x, aeq.y - 0.5 * (kq * kq) * F.g[0].y);
+        au = cadd(au, cmi(k, F.f[1]));
+        auq = cadd(auq, cmi(kq, F.g[1]));
+      } else {
+        // -i k (eta u)^ and -i k (u^2 - (M0 u)^2)^ / 2
+        ae = cmi(k, F.f[0]);
+        aeq = cmi(kq, F.g[0]);
+        au = cmi(0.5 * k, F.f[2]);
+        auq = cmi(0.5 * kq, F.g[2]);
+      }
+      q = CUBIC ? F.f[2] : F.f[1];
+      qq = CUBIC ? F.g[2] : F.g[1];
+      if (!last) {
+        Q[r.p] = q;
+        Q[r.pp] = qq;
+      }
+      if (K > 0) {
+        s = cscale(F.f[3], back.c[3]);
+        sq = cscale(F.g[3], back.cq[3]);
+      } else {   // flat: the operator's multiplier is the table's
+        s = q;
+        sq = qq;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        s = cadd(s, cscale(F.f[i], back.c[i]));
+        sq = cadd(sq, cscale(F.g[i], back.cq[i]));
+      }
+    }
+    if (last) {
+      // L q^ = k^2 HSS / g: minus L (eta M0 u)^, or plus L (A3 + B3 / 2)^
+      const double2 l = cscale(s, L), lq = cscale(sq, Lq);
+      ae = CUBIC ? cadd(ae, l) : csub(ae, l);
+      aeq = CUBIC ? cadd(aeq, lq) : csub(aeq, lq);
+      if (final_sweep) {
+        emit_pair(A, pb.Aq, r, ae, aeq, au, auq, invN);   // into the nonlinear adjustment
+      } else {
+        emit_pair(A, pb.Aq, r, l, lq, brk ? hilbert_hat(k, e) : czero(), brk ? hilbert_hat(kq, ep) : czero(), invN);
+      }
+    } else {
+      acc[r.p] = s;
+      acc[r.pp] = sq;
+      emit_refs(A, pb.Aq, B, pb.Bq, r, next, nnext, q, qq, invN);
+    }
+    if (it == 0 || (last && !final_sweep)) {
+      AE[r.p] = ae;
+      AE[r.pp] = aeq;
+      AU[r.p] = au;
+      AU[r.pp] = auq;
+    }
+  }
+}
 
-  if (brk) breaking_reset(X);
-  if (X.tid == 0) *X.ncand = 0;
-  if (d.model == 1) {
-    stage_phase(X, kWithNone);
-    meet<M>(X, 1, 1, OpLinear<M>{d.damp});
-    lead_and_influx(X, t, PE, &PM[0].y);
+template <int M, bool CUBIC>
+__device__ __forceinline__ void rest_sweep(Ctx<M> X, double t) {
+  const int nit = rest_plan(refs(X)).nit;
+  const bool final_sweep = CUBIC || X.d.model != 3;
+  for (int it = 0; it < nit; ++it) {
+    const int K = refs(X), nout = rest_plan(K).at + 1 - 4 * it > 2 ? 2 : 1;
+    const int nin = it == 0 ? (!CUBIC && K == 0 ? 2 : 1) : (K - 4 * (it - 1) > 2 ? 2 : 1);
+    meet<M, OpRest<M, CUBIC>>(X, nin, nout, it);
+    // breaking criterion on eta, u, H(eta), complete member-wide by now
+    const bool done = final_sweep && it + 1 == nit;
+    const double* Heta = X.d.model == 3 ? &X.d.sc[7][0].y : &X.d.sc[1][0].y;
+    if (X.d.brk && done) breaking_scan(X, X.d.sc[0], Heta, 2);
+    member_sync(X.d.C);
+    rest_spectral<M, CUBIC>(X, it, nout);
+    if (done) lead_and_influx(X, t, X.d.sc[0], Heta);
+    if (X.d.C > 1) cg::this_cluster().sync();
+  }
+}
+
+// Scratch fields: sc[0] eta, u in physical space; sc[1] M0 u with H(eta) or d_x u; sc[2], sc[3]
+// spectral terms; sc[4] spectral and sc[5] physical sum of an HSS; sc[6] M0 u^; sc[7] L (eta M0 u)
+// with H(eta); sc[10] the operand's spectrum.
+template <int M>
+__device__ __noinline__ void rhs_gen(Ctx<M> X, double t, double2* __restrict__ dz) {
+  const int C = X.d.C;
+  if (X.d.brk) breaking_reset(X);
+  if (threadIdx.x == 0) X.sc->ncand = 0;
+  if (X.d.model == 1) {
+    stage_phase<M, kWithNone>(X);
+    meet<M, OpLinear<M>>(X, 1, 1, 0);
+    lead_and_influx(X, t, nullptr, nullptr);
     member_sync(C);
     assemble<M, kAsmLinear, false>(X, dz, nullptr, nullptr, nullptr, nullptr);
     member_sync(C);
     return;
   }
-  stage_phase(X, K > 0 ? kWithRefs : kWithM0Dx);
-  if (K > 0) {
-    const int at = K % 4 == 3 ? K + 1 : K, nit = at / 4 + 1;
+  if (X.d.flat) {
+    stage_phase<M, kWithM0Dx>(X);
+  } else {
+    stage_phase<M, kWithRefs>(X);
+    const int nit = first_plan(X.d.nref).nit;
     for (int it = 0; it < nit; ++it) {
-      const int nin = K + 2 - 4 * it > 2 ? 2 : 1, nout = at + 1 - 4 * it > 2 ? 2 : 1, last = it == nit - 1;
-      meet<M>(X, nin, nout, OpFirst<M>{d.gam, PE, S, N, K, it, at, !last, Listing<M>(X)});
+      const int K = X.d.nref, nin = K + 2 - 4 * it > 2 ? 2 : 1, nout = first_plan(K).at + 1 - 4 * it > 2 ? 2 : 1;
+      meet<M, OpFirst<M>>(X, nin, nout, it);
       member_sync(C);
-      const int nnext = K + 2 - 4 * (it + 1) > 2 ? 2 : 1;
-#pragma unroll 1
-      for (int u = 0; u < kPts / 2; ++u) {
-        const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
-        RefRows back, next;
-        back.load(d.Csq, N, K, 4 * it, r);
-        back.add_sum(at - 4 * it);
-        double2 s = czero(), sq = czero();
-        if (it > 0) {
-          s = acc[r.p];
-          sq = acc[r.pp];
-        }
-        // the next input's operands: u^ again, or (last) eta^ and u^ with k
-        const double2 w = ZU[r.p], wp = ZU[r.pp], e = ZE[r.p], ep = ZE[r.pp];
-        const double k = kt[r.p], kq = kt[r.pp];
-        if (!last) next.load(d.Csq, N, K, 4 * it + 2, r);
-        const double2 y = nout == 2 ? B[pidx(r.i)] : czero(), yp = nout == 2 ? pb.Bq[pidx(r.j)] : czero();
-        const Four F(r, A[pidx(r.i)], pb.Aq[pidx(r.j)], y, yp);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          s = cadd(s, cscale(F.f[i], back.c[i]));
-          sq = cadd(sq, cscale(F.g[i], back.cq[i]));
-        }
-        if (!last) {
-          acc[r.p] = s;
-          acc[r.pp] = sq;
-          emit_refs(A, pb.Aq, B, pb.Bq, r, next, nnext, w, wp, invN);
-        } else {
-          // M0 u^ = -i k HSS / g
-          const double2 m = cmi(0.5 / kG * k, s), mq = cmi(0.5 / kG * kq, sq);
-          M0h[r.p] = m;
-          M0h[r.pp] = mq;
-          double2 h = czero(), hq = czero();
-          if (hs3) {
-            h = cmi(-k, w);
-            hq = cmi(-kq, wp);
-          } else if (brk) {
-            h = hilbert_hat(k, e);
-            hq = hilbert_hat(kq, ep);
-          }
-          emit_pair(A, pb.Aq, r, m, mq, h, hq, invN);
-        }
-      }
+      first_spectral(X, it, nout);
       if (C > 1) cg::this_cluster().sync();
     }
   }
-  // images come from iteration 1 on, four to an iteration; the sum goes back with the
-  // last of them, or after the last gam_j q
-  const int nimg = (K + 3) / 4;
-  const int at = K > 0 ? (3 + K > 4 * nimg ? 3 + K : 4 * nimg) : 3, nit = at / 4 + 1;
-  auto sweep = [&](auto cubic) {
-    constexpr bool CUBIC = decltype(cubic)::value;
-    const bool final_sweep = CUBIC || !hs3;
-    for (int it = 0; it < nit; ++it) {
-      const int start = !CUBIC && K == 0 && it == 0, last = it == nit - 1;
-      const int nin = it == 0 ? (start ? 2 : 1) : (K - 4 * (it - 1) > 2 ? 2 : 1);
-      const int nout = at + 1 - 4 * it > 2 ? 2 : 1;
-      meet<M>(X, nin, nout, OpRest<M, CUBIC>{d.gam, PE, PM, PA, S, N, K, it, at, !last, start, Listing<M>(X)});
-      // breaking criterion on eta, u, H(eta), complete member-wide by now
-      const double* Heta = hs3 ? &PA[0].y : &PM[0].y;
-      if (brk && final_sweep && last) breaking_scan(X, PE, Heta, 2);
-      member_sync(C);
-      const int nnext = K - 4 * it > 2 ? 2 : 1;
-#pragma unroll 1
-      for (int u = 0; u < kPts / 2; ++u) {
-        const PairAt r = pair_at<M>(X.c, pb.cq, X.tid + u * T);
-        RefRows back, next;
-        back.load(d.Csq, N, K, 4 * it - 3, r);
-        if (K > 0) back.add_sum(at - 4 * it);
-        double2 s = czero(), sq = czero(), q = czero(), qq = czero(), ae = czero(), aeq = czero(), au = czero(),
-                auq = czero(), e = czero(), ep = czero();
-        if (it > 0) {
-          s = acc[r.p];
-          sq = acc[r.pp];
-          q = Q[r.p];
-          qq = Q[r.pp];
-        }
-        const double k = kt[r.p], kq = kt[r.pp];
-        const double L = K > 0 ? 0.5 / kG * (k * k) : k * c1t[r.p], Lq = K > 0 ? 0.5 / kG * (kq * kq) : kq * c1t[r.pp];
-        if (CUBIC || it > 0) {
-          ae = AE[r.p];
-          aeq = AE[r.pp];
-          au = AU[r.p];
-          auq = AU[r.pp];
-        }
-        if (!CUBIC && hs3 && brk && last) {
-          e = ZE[r.p];
-          ep = ZE[r.pp];
-        }
-        if (!last) next.load(d.Csq, N, K, 4 * it, r);
-        const double2 y = nout == 2 ? B[pidx(r.i)] : czero(), yp = nout == 2 ? pb.Bq[pidx(r.j)] : czero();
-        const Four F(r, A[pidx(r.i)], pb.Aq[pidx(r.j)], y, yp);
-        if (it == 0) {
-          if (CUBIC) {
-            // D3, F3: -k^2 D3^ / 2 and -i k F3^
-            ae = make_double2(ae.x - 0.5 * (k * k) * F.f[0].x, ae.y - 0.5 * (k * k) * F.f[0].y);
-            aeq = make_double2(aeq.x - 0.5 * (kq * kq) * F.g[0].x, aeq.y - 0.5 * (kq * kq) * F.g[0].y);
-            au = cadd(au, cmi(k, F.f[1]));
-            auq = cadd(auq, cmi(kq, F.g[1]));
-          } else {
-            // -i k (eta u)^ and -i k (u^2 - (M0 u)^2)^ / 2
-            ae = cmi(k, F.f[0]);
-            aeq = cmi(kq, F.g[0]);
-            au = cmi(0.5 * k, F.f[2]);
-            auq = cmi(0.5 * kq, F.g[2]);
-          }
-          q = CUBIC ? F.f[2] : F.f[1];
-          qq = CUBIC ? F.g[2] : F.g[1];
-          if (!last) {
-            Q[r.p] = q;
-            Q[r.pp] = qq;
-          }
-          if (K > 0) {
-            s = cscale(F.f[3], back.c[3]);
-            sq = cscale(F.g[3], back.cq[3]);
-          } else {   // flat: the operator's multiplier is the table's
-            s = q;
-            sq = qq;
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            s = cadd(s, cscale(F.f[i], back.c[i]));
-            sq = cadd(sq, cscale(F.g[i], back.cq[i]));
-          }
-        }
-        if (last) {
-          // L q^ = k^2 HSS / g: minus L (eta M0 u)^, or plus L (A3 + B3 / 2)^
-          const double2 l = cscale(s, L), lq = cscale(sq, Lq);
-          ae = CUBIC ? cadd(ae, l) : csub(ae, l);
-          aeq = CUBIC ? cadd(aeq, lq) : csub(aeq, lq);
-          if (final_sweep) {
-            emit_pair(A, pb.Aq, r, ae, aeq, au, auq, invN);   // into the nonlinear adjustment
-          } else {
-            emit_pair(A, pb.Aq, r, l, lq, brk ? hilbert_hat(k, e) : czero(), brk ? hilbert_hat(kq, ep) : czero(), invN);
-          }
-        } else {
-          acc[r.p] = s;
-          acc[r.pp] = sq;
-          emit_refs(A, pb.Aq, B, pb.Bq, r, next, nnext, q, qq, invN);
-        }
-        if (it == 0 || (last && !final_sweep)) {
-          AE[r.p] = ae;
-          AE[r.pp] = aeq;
-          AU[r.p] = au;
-          AU[r.pp] = auq;
-        }
-      }
-      if (final_sweep && last) lead_and_influx(X, t, PE, Heta);
-      if (C > 1) cg::this_cluster().sync();
-    }
-  };
-  sweep(std::false_type{});
-  if (hs3) sweep(std::true_type{});
-  finish_rhs(X, dz, M0h);
+  rest_sweep<M, false>(X, t);
+  if (X.d.model == 3) rest_sweep<M, true>(X, t);
+  finish_rhs(X, dz, X.d.flat ? nullptr : X.d.sc[6]);
 }
 
 }  // namespace hwdev

@@ -11,30 +11,24 @@
 
 namespace hwdev {
 
-struct Bufs {
-  double2* y;
-  double2* yn;
-  double2* k[7];   // k1..k6, kout
-};
-
 // max over the member (all CTAs of the cluster); identical result in every thread
 template <int M>
-__device__ __forceinline__ double member_max(Ctx<M>& X, double v) {
+__device__ __forceinline__ double member_max(Ctx<M> X, double v) {
   const DevMember& d = X.d;
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int w = X.tid >> 5;
+  const int w = int(threadIdx.x) >> 5;
   constexpr int NW = Ctx<M>::T / 32;
   __syncthreads();
-  if ((X.tid & 31) == 0) X.red[w] = v;
+  if ((int(threadIdx.x) & 31) == 0) X.sc->red[w] = v;
   __syncthreads();
-  double m = X.red[0];
-  for (int i = 1; i < NW; ++i) m = fmax(m, X.red[i]);
+  double m = X.sc->red[0];
+  for (int i = 1; i < NW; ++i) m = fmax(m, X.sc->red[i]);
   if (d.C > 1) {
     cg::cluster_group cl = cg::this_cluster();
-    if (X.tid == 0) X.red[NW] = m;
+    if (int(threadIdx.x) == 0) X.sc->red[NW] = m;
     cl.sync();
-    m = *cl.map_shared_rank(X.red + NW, 0);
-    for (int r = 1; r < d.C; ++r) m = fmax(m, *cl.map_shared_rank(X.red + NW, r));
+    m = *cl.map_shared_rank(X.sc->red + NW, 0);
+    for (int r = 1; r < d.C; ++r) m = fmax(m, *cl.map_shared_rank(X.sc->red + NW, r));
     cl.sync();
   }
   return m;
@@ -45,8 +39,9 @@ __device__ __forceinline__ double member_max(Ctx<M>& X, double v) {
 // zero, so ynew = y there (both buffers hold it since the launch began) and yerr = 0.
 // A thread keeps the numerator and denominator of its largest ratio and divides once.
 template <int M>
-__device__ __noinline__ double final_combine(Ctx<M>& X, const Bufs& B, double h) {
+__device__ __noinline__ double final_combine(Ctx<M> X, double h) {
   const DevMember& d = X.d;
+  const Bufs& B = X.sc->bufs;
   constexpr int T = Ctx<M>::T;
   const double2* __restrict__ ys = B.y;
   const double2* __restrict__ k1 = B.k[0];
@@ -75,7 +70,7 @@ __device__ __noinline__ double final_combine(Ctx<M>& X, const Bufs& B, double h)
   };
 #pragma unroll 1
   for (int u = 0; u < kPts / 2; ++u) {
-    const PairAt r = pair_at<M>(X.c, cq, X.tid + u * T);
+    const PairAt r = pair_at<M>(X.c, cq, int(threadIdx.x) + u * T);
     if (r.i >= act) continue;
 #pragma unroll 1
     for (int off = 0; off <= N; off += N) {
@@ -94,11 +89,11 @@ __device__ __noinline__ double final_combine(Ctx<M>& X, const Bufs& B, double h)
 // Outside the alias band every k_i is zero and the state stays what it is: the second
 // state buffer and the stage input take those points once, when a launch begins.
 template <int M>
-__device__ __forceinline__ void spread_unmoved(Ctx<M>& X) {
+__device__ __forceinline__ void spread_unmoved(Ctx<M> X) {
   const DevMember& d = X.d;
   const int cq = (d.C - X.c) & (d.C - 1);
   for (int u = 0; u < kPts / 2; ++u) {
-    const PairAt r = pair_at<M>(X.c, cq, X.tid + u * Ctx<M>::T);
+    const PairAt r = pair_at<M>(X.c, cq, int(threadIdx.x) + u * Ctx<M>::T);
     if (r.i < d.act) continue;
     for (int off = 0; off <= d.N; off += d.N) {
       d.ynew[r.p + off] = d.zs[r.p + off] = d.y[r.p + off];
@@ -113,25 +108,29 @@ struct StepState {
   long long rhs, acc, rej;
 };
 
+// stage s of a step of size h as the coming RHS's input: y + h sum_j b_sj k_j, or (s = 1)
+// the state y itself; the RHS's first barrier makes it known
 template <int M>
-__device__ __forceinline__ void rhs_into(Ctx<M>& X, StepState& S, double t, double2* out) {
-  rhs_eval<M>(X, t, out);
-  ++S.rhs;
+__device__ __forceinline__ void set_stage(Ctx<M> X, const double2* y, int s, double h) {
+  if (threadIdx.x == 0) {
+    const Bufs& B = X.sc->bufs;
+    X.sc->stg = StageSrc{y, {B.k[0], B.k[1], B.k[2], B.k[3], B.k[4]}, s, h};
+  }
 }
 
 // one RHS evaluation at the state src itself (the RHS copies it into zs)
 template <int M>
-__device__ __forceinline__ void rhs_at(Ctx<M>& X, StepState& S, double t, const double2* src, double2* out) {
-  const StageSrc st{src, {nullptr, nullptr, nullptr, nullptr, nullptr}, 1, 0.0};
-  X.stg = &st;
-  rhs_into(X, S, t, out);
-  X.stg = nullptr;
+__device__ __forceinline__ void rhs_at(Ctx<M> X, StepState& S, double t, const double2* src, double2* out) {
+  set_stage(X, src, 1, 0.0);
+  rhs_eval<M>(X, t, out);
+  ++S.rhs;
 }
 
 // gsl_odeiv_evolve_apply with rkf45 and control_y, one member
 template <int M>
-__device__ __noinline__ void evolve_apply(Ctx<M>& X, Bufs& B, StepState& S, double t1) {
+__device__ __noinline__ void evolve_apply(Ctx<M> X, StepState& S, double t1) {
   const DevMember& d = X.d;
+  Bufs& B = X.sc->bufs;
   const double t0 = S.t;
   double h0 = S.h;
   const double dt = t1 - t0;
@@ -143,13 +142,12 @@ __device__ __noinline__ void evolve_apply(Ctx<M>& X, Bufs& B, StepState& S, doub
     if ((dt >= 0.0 && h0 > dt) || (dt < 0.0 && h0 < dt)) { h0 = dt; final_step = true; }
     for (int s = 2; s <= 6; ++s) {
       // the RHS forms its own stage input from y and the k's (into zs as well)
-      const StageSrc st{B.y, {B.k[0], B.k[1], B.k[2], B.k[3], B.k[4]}, s, h0};
-      X.stg = &st;
-      rhs_into(X, S, t0 + RK_ah[s - 2] * h0, B.k[s - 1]);
-      X.stg = nullptr;
+      set_stage(X, B.y, s, h0);
+      rhs_eval<M>(X, t0 + RK_ah[s - 2] * h0, B.k[s - 1]);
+      ++S.rhs;
     }
     member_sync(d.C);
-    const double rmax = final_combine(X, B, h0);
+    const double rmax = final_combine(X, h0);
     if (d.exact) rhs_at(X, S, t0 + h0, B.yn, B.k[6]);
     const double tn = final_step ? t1 : t0 + h0;
     // std_control_hadjust (order 5)
@@ -186,7 +184,6 @@ __device__ __noinline__ void evolve_apply(Ctx<M>& X, Bufs& B, StepState& S, doub
       const double tk = t0 + h0;
       if (tk == tn) {
         rhs_at(X, S, tk, B.yn, B.k[6]);
-        double2* tmp = B.k[0]; B.k[0] = B.k[6]; B.k[6] = tmp;
         S.k1_valid = 1;
       } else {
         S.k1_valid = 0;
@@ -194,7 +191,12 @@ __device__ __noinline__ void evolve_apply(Ctx<M>& X, Bufs& B, StepState& S, doub
     } else {
       S.k1_valid = 0;
     }
-    double2* ty = B.y; B.y = B.yn; B.yn = ty;
+    __syncthreads();   // every thread has read the buffers' addresses
+    if (threadIdx.x == 0) {
+      double2* ty = B.y; B.y = B.yn; B.yn = ty;
+      if (S.k1_valid) { double2* tk = B.k[0]; B.k[0] = B.k[6]; B.k[6] = tk; }
+    }
+    __syncthreads();
     S.t = tn;
     S.h = hn;
     ++S.acc;
