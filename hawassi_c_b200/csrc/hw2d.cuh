@@ -440,31 +440,48 @@ __device__ __forceinline__ double eta_loss(const Tab2& tb, const Work2& w, size_
 // pass D runs, all three as spectra (2)
 __device__ __forceinline__ int damp_fields(const Tab2& tb, const Work2& w) { return tb.chi_one ? 2 : (w.dph ? 1 : 0); }
 
-// the loss fields of a physical point into slices s0 + 2 f + k
-__device__ __forceinline__ void emit_loss(double2* sm, int M, int s0, int nd, const ColPt& p, const Tab2& tb, const Work2& w,
-                                          double eta, double u, double v) {
+// Column pass: the loss fields from physical space to w.Q's fields f0..., once the slices'
+// own fields are stored (a batch of their own keeps every pass at six slices, two CTAs to
+// an SM at 1024 points)
+template <int M, int NT>
+__device__ __forceinline__ void send_loss(double2* sm, int f0, int nd, const Tab2& tb, const Work2& w, int c, size_t n) {
   if (nd == 0) return;
-  const double dm = tb.damp[p.q];
-  put(sm, M, s0 + p.k, p.y, make_double2(eta_loss(tb, w, p.q, p.y, dm, eta), nd == 2 ? dm * u : 0.0));
-  if (nd == 2) put(sm, M, s0 + 2 + p.k, p.y, make_double2(dm * v, 0.0));
+  __syncthreads();
+#pragma unroll 2
+  for (int t = threadIdx.x; t < 2 * M; t += NT) {
+    const ColPt p(t, c, tb.nx);
+    const double dm = tb.damp[p.q];
+    put(sm, M, p.k, p.y, make_double2(eta_loss(tb, w, p.q, p.y, dm, w.phys[p.q]), nd == 2 ? dm * w.phys[n + p.q] : 0.0));
+    if (nd == 2) put(sm, M, 2 + p.k, p.y, make_double2(dm * w.phys[2 * n + p.q], 0.0));
+  }
+  fft_slices<M, NT>(sm, 0, 2 * nd, tb.twy, -1);
+  col_store<M, NT>(sm, 0, nd, w.Q + f0 * n, tb.nx, c, n);
 }
-// and their spectra, at all of a quad's points, into w.D
-__device__ __forceinline__ void store_loss(const double2* sm, int M, int s0, int nd, const Quad& Q, int Nx, const Work2& w,
-                                           size_t n) {
+// Row pass: their spectra into w.D, ahead of the pass's own fields
+template <int M, int NT>
+__device__ __forceinline__ void store_loss(double2* sm, int f0, int nd, const Tab2& tb, const Work2& w, const Pair& P, size_t n) {
   if (nd == 0) return;
+  row_load<M, NT>(sm, 0, nd, w.Q + f0 * n, P, n);
+  fft_slices<M, NT>(sm, 0, 2 * nd, tb.twx, -1);
+#pragma unroll 1
+  for (int j = threadIdx.x; j < M / 2; j += NT) {
+    const Quad Q(P, j, M);
 #pragma unroll
-  for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 2; ++k)
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      double2 a, b;
-      split_at(sm, M, s0, Q, k, s, a, b);
-      w.D[Q.at(k, s, Nx)] = a;
-      if (nd == 2) {
-        w.D[n + Q.at(k, s, Nx)] = b;
-        split_at(sm, M, s0 + 2, Q, k, s, a, b);
-        w.D[2 * n + Q.at(k, s, Nx)] = a;
+      for (int s = 0; s < 2; ++s) {
+        const size_t q = Q.at(k, s, M);
+        double2 a, b;
+        split_at(sm, M, 0, Q, k, s, a, b);
+        w.D[q] = a;
+        if (nd == 2) {
+          w.D[n + q] = b;
+          split_at(sm, M, 2, Q, k, s, a, b);
+          w.D[2 * n + q] = a;
+        }
       }
-    }
+  }
+  __syncthreads();
 }
 
 // the adjustment's input at a quad: S(i kx dH), S(i ky dH), S(a) into slices 0..5
@@ -597,10 +614,10 @@ k2_colB(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
     w.phys[2 * n + p.q] = v;
     put(sm, M, p.k, p.y, make_double2(eta * lphi * wc, eta * u * wc));
     put(sm, M, 2 + p.k, p.y, make_double2(eta * v * wc, 0.5 * ((u * u + v * v) - lphi * lphi) * wc));
-    emit_loss(sm, M, 2 * np, nd, p, tb, w, eta, u, v);
   }
-  fft_slices<M, NT>(sm, 0, 2 * (np + nd), tb.twy, -1);
-  col_store<M, NT>(sm, 0, np + nd, w.Q, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 2 * np, tb.twy, -1);
+  col_store<M, NT>(sm, 0, np, w.Q, Nx, c, n);
+  send_loss<M, NT>(sm, np, nd, tb, w, c, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -620,13 +637,13 @@ k2_rowC(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   const bool hs3 = tb.model == 3;
   const int np = hs3 ? 3 : 2;
   const Pair P = row_pair(blockIdx.x, Ny);
-  row_load<M, NT>(sm, 0, np + nd, w.Q, P, n);
-  fft_slices<M, NT>(sm, 0, 2 * (np + nd), tb.twx, -1);
+  store_loss<M, NT>(sm, np, nd, tb, w, P, n);
+  row_load<M, NT>(sm, 0, np, w.Q, P, n);
+  fft_slices<M, NT>(sm, 0, 2 * np, tb.twx, -1);
 #pragma unroll 1
   for (int j = threadIdx.x; j < Nx / 2; j += NT) {
     const Quad Q(P, j, Nx);
     double2 dH[2][2], a[2][2], lq[2][2], dv[2][2];
-    store_loss(sm, M, 2 * np, nd, Q, Nx, w, n);
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -832,7 +849,9 @@ k2_colH1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
       u = a.y * invN;
       v = b.x * invN;
     }
-    emit_loss(sm, M, 0, 2, p, tb, w, eta, u, v);
+    const double dm = tb.damp[p.q];
+    put(sm, M, p.k, p.y, make_double2(eta_loss(tb, w, p.q, p.y, dm, eta), dm * u));
+    put(sm, M, 2 + p.k, p.y, make_double2(dm * v, 0.0));
   }
   fft_slices<M, NT>(sm, 0, 4, tb.twy, -1);
   col_store<M, NT>(sm, 0, 2, w.Q, Nx, c, n);

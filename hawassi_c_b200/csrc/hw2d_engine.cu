@@ -39,41 +39,37 @@ constexpr long long kMaxAttemptsPerRun = 2000000;
 template <int M>
 size_t smem_bytes(int slices) { return (size_t)slices * hwdev::padded(M) * sizeof(double2); }
 
-template <class Kernel>
-void allow(Kernel* k, size_t bytes) {
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-// the most slices that each pass takes
+// the slices of each pass
 template <int M>
 void set_attrs() {
-  allow(hw2d::k2_rowA<M>, smem_bytes<M>(2));
-  allow(hw2d::k2_colB<M>, smem_bytes<M>(10));
-  allow(hw2d::k2_rowC<M>, smem_bytes<M>(10));
-  allow(hw2d::k2_colD<M>, smem_bytes<M>(2));
-  allow(hw2d::k2_rowE<M>, smem_bytes<M>(2));
-  allow(hw2d::k2_colH3<M>, smem_bytes<M>(2));
-  allow(hw2d::k2_rowI3<M>, smem_bytes<M>(6));
-  allow(hw2d::k2_colH1<M>, smem_bytes<M>(4));
-  allow(hw2d::k2_rowH1<M>, smem_bytes<M>(4));
-  allow(hw2d::k2v_row1<M>, smem_bytes<M>(2));
-  allow(hw2d::k2v_col2<M>, smem_bytes<M>(6));
-  allow(hw2d::k2v_row3<M>, smem_bytes<M>(8));
-  allow(hw2d::k2v_col4<M>, smem_bytes<M>(10));
-  allow(hw2d::k2v_row5<M>, smem_bytes<M>(10));
-  allow(hw2d::k2v_col6<M>, smem_bytes<M>(6));
-  allow(hw2d::k2v_row7<M>, smem_bytes<M>(6));
-  allow(hw2d::k2b_rowI<M>, smem_bytes<M>(2));
-  allow(hw2d::k2b_colI<M>, smem_bytes<M>(2));
-  allow(hw2d::k2b_sbcol<M>, smem_bytes<M>(2));
-  allow(hw2d::k2b_sbrow<M>, smem_bytes<M>(2));
-  allow(hw2d::k2w_row1<M>, smem_bytes<M>(2));
-  allow(hw2d::k2w_col2<M>, smem_bytes<M>(2));
-  allow(hw2d::k2w_row3<M>, smem_bytes<M>(2));
-  allow(hw2d::k2w_rowV1<M>, smem_bytes<M>(4));
-  allow(hw2d::k2w_colV2<M>, smem_bytes<M>(4));
-  allow(hw2d::k2w_rowV3<M>, smem_bytes<M>(2));
-  allow(hw2d::k2o_row<M>, smem_bytes<M>(4));
-  allow(hw2d::k2o_col<M>, smem_bytes<M>(4));
+  cudaFuncSetAttribute(hw2d::k2_rowA<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2_colB<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2_rowC<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2_colD<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2_rowE<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2_colH3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2_rowI3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2_colH1<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
+  cudaFuncSetAttribute(hw2d::k2_rowH1<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
+  cudaFuncSetAttribute(hw2d::k2v_row1<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2v_col2<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2v_row3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2v_col4<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2v_row5<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2v_col6<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2v_row7<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(6));
+  cudaFuncSetAttribute(hw2d::k2b_rowI<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2b_colI<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2b_sbcol<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2b_sbrow<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2w_row1<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2w_col2<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2w_row3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2w_rowV1<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
+  cudaFuncSetAttribute(hw2d::k2w_colV2<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
+  cudaFuncSetAttribute(hw2d::k2w_rowV3<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(2));
+  cudaFuncSetAttribute(hw2d::k2o_row<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
+  cudaFuncSetAttribute(hw2d::k2o_col<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<M>(4));
 }
 
 // the output stage's two passes (row M = nx, column M = ny)
@@ -169,36 +165,36 @@ struct PassArgs {
 template <int M>
 void launch_row(RowPass which, int cubic, const PassArgs& a) {
   const Tab2& tb = a.tb;
-  const int nb = tb.ny / 2, nd = tb.chi_one ? 2 : (a.w.dph ? 1 : 0), np = (tb.model == 3 ? 3 : 2) + nd;
+  const int nb = tb.ny / 2;
   const int t2 = hw2d::thr2(M), t4 = hw2d::thr4(M);
   switch (which) {
     case kRowA:
       hw2d::k2_rowA<M><<<dim3(nb, tb.model == 3 ? 3 : 2), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.ctl, a.mode, a.cond);
       break;
-    case kRowC: hw2d::k2_rowC<M><<<nb, t4, smem_bytes<M>(std::max(6, 2 * np)), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kRowC: hw2d::k2_rowC<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
     case kRowE: hw2d::k2_rowE<M><<<dim3(nb, 3), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.rk, a.ctl, a.mode, a.cond, a.out); break;
     case kRowI3: hw2d::k2_rowI3<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
     case kRowH1: hw2d::k2_rowH1<M><<<nb, t4, smem_bytes<M>(4), a.s>>>(tb, a.w, a.rk, a.ctl, a.mode, a.cond, a.out); break;
     case kRowV1:
       hw2d::k2v_row1<M><<<dim3(nb, 2 + tb.nk), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.ctl, a.mode, a.cond);
       break;
-    case kRowV3: hw2d::k2v_row3<M><<<nb, t4, smem_bytes<M>(tb.model == 3 ? 8 : 6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
-    case kRowV5: hw2d::k2v_row5<M><<<nb, t4, smem_bytes<M>(std::max(6, cubic ? 2 : 2 * np)), a.s>>>(tb, a.w, a.ctl, a.cond, cubic); break;
+    case kRowV3: hw2d::k2v_row3<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kRowV5: hw2d::k2v_row5<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond, cubic); break;
     case kRowV7: hw2d::k2v_row7<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond, cubic); break;
   }
 }
 template <int M>
 void launch_col(ColPass which, int cubic, const PassArgs& a) {
   const Tab2& tb = a.tb;
-  const int nb = tb.nx / 2, nd = tb.chi_one ? 2 : (a.w.dph ? 1 : 0), np = (tb.model == 3 ? 3 : 2) + nd;
+  const int nb = tb.nx / 2;
   const int t2 = hw2d::thr2(M), t4 = hw2d::thr4(M);
   switch (which) {
-    case kColB: hw2d::k2_colB<M><<<nb, t4, smem_bytes<M>(std::max(tb.model == 3 ? 6 : 4, 2 * np)), a.s>>>(tb, a.w, a.ctl, a.cond); break;
+    case kColB: hw2d::k2_colB<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
     case kColD: hw2d::k2_colD<M><<<dim3(nb, 3), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.cond); break;
     case kColH3: hw2d::k2_colH3<M><<<nb, t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.cond); break;
     case kColH1: hw2d::k2_colH1<M><<<nb, t4, smem_bytes<M>(4), a.s>>>(tb, a.w, a.ctl, a.cond); break;
     case kColV2: hw2d::k2v_col2<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
-    case kColV4: hw2d::k2v_col4<M><<<nb, t4, smem_bytes<M>(std::max(4, cubic ? 2 : 2 * np)), a.s>>>(tb, a.w, a.ctl, a.cond, cubic); break;
+    case kColV4: hw2d::k2v_col4<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond, cubic); break;
     case kColV6: hw2d::k2v_col6<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
   }
 }

@@ -114,8 +114,9 @@ k2v_col2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   col_store<M, NT>(sm, 0, 1, w.Q, Nx, c, n);
 }
 
-// V3: slices 0..3 two fields at a time, 4, 5 the sum kx (.) + ky (.), under HS3 6, 7 its
-// kx part at the points that the symmetrisation keeps (columns up to Nx / 2)
+// V3: slices 0..3 two fields at a time, 4, 5 the sum kx (.) + ky (.); under HS3 0, 1 one field
+// at a time, 2, 3 the sum's kx part at the points that the symmetrisation keeps (columns up
+// to Nx / 2)
 template <int M>
 __global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
 k2v_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
@@ -126,8 +127,9 @@ k2v_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   const size_t n = (size_t)tb.n;
   const bool hs3 = tb.model == 3;
   const Pair P = row_pair(blockIdx.x, tb.ny);
-  for (int f = 0; f <= K; f += 2) {
-    const int nf = K + 1 - f > 1 ? 2 : 1;
+  const int step = hs3 ? 1 : 2;
+  for (int f = 0; f <= K; f += step) {
+    const int nf = K + 1 - f < step ? 1 : step;
     __syncthreads();
     row_load<M, NT>(sm, 0, nf, w.Q + f * n, P, n);
     fft_slices<M, NT>(sm, 0, 2 * nf, tb.twx, -1);
@@ -155,8 +157,8 @@ k2v_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
           put(sm, M, 4 + k, Q.cc[s], t);
           if (hs3 && Q.has(s)) {
             double2 tu = cscale(pu, kx);
-            if (f > 0) tu = cadd(tu, slot(sm, M, 6 + k, Q.cc[s]));
-            put(sm, M, 6 + k, Q.cc[s], tu);
+            if (f > 0) tu = cadd(tu, slot(sm, M, 2 + k, Q.cc[s]));
+            put(sm, M, 2 + k, Q.cc[s], tu);
           }
         }
     }
@@ -177,7 +179,7 @@ k2v_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
         x[k][s] = t;
         y[k][s] = zero2();
         if (hs3) {
-          x[k][s] = mul_mi(slot(sm, M, 6 + k, Q.cc[s]), h);
+          x[k][s] = mul_mi(slot(sm, M, 2 + k, Q.cc[s]), h);
           y[k][s] = csub(t, x[k][s]);
         }
       }
@@ -188,8 +190,8 @@ k2v_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   row_store<M, NT>(sm, 4, 1, w.R, P, n);
 }
 
-// where pass V4 puts its fields in w.Q: the products, the loss fields, then the gam_j pairs
-__device__ __forceinline__ int first_pair(const Tab2& tb, int nd, int cubic) { return cubic ? 1 : (tb.model == 3 ? 3 : 2) + nd; }
+// the products' fields of pass V4 in w.Q; the loss fields and the gam_j pairs follow
+__device__ __forceinline__ int products(const Tab2& tb, int cubic) { return cubic ? 1 : (tb.model == 3 ? 3 : 2); }
 
 // V4: column pass, inverse -> products -> forward; then gam_j q, four references at a time.
 // cubic = 0: L phi (HS3: M0u, M0v) in; fields 0 (q, eta u), 1 (eta v, deletaH2), under HS3
@@ -204,7 +206,7 @@ k2v_col4(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
   const int Nx = tb.nx, c = blockIdx.x, K = tb.nk, nd = cubic ? 0 : damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
   const bool hs3 = tb.model == 3;
-  const int f0 = first_pair(tb, nd, cubic);
+  const int np = products(tb, cubic), f0 = np + nd;
   const double invN = 1.0 / ((double)tb.n);
   col_load<M, NT>(sm, 0, 1, w.R, Nx, c, n);
   fft_slices<M, NT>(sm, 0, 2, tb.twy, +1);
@@ -227,11 +229,11 @@ k2v_col4(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
         put(sm, M, 4 + p.k, p.y, make_double2(eta * eta * a.x * wc, eta * eta * a.y * wc));
         w.op[n + p.q] = lphi;
       }
-      emit_loss(sm, M, 2 * (hs3 ? 3 : 2), nd, p, tb, w, eta, u, v);
     }
   }
-  fft_slices<M, NT>(sm, 0, 2 * f0, tb.twy, -1);
-  col_store<M, NT>(sm, 0, f0, w.Q, Nx, c, n);
+  fft_slices<M, NT>(sm, 0, 2 * np, tb.twy, -1);
+  col_store<M, NT>(sm, 0, np, w.Q, Nx, c, n);
+  send_loss<M, NT>(sm, np, nd, tb, w, c, n);
   for (int j = 0; j < K; j += 4) {
     const int nf = K - j > 2 ? 2 : 1;
     __syncthreads();
@@ -262,14 +264,14 @@ k2v_row5(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
   const int Nx = M, K = tb.nk, nd = cubic ? 0 : damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
   const bool hs3 = tb.model == 3;
-  const int f0 = first_pair(tb, nd, cubic), np = cubic ? 1 : (hs3 ? 3 : 2);
+  const int np = products(tb, cubic), f0 = np + nd;
   const Pair P = row_pair(blockIdx.x, tb.ny);
-  row_load<M, NT>(sm, 0, f0, w.Q, P, n);
-  fft_slices<M, NT>(sm, 0, 2 * f0, tb.twx, -1);
+  store_loss<M, NT>(sm, np, nd, tb, w, P, n);
+  row_load<M, NT>(sm, 0, np, w.Q, P, n);
+  fft_slices<M, NT>(sm, 0, 2 * np, tb.twx, -1);
 #pragma unroll 1
   for (int j = threadIdx.x; j < Nx / 2; j += NT) {
     const Quad Q(P, j, Nx);
-    if (!cubic) store_loss(sm, M, 2 * np, nd, Q, Nx, w, n);
     double2 keep[2][2];
 #pragma unroll
     for (int k = 0; k < 2; ++k)
