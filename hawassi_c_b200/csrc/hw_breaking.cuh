@@ -35,21 +35,20 @@ __device__ __forceinline__ void crest_clear(Crest* a, int n) {  // set_init_CB (
   }
 }
 
-// breaking_criterion's test at a local maximum J (1d/breaking.c:72-95): local
-// wavenumber K = (eta dH/dx - H deta/dx) / (eta^2 + H^2) from the Hilbert transform
-// H of eta (centred differences, 1d/functions.c:1850), crest speed c(K, h + eta),
+// breaking_criterion's test at a local maximum (1d/breaking.c:72-95), from the values
+// around it: local wavenumber K = (eta dH/dx - H deta/dx) / (eta^2 + H^2) from the Hilbert
+// transform H of eta (centred differences, 1d/functions.c:1850), crest speed c(K, h + eta),
 // breaking if |u| > KBC |c|.  Products and sums are rounded one by one (no fused
 // multiply-add), in the reference's order, as the reference's x86-64 build rounds.
-__device__ __forceinline__ bool crest_breaks(const DevMember& d, const double2* PE, const double* Heta, int hs,
-                                             int J) {
-  const double eJ = PE[J].x, hJ = Heta[size_t(hs) * J];
+__device__ __forceinline__ bool crest_breaks(const DevMember& d, double2 e, double el, double er, double h, double hl,
+                                             double hr, double depth) {
   const double dx2 = 2 * d.dx;
-  const double gH = __ddiv_rn(__dsub_rn(Heta[size_t(hs) * (J + 1)], Heta[size_t(hs) * (J - 1)]), dx2);
-  const double ge = __ddiv_rn(__dsub_rn(PE[J + 1].x, PE[J - 1].x), dx2);
-  const double KxJ = __ddiv_rn(__dsub_rn(__dmul_rn(eJ, gH), __dmul_rn(hJ, ge)),
-                               __dadd_rn(__dmul_rn(eJ, eJ), __dmul_rn(hJ, hJ)));
-  const double Cc = phase_velocity_dev(KxJ, __dadd_rn(d.depth[J], eJ));
-  return fabs(PE[J].y) > __dmul_rn(d.KBC, fabs(Cc));
+  const double gH = __ddiv_rn(__dsub_rn(hr, hl), dx2);
+  const double ge = __ddiv_rn(__dsub_rn(er, el), dx2);
+  const double KxJ = __ddiv_rn(__dsub_rn(__dmul_rn(e.x, gH), __dmul_rn(h, ge)),
+                               __dadd_rn(__dmul_rn(e.x, e.x), __dmul_rn(h, h)));
+  const double Cc = phase_velocity_dev(KxJ, __dadd_rn(depth, e.x));
+  return fabs(e.y) > __dmul_rn(d.KBC, fabs(Cc));
 }
 
 // the sequential part of breaking_process, run by one thread
@@ -226,62 +225,74 @@ static __device__ __noinline__ void breaking_leader(const DevMember& d, BrkDev* 
   bk->npk = bk->n_touched;
 }
 
+// whether the machine's records are all clear: with no crest passing, a call then changes
+// nothing but the output interval's counter
+__device__ __forceinline__ bool records_clear(const BrkDev* bk) {
+  const int flag = bk->flag, touched = bk->n_touched, cb = bk->dirty_cb, cbn = bk->dirty_cbn;
+  return (flag | touched | cb | cbn) == 0;
+}
+
 // The parts of one RHS's breaking work, so that a caller can place them between
 // its own phases:
-//   breaking_reset  (leader) before a barrier that precedes the scan;
+//   breaking_reset  (every CTA's first thread) before a barrier that precedes the listing;
 //   breaking_scan   (all threads) once eta, u and H(eta) are complete member-wide;
-//   breaking_lead   (leader) after a barrier that follows the scan; it leaves the
-//                   count of nodes with B != 0 in bk->npk (0: no force);
+//   breaking_lead   (leader) after a barrier that follows the scan; it sets `live` in
+//                   every CTA where some node has B != 0;
 //   breaking_force  (all threads) after a barrier that follows the leader.
 template <int M>
 __device__ __forceinline__ void breaking_reset(Ctx<M> X) {
-  if (X.c == 0 && int(threadIdx.x) == 0) {
-    X.d.bk->npk = 0;
-    X.d.bk->any_above = 0;
-  }
+  if (threadIdx.x == 0) X.sc->ncand = X.sc->npk = X.sc->above = X.sc->live = 0;
 }
 
 // criterion scan (1d/breaking.c:36-61,72) over the listed points of the window
 // [xbstart, xbstart + lenIF) that are not below the threshold (the threads that formed
 // eta listed them): a few in a hundred, so one sweep of the CTA takes them, where a
 // thread that walked its own eight points waited for each crest in turn
-// (21 against 7 thousand cycles an RHS in the 256-member ensemble)
+// (21 against 6 thousand cycles an RHS in the 256-member ensemble).  All that a point's
+// test can need is loaded at once.
 template <int M>
 __device__ __forceinline__ void breaking_scan(Ctx<M> X, const double2* PE, const double* Heta, int hs) {
   const DevMember& d = X.d;
-  BrkDev* bk = d.bk;
   const int N = d.N, n = X.sc->ncand;
   const int w0 = d.xbstart, w1 = d.xbstart + d.lenIF;
-  bool above = false;
-  for (int q = int(threadIdx.x); q < n; q += Ctx<M>::T) {
+  for (int q = threadIdx.x; q < n; q += Ctx<M>::T) {
     const int p = X.sc->cand[q];
     const bool inner = p >= w0 + 1 && p <= w1 - 2;
-    const double e = PE[p].x, el = inner ? PE[p - 1].x : 0.0, er = inner ? PE[p + 1].x : 0.0;
-    if (e > d.MaxEtaInit) above = true;
-    if (inner && e > er && e > el && crest_breaks(d, PE, Heta, hs, p)) {
-      const int slot = atomicAdd(&bk->npk, 1);
-      if (slot < N) bk->pk[slot] = p;
+    const int l = inner ? p - 1 : p, r = inner ? p + 1 : p;
+    const double2 e = PE[p];
+    const double el = PE[l].x, er = PE[r].x, h = Heta[size_t(hs) * p], hl = Heta[size_t(hs) * l], hr = Heta[size_t(hs) * r];
+    const double depth = d.depth[p];
+    Scratch<M>* lead = d.C > 1 ? cg::this_cluster().map_shared_rank(X.sc, 0) : X.sc;
+    if (e.x > d.MaxEtaInit) lead->above = 1;
+    if (inner && e.x > er && e.x > el && crest_breaks(d, e, el, er, h, hl, hr, depth)) {
+      const int slot = atomicAdd(&lead->npk, 1);
+      if (slot < N) d.bk->pk[slot] = p;
     }
   }
-  // one flag update per warp
-  if (__any_sync(0xffffffffu, above) && (int(threadIdx.x) & 31) == 0) atomicOr(&bk->any_above, 1);
 }
 
 template <int M>
 __device__ __forceinline__ void breaking_lead(Ctx<M> X, double t, const double2* PE, const double* Heta, int hs) {
-  if (X.c == 0 && int(threadIdx.x) == 0) {
+  if (X.c == 0 && threadIdx.x == 0) {
     BrkDev* bk = X.d.bk;
-    const int npk = bk->npk, flag = bk->flag, touched = bk->n_touched, it = bk->ITERbdt;
-    const int dirty = bk->dirty_cb | bk->dirty_cbn;
-    if (npk == 0 && flag == 0 && touched == 0 && dirty == 0) {
-      // no crest passes and none is tracked: every record is clear, and all that
-      // breaking_leader would change is the output interval's counter
-      if (t > (it * X.d.dt_in)) bk->ITERbdt = it + 1;
-    } else {
-      if (npk > X.d.N) bk->npk = X.d.N;
-      breaking_leader(X.d, bk, t, PE, Heta, hs);
+    Scratch<M>& sc = *X.sc;
+    if (sc.idle < 0) {
+      sc.idle = records_clear(bk);
+      sc.iter = bk->ITERbdt;
     }
-    __threadfence();
+    if (sc.npk == 0 && sc.idle) {
+      // no crest passes and none is tracked
+      if (t > (sc.iter * X.d.dt_in)) bk->ITERbdt = ++sc.iter;
+    } else {
+      bk->npk = sc.npk < X.d.N ? sc.npk : X.d.N;
+      bk->any_above = sc.above;
+      breaking_leader(X.d, bk, t, PE, Heta, hs);
+      sc.idle = records_clear(bk);
+      sc.iter = bk->ITERbdt;
+      if (bk->npk > 0)   // nodes touched by this call
+        for (int r = 0; r < X.d.C; ++r) (X.d.C > 1 ? cg::this_cluster().map_shared_rank(X.sc, r) : X.sc)->live = 1;
+      __threadfence();
+    }
   }
 }
 

@@ -218,9 +218,9 @@ __device__ __forceinline__ void slice_fft(double2* buf, int xo, const double2* _
     slice_pass<M, 16>(buf, xo, 8, tw, tw_stride, sign, tid, g, act);
     slice_pass<M, 16>(buf, xo, 128, tw, tw_stride, sign, tid, g, act);
   } else if constexpr (M == 1024) {
-    slice_pass<M, 8>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
-    slice_pass<M, 8>(buf, xo, 8, tw, tw_stride, sign, tid, g, act);
-    slice_pass<M, 16>(buf, xo, 64, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 16>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 8>(buf, xo, 16, tw, tw_stride, sign, tid, g, act);
+    slice_pass<M, 8>(buf, xo, 128, tw, tw_stride, sign, tid, g, act);
   } else if constexpr (M == 512) {
     slice_pass<M, 8>(buf, xo, 1, tw, tw_stride, sign, tid, g, act);
     slice_pass<M, 8>(buf, xo, 8, tw, tw_stride, sign, tid, g, act);

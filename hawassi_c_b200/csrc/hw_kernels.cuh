@@ -28,6 +28,7 @@ __device__ __forceinline__ void evolve_member(DevMember* mems, int mi, int mode,
     sc.bufs.yn = sd.ynew;
     for (int i = 0; i < 7; ++i) sc.bufs.k[i] = sd.kb[i];
     sc.full = 0;
+    sc.idle = -1;
   }
   // a cluster barrier, not only the CTA's: the RHS's first phase writes into the
   // partner CTA's shared memory, which must be running
@@ -116,7 +117,9 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs(DevMember* mems, c
   if (threadIdx.x == 0) {
     sd = mems[mi];
     sc.stg.s = 0;
+    sc.stg.sig = -1;
     sc.full = 1;
+    sc.idle = -1;
   }
   __syncthreads();
   Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);

@@ -56,7 +56,9 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs_noalloc(DevMember*
     sd.kb[6] = scratch + 2 * N;
     for (int i = 0; i < kScratch; ++i) sd.sc[i] = scratch + size_t(4 + i) * N;
     sc.stg.s = 0;
+    sc.stg.sig = -1;
     sc.full = 1;
+    sc.idle = -1;
   }
   __syncthreads();
   Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);

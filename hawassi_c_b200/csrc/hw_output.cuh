@@ -39,7 +39,7 @@ __device__ __noinline__ void output_stage(Ctx<M> X, StepState& S, int row) {
   const double2* dy = B.k[6];
   if (!d.exact && !none) {
     if (!S.k1_valid) {
-      rhs_at(X, S, S.t, B.y, B.k[0]);
+      rhs_at(X, S, S.t, B.y, B.k[0], -1);
       S.k1_valid = 1;
     }
     dy = B.k[0];

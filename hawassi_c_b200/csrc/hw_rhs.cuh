@@ -33,6 +33,7 @@ struct StageSrc {
   const double2* y;
   const double2* k[5];
   int s;
+  int sig;      // entry of the step's influx signals at this stage's time (-1: not formed)
   double h;
 };
 
@@ -97,6 +98,11 @@ struct Scratch {
   StageSrc stg;         // stage input of the coming RHS (stg.s = 0: zs holds it)
   Bufs bufs;
   int full;             // dz is written outside the alias band too (as zeros)
+  double2 sig[7];       // influx signal and its integral at the step's times: k1, stages 2..6, kout
+  // breaking (CTA 0's counters serve the member; live in every CTA)
+  int npk, above;       // crests that passed the test, eta above the threshold somewhere
+  int live;             // some node breaks: the force is not zero
+  int idle, iter;       // no crest is tracked and every record clear (-1: not known); ITERbdt
   int ncand;
   unsigned short cand[M];   // grid points of this CTA's threads above the breaking threshold
 };

@@ -326,7 +326,8 @@ __device__ __noinline__ void assemble(Ctx<M> X, double2* __restrict__ dz, const 
   const double* __restrict__ aalt = d.aal;
   const double2* __restrict__ gxt = d.gamX;
   const double2* __restrict__ gst = d.gamXs;
-  const double pv = X.sc->red[kRedPv], ps = X.sc->red[kRedPs];
+  const int sig = X.sc->stg.sig;
+  const double pv = sig < 0 ? X.sc->red[kRedPv] : X.sc->sig[sig].x, ps = sig < 0 ? X.sc->red[kRedPs] : X.sc->sig[sig].y;
 #pragma unroll 1
   for (int u = 0; u < kPts / 2; ++u) {
     const PairAt r = pair_at<M>(c, pb.cq, int(threadIdx.x) + u * T);
@@ -375,12 +376,13 @@ __device__ __noinline__ void assemble(Ctx<M> X, double2* __restrict__ dz, const 
   }
 }
 
-// beside the last spectral phase: the breaking machine's leader and, by another thread,
-// the influx signals at the stage time (read after the phase's barrier)
+// beside the last spectral phase: the breaking machine's leader and, where the step has not
+// formed them, by another thread the influx signals at the stage time (read after the
+// phase's barrier)
 template <int M>
 __device__ __forceinline__ void lead_and_influx(Ctx<M> X, double t, const double2* PE, const double* Heta) {
   if (X.d.brk) breaking_lead(X, t, PE, Heta, 2);
-  if (X.d.has_influx && int(threadIdx.x) == Ctx<M>::T - 1) {
+  if (X.d.has_influx && X.sc->stg.sig < 0 && int(threadIdx.x) == Ctx<M>::T - 1) {
     const double2 s = influx_at(X.d, t);
     X.sc->red[kRedPv] = s.x;
     X.sc->red[kRedPs] = s.y;
@@ -418,8 +420,8 @@ __device__ __noinline__ void finish_rhs(Ctx<M> X, double2* __restrict__ dz, cons
     fft_forward2<M>(A, Bf, d.tw, d.N, C, X.c);
   }
   member_sync(C);
-  // the leader's node count is visible member-wide after the transforms' barriers
-  const bool rb_live = d.brk != 0 && d.bk->npk > 0;
+  // (the leader's word is in every CTA since the transforms' barriers)
+  const bool rb_live = d.brk != 0 && X.sc->live;
   if (!rb_live) {
     if (M0h) assemble<M, kAsmSlices, true>(X, dz, M0h, nullptr, nullptr, nullptr);
     else assemble<M, kAsmSlices, false>(X, dz, nullptr, nullptr, nullptr, nullptr);
@@ -460,8 +462,7 @@ __device__ __noinline__ void rhs_hs2_flat(Ctx<M> X, double t, double2* __restric
   const PairBufs<M> pb(X);
 
   // (0)-(1) stage input and its packing
-  if (brk) breaking_reset(X);
-  if (int(threadIdx.x) == 0) X.sc->ncand = 0;
+  breaking_reset(X);
   stage_phase<M, kWithM0Hilbert>(X);
   // (2) products in physical space (1d/functions.c:1486-1498)
   const bool fused = C == 2 || C == 4 || C == 8;

@@ -500,8 +500,7 @@ __device__ __forceinline__ void rest_sweep(Ctx<M> X, double t) {
 template <int M>
 __device__ __noinline__ void rhs_gen(Ctx<M> X, double t, double2* __restrict__ dz) {
   const int C = X.d.C;
-  if (X.d.brk) breaking_reset(X);
-  if (threadIdx.x == 0) X.sc->ncand = 0;
+  breaking_reset(X);
   if (X.d.model == 1) {
     stage_phase<M, kWithNone>(X);
     meet<M, OpLinear<M>>(X, 1, 1, 0);

@@ -109,19 +109,20 @@ struct StepState {
 };
 
 // stage s of a step of size h as the coming RHS's input: y + h sum_j b_sj k_j, or (s = 1)
-// the state y itself; the RHS's first barrier makes it known
+// the state y itself, and entry sig of the step's influx signals; the RHS's first barrier
+// makes it known
 template <int M>
-__device__ __forceinline__ void set_stage(Ctx<M> X, const double2* y, int s, double h) {
+__device__ __forceinline__ void set_stage(Ctx<M> X, const double2* y, int s, int sig, double h) {
   if (threadIdx.x == 0) {
     const Bufs& B = X.sc->bufs;
-    X.sc->stg = StageSrc{y, {B.k[0], B.k[1], B.k[2], B.k[3], B.k[4]}, s, h};
+    X.sc->stg = StageSrc{y, {B.k[0], B.k[1], B.k[2], B.k[3], B.k[4]}, s, X.d.has_influx ? sig : -1, h};
   }
 }
 
 // one RHS evaluation at the state src itself (the RHS copies it into zs)
 template <int M>
-__device__ __forceinline__ void rhs_at(Ctx<M> X, StepState& S, double t, const double2* src, double2* out) {
-  set_stage(X, src, 1, 0.0);
+__device__ __forceinline__ void rhs_at(Ctx<M> X, StepState& S, double t, const double2* src, double2* out, int sig) {
+  set_stage(X, src, 1, sig, 0.0);
   rhs_eval<M>(X, t, out);
   ++S.rhs;
 }
@@ -135,20 +136,29 @@ __device__ __noinline__ void evolve_apply(Ctx<M> X, StepState& S, double t1) {
   double h0 = S.h;
   const double dt = t1 - t0;
   if ((dt < 0.0 && h0 > 0.0) || (dt > 0.0 && h0 < 0.0)) { S.status = kStepFailed; return; }
-  if (d.exact || !S.k1_valid) rhs_at(X, S, t0, B.y, B.k[0]);
+  bool need_k1 = d.exact || !S.k1_valid;
   int attempts = 0;
   for (;;) {
     bool final_step = false;
     if ((dt >= 0.0 && h0 > dt) || (dt < 0.0 && h0 < dt)) { h0 = dt; final_step = true; }
+    // The influx signals at the attempt's seven times, each by a thread of its own: one
+    // wait for the samples and divisions an attempt instead of one an RHS (4 thousand
+    // cycles of an RHS's 40 in a single tank)
+    if (d.has_influx && threadIdx.x < 7) {
+      const int j = threadIdx.x;
+      X.sc->sig[j] = influx_at(d, j == 0 ? t0 : (j == 6 ? t0 + h0 : t0 + RK_ah[j - 1] * h0));
+    }
+    if (need_k1) rhs_at(X, S, t0, B.y, B.k[0], 0);
+    need_k1 = false;
     for (int s = 2; s <= 6; ++s) {
       // the RHS forms its own stage input from y and the k's (into zs as well)
-      set_stage(X, B.y, s, h0);
+      set_stage(X, B.y, s, s - 1, h0);
       rhs_eval<M>(X, t0 + RK_ah[s - 2] * h0, B.k[s - 1]);
       ++S.rhs;
     }
     member_sync(d.C);
     const double rmax = final_combine(X, h0);
-    if (d.exact) rhs_at(X, S, t0 + h0, B.yn, B.k[6]);
+    if (d.exact) rhs_at(X, S, t0 + h0, B.yn, B.k[6], 6);
     const double tn = final_step ? t1 : t0 + h0;
     // std_control_hadjust (order 5)
     const double h_old = h0;
@@ -183,7 +193,7 @@ __device__ __noinline__ void evolve_apply(Ctx<M> X, StepState& S, double t1) {
       // next call starts exactly at t0 + h0
       const double tk = t0 + h0;
       if (tk == tn) {
-        rhs_at(X, S, tk, B.yn, B.k[6]);
+        rhs_at(X, S, tk, B.yn, B.k[6], 6);
         S.k1_valid = 1;
       } else {
         S.k1_valid = 0;
