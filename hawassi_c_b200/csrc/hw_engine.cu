@@ -475,8 +475,31 @@ bool hw_ctx::init(const std::vector<std::string>& dirs, const hw_opts* o, const 
       return false;
     }
     h.N = N;
-    const int slice = (member_slice && member_slice[i] > 0) ? member_slice[i] : (opt.slice > 0 ? opt.slice : 2048);
-    int C = opt.cluster > 0 ? opt.cluster : std::max(1, N / slice);
+    maxN = std::max(maxN, N);
+  }
+  // Slices.  2048 points fill the GPU best when there are members for every SM.  When
+  // there are not, a member's time is its CTA's, and smaller slices put more SMs on it:
+  // 512 points, or the eighth of the grid (clusters of 2, 4 and 8 have the fused cross-CTA
+  // steps), as long as no SM is given two CTAs.  Grids of up to 1024 points stay in one
+  // CTA, where no step crosses the cluster.  One flat HS2 member, us an RHS: 2048 points
+  // 28.4 (one CTA) 23.4 (512-point slices), 4096 points 38.0 (2048) 27.9 (1024) 24.0 (512);
+  // 1024 points 20.3 in one CTA, 24.1 in two.
+  auto points = [&](size_t i, int least) {
+    const int N = mem[i].N;
+    if (member_slice && member_slice[i] > 0) return member_slice[i];
+    if (opt.slice > 0) return opt.slice;
+    return N <= 1024 ? N : std::min(2048, std::max(least, N / 8));
+  };
+  int least = 512;
+  for (; least < 2048; least *= 2) {
+    long long ctas = 0;
+    for (size_t i = 0; i < mem.size(); ++i) ctas += std::max(1, mem[i].N / points(i, least));
+    if (ctas <= 148) break;
+  }
+  for (size_t i = 0; i < dirs.size(); ++i) {
+    HostMember& h = mem[i];
+    const int N = h.N;
+    int C = opt.cluster > 0 ? opt.cluster : std::max(1, N / points(i, least));
     if ((C & (C - 1)) != 0 || N / C < 256 || N / C > 2048 || C > 16) {
       err = "invalid cluster size " + std::to_string(C) + " for Nx=" + std::to_string(N);
       return false;
@@ -485,7 +508,6 @@ bool hw_ctx::init(const std::vector<std::string>& dirs, const hw_opts* o, const 
     h.M = N / C;
     h.logC = 0;
     while ((1 << h.logC) < C) ++h.logC;
-    maxN = std::max(maxN, N);
     if (!upload_member(h)) return false;
     if (opt.exact_sequence) h.d.exact = 1;
   }

@@ -32,7 +32,8 @@ typedef struct hw_opts {
     int exact_sequence;      /* 1: evaluate the RHS exactly where GSL does even when it is stateless */
     int cluster;             /* CTAs per member, power of two (0 = automatic) */
     int device;              /* CUDA device ordinal */
-    int slice;               /* grid points per CTA when cluster == 0 (0 = 2048) */
+    int slice;               /* grid points per CTA when cluster == 0 (0: 2048, or less where the
+                                members' CTAs would leave SMs idle) */
     int resident;            /* evolve launches of an ensemble: 0 = one cluster per member
                                 (members started longest first); -1 = a persistent grid per
                                 grid-size class, its clusters pulling members (longest first)
