@@ -1019,8 +1019,10 @@ __global__ void k2_begin(Ctl2* c, double t1) {
   if (!c->done) set_prologue(c);
 }
 
-// reference layout [Re eta | Im eta | Re u | Im u | Re v | Im v] <-> 3 double2 fields
-__global__ void k2_to_internal(const double* __restrict__ yr, double2* __restrict__ yi, size_t n) {
+// reference layout [Re eta | Im eta | Re u | Im u | Re v | Im v] <-> 3 double2 fields; with a
+// control block, the time of a direct right-hand side as well
+__global__ void k2_to_internal(const double* __restrict__ yr, double2* __restrict__ yi, size_t n, Ctl2* ctl, double t) {
+  if (ctl && blockIdx.x == 0 && threadIdx.x == 0) ctl->t_direct = t;
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < 3 * n; q += (size_t)gridDim.x * blockDim.x) {
     const size_t f = q / n, p = q - f * n;
     yi[q] = make_double2(yr[2 * f * n + p], yr[(2 * f + 1) * n + p]);

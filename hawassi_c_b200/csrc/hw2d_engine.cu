@@ -253,6 +253,7 @@ struct hw2d_ctx {
   Ctl2* hctl = nullptr;    // pinned host copy
   hw2d::Brk2 brk{};        // kinematic breaking (brk.on = 0: off)
   double* dref = nullptr;  // 6n staging for reference-layout transfers
+  double* href = nullptr;  // the same on small grids, mapped and pinned, for hw2d_rhs (behind hctl)
   double2* dout = nullptr; // 3n direct RHS output
   std::vector<void*> allocs;
   cudaGraphExec_t attempt = nullptr;
@@ -271,6 +272,10 @@ struct hw2d_ctx {
   int per_rhs = 5;
   std::string err;
 
+  // Grids whose right-hand side moves through a mapped buffer: one call in copies and so,
+  // 64x64 97 and 78 us, 128x64 121 and 97, 128x128 175 and 172, 256x128 270 and 312 (the
+  // host's own copy into the buffer costs more than the driver's staging)
+  static constexpr size_t kMappedPoints = 128 * 64;
   template <class T>
   T* dalloc(size_t count) {
     void* p = nullptr;
@@ -722,7 +727,15 @@ hw2d_ctx* hw2d_create(const hw2d_tables* t, const hw_opts* o) {
                               (var || (w.WP && tb.c2d && (!tb.refl_one || (tb.gwx && tb.gwy))))));
   for (int i = 0; i < 2; ++i) ok = ok && rk.y[i] && rk.kk[i];
   for (int i = 0; i < 5; ++i) ok = ok && rk.ks[i];
-  if (!ok || cudaMallocHost(&c->hctl, sizeof(Ctl2)) != cudaSuccess) {
+  // the pinned control block, with the mapped buffer behind it where there is one
+  const size_t mapped = n <= hw2d_ctx::kMappedPoints ? 6 * n : 0;
+  static_assert(sizeof(Ctl2) % sizeof(double) == 0, "the buffer follows aligned");
+  if (ok && cudaHostAlloc(&c->hctl, sizeof(Ctl2) + mapped * sizeof(double), cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    ok = false;
+  }
+  if (ok && mapped) c->href = reinterpret_cast<double*>(c->hctl + 1);
+  if (!ok) {
     g_err2d = "hw2d_create: device allocation failed";
     delete c;
     return nullptr;
@@ -761,15 +774,18 @@ int hw2d_rhs(hw2d_ctx* c, double t, const double* y, double* dydt) {
   if (!c || !y || !dydt) return 1;
   cudaSetDevice(c->device);
   const size_t n = c->n;
-  cudaMemcpyAsync(c->dref, y, 6 * n * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-  hw2d::k2_to_internal<<<592, 256, 0, c->stream>>>(c->dref, c->w.z, n);
-  cudaMemcpyAsync(&c->ctl->t_direct, &t, sizeof(double), cudaMemcpyHostToDevice, c->stream);
+  // the mapped buffer where there is one: the layout kernels read and write it over PCIe
+  double* ref = c->href ? c->href : c->dref;
+  if (c->href) std::memcpy(ref, y, 6 * n * sizeof(double));
+  else cudaMemcpyAsync(ref, y, 6 * n * sizeof(double), cudaMemcpyHostToDevice, c->stream);
+  hw2d::k2_to_internal<<<592, 256, 0, c->stream>>>(ref, c->w.z, n, c->ctl, t);
   c->rhs_launch(0, hw2d::kAlways, c->stream, c->dout);
-  hw2d::k2_to_reference<<<592, 256, 0, c->stream>>>(c->dout, c->dref, n);
+  hw2d::k2_to_reference<<<592, 256, 0, c->stream>>>(c->dout, ref, n);
   c->launches += c->per_rhs + 2;
-  cudaMemcpyAsync(dydt, c->dref, 6 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
+  if (!c->href) cudaMemcpyAsync(dydt, ref, 6 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
   if (const cudaError_t e = cudaStreamSynchronize(c->stream); e != cudaSuccess) return c->fail("hw2d_rhs", e);
   if (!c->check("hw2d_rhs")) return 1;
+  if (c->href) std::memcpy(dydt, ref, 6 * n * sizeof(double));
   if (c->brk.on) {
     hw2d::BrkSt st{};
     if (const cudaError_t e = cudaMemcpy(&st, c->brk.st, sizeof st, cudaMemcpyDeviceToHost); e != cudaSuccess)
@@ -800,7 +816,7 @@ int hw2d_set_state(hw2d_ctx* c, double t, double h, const double* y) {
   s.status = hw2d::kOk;
   *c->hctl = s;
   cudaMemcpyAsync(c->dref, y, 6 * c->n * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-  hw2d::k2_to_internal<<<592, 256, 0, c->stream>>>(c->dref, c->rk.y[0], c->n);
+  hw2d::k2_to_internal<<<592, 256, 0, c->stream>>>(c->dref, c->rk.y[0], c->n, nullptr, 0.0);
   c->launches += 1;
   cudaMemcpyAsync(c->ctl, c->hctl, sizeof(Ctl2), cudaMemcpyHostToDevice, c->stream);
   if (const cudaError_t e = cudaStreamSynchronize(c->stream); e != cudaSuccess) return c->fail("hw2d_set_state", e);

@@ -104,18 +104,27 @@ __global__ void __launch_bounds__(M / kPts, HW_EVOLVE_MIN_BLOCKS(M))
   member_sync(C);
 }
 
-// single RHS evaluation of member mi: kout = f(t, zs)
+// Single RHS evaluation of member mi: kout = f(t, zs).  With y_ref the state comes from
+// there and the result goes to dy_ref, both in the reference layout (4N doubles); with
+// scratch, the member's zs, kout and fields are in that array.
 template <int M>
-__global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs(DevMember* mems, const int* list, double t) {
+__global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs(DevMember* mems, int mi, double t,
+                                                              const double* y_ref, double* dy_ref,
+                                                              double2* scratch) {
   extern __shared__ double2 smem_buf[];
   __shared__ DevMember sd;
   __shared__ Scratch<M> sc;
   cg::cluster_group cl = cg::this_cluster();
   const int C = int(cl.num_blocks());
   const int rank = int(cl.block_rank());
-  const int mi = list[blockIdx.x / C];
   if (threadIdx.x == 0) {
     sd = mems[mi];
+    const int N = sd.N;
+    if (scratch) {
+      sd.zs = scratch;
+      sd.kb[6] = scratch + 2 * N;
+      for (int i = 0; i < kScratch; ++i) sd.sc[i] = scratch + size_t(4 + i) * N;
+    }
     sc.stg.s = 0;
     sc.stg.sig = -1;
     sc.full = 1;
@@ -123,11 +132,29 @@ __global__ void __launch_bounds__(M / kPts, (4096 / M)) k_rhs(DevMember* mems, c
   }
   __syncthreads();
   Ctx<M> X = make_ctx<M>(sd, smem_buf, sc, rank);
+  const int N = sd.N;
+  if (y_ref) {
+    // reference layout -> this CTA's spectral slice of the stage input
+    HW_FOREACH(X) {
+      const int kk = X.c + (idx << sd.logC);
+      sd.zs[p] = make_double2(y_ref[kk], y_ref[N + kk]);
+      sd.zs[N + p] = make_double2(y_ref[2 * N + kk], y_ref[3 * N + kk]);
+    }
+  }
   rhs_eval<M>(X, t, sd.kb[6]);
+  if (dy_ref) {
+    HW_FOREACH(X) {
+      const int kk = X.c + (idx << sd.logC);
+      const double2 e = sd.kb[6][p], u = sd.kb[6][N + p];
+      dy_ref[kk] = e.x;
+      dy_ref[N + kk] = e.y;
+      dy_ref[2 * N + kk] = u.x;
+      dy_ref[3 * N + kk] = u.y;
+    }
+  }
   member_sync(C);
   if (rank == 0 && threadIdx.x == 0) mems[mi].rhs_calls += 1;
 }
-
 
 template <int M>
 cudaError_t set_attrs() {
@@ -161,13 +188,11 @@ int max_clusters(int C) {
   return n;
 }
 
-// mode 0/1: evolve (nmem list entries; with a queue, ngrid resident clusters pull them);
-// mode 2: one RHS of each listed member
-template <int M>
-cudaError_t launch(int mode, DevMember* mems, const int* list, int nmem, int C, double t, cudaStream_t s,
-                   int* queue, int ngrid) {
+// a launch of `clusters` clusters of C CTAs
+template <int M, typename... P, typename... A>
+cudaError_t launch_clusters(void (*kernel)(P...), int clusters, int C, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned((queue && mode != 2 ? ngrid : nmem) * C));
+  cfg.gridDim = dim3(unsigned(clusters * C));
   cfg.blockDim = dim3(M / kPts);
   cfg.dynamicSmemBytes = slice_smem_bytes(M);
   cfg.stream = s;
@@ -178,16 +203,20 @@ cudaError_t launch(int mode, DevMember* mems, const int* list, int nmem, int C, 
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (mode == 2) return cudaLaunchKernelEx(&cfg, k_rhs<M>, mems, list, t);
-  return cudaLaunchKernelEx(&cfg, k_evolve<M>, mems, list, mode, queue, nmem);
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 }  // namespace hwdev
 
 #define HW_INSTANTIATE(MM)                                                                          \
   cudaError_t hw_attr_##MM() { return hwdev::set_attrs<MM>(); }                                    \
-  cudaError_t hw_launch_##MM(int mode, hwdev::DevMember* mems, const int* list, int nmem, int C,  \
-                             double t, cudaStream_t s, int* queue, int ngrid) {                     \
-    return hwdev::launch<MM>(mode, mems, list, nmem, C, t, s, queue, ngrid);                        \
+  cudaError_t hw_evolve_##MM(int mode, hwdev::DevMember* mems, const int* list, int nmem, int C,   \
+                             cudaStream_t s, int* queue, int ngrid) {                               \
+    return hwdev::launch_clusters<MM>(hwdev::k_evolve<MM>, queue ? ngrid : nmem, C, s, mems, list,  \
+                                      mode, queue, nmem);                                           \
+  }                                                                                                 \
+  cudaError_t hw_rhs_##MM(hwdev::DevMember* mems, int mi, int C, double t, const double* y,         \
+                          double* dy, double2* scratch, cudaStream_t s) {                           \
+    return hwdev::launch_clusters<MM>(hwdev::k_rhs<MM>, 1, C, s, mems, mi, t, y, dy, scratch);      \
   }                                                                                                 \
   int hw_max_clusters_##MM(int C) { return hwdev::max_clusters<MM>(C); }

@@ -7,8 +7,11 @@
 
 #define HW_DECLARE(MM)                                                                             \
   cudaError_t hw_attr_##MM();                                                                      \
-  cudaError_t hw_launch_##MM(int mode, hwdev::DevMember* mems, const int* list, int nmem, int C, \
-                             double t, cudaStream_t s, int* queue, int ngrid);                    \
+  /* mode 0 run, 1 one step, of the nmem listed members; with a queue, ngrid clusters pull them */ \
+  cudaError_t hw_evolve_##MM(int mode, hwdev::DevMember* mems, const int* list, int nmem, int C, \
+                             cudaStream_t s, int* queue, int ngrid);                              \
+  cudaError_t hw_rhs_##MM(hwdev::DevMember* mems, int mi, int C, double t, const double* y,       \
+                          double* dy, double2* scratch, cudaStream_t s);                          \
   int hw_max_clusters_##MM(int C);
 HW_DECLARE(256)
 HW_DECLARE(512)
