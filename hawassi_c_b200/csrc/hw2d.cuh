@@ -362,8 +362,6 @@ __device__ __forceinline__ double2 stage_value(const RK2& B, const Ctl2* c, int 
                           rm2(A2_b6[4], c5.y)))));
 }
 
-// ---------------------------------------------------------------------------
-// stage input z = y + h sum_j b_sj k_j of every point, a streaming pass ahead of the
 // the buffer an RHS of the given mode writes
 __device__ __forceinline__ double2* rhs_out(const RK2& rk, const Ctl2* ctl, int mode, double2* direct_out) {
   if (mode == 0) return direct_out;
@@ -372,13 +370,34 @@ __device__ __forceinline__ double2* rhs_out(const RK2& rk, const Ctl2* ctl, int 
   return rk.ks[mode - 2];
 }
 
-// first row pass (mode 1 and 7: z = y)
+// ---------------------------------------------------------------------------
+// Stage input z = y + h sum_j b_sj k_j, a streaming pass ahead of the first row pass (mode 1
+// and 7: z = y).  It and the combination move the points inside the alias mask alone:
+// outside it every k_j is zero, so z and both states are what they were when the run
+// began, which is when k2_spread writes them.  Bound by memory: at 1024^2 points, 39 in a
+// hundred of them inside, a right-hand side with its stage took 670 us, 650 so.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-k2_stage(RK2 rk, Work2 w, const Ctl2* __restrict__ ctl, int mode, int cond, size_t n3) {
+k2_stage(const double* __restrict__ aal, RK2 rk, Work2 w, const Ctl2* __restrict__ ctl, int mode, int cond, size_t n) {
   if (!rhs_active(ctl, cond)) return;
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n3; q += (size_t)gridDim.x * blockDim.x)
-    w.z[q] = stage_value(rk, ctl, mode, q);
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
+    if (aal[q] == 0.0) continue;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) w.z[f * n + q] = stage_value(rk, ctl, mode, f * n + q);
+  }
+}
+
+// the points outside the alias mask, in the stage input and the other state
+__global__ void __launch_bounds__(256)
+k2_spread(const double* __restrict__ aal, RK2 rk, Work2 w, const Ctl2* __restrict__ ctl, size_t n) {
+  if (ctl->done) return;
+  const double2* __restrict__ y = rk.y[ctl->cur];
+  double2* __restrict__ yn = rk.y[ctl->cur ^ 1];
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
+    if (aal[q] != 0.0) continue;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) w.z[f * n + q] = yn[f * n + q] = y[f * n + q];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -896,7 +915,7 @@ constexpr int kCombThreads = 256;
 
 // y_new = y + h0 sum c_i k_i into y[cur ^ 1]; per-block max of |yerr| / D0
 __global__ void __launch_bounds__(kCombThreads)
-k2_combine(RK2 rk, Work2 w, const Ctl2* __restrict__ ctl, size_t n3) {
+k2_combine(const double* __restrict__ aal, RK2 rk, Work2 w, const Ctl2* __restrict__ ctl, size_t n) {
   __shared__ double red[kCombThreads / 32];
   __shared__ int badw[kCombThreads / 32];
   if (ctl->done) return;
@@ -906,22 +925,27 @@ k2_combine(RK2 rk, Work2 w, const Ctl2* __restrict__ ctl, size_t n3) {
   const double2* __restrict__ k1 = rk.kk[ctl->k1i];
   double rm = 2.2250738585072014e-308;
   int bad = 0;
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n3; q += (size_t)gridDim.x * blockDim.x) {
-    const double2 a = k1[q], c = rk.ks[1][q], e = rk.ks[2][q], f = rk.ks[3][q], g = rk.ks[4][q], yy = y[q];
-    const double dix = ra2(ra2(ra2(ra2(rm2(A2_c[0], a.x), rm2(A2_c[1], c.x)), rm2(A2_c[2], e.x)), rm2(A2_c[3], f.x)),
-                           rm2(A2_c[4], g.x));
-    const double diy = ra2(ra2(ra2(ra2(rm2(A2_c[0], a.y), rm2(A2_c[1], c.y)), rm2(A2_c[2], e.y)), rm2(A2_c[3], f.y)),
-                           rm2(A2_c[4], g.y));
-    const double2 nv = make_double2(ra2(yy.x, rm2(h, dix)), ra2(yy.y, rm2(h, diy)));
-    yn[q] = nv;
-    const double ex = rm2(h, ra2(ra2(ra2(ra2(rm2(A2_ec[0], a.x), rm2(A2_ec[1], c.x)), rm2(A2_ec[2], e.x)),
-                                     rm2(A2_ec[3], f.x)), rm2(A2_ec[4], g.x)));
-    const double ey = rm2(h, ra2(ra2(ra2(ra2(rm2(A2_ec[0], a.y), rm2(A2_ec[1], c.y)), rm2(A2_ec[2], e.y)),
-                                     rm2(A2_ec[3], f.y)), rm2(A2_ec[4], g.y)));
-    const double rx = fabs(ex) / fabs(ra2(rm2(er, fabs(nv.x)), ea));
-    const double ry = fabs(ey) / fabs(ra2(rm2(er, fabs(nv.y)), ea));
-    bad |= (!(rx == rx) || !(ry == ry) || isinf(nv.x) || isinf(nv.y)) ? 1 : 0;
-    rm = fmax(rm, fmax(rx, ry));
+  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
+    if (aal[p] == 0.0) continue;
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      const size_t q = s * n + p;
+      const double2 a = k1[q], c = rk.ks[1][q], e = rk.ks[2][q], f = rk.ks[3][q], g = rk.ks[4][q], yy = y[q];
+      const double dix = ra2(ra2(ra2(ra2(rm2(A2_c[0], a.x), rm2(A2_c[1], c.x)), rm2(A2_c[2], e.x)), rm2(A2_c[3], f.x)),
+                             rm2(A2_c[4], g.x));
+      const double diy = ra2(ra2(ra2(ra2(rm2(A2_c[0], a.y), rm2(A2_c[1], c.y)), rm2(A2_c[2], e.y)), rm2(A2_c[3], f.y)),
+                             rm2(A2_c[4], g.y));
+      const double2 nv = make_double2(ra2(yy.x, rm2(h, dix)), ra2(yy.y, rm2(h, diy)));
+      yn[q] = nv;
+      const double ex = rm2(h, ra2(ra2(ra2(ra2(rm2(A2_ec[0], a.x), rm2(A2_ec[1], c.x)), rm2(A2_ec[2], e.x)),
+                                       rm2(A2_ec[3], f.x)), rm2(A2_ec[4], g.x)));
+      const double ey = rm2(h, ra2(ra2(ra2(ra2(rm2(A2_ec[0], a.y), rm2(A2_ec[1], c.y)), rm2(A2_ec[2], e.y)),
+                                       rm2(A2_ec[3], f.y)), rm2(A2_ec[4], g.y)));
+      const double rx = fabs(ex) / fabs(ra2(rm2(er, fabs(nv.x)), ea));
+      const double ry = fabs(ey) / fabs(ra2(rm2(er, fabs(nv.y)), ea));
+      bad |= (!(rx == rx) || !(ry == ry) || isinf(nv.x) || isinf(nv.y)) ? 1 : 0;
+      rm = fmax(rm, fmax(rx, ry));
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     rm = fmax(rm, __shfl_xor_sync(0xffffffffu, rm, o));

@@ -305,7 +305,7 @@ struct hw2d_ctx {
   }
   void rhs_launch(int mode, int cond, cudaStream_t s, double2* out) {
     const int rows = ny / 2, cols = nx / 2;
-    if (mode != 0) hw2d::k2_stage<<<hw2d::kCombBlocks, 256, 0, s>>>(rk, w, ctl, mode, cond, 3 * n);
+    if (mode != 0) hw2d::k2_stage<<<hw2d::kCombBlocks, 256, 0, s>>>(tb.aal, rk, w, ctl, mode, cond, n);
     per_rhs = 1;
     const PassArgs a{s, tb, w, rk, ctl, mode, cond, out};
     auto row = [&](RowPass p, int cubic = 0) { row_pass(p, a, cubic); ++per_rhs; };
@@ -362,19 +362,22 @@ struct hw2d_ctx {
     brk_row(nx, 1, rows, s, tb, w, brk, rk, ctl, mode, cond, out);
     per_rhs += 8;
   }
-  long long kernels_per_attempt() const { return 7LL * per_rhs + 3; }
+  long long kernels_per_attempt() const { return (brk.on ? 7LL : 6LL) * per_rhs + 3; }
+  // One attempt of a step.  Without breaking only a run's first attempt forms its own k1
+  // (an accepted one leaves the next one's), so that right-hand side is launched ahead of the
+  // attempts: as a conditional part of each it was six to thirteen empty kernels of 1.3 us.
   void attempt_launch(cudaStream_t s) {
-    rhs_launch(1, hw2d::kIfK1, s, nullptr);
+    if (brk.on) rhs_launch(1, hw2d::kIfK1, s, nullptr);
     for (int st = 2; st <= 6; ++st) rhs_launch(st, hw2d::kIfStage, s, nullptr);
     if (brk.on) {
       // gsl_odeiv2's order: dydt_out of the candidate state before the step control
-      hw2d::k2_combine<<<hw2d::kCombBlocks, hw2d::kCombThreads, 0, s>>>(rk, w, ctl, 3 * n);
+      hw2d::k2_combine<<<hw2d::kCombBlocks, hw2d::kCombThreads, 0, s>>>(tb.aal, rk, w, ctl, n);
       rhs_launch(8, hw2d::kIfStage, s, nullptr);
       hw2d::k2_control<<<1, 256, 0, s>>>(ctl, w, hw2d::kCombBlocks);
       hw2d::k2_finalize<<<1, 1, 0, s>>>(ctl);
       return;
     }
-    hw2d::k2_combine<<<hw2d::kCombBlocks, hw2d::kCombThreads, 0, s>>>(rk, w, ctl, 3 * n);
+    hw2d::k2_combine<<<hw2d::kCombBlocks, hw2d::kCombThreads, 0, s>>>(tb.aal, rk, w, ctl, n);
     hw2d::k2_control<<<1, 256, 0, s>>>(ctl, w, hw2d::kCombBlocks);
     rhs_launch(7, hw2d::kIfKout, s, nullptr);
     hw2d::k2_finalize<<<1, 1, 0, s>>>(ctl);
@@ -414,18 +417,26 @@ struct hw2d_ctx {
   int run(double t1, bool one_step) {
     if (!build_graph()) return 1;
     hw2d::k2_begin<<<1, 1, 0, stream>>>(ctl, t1);
-    launches += 1;
+    hw2d::k2_spread<<<hw2d::kCombBlocks, 256, 0, stream>>>(tb.aal, rk, w, ctl, n);
+    launches += 2;
     if (!check("begin")) return 1;
     if (!read_ctl()) return 1;
     const long long acc0 = hctl->acc;
-    int batch = one_step ? 1 : 2;
     long long launched = 0;
+    if (!brk.on && !hctl->done && hctl->need_k1) {
+      rhs_launch(1, hw2d::kIfK1, stream, nullptr);
+      launches += per_rhs;
+      if (!check("first right-hand side")) return 1;
+    }
     for (;;) {
       if (hctl->done) break;
       if (launched > kMaxAttemptsPerRun) {
         err = "time integration stopped: attempt budget of one run exceeded (step size collapsed)";
         return 1;
       }
+      // as many attempts as the present step asks for, sixteen at most: one past the end is
+      // some forty empty kernels (50 us), one short another read of the control block (15 us)
+      const int batch = one_step ? 1 : (int)std::min(16.0, std::max(1.0, std::ceil((t1 - hctl->t) / hctl->h - 0.01)));
       launched += batch;
       for (int b = 0; b < batch; ++b)
         if (const cudaError_t e = cudaGraphLaunch(attempt, stream); e != cudaSuccess) return fail("graph launch", e);
@@ -436,7 +447,6 @@ struct hw2d_ctx {
         // stop here: the next call recomputes its dydt_in like GSL's evolve_apply
         break;
       }
-      if (!one_step && batch < 16) batch *= 2;
     }
     if (hctl->status == hw2d::kNonFinite) { err = "non-finite state (the step size collapsed)"; return 1; }
     if (hctl->status == hw2d::kStepFailed) { err = "time integration failed (too many rejected steps)"; return 1; }
