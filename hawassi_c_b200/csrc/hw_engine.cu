@@ -532,17 +532,18 @@ bool hw_ctx::init(const std::vector<std::string>& dirs, const hw_opts* o, const 
     maxN = std::max(maxN, N);
   }
   // Slices.  2048 points fill the GPU best when there are members for every SM.  When
-  // there are not, a member's time is its CTA's, and smaller slices put more SMs on it:
-  // 512 points, or the eighth of the grid (clusters of 2, 4 and 8 have the fused cross-CTA
-  // steps), as long as no SM is given two CTAs.  Grids of up to 1024 points stay in one
-  // CTA, where no step crosses the cluster.  One flat HS2 member, us an RHS: 2048 points
-  // 28.4 (one CTA) 23.4 (512-point slices), 4096 points 38.0 (2048) 27.9 (1024) 24.0 (512);
-  // 1024 points 20.3 in one CTA, 24.1 in two.
+  // there are not, a member's time is its CTA's, and smaller slices put more SMs on it, as
+  // long as no SM is given two CTAs: 512 points up to eight CTAs, 1024 up to sixteen.  Grids
+  // of up to 1024 points stay in one CTA, where no step crosses the cluster.  One member, us an
+  // RHS in slices of 2048, 1024, 512 and 256 points: flat HS2 of 2048 points 27 27 24 24, of
+  // 4096 37 28 24 30, of 8192 39 28 30, of 16384 41 36; HS3 on a slope (sixteen reference
+  // depths) of 4096 367 275 253 302, of 8192 395 303 302, of 16384 430 359; flat of 1024 in
+  // one CTA 20, in two 24.
   auto points = [&](size_t i, int least) {
     const int N = mem[i].N;
     if (member_slice && member_slice[i] > 0) return member_slice[i];
     if (opt.slice > 0) return opt.slice;
-    return N <= 1024 ? N : std::min(2048, std::max(least, N / 8));
+    return N <= 1024 ? N : std::min(2048, std::max({least, N / 16, std::min(N / 8, 1024)}));
   };
   int least = 512;
   for (; least < 2048; least *= 2) {

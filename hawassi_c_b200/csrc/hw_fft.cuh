@@ -306,64 +306,137 @@ __device__ __forceinline__ void local_fft(double2* buf, const double2* __restric
 // the thread owning position i gathers the C values at i from every CTA's slice,
 // applies the C-point DFT (forward: then the twiddles W_N^(i k1); inverse: the
 // twiddles W_N^-(i k1) first) and stores output j into CTA j's slice at i.
-// Every position is owned by exactly one thread of the cluster, which reads and
-// then rewrites it in every CTA, so the scatter needs no barrier after the gather:
-// one cluster barrier before (the slices are complete) and one after.
+// Every position is owned by exactly one thread of the cluster -- with sixteen CTAs by two
+// neighbouring lanes, which have eight of its sixteen values each -- so the values are
+// rewritten without a barrier after they were read: one cluster barrier before (the slices
+// are complete) and one after.
+// (A sum over sixteen peers for each point instead, with two barriers more and the products
+// in shared memory, left sixteen CTAs slower than eight; now 16384 points on a slope take
+// 359 us an RHS in sixteen and 430 in eight.)
+template <int C>
+struct Cross {
+  static constexpr int H = C > kPts ? C / kPts : 1;   // threads to a position
+  static constexpr int R = C / H;                     // values to a thread
+  static constexpr int PER = kPts / R;                // positions to a thread
+  static_assert(H == 1 || H == 2, "clusters of up to 16 CTAs");
+  static __device__ __forceinline__ int half() { return H > 1 ? int(threadIdx.x) & (H - 1) : 0; }
+  // the q-th position of this thread in CTA c; value e's CTA on the spectral and the physical side
+  template <int T>
+  static __device__ __forceinline__ int at(int c, int q) {
+    return c * (T / H) + int(threadIdx.x) / H + q * (C * T / H);
+  }
+  static __device__ __forceinline__ int spectral(int e) { return e * H + half(); }
+  static __device__ __forceinline__ int physical(int e) { return e + R * half(); }
+};
+
+// values v of one position from the spectral to the physical side, and back.  The twiddles
+// are formed anew on each side: kept across the pointwise work they took the registers that
+// its loads need.  With two threads to a position the 16-point DFT is two 8-point ones
+// (even and odd CTAs) and a butterfly between the lanes; each lane stores only after the
+// exchange, and so after its partner's loads.
+__device__ __forceinline__ double2 lane_swap(double2 v) {
+  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, 1), __shfl_xor_sync(0xffffffffu, v.y, 1));
+}
+// x exp(sign 2 pi i n / 16), n = 0..7
+template <int N16>
+__device__ __forceinline__ double2 rot16(double2 a, int sign) {
+  constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173, r = 0.70710678118654752440;
+  constexpr double co[8] = {1.0, c1, r, s1, 0.0, -s1, -r, -c1}, si[8] = {0.0, s1, r, c1, 1.0, c1, r, s1};
+  if constexpr (N16 == 0) return a;
+  if constexpr (N16 == 4) return mul_pm_i(a, sign);
+  const double sg = double(sign), c = co[N16], t = si[N16];
+  return make_double2(c * a.x - sg * t * a.y, c * a.y + sg * t * a.x);
+}
+template <int N16 = 0>
+__device__ __forceinline__ void lanes_in(double2* v, int h) {
+  if constexpr (N16 < 8) {
+    if (h) v[N16] = rot16<N16>(v[N16], +1);
+    const double2 p = lane_swap(v[N16]);
+    v[N16] = h ? csub(p, v[N16]) : cadd(v[N16], p);
+    lanes_in<N16 + 1>(v, h);
+  }
+}
+template <int N16 = 0>
+__device__ __forceinline__ void lanes_out(double2* v, int h) {
+  if constexpr (N16 < 8) {
+    const double2 p = lane_swap(v[N16]);
+    v[N16] = h ? rot16<N16>(csub(p, v[N16]), -1) : cadd(v[N16], p);
+    lanes_out<N16 + 1>(v, h);
+  }
+}
+// the position's twiddles: value e times W_N^(sign i spectral(e))
+template <int C>
+__device__ __forceinline__ void cross_twiddle(double2* v, const double2* __restrict__ tw, int i, int sign) {
+  using X = Cross<C>;
+  double2 w[X::R > 1 ? X::R : 2];
+  twiddle_powers<X::R>(twd(tw, X::H * i, sign), w);
+#pragma unroll
+  for (int e = 1; e < X::R; ++e) v[e] = cmul(v[e], w[e]);
+  if constexpr (X::H > 1) {
+    if (X::half()) {
+      const double2 w1 = twd(tw, i, sign);
+#pragma unroll
+      for (int e = 0; e < X::R; ++e) v[e] = cmul(v[e], w1);
+    }
+  }
+}
+template <int C>
+__device__ __forceinline__ void cross_in(double2* v, const double2* __restrict__ tw, int i) {
+  cross_twiddle<C>(v, tw, i, +1);
+  dft_small<Cross<C>::R>(v, +1);
+  if constexpr (Cross<C>::H > 1) lanes_in(v, Cross<C>::half());
+}
+template <int C>
+__device__ __forceinline__ void cross_out(double2* v, const double2* __restrict__ tw, int i) {
+  if constexpr (Cross<C>::H > 1) lanes_out(v, Cross<C>::half());
+  dft_small<Cross<C>::R>(v, -1);
+  cross_twiddle<C>(v, tw, i, -1);
+}
+
 template <int M, int C, int NBUF>
 __device__ __forceinline__ void cross_gs(double2* A, double2* B, const double2* __restrict__ tw, int c, int sign) {
+  using X = Cross<C>;
   constexpr int T = M / kPts;
-  constexpr int PER = kPts / C;   // positions per thread
   cg::cluster_group cl = cg::this_cluster();
-  double2 va[PER][C], vb[PER][C];
+  double2 va[X::PER][X::R], vb[X::PER][X::R];
   cl.sync();
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int i = c * T + threadIdx.x + q * (C * T);
+  for (int q = 0; q < X::PER; ++q) {
+    const int i = X::template at<T>(c, q);
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      va[q][r] = cl.map_shared_rank(A, r)[pidx(i)];
-      if constexpr (NBUF == 2) vb[q][r] = cl.map_shared_rank(B, r)[pidx(i)];
+    for (int e = 0; e < X::R; ++e) {
+      const int r = sign > 0 ? X::spectral(e) : X::physical(e);
+      va[q][e] = cl.map_shared_rank(A, r)[pidx(i)];
+      if constexpr (NBUF == 2) vb[q][e] = cl.map_shared_rank(B, r)[pidx(i)];
     }
   }
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int i = c * T + threadIdx.x + q * (C * T);
-    double2 w[C > 1 ? C : 2];
-    if (sign > 0) {   // inverse: twiddle by W_N^(+i k1) before the DFT over k1
-      twiddle_powers<C>(twd(tw, i, +1), w);
-#pragma unroll
-      for (int r = 1; r < C; ++r) {
-        va[q][r] = cmul(va[q][r], w[r]);
-        if constexpr (NBUF == 2) vb[q][r] = cmul(vb[q][r], w[r]);
-      }
-    }
-    dft_small<C>(va[q], sign);
-    if constexpr (NBUF == 2) dft_small<C>(vb[q], sign);
-    if (sign < 0) {   // forward: output k1 gets W_N^(-i k1)
-      twiddle_powers<C>(twd(tw, i, -1), w);
-#pragma unroll
-      for (int r = 1; r < C; ++r) {
-        va[q][r] = cmul(va[q][r], w[r]);
-        if constexpr (NBUF == 2) vb[q][r] = cmul(vb[q][r], w[r]);
-      }
+  for (int q = 0; q < X::PER; ++q) {
+    const int i = X::template at<T>(c, q);
+    if (sign > 0) {
+      cross_in<C>(va[q], tw, i);
+      if constexpr (NBUF == 2) cross_in<C>(vb[q], tw, i);
+    } else {
+      cross_out<C>(va[q], tw, i);
+      if constexpr (NBUF == 2) cross_out<C>(vb[q], tw, i);
     }
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      cl.map_shared_rank(A, r)[pidx(i)] = va[q][r];
-      if constexpr (NBUF == 2) cl.map_shared_rank(B, r)[pidx(i)] = vb[q][r];
+    for (int e = 0; e < X::R; ++e) {
+      const int r = sign > 0 ? X::physical(e) : X::spectral(e);
+      cl.map_shared_rank(A, r)[pidx(i)] = va[q][e];
+      if constexpr (NBUF == 2) cl.map_shared_rank(B, r)[pidx(i)] = vb[q][e];
     }
   }
   cl.sync();
 }
 
-// dispatch on the cluster size (2, 4, 8); returns false for other sizes
+// dispatch on the cluster size
 template <int M, int NBUF>
-__device__ __forceinline__ bool cross_fast(double2* A, double2* B, const double2* __restrict__ tw, int C, int c,
-                                           int sign) {
-  if (C == 2) { cross_gs<M, 2, NBUF>(A, B, tw, c, sign); return true; }
-  if (C == 4) { cross_gs<M, 4, NBUF>(A, B, tw, c, sign); return true; }
-  if (C == 8) { cross_gs<M, 8, NBUF>(A, B, tw, c, sign); return true; }
-  return false;
+__device__ __forceinline__ void cross_step(double2* A, double2* B, const double2* __restrict__ tw, int C, int c, int sign) {
+  if (C == 2) cross_gs<M, 2, NBUF>(A, B, tw, c, sign);
+  else if (C == 4) cross_gs<M, 4, NBUF>(A, B, tw, c, sign);
+  else if (C == 8) cross_gs<M, 8, NBUF>(A, B, tw, c, sign);
+  else cross_gs<M, 16, NBUF>(A, B, tw, c, sign);
 }
 
 // cluster-wide barrier (block barrier when the member is a single CTA)
@@ -374,139 +447,34 @@ __device__ __forceinline__ void member_sync(int C) {
 
 // Forward FFT: physical block slice in buf -> spectral cyclic slice in buf.
 template <int M>
-__device__ __noinline__ void fft_forward(double2* buf, const double2* __restrict__ tw, int N, int C, int c) {
-  if (C == 1) __syncthreads();
-  if (C > 1 && cross_fast<M, 1>(buf, buf, tw, C, c, -1)) {
-    local_fft<M>(buf, tw, C, -1);
-    return;
-  }
-  if (C > 1) {
-    constexpr int T = M / kPts;
-    cg::cluster_group cl = cg::this_cluster();
-    cl.sync();
-    double2 acc[kPts];
-    const int NC = N / C;
-#pragma unroll
-    for (int u = 0; u < kPts; ++u) {
-      const int i = threadIdx.x + u * T;
-      double2 s = make_double2(0.0, 0.0);
-      for (int n1 = 0; n1 < C; ++n1) {
-        const double2* pb = cl.map_shared_rank(buf, n1);
-        double2 x = pb[pidx(i)];
-        s = cadd(s, cmul(x, twd(tw, ((n1 * c) % C) * NC, -1)));
-      }
-      acc[u] = cmul(s, twd(tw, i * c, -1));
-    }
-    cl.sync();
-#pragma unroll
-    for (int u = 0; u < kPts; ++u) buf[pidx(threadIdx.x + u * T)] = acc[u];
-    __syncthreads();
-  }
+__device__ __noinline__ void fft_forward(double2* buf, const double2* __restrict__ tw, int C, int c) {
+  if (C > 1) cross_step<M, 1>(buf, buf, tw, C, c, -1);
+  else __syncthreads();
   local_fft<M>(buf, tw, C, -1);
 }
 
 // Inverse FFT (unnormalised): spectral cyclic slice in buf -> physical block slice in buf.
 template <int M>
-__device__ __noinline__ void fft_inverse(double2* buf, const double2* __restrict__ tw, int N, int C, int c) {
+__device__ __noinline__ void fft_inverse(double2* buf, const double2* __restrict__ tw, int C, int c) {
   __syncthreads();
   local_fft<M>(buf, tw, C, +1);
-  if (C > 1 && cross_fast<M, 1>(buf, buf, tw, C, c, +1)) {
-    __syncthreads();
-    return;
-  }
-  if (C > 1) {
-    constexpr int T = M / kPts;
-    cg::cluster_group cl = cg::this_cluster();
-    cl.sync();
-    double2 acc[kPts];
-    const int NC = N / C;
-#pragma unroll
-    for (int u = 0; u < kPts; ++u) {
-      const int i = threadIdx.x + u * T;
-      double2 s = make_double2(0.0, 0.0);
-      for (int k1 = 0; k1 < C; ++k1) {
-        const double2* pb = cl.map_shared_rank(buf, k1);
-        double2 z = cmul(pb[pidx(i)], twd(tw, i * k1, +1));
-        s = cadd(s, cmul(z, twd(tw, ((c * k1) % C) * NC, +1)));
-      }
-      acc[u] = s;
-    }
-    cl.sync();
-#pragma unroll
-    for (int u = 0; u < kPts; ++u) buf[pidx(threadIdx.x + u * T)] = acc[u];
-    __syncthreads();
-  }
+  if (C > 1) cross_step<M, 1>(buf, buf, tw, C, c, +1);
 }
 
-}  // namespace hwdev
-
-namespace hwdev {
-
-// ---------------------------------------------------------------------------
 // Dual transforms: two M-point slices (A and B) in one sweep -- twice the
 // independent work per thread, one set of twiddle loads and barriers for both.
-// ---------------------------------------------------------------------------
-// cross-CTA step of the distributed transform for both slices (see fft_forward /
-// fft_inverse): forward = C-point DFT then twiddle, inverse = twiddle then DFT.
 template <int M>
-__device__ __forceinline__ void cross_step2(double2* A, double2* B, const double2* __restrict__ tw, int N, int C,
-                                            int c, int sign) {
-  constexpr int T = M / kPts;
-  cg::cluster_group cl = cg::this_cluster();
-  cl.sync();
-  double2 sa[kPts], sb[kPts];
-  const int NC = N / C;
-#pragma unroll
-  for (int u = 0; u < kPts; ++u) {
-    const int i = threadIdx.x + u * T;
-    double2 a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
-    for (int r = 0; r < C; ++r) {
-      const double2* pa = cl.map_shared_rank(A, r);
-      const double2* pb = cl.map_shared_rank(B, r);
-      double2 xa = pa[pidx(i)], xb = pb[pidx(i)];
-      if (sign > 0) {   // inverse: peer r is the spectral class k1 = r
-        const double2 w = twd(tw, i * r, +1);
-        xa = cmul(xa, w);
-        xb = cmul(xb, w);
-      }
-      const double2 wc = twd(tw, ((r * c) % C) * NC, sign);
-      a = cadd(a, cmul(xa, wc));
-      b = cadd(b, cmul(xb, wc));
-    }
-    if (sign < 0) {
-      const double2 w = twd(tw, i * c, -1);
-      a = cmul(a, w);
-      b = cmul(b, w);
-    }
-    sa[u] = a;
-    sb[u] = b;
-  }
-  cl.sync();
-#pragma unroll
-  for (int u = 0; u < kPts; ++u) {
-    A[pidx(threadIdx.x + u * T)] = sa[u];
-    B[pidx(threadIdx.x + u * T)] = sb[u];
-  }
-  __syncthreads();
-}
-
-template <int M>
-__device__ __noinline__ void fft_forward2(double2* A, double2* B, const double2* __restrict__ tw, int N, int C,
-                                          int c) {
-  __syncthreads();
-  if (C > 1 && !cross_fast<M, 2>(A, B, tw, C, c, -1)) cross_step2<M>(A, B, tw, N, C, c, -1);
+__device__ __noinline__ void fft_forward2(double2* A, double2* B, const double2* __restrict__ tw, int C, int c) {
+  if (C > 1) cross_step<M, 2>(A, B, tw, C, c, -1);
+  else __syncthreads();
   local_fft2<M>(A, B, tw, C, -1);
 }
 
 template <int M>
-__device__ __noinline__ void fft_inverse2(double2* A, double2* B, const double2* __restrict__ tw, int N, int C,
-                                          int c) {
+__device__ __noinline__ void fft_inverse2(double2* A, double2* B, const double2* __restrict__ tw, int C, int c) {
   __syncthreads();
   local_fft2<M>(A, B, tw, C, +1);
-  if (C > 1) {
-    if (!cross_fast<M, 2>(A, B, tw, C, c, +1)) cross_step2<M>(A, B, tw, N, C, c, +1);
-    __syncthreads();
-  }
+  if (C > 1) cross_step<M, 2>(A, B, tw, C, c, +1);
 }
 
 // The local (in-CTA) part of a distributed transform alone, for callers that do the

@@ -70,7 +70,7 @@ __device__ __noinline__ void output_stage(Ctx<M> X, StepState& S, int row) {
     (void)p;
     A[pidx(idx)] = va[u];
   }
-  fft_inverse<M>(A, d.tw, N, C, X.c);
+  fft_inverse<M>(A, d.tw, C, X.c);
   member_sync(C);
   // A: (eta, d eta / dt) at grid points c*M + i
   double* fr = d.fields ? d.fields + (size_t)row * 3 * N : nullptr;
@@ -180,7 +180,7 @@ __device__ __noinline__ void output_stage(Ctx<M> X, StepState& S, int row) {
     (void)p;
     A[pidx(idx)] = va[u];
   }
-  fft_inverse<M>(A, d.tw, N, C, X.c);
+  fft_inverse<M>(A, d.tw, C, X.c);
   member_sync(C);
   HW_FOREACH(X) {
     (void)p;

@@ -187,7 +187,7 @@ __device__ __forceinline__ double2 mul_ik(double a, double2 b) {
 template <int M, class F>
 __device__ __forceinline__ void fft_forward_split(Ctx<M> X, F&& f) {
   const DevMember& d = X.d;
-  fft_forward<M>(X.buf, d.tw, d.N, d.C, X.c);
+  fft_forward<M>(X.buf, d.tw, d.C, X.c);
   const double2* pb = X.buf;
   if (d.C > 1) {
     cg::cluster_group cl = cg::this_cluster();
@@ -209,7 +209,7 @@ __device__ __forceinline__ void fft_forward_split(Ctx<M> X, F&& f) {
 template <int M, class G>
 __device__ __forceinline__ void fft_inverse_then(Ctx<M> X, G&& g) {
   const DevMember& d = X.d;
-  fft_inverse<M>(X.buf, d.tw, d.N, d.C, X.c);
+  fft_inverse<M>(X.buf, d.tw, d.C, X.c);
   HW_FOREACH(X) { g(u, idx, p, X.buf[pidx(idx)]); }
 }
 

@@ -176,25 +176,6 @@ __device__ __forceinline__ double2 source_term(int mode, double2 gx, double2 gs,
 // forward C-point DFT, twiddle, scatter.  Two cluster barriers replace four and the
 // physical fields never pass through shared memory.
 
-// The twiddles are formed anew on each side: kept across the pointwise work they took
-// the registers that its loads need.
-template <int C>
-__device__ __forceinline__ void cross_in(double2* v, const double2* __restrict__ tw, int i) {
-  double2 w[C > 1 ? C : 2];
-  twiddle_powers<C>(twd(tw, i, +1), w);
-#pragma unroll
-  for (int r = 1; r < C; ++r) v[r] = cmul(v[r], w[r]);
-  dft_small<C>(v, +1);
-}
-template <int C>
-__device__ __forceinline__ void cross_out(double2* v, const double2* __restrict__ tw, int i) {
-  double2 w[C > 1 ? C : 2];
-  dft_small<C>(v, -1);
-  twiddle_powers<C>(twd(tw, i, -1), w);
-#pragma unroll
-  for (int r = 1; r < C; ++r) v[r] = cmul(v[r], w[r]);
-}
-
 // What the first meeting does at physical point n (1d/functions.c:1486-1498), given
 // e = (eta, u), m = (M0 u, H(eta)): a <- (eta u) + i (eta M0 u), b <- u^2 - (M0 u)^2.
 // (eta, u) goes to global memory where the damping zones read it back, and with
@@ -228,32 +209,33 @@ __device__ __forceinline__ void adjust_point(const double2* PE, int n, double ch
 
 template <int M, int C>
 __device__ __forceinline__ void cross_products(Ctx<M> X, double2* A, double2* B, double2* PE, double2* PM) {
-  constexpr int T = M / kPts;
-  constexpr int PER = kPts / C;
+  using P = Cross<C>;
+  constexpr int T = M / kPts, R = P::R;
   const DevMember& d = X.d;
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int i = X.c * T + int(threadIdx.x) + q * (C * T);
-    double2 va[C], vb[C];
-    double dm[C];
+  for (int q = 0; q < P::PER; ++q) {
+    const int i = P::template at<T>(X.c, q);
+    double2 va[R], vb[R];
+    double dm[R];
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      va[r] = cl.map_shared_rank(A, r)[pidx(i)];
-      vb[r] = cl.map_shared_rank(B, r)[pidx(i)];
-      dm[r] = __ldg(d.damp + r * M + i);
+    for (int e = 0; e < R; ++e) {
+      va[e] = cl.map_shared_rank(A, P::spectral(e))[pidx(i)];
+      vb[e] = cl.map_shared_rank(B, P::spectral(e))[pidx(i)];
+      dm[e] = __ldg(d.damp + P::physical(e) * M + i);
     }
     cross_in<C>(va, d.tw, i);
     cross_in<C>(vb, d.tw, i);
 #pragma unroll
-    for (int r = 0; r < C; ++r) product_point<M>(X, r * M + i, va[r], vb[r], dm[r], PE, PM, va[r], vb[r]);
+    for (int e = 0; e < R; ++e)
+      product_point<M>(X, P::physical(e) * M + i, va[e], vb[e], dm[e], PE, PM, va[e], vb[e]);
     cross_out<C>(va, d.tw, i);
     cross_out<C>(vb, d.tw, i);
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      cl.map_shared_rank(A, r)[pidx(i)] = va[r];
-      cl.map_shared_rank(B, r)[pidx(i)] = vb[r];
+    for (int e = 0; e < R; ++e) {
+      cl.map_shared_rank(A, P::spectral(e))[pidx(i)] = va[e];
+      cl.map_shared_rank(B, P::spectral(e))[pidx(i)] = vb[e];
     }
   }
   cl.sync();
@@ -261,31 +243,31 @@ __device__ __forceinline__ void cross_products(Ctx<M> X, double2* A, double2* B,
 
 template <int M, int C>
 __device__ __forceinline__ void cross_adjust(Ctx<M> X, double2* A, double2* B, const double2* PE) {
-  constexpr int T = M / kPts;
-  constexpr int PER = kPts / C;
+  using P = Cross<C>;
+  constexpr int T = M / kPts, R = P::R;
   const DevMember& d = X.d;
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int i = X.c * T + int(threadIdx.x) + q * (C * T);
-    double2 va[C], vb[C];
-    double dm[C], ch[C];
+  for (int q = 0; q < P::PER; ++q) {
+    const int i = P::template at<T>(X.c, q);
+    double2 va[R], vb[R];
+    double dm[R], ch[R];
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      va[r] = cl.map_shared_rank(A, r)[pidx(i)];
-      dm[r] = __ldg(d.damp + r * M + i);
-      ch[r] = __ldg(d.chi + r * M + i);
+    for (int e = 0; e < R; ++e) {
+      va[e] = cl.map_shared_rank(A, P::spectral(e))[pidx(i)];
+      dm[e] = __ldg(d.damp + P::physical(e) * M + i);
+      ch[e] = __ldg(d.chi + P::physical(e) * M + i);
     }
     cross_in<C>(va, d.tw, i);
 #pragma unroll
-    for (int r = 0; r < C; ++r) adjust_point(PE, r * M + i, ch[r], dm[r], va[r], vb[r]);
+    for (int e = 0; e < R; ++e) adjust_point(PE, P::physical(e) * M + i, ch[e], dm[e], va[e], vb[e]);
     cross_out<C>(va, d.tw, i);
     cross_out<C>(vb, d.tw, i);
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      cl.map_shared_rank(A, r)[pidx(i)] = va[r];
-      cl.map_shared_rank(B, r)[pidx(i)] = vb[r];
+    for (int e = 0; e < R; ++e) {
+      cl.map_shared_rank(A, P::spectral(e))[pidx(i)] = va[e];
+      cl.map_shared_rank(B, P::spectral(e))[pidx(i)] = vb[e];
     }
   }
   cl.sync();
@@ -295,13 +277,15 @@ template <int M>
 __device__ __forceinline__ void cross_products_any(Ctx<M> X, double2* A, double2* B, double2* PE, double2* PM) {
   if (X.d.C == 2) cross_products<M, 2>(X, A, B, PE, PM);
   else if (X.d.C == 4) cross_products<M, 4>(X, A, B, PE, PM);
-  else cross_products<M, 8>(X, A, B, PE, PM);
+  else if (X.d.C == 8) cross_products<M, 8>(X, A, B, PE, PM);
+  else cross_products<M, 16>(X, A, B, PE, PM);
 }
 template <int M>
 __device__ __forceinline__ void cross_adjust_any(Ctx<M> X, double2* A, double2* B, const double2* PE) {
   if (X.d.C == 2) cross_adjust<M, 2>(X, A, B, PE);
   else if (X.d.C == 4) cross_adjust<M, 4>(X, A, B, PE);
-  else cross_adjust<M, 8>(X, A, B, PE);
+  else if (X.d.C == 8) cross_adjust<M, 8>(X, A, B, PE);
+  else cross_adjust<M, 16>(X, A, B, PE);
 }
 
 // Assembly of dz (1d/rhs.c:217-228, 373-385, 73-83): delta H1 + adjusted nonlinear terms
@@ -399,7 +383,7 @@ __device__ __noinline__ void finish_rhs(Ctx<M> X, double2* __restrict__ dz, cons
   double2* A = X.buf;
   double2* Bf = X.buf2();
   const double2* PE = d.sc[0];
-  if (C == 2 || C == 4 || C == 8) {
+  if (C > 1) {
     fft_local<M>(A, d.tw, C, +1);
     cross_adjust_any<M>(X, A, Bf, PE);
     fft_local2<M>(A, Bf, d.tw, C, -1);
@@ -410,14 +394,14 @@ __device__ __noinline__ void finish_rhs(Ctx<M> X, double2* __restrict__ dz, cons
       dm[u] = __ldg(d.damp + p);
       ch[u] = __ldg(d.chi + p);
     }
-    fft_inverse<M>(A, d.tw, d.N, C, X.c);
+    fft_inverse<M>(A, d.tw, C, X.c);
     HW_FOREACH(X) {
       double2 a = A[pidx(idx)], b;
       adjust_point(PE, p, ch[u], dm[u], a, b);
       A[pidx(idx)] = a;
       Bf[pidx(idx)] = b;
     }
-    fft_forward2<M>(A, Bf, d.tw, d.N, C, X.c);
+    fft_forward2<M>(A, Bf, d.tw, C, X.c);
   }
   member_sync(C);
   // (the leader's word is in every CTA since the transforms' barriers)
@@ -465,7 +449,7 @@ __device__ __noinline__ void rhs_hs2_flat(Ctx<M> X, double t, double2* __restric
   breaking_reset(X);
   stage_phase<M, kWithM0Hilbert>(X);
   // (2) products in physical space (1d/functions.c:1486-1498)
-  const bool fused = C == 2 || C == 4 || C == 8;
+  const bool fused = C > 1;
   if (fused) {
     fft_local2<M>(A, Bf, d.tw, C, +1);
     cross_products_any<M>(X, A, Bf, PE, PM);
@@ -476,14 +460,14 @@ __device__ __noinline__ void rhs_hs2_flat(Ctx<M> X, double t, double2* __restric
       (void)idx;
       dm[u] = __ldg(d.damp + p);
     }
-    fft_inverse2<M>(A, Bf, d.tw, d.N, C, X.c);
+    fft_inverse2<M>(A, Bf, d.tw, C, X.c);
     HW_FOREACH(X) {
       double2 a, b;
       product_point<M>(X, p, A[pidx(idx)], Bf[pidx(idx)], dm[u], PE, PM, a, b);
       A[pidx(idx)] = a;
       Bf[pidx(idx)] = b;
     }
-    fft_forward2<M>(A, Bf, d.tw, d.N, C, X.c);
+    fft_forward2<M>(A, Bf, d.tw, C, X.c);
   }
   // breaking criterion (1d/breaking.c:36-95) on eta, u, H(eta): the transform's
   // barriers made PE / PM complete member-wide

@@ -31,35 +31,36 @@ namespace hwdev {
 // together.  The meeting of cross-CTA steps is cross_products'.
 template <int M, int C, class Op>
 __device__ __forceinline__ void meet_cross(Ctx<M> X, int nin, int nout, const Op& op) {
-  constexpr int T = M / kPts;
-  constexpr int PER = kPts / C;
+  using P = Cross<C>;
+  constexpr int T = M / kPts, R = P::R;
   const DevMember& d = X.d;
   double2 *A = X.buf, *B = X.buf2();
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
 #pragma unroll 1
-  for (int q = 0; q < PER; ++q) {
-    const int i = X.c * T + int(threadIdx.x) + q * (C * T);
-    double2 va[C], vb[C];
+  for (int q = 0; q < P::PER; ++q) {
+    const int i = P::template at<T>(X.c, q);
+    double2 va[R], vb[R];
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      va[r] = cl.map_shared_rank(A, r)[pidx(i)];
-      vb[r] = nin == 2 ? cl.map_shared_rank(B, r)[pidx(i)] : czero();
+    for (int e = 0; e < R; ++e) {
+      va[e] = cl.map_shared_rank(A, P::spectral(e))[pidx(i)];
+      vb[e] = nin == 2 ? cl.map_shared_rank(B, P::spectral(e))[pidx(i)] : czero();
     }
     cross_in<C>(va, d.tw, i);
     if (nin == 2) cross_in<C>(vb, d.tw, i);
 #pragma unroll
-    for (int r = 0; r < C; r += 2) {
-      const typename Op::L l0 = op.load(r * M + i), l1 = op.load((r + 1) * M + i);
-      op(r * M + i, l0, va[r], vb[r]);
-      op((r + 1) * M + i, l1, va[r + 1], vb[r + 1]);
+    for (int e = 0; e < R; e += 2) {
+      const int n0 = P::physical(e) * M + i, n1 = P::physical(e + 1) * M + i;
+      const typename Op::L l0 = op.load(n0), l1 = op.load(n1);
+      op(n0, l0, va[e], vb[e]);
+      op(n1, l1, va[e + 1], vb[e + 1]);
     }
     cross_out<C>(va, d.tw, i);
     if (nout == 2) cross_out<C>(vb, d.tw, i);
 #pragma unroll
-    for (int r = 0; r < C; ++r) {
-      cl.map_shared_rank(A, r)[pidx(i)] = va[r];
-      if (nout == 2) cl.map_shared_rank(B, r)[pidx(i)] = vb[r];
+    for (int e = 0; e < R; ++e) {
+      cl.map_shared_rank(A, P::spectral(e))[pidx(i)] = va[e];
+      if (nout == 2) cl.map_shared_rank(B, P::spectral(e))[pidx(i)] = vb[e];
     }
   }
   cl.sync();
@@ -71,18 +72,19 @@ template <int M, class Op>
 __device__ __noinline__ void meet(Ctx<M> X, int nin, int nout, int it) {
   const DevMember& d = X.d;
   const int C = d.C;
-  if (C == 2 || C == 4 || C == 8) {
+  if (C > 1) {
     if (nin == 2) fft_local2<M>(X.buf, X.buf2(), d.tw, C, +1);
     else fft_local<M>(X.buf, d.tw, C, +1);
     if (C == 2) meet_cross<M, 2>(X, nin, nout, Op(X, it));
     else if (C == 4) meet_cross<M, 4>(X, nin, nout, Op(X, it));
-    else meet_cross<M, 8>(X, nin, nout, Op(X, it));
+    else if (C == 8) meet_cross<M, 8>(X, nin, nout, Op(X, it));
+    else meet_cross<M, 16>(X, nin, nout, Op(X, it));
     if (nout == 2) fft_local2<M>(X.buf, X.buf2(), d.tw, C, -1);
     else fft_local<M>(X.buf, d.tw, C, -1);
     return;
   }
-  if (nin == 2) fft_inverse2<M>(X.buf, X.buf2(), d.tw, d.N, C, X.c);
-  else fft_inverse<M>(X.buf, d.tw, d.N, C, X.c);
+  if (nin == 2) fft_inverse2<M>(X.buf, X.buf2(), d.tw, C, X.c);
+  else fft_inverse<M>(X.buf, d.tw, C, X.c);
   {
     const Op op(X, it);
     double2 *A = X.buf, *B = X.buf2();
@@ -102,8 +104,8 @@ __device__ __noinline__ void meet(Ctx<M> X, int nin, int nout, int it) {
       }
     }
   }
-  if (nout == 2) fft_forward2<M>(X.buf, X.buf2(), d.tw, d.N, C, X.c);
-  else fft_forward<M>(X.buf, d.tw, d.N, C, X.c);
+  if (nout == 2) fft_forward2<M>(X.buf, X.buf2(), d.tw, C, X.c);
+  else fft_forward<M>(X.buf, d.tw, C, X.c);
 }
 
 // How K reference depths fill a sweep's iterations.  First sweep: fields in 0 eta, 1 u, then
