@@ -51,16 +51,11 @@ struct DevMember {
   const double* k;
   const double* aal;
   const double* c1;     // (Csqr/g) k
-  const double* gk;     // g k
-  const double* M0im;   // -k Csqr/g
-  const double* L;      // k^2 Csqr / g
   const double2* gamX;
   const double2* gamXs;
   const double* Csq;    // [nref][N]
   // physical tables, natural order
-  const double* dcoef;
-  const double* dchar;
-  const double* damp;   // dcoef dchar
+  const double* damp;   // damping coefficient times characteristic function
   const double* chi;
   const double* depth;
   const double* gam;    // [nref][N]
@@ -95,7 +90,6 @@ struct DevMember {
   int i_out, i_stop;    // next output index, stop index (exclusive)
   int status, k1_valid;
   long long rhs_calls, accepted, rejected, rhs_budget;
-  double last_rmax;
 };
 
 }  // namespace hwdev

@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -162,6 +163,58 @@ __global__ void k_states_to_reference(const DevMember* __restrict__ mems, double
 // ---------------------------------------------------------------------------
 // host engine
 // ---------------------------------------------------------------------------
+// The mapped pinned buffers of the host calls, kept past their contexts: a new one cost 0.15 to
+// 2.6 ms, a context of 512 points without it 0.9.  At most kKept buffers wait here (of 1 MiB
+// each at most: 4 x 32768 doubles), the others are freed; a buffer whose device was reset
+// meanwhile is no longer pinned and is let go.
+class PinnedBuffers {
+ public:
+  struct Block {
+    double* p = nullptr;
+    size_t n = 0;
+  };
+  cudaError_t take(size_t n, Block& out) {
+    {
+      std::lock_guard<std::mutex> lk(m_);
+      for (size_t i = 0; i < kept_.size();) {
+        unsigned flags = 0;
+        if (cudaHostGetFlags(&flags, kept_[i].p) != cudaSuccess) {
+          cudaGetLastError();
+          kept_.erase(kept_.begin() + long(i));
+        } else if (kept_[i].n >= n) {
+          out = kept_[i];
+          kept_.erase(kept_.begin() + long(i));
+          return cudaSuccess;
+        } else {
+          ++i;
+        }
+      }
+    }
+    out.n = std::max<size_t>(n, 4096);
+    return cudaHostAlloc(&out.p, sizeof(double) * out.n, cudaHostAllocMapped | cudaHostAllocPortable);
+  }
+  void give(Block b) {
+    if (!b.p) return;
+    {
+      std::lock_guard<std::mutex> lk(m_);
+      if (kept_.size() < kKept) {
+        kept_.push_back(b);
+        return;
+      }
+    }
+    cudaFreeHost(b.p);
+  }
+ private:
+  static constexpr size_t kKept = 4;
+  std::mutex m_;
+  std::vector<Block> kept_;
+};
+// (never destroyed: contexts may outlive the statics)
+PinnedBuffers& pinned_buffers() {
+  static PinnedBuffers* p = new PinnedBuffers;
+  return *p;
+}
+
 #define HW_CUDA(call)                                                                       \
   do {                                                                                      \
     cudaError_t e_ = (call);                                                                \
@@ -218,6 +271,7 @@ struct hw_ctx {
   int* d_stops = nullptr;     // stop index of every member for the next launch
   long long* d_prev_rhs = nullptr;   // each member's RHS count when its class was last ordered
   double* d_ref = nullptr;    // 4*maxN staging for reference-layout transfers
+  PinnedBuffers::Block pinned;
   double* h_ref = nullptr;    // the same, mapped and pinned, with a step's (t, h, status)
   int maxN = 0;
   double* d_stage = nullptr;  // all members' states, reference layout, concatenated
@@ -289,7 +343,7 @@ bool hw_ctx::upload_member(HostMember& h) {
   // size the arena
   size_t bytes = 0;
   auto add = [&](size_t b) { bytes += ((b + 255) / 256) * 256; };
-  for (int i = 0; i < 10 + 3; ++i) add(sizeof(double) * N);                 // real tables
+  for (int i = 0; i < 6; ++i) add(sizeof(double) * N);                       // k, aal, c1, damp, chi, depth
   add(sizeof(double2) * N * 2);                                              // gamX, gamXs
   add(sizeof(double) * size_t(N) * std::max(K, 1) * 2);                      // Csq, gam
   for (int i = 0; i < 5; ++i) add(sizeof(double) * std::max(n, 2));          // splines
@@ -326,15 +380,11 @@ bool hw_ctx::upload_member(HostMember& h) {
     if (!v.empty()) cudaMemcpy(p, v.data(), sizeof(double) * std::min(cnt, v.size()), cudaMemcpyHostToDevice);
     return p;
   };
-  std::vector<double> c1(N), gk(N);
-  for (int i = 0; i < N; ++i) {
-    c1[i] = (m.Csqr[i] / hwdev::kG) * m.k[i];
-    gk[i] = hwdev::kG * m.k[i];
-  }
+  std::vector<double> c1(N);
+  for (int i = 0; i < N; ++i) c1[i] = (m.Csqr[i] / hwdev::kG) * m.k[i];
   d.k = up(permute(m.k, N, C, M), N);
   d.aal = up(permute(m.aal, N, C, M), N);
   d.c1 = up(permute(c1, N, C, M), N);
-  d.gk = up(permute(gk, N, C, M), N);
   // first pair index outside the alias band (pair_at's ownership: partners count as
   // their pair's first index; position M / 2 of CTA 0 goes with position 0)
   for (int q = 0; q < N; ++q) {
@@ -343,8 +393,6 @@ bool hw_ctx::upload_member(HostMember& h) {
     const int first = i < M / 2 ? i : (c == 0 ? (M - i) % (M / 2) : M - 1 - i);
     d.act = std::max(d.act, first + 1);
   }
-  d.M0im = up(permute(m.M0im, N, C, M), N);
-  d.L = up(permute(m.L, N, C, M), N);
   {
     std::vector<double> g(2 * N), s(2 * N);
     std::vector<double> pr = permute(m.gamX_re, N, C, M), pi = permute(m.gamX_im, N, C, M);
@@ -363,8 +411,6 @@ bool hw_ctx::upload_member(HostMember& h) {
     d.Csq = up(cs, cs.size());
     d.gam = up(gm, gm.size());
   }
-  d.dcoef = up(m.dampcoef, N);
-  d.dchar = up(m.dampchar, N);
   std::vector<double> damp(N);
   for (int i = 0; i < N; ++i) damp[i] = m.dampcoef[i] * m.dampchar[i];
   d.damp = up(damp, N);
@@ -533,12 +579,13 @@ bool hw_ctx::init(const std::vector<std::string>& dirs, const hw_opts* o, const 
   }
   // Slices.  2048 points fill the GPU best when there are members for every SM.  When
   // there are not, a member's time is its CTA's, and smaller slices put more SMs on it, as
-  // long as no SM is given two CTAs: 512 points up to eight CTAs, 1024 up to sixteen.  Grids
+  // long as few SMs are given two CTAs: 512 points up to eight CTAs, 1024 up to sixteen.  Grids
   // of up to 1024 points stay in one CTA, where no step crosses the cluster.  One member, us an
   // RHS in slices of 2048, 1024, 512 and 256 points: flat HS2 of 2048 points 27 27 24 24, of
   // 4096 37 28 24 30, of 8192 39 28 30, of 16384 41 36; HS3 on a slope (sixteen reference
   // depths) of 4096 367 275 253 302, of 8192 395 303 302, of 16384 430 359; flat of 1024 in
-  // one CTA 20, in two 24.
+  // one CTA 20, in two 24.  Slices of 1024 points may put two CTAs on a few SMs: a run of 17
+  // bathymetries 63 ms in 160 CTAs, 75 in 80 of 2048 points; of 24, 84 in 224 and 79 in 112.
   auto points = [&](size_t i, int least) {
     const int N = mem[i].N;
     if (member_slice && member_slice[i] > 0) return member_slice[i];
@@ -549,7 +596,7 @@ bool hw_ctx::init(const std::vector<std::string>& dirs, const hw_opts* o, const 
   for (; least < 2048; least *= 2) {
     long long ctas = 0;
     for (size_t i = 0; i < mem.size(); ++i) ctas += std::max(1, mem[i].N / points(i, least));
-    if (ctas <= 148) break;
+    if (ctas <= (least == 512 ? 148 : 185)) break;
   }
   for (size_t i = 0; i < dirs.size(); ++i) {
     HostMember& h = mem[i];
@@ -577,7 +624,8 @@ bool hw_ctx::init(const std::vector<std::string>& dirs, const hw_opts* o, const 
   for (size_t i = 0; i < mem.size(); ++i) ids[i] = int(i);
   HW_CUDA(cudaMemcpy(d_single, ids.data(), sizeof(int) * ids.size(), cudaMemcpyHostToDevice));
   HW_CUDA(cudaMalloc(&d_ref, sizeof(double) * 4 * maxN));
-  HW_CUDA(cudaHostAlloc(&h_ref, sizeof(double) * (4 * maxN + kStageTail), cudaHostAllocMapped));
+  HW_CUDA(pinned_buffers().take(size_t(4 * maxN + kStageTail), pinned));
+  h_ref = pinned.p;
   HW_CUDA(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
   stream = own_stream;
   HW_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
@@ -725,7 +773,7 @@ hw_ctx::~hw_ctx() {
   if (d_stops) cudaFree(d_stops);
   if (d_prev_rhs) cudaFree(d_prev_rhs);
   if (d_ref) cudaFree(d_ref);
-  if (h_ref) cudaFreeHost(h_ref);
+  pinned_buffers().give(pinned);
   if (fork) cudaEventDestroy(fork);
   if (own_stream) cudaStreamDestroy(own_stream);
 }
