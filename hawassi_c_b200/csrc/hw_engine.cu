@@ -19,6 +19,7 @@
 #include "../../include/hawassi_b200.h"
 #include "hw_kernels.h"
 #include "hw_kin.h"
+#include "hw_slices.hpp"
 #include "hw_setup.hpp"
 
 using namespace hwdev;
@@ -577,31 +578,24 @@ bool hw_ctx::init(const std::vector<std::string>& dirs, const hw_opts* o, const 
     h.N = N;
     maxN = std::max(maxN, N);
   }
-  // Slices.  2048 points fill the GPU best when there are members for every SM.  When
-  // there are not, a member's time is its CTA's, and smaller slices put more SMs on it, as
-  // long as few SMs are given two CTAs: 512 points up to eight CTAs, 1024 up to sixteen.  Grids
-  // of up to 1024 points stay in one CTA, where no step crosses the cluster.  One member, us an
-  // RHS in slices of 2048, 1024, 512 and 256 points: flat HS2 of 2048 points 27 27 24 24, of
-  // 4096 37 28 24 30, of 8192 39 28 30, of 16384 41 36; HS3 on a slope (sixteen reference
-  // depths) of 4096 367 275 253 302, of 8192 395 303 302, of 16384 430 359; flat of 1024 in
-  // one CTA 20, in two 24.  Slices of 1024 points may put two CTAs on a few SMs: a run of 17
-  // bathymetries 63 ms in 160 CTAs, 75 in 80 of 2048 points; of 24, 84 in 224 and 79 in 112.
-  auto points = [&](size_t i, int least) {
-    const int N = mem[i].N;
-    if (member_slice && member_slice[i] > 0) return member_slice[i];
-    if (opt.slice > 0) return opt.slice;
-    return N <= 1024 ? N : std::min(2048, std::max({least, N / 16, std::min(N / 8, 1024)}));
-  };
-  int least = 512;
-  for (; least < 2048; least *= 2) {
-    long long ctas = 0;
-    for (size_t i = 0; i < mem.size(); ++i) ctas += std::max(1, mem[i].N / points(i, least));
-    if (ctas <= (least == 512 ? 148 : 185)) break;
+  int sms = 0;
+  HW_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  std::vector<int> nx(mem.size()), named(mem.size());
+  for (size_t i = 0; i < mem.size(); ++i) {
+    nx[i] = mem[i].N;
+    named[i] = member_slice && member_slice[i] > 0 ? member_slice[i] : std::max(opt.slice, 0);
   }
+  int fits[9];   // by M / 256, asked once: a query is tens of microseconds
+  std::fill(fits, fits + 9, -1);
+  const std::vector<int> slices = hw::choose_slices(nx, named, sms, [&](int M) {
+    int& f = fits[M / 256];
+    if (f < 0) f = max_clusters_any(M, 16);
+    return f > 0;
+  });
   for (size_t i = 0; i < dirs.size(); ++i) {
     HostMember& h = mem[i];
     const int N = h.N;
-    int C = opt.cluster > 0 ? opt.cluster : std::max(1, N / points(i, least));
+    int C = opt.cluster > 0 ? opt.cluster : std::max(1, N / slices[i]);
     if ((C & (C - 1)) != 0 || N / C < 256 || N / C > 2048 || C > 16) {
       err = "invalid cluster size " + std::to_string(C) + " for Nx=" + std::to_string(N);
       return false;
@@ -833,6 +827,11 @@ int hw_members(const hw_ctx* ctx) { return ctx ? int(ctx->mem.size()) : 0; }
 int hw_nx(const hw_ctx* ctx, int m) {
   if (!ctx || m < 0 || m >= int(ctx->mem.size())) return -1;
   return ctx->mem[size_t(m)].N;
+}
+
+int hw_slice(const hw_ctx* ctx, int m) {
+  if (!ctx || m < 0 || m >= int(ctx->mem.size())) return 0;
+  return ctx->mem[size_t(m)].M;
 }
 
 int hw_nt(const hw_ctx* ctx, int m) {

@@ -33,7 +33,7 @@ def library_path():
 
 
 EXPORTS = [
-    "hw_create", "hw_ensemble_create", "hw_ensemble_create_sliced", "hw_destroy", "hw_last_error", "hw_members", "hw_nx", "hw_nt",
+    "hw_create", "hw_ensemble_create", "hw_ensemble_create_sliced", "hw_destroy", "hw_last_error", "hw_members", "hw_nx", "hw_slice", "hw_nt",
     "hw_initial_state", "hw_rhs", "hw_gsl_rhs", "hw_evolve_apply", "hw_run", "hw_run_to_time",
     "hw_get_state", "hw_set_state", "hw_reset", "hw_member_stats", "hw_last_dydt", "hw_breaking_log",
     "hw_set_stream", "hw_synchronize", "hw_deck_table", "hw_get_states", "hw_set_states",
@@ -68,6 +68,7 @@ def load_library():
     L.hw_last_error.argtypes = [vp]
     L.hw_members.argtypes = [vp]
     L.hw_nx.argtypes = [vp, ip]
+    L.hw_slice.argtypes = [vp, ip]
     L.hw_nt.argtypes = [vp, ip]
     L.hw_initial_state.argtypes = [vp, ip, dp]
     L.hw_rhs.argtypes = [vp, ip, dd, dp, dp]
@@ -127,7 +128,9 @@ class Engine:
     def __init__(self, decks, eps_abs=0.0, eps_rel=0.0, h0=0.0, seed=0, nref=0, exact_sequence=False,
                  cluster=0, device=0, slice=0, slices=None, resident=0):
         """slices: grid points per CTA per grid size ({Nx: points}, e.g. from
-        autotune.autotune_slices) or per member (a list); others use `slice`.
+        autotune.autotune_slices) or per member (a list); others use `slice`
+        (0: by the number of members; Engine.slices says what was taken).  A slice
+        named by the caller gives a deck the same digits in any company.
         resident: the evolve launches' grid (hw_opts.resident): 0 one cluster per
         member, -1 a persistent grid of resident clusters pulling members from a
         queue (sized to the class's share), n > 0 at most n such clusters per class."""
@@ -152,6 +155,7 @@ class Engine:
         self.members = L.hw_members(self._h)
         self.nx = [L.hw_nx(self._h, i) for i in range(self.members)]
         self.nt = [L.hw_nt(self._h, i) for i in range(self.members)]
+        self.slices = [L.hw_slice(self._h, i) for i in range(self.members)]
 
     # -- lifetime ---------------------------------------------------------
     def close(self):

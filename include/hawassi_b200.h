@@ -33,7 +33,12 @@ typedef struct hw_opts {
     int cluster;             /* CTAs per member, power of two (0 = automatic) */
     int device;              /* CUDA device ordinal */
     int slice;               /* grid points per CTA when cluster == 0 (0: 2048, or less where the
-                                members' CTAs would leave SMs idle) */
+                                members' CTAs would leave SMs idle; hw_slice says which).  The
+                                slice sets the order of a transform's sums: with 0 a member's
+                                last digits -- and over a long run its step sequence, in a
+                                breaking run its node decisions -- depend on the members beside
+                                it.  A fixed slice gives a deck the same digits alone, in any
+                                ensemble and in any split of one over ranks */
     int resident;            /* evolve launches of an ensemble: 0 = one cluster per member
                                 (members started longest first); -1 = a persistent grid per
                                 grid-size class, its clusters pulling members (longest first)
@@ -58,6 +63,7 @@ void        hw_destroy(hw_ctx* ctx);
 const char* hw_last_error(const hw_ctx* ctx);   /* ctx may be NULL (last create error) */
 int         hw_members(const hw_ctx* ctx);
 int         hw_nx(const hw_ctx* ctx, int member);
+int         hw_slice(const hw_ctx* ctx, int member); /* grid points per CTA of the member; 0: no such member */
 int         hw_nt(const hw_ctx* ctx, int member); /* output/influx samples of the member */
 
 /* Initial spectral state of set_initial_ode (1d/functions.c:314). */
