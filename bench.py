@@ -91,20 +91,37 @@ def fp64_roofline(flops, ms, device, kernel, basis):
 T_START = time.time()
 
 
-def profile_traffic(workload):
+def profile_traffic(workload, kernel=None):
     """DRAM bytes per RHS grid point of a workload's dominant kernel, from the ncu
     capture recorded in profiles/traffic.json (dram__bytes_read.sum +
     dram__bytes_write.sum of a small capture of the same kernel, divided by the RHS
     points it evaluated).  Returns (bytes per point or None, provenance text); the
     bench scales it to the launch it times, so the figure is profile-derived, not
-    measured in this run."""
+    measured in this run.  `kernel`: what this run launched; a capture of another
+    kernel says nothing about it."""
     try:
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
             rec = json.load(f)[workload]
+        if kernel is not None and rec["kernel"] != kernel:
+            return None, f"no ncu capture of {kernel} (recorded: {rec['kernel']})"
         return float(rec["dram_bytes_per_rhs_pt"]), (
             f"profile-derived: {rec['capture']} ({rec['build']}), scaled by this launch's RHS points")
     except (OSError, KeyError, ValueError, TypeError) as e:
         return None, f"no ncu capture recorded for this workload ({type(e).__name__})"
+
+
+def slices_used(eng):
+    """Grid points per CTA that the engine took, by grid size (a list where members of
+    one grid size differ)."""
+    by = {}
+    for n, m in sorted(set(zip(eng.nx, eng.slices))):
+        by.setdefault(str(n), []).append(m)
+    return {n: m[0] if len(m) == 1 else m for n, m in by.items()}
+
+
+def evolve_kernels(eng):
+    """The evolve kernels of the engine's launches, one instance per slice."""
+    return ", ".join(f"k_evolve<{m}>" for m in sorted(set(eng.slices), reverse=True))
 
 
 def log(msg):
@@ -807,7 +824,7 @@ def main_c2(args, rank, world, local):
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f64",
             "data": "synthetic seeded deck (JONSWAP influx) in the reference input format",
-            "config": {"workload": workload_text, "step_samples": step_samples, "slice": slice_ or 2048,
+            "config": {"workload": workload_text, "step_samples": step_samples, "slice": eng.slices[0],
                        "l2": "single member resident in L2: latency-bound, no roofline claim"},
             "sim_s_per_wall_s": sim / (ms / 1e3), "rhs_calls": s1["rhs_calls"] - s0["rhs_calls"],
             "accepted": s1["accepted"] - s0["accepted"], "rejected": s1["rejected"] - s0["rejected"],
@@ -988,16 +1005,17 @@ def main():
     except OSError:
         pass
     peak = float(peaks.get("hbm_gbs", 6650.0))
-    per_pt, traffic_source = profile_traffic("ensemble")
+    slices_run, kernels = slices_used(eng), evolve_kernels(eng)
+    per_pt, traffic_source = profile_traffic("ensemble", kernels)
     traffic = per_pt * grp_pts if per_pt else None   # bytes over the launch group
     classes = eng.class_timing()
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic, "traffic_source": traffic_source, "kernel": "k_evolve<2048>",
+            "traffic": traffic, "traffic_source": traffic_source, "kernel": kernels,
             "launch": f"one step = {len(classes)} concurrent launches (one per grid-size class), "
                       f"{gms:.2f} ms, {grp_pts:.3e} RHS grid points, {BYTES_PER_RHS_PT:.1f} algorithmic B/point",
             "class_ms": [round(c[0], 3) for c in classes],
             "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if "hbm_gbs" in peaks else "fallback"}
-    roof_fp64 = fp64_roofline(rhs_flops() - flops_a, gms, local, "k_evolve<2048>",
+    roof_fp64 = fp64_roofline(rhs_flops() - flops_a, gms, local, kernels,
                               f"{FFTS_PER_RHS_1D} c2c transforms x 5 log2(Nx) + {POINTWISE_FLOPS:.0f} "
                               "pointwise flops per RHS point, per member")
 
@@ -1054,7 +1072,7 @@ def main():
             "dtype": "f64",
             "data": "synthetic seeded decks (JONSWAP influx, flat depths) in the reference input format",
             "config": ensemble_config(args),
-            "slices": ({str(k): v for k, v in slices.items()} if slices else "2048 (default)"),
+            "slices": slices_run,
             "ensemble_summary": summary,
             "rhs_points_per_step": tot_pts / args.steps,
             "sim_s_per_wall_s": tot_sim / (ms / 1e3),
