@@ -7,8 +7,8 @@ whole ensemble the highest RHS throughput, measured on the device.
 
 The grid-size classes run concurrently and share the GPU, so a class's best shape
 depends on the others: the tuner does coordinate descent on the whole ensemble,
-starting from the default shape (2048-point slices), changing one class's slice at a
-time and keeping a change only when the ensemble's throughput over the same simulated
+starting from the slices that the engine takes by itself, changing one class's slice at
+a time and keeping a change only when the ensemble's throughput over the same simulated
 interval (`warm` windows, then a timed window of `window` output samples) improves.
 """
 import time
@@ -34,7 +34,7 @@ def _measure(decks, nxs, slices, window, warm, device, eps_abs, eps_rel):
         eng.run(i_stop, sync=True)
         dt = time.perf_counter() - t0
         p1 = sum(eng.stats(m)["rhs_calls"] * nxs[m] for m in range(eng.members))
-        return (p1 - p0) / max(dt, 1e-12)
+        return (p1 - p0) / max(dt, 1e-12), dict(zip(nxs, eng.slices))
     finally:
         eng.close()
 
@@ -44,9 +44,8 @@ def autotune_slices(decks, candidates=(2048, 1024, 512), window=5, warm=2, devic
     """Returns ({Nx: slice}, [(slices tried, RHS grid points / s), ...])."""
     nxs = [int(deck_table(d, "Nx")[0]) for d in decks]
     classes = sorted(set(nxs), reverse=True)
-    cur = {nx: next(s for s in (2048, 1024, 512, 256) if _valid(nx, s)) for nx in classes}
     trials = []
-    best = _measure(decks, nxs, dict(cur), window, warm, device, eps_abs, eps_rel)
+    best, cur = _measure(decks, nxs, None, window, warm, device, eps_abs, eps_rel)
     trials.append((dict(cur), best))
     if log:
         log(f"autotune start {cur}: {best:.3e} RHS-pt/s")
@@ -57,7 +56,7 @@ def autotune_slices(decks, candidates=(2048, 1024, 512), window=5, warm=2, devic
             trial = dict(cur)
             trial[nx] = s
             try:
-                v = _measure(decks, nxs, trial, window, warm, device, eps_abs, eps_rel)
+                v, _ = _measure(decks, nxs, trial, window, warm, device, eps_abs, eps_rel)
             except EngineError:
                 continue
             trials.append((dict(trial), v))
