@@ -12,13 +12,13 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/hawassi_b200.h"
 #include "hw_kernels.h"
 #include "hw_kin.h"
+#include "hw_pinned.hpp"
 #include "hw_slices.hpp"
 #include "hw_setup.hpp"
 
@@ -164,55 +164,9 @@ __global__ void k_states_to_reference(const DevMember* __restrict__ mems, double
 // ---------------------------------------------------------------------------
 // host engine
 // ---------------------------------------------------------------------------
-// The mapped pinned buffers of the host calls, kept past their contexts: a new one cost 0.15 to
-// 2.6 ms, a context of 512 points without it 0.9.  At most kKept buffers wait here (of 1 MiB
-// each at most: 4 x 32768 doubles), the others are freed; a buffer whose device was reset
-// meanwhile is no longer pinned and is let go.
-class PinnedBuffers {
- public:
-  struct Block {
-    double* p = nullptr;
-    size_t n = 0;
-  };
-  cudaError_t take(size_t n, Block& out) {
-    {
-      std::lock_guard<std::mutex> lk(m_);
-      for (size_t i = 0; i < kept_.size();) {
-        unsigned flags = 0;
-        if (cudaHostGetFlags(&flags, kept_[i].p) != cudaSuccess) {
-          cudaGetLastError();
-          kept_.erase(kept_.begin() + long(i));
-        } else if (kept_[i].n >= n) {
-          out = kept_[i];
-          kept_.erase(kept_.begin() + long(i));
-          return cudaSuccess;
-        } else {
-          ++i;
-        }
-      }
-    }
-    out.n = std::max<size_t>(n, 4096);
-    return cudaHostAlloc(&out.p, sizeof(double) * out.n, cudaHostAllocMapped | cudaHostAllocPortable);
-  }
-  void give(Block b) {
-    if (!b.p) return;
-    {
-      std::lock_guard<std::mutex> lk(m_);
-      if (kept_.size() < kKept) {
-        kept_.push_back(b);
-        return;
-      }
-    }
-    cudaFreeHost(b.p);
-  }
- private:
-  static constexpr size_t kKept = 4;
-  std::mutex m_;
-  std::vector<Block> kept_;
-};
 // (never destroyed: contexts may outlive the statics)
-PinnedBuffers& pinned_buffers() {
-  static PinnedBuffers* p = new PinnedBuffers;
+hw::PinnedBuffers& pinned_buffers() {
+  static hw::PinnedBuffers* p = new hw::PinnedBuffers;
   return *p;
 }
 
@@ -272,8 +226,9 @@ struct hw_ctx {
   int* d_stops = nullptr;     // stop index of every member for the next launch
   long long* d_prev_rhs = nullptr;   // each member's RHS count when its class was last ordered
   double* d_ref = nullptr;    // 4*maxN staging for reference-layout transfers
-  PinnedBuffers::Block pinned;
-  double* h_ref = nullptr;    // the same, mapped and pinned, with a step's (t, h, status)
+  hw::PinnedBuffers::Block pinned;
+  double* h_ref = nullptr;    // the same, mapped and pinned, with a step's (t, h, status);
+  double* h_ref_dev = nullptr;   // the device's address of it
   int maxN = 0;
   double* d_stage = nullptr;  // all members' states, reference layout, concatenated
   long long* d_off = nullptr; // offset of each member in d_stage
@@ -620,6 +575,7 @@ bool hw_ctx::init(const std::vector<std::string>& dirs, const hw_opts* o, const 
   HW_CUDA(cudaMalloc(&d_ref, sizeof(double) * 4 * maxN));
   HW_CUDA(pinned_buffers().take(size_t(4 * maxN + kStageTail), pinned));
   h_ref = pinned.p;
+  h_ref_dev = pinned.dev;
   HW_CUDA(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
   stream = own_stream;
   HW_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
@@ -853,10 +809,10 @@ int hw_rhs(hw_ctx* ctx, int m, double t, const double* y, double* dydt) {
     HostMember& h = ctx->mem[size_t(m)];
     const int N = h.N;
     std::memcpy(ctx->h_ref, y, sizeof(double) * 4 * N);
-    k_to_internal<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ctx->h_ref, h.d.zs, N, h.logC, h.M);
+    k_to_internal<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ctx->h_ref_dev, h.d.zs, N, h.logC, h.M);
     HW_CUDA(cudaGetLastError());
     HW_CUDA(rhs_any(h.M, ctx->d_mems, m, h.C, t, ctx->stream));
-    k_call_end<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ctx->d_mems, m, false, ctx->h_ref);
+    k_call_end<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ctx->d_mems, m, false, ctx->h_ref_dev);
     HW_CUDA(cudaGetLastError());
     HW_CUDA(cudaStreamSynchronize(ctx->stream));
     std::memcpy(dydt, ctx->h_ref, sizeof(double) * 4 * N);
@@ -924,10 +880,10 @@ int hw_evolve_apply(hw_ctx* ctx, int m, double* t, double t1, double* h, double*
     const HostMember& hm = ctx->mem[size_t(m)];
     const int N = hm.N;
     std::memcpy(ctx->h_ref, y, sizeof(double) * 4 * N);
-    k_step_begin<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ctx->d_mems, m, ctx->h_ref, *t, *h, t1);
+    k_step_begin<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ctx->d_mems, m, ctx->h_ref_dev, *t, *h, t1);
     HW_CUDA(cudaGetLastError());
     HW_CUDA(evolve_any(hm.M, 1, ctx->d_mems, ctx->d_single + m, 1, hm.C, ctx->stream));
-    k_call_end<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ctx->d_mems, m, true, ctx->h_ref);
+    k_call_end<<<(N + 255) / 256, 256, 0, ctx->stream>>>(ctx->d_mems, m, true, ctx->h_ref_dev);
     HW_CUDA(cudaGetLastError());
     HW_CUDA(cudaStreamSynchronize(ctx->stream));
     const double* tail = ctx->h_ref + 4 * N;
