@@ -418,11 +418,12 @@ bool room(float*& p, size_t& have, size_t count) {
 // go to the device minibatch by minibatch while the first epoch's steps run, and nothing
 // waits for a step's loss: the minibatches' sums come back once, at the end.
 int hw_mlp_train(hw_mlp* mlp, const float* data_host, int n, int epochs, int batch, float lr, float* losses) {
-  if (n < 0 || batch <= 0) { mlp->err = "training: n must not be negative, batch must be positive"; return 1; }
-  if (n == 0 || epochs <= 0) {   // no step to take: the mean loss of no records
+  if (n < 0) { mlp->err = "training: n must not be negative"; return 1; }
+  if (n == 0 || epochs <= 0) {   // no step to take, whatever the batch: the mean loss of no records
     for (int ep = 0; losses && ep < epochs; ++ep) losses[ep] = std::nanf("");
     return 0;
   }
+  if (batch <= 0) { mlp->err = "training: batch must be positive"; return 1; }
   const int per = (n - 1) / batch + 1;
   if (!room(mlp->records, mlp->record_floats, size_t(n) * kRec) ||
       !room(mlp->losses, mlp->loss_floats, size_t(per) * epochs)) {
