@@ -154,8 +154,7 @@ __device__ __forceinline__ void put(double2* sm, int M, int s, int i, double2 v)
 // CTAs that an SM's registers hold at 128 a thread (16 points and their twiddles).
 // 256 and 512 threads at 1024 points, one CTA less an SM, took 764 us an RHS against 665.
 __host__ __device__ constexpr int ctas(int threads) { return 512 / threads; }
-__host__ __device__ constexpr int thr2(int) { return 128; }
-__host__ __device__ constexpr int thr4(int) { return 256; }
+constexpr int kThr2 = 128, kThr4 = 256;
 
 // slices [s0, s0 + ns) by a CTA of NT threads, NT / (M/16) at a time; CTA-wide
 // barriers on entry and exit (the phases around read and write every slice).  Sixteen
@@ -560,11 +559,11 @@ __device__ __forceinline__ void stage_extras(const Tab2& tb, const Work2& w, con
 //    0 (eta, u); 1 (v, L phi) under HS2, (v, M0u) under HS3, (v, -) under HS1; 2 (M0v, -)
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2_rowA(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, Ctl2* ctlw, int mode, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = M, Ny = tb.ny, f = blockIdx.y;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, Ny);
@@ -603,11 +602,11 @@ k2_rowA(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, Ctl2* ctlw, int mode, in
 //    1 (eta v, deletaH2), under HS3 2 (eta^2 M0u, eta^2 M0v), then the loss fields.
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2_colB(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = tb.nx, c = blockIdx.x, nd = damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
   const bool hs3 = tb.model == 3;
@@ -646,11 +645,11 @@ k2_colB(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 //    goes to physical space.
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2_rowC(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = M, Ny = tb.ny, nd = damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
   const bool hs3 = tb.model == 3;
@@ -707,11 +706,11 @@ __device__ __forceinline__ double2 cubic_products(const Tab2& tb, const Work2& w
   return make_double2(eta * lel + 0.5 * (eta * eta * divg * wc), lphi * eta * divg + lphi * lel);
 }
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2_colH3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, c = blockIdx.x;
   const size_t n = (size_t)tb.n;
   col_load<M, NT>(sm, 0, 1, w.R, Nx, c, n);
@@ -727,11 +726,11 @@ k2_colH3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   col_store<M, NT>(sm, 0, 1, w.Q, Nx, c, n);
 }
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2_rowI3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = M;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, tb.ny);
@@ -763,11 +762,11 @@ k2_rowI3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 //    intermediate is kept (the Nyquist column of S(A) is not Hermitian).
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2_colD(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, c = blockIdx.x, f = blockIdx.y;
   const size_t n = (size_t)tb.n;
   const bool loss = f < 2 || !w.dph;
@@ -802,11 +801,11 @@ __device__ __forceinline__ double2 delphi_h1(const Tab2& tb, const Work2& w, siz
   return cadd(mul_mi(w.z[n + q], cg * kx), mul_mi(w.z[2 * n + q], cg * ky));
 }
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2_rowE(Tab2 tb, Work2 w, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int cond, double2* __restrict__ direct_out) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = M, f = blockIdx.y;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, tb.ny);
@@ -842,11 +841,11 @@ k2_rowE(Tab2 tb, Work2 w, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int co
 // physical space) -> their damping; row pass: dt Z.
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2_colH1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = tb.nx, c = blockIdx.x;
   const size_t n = (size_t)tb.n;
   if (!tb.var) {
@@ -876,11 +875,11 @@ k2_colH1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   col_store<M, NT>(sm, 0, 2, w.Q, Nx, c, n);
 }
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2_rowH1(Tab2 tb, Work2 w, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int cond, double2* __restrict__ direct_out) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = M;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, tb.ny);

@@ -170,12 +170,12 @@ __device__ __forceinline__ double gyat(const double* a, int st, int Nx, int Ny, 
 // rowI: S(delphiH^) into dt eta^, and E(S(delphiH^)) + i E(S(HilbEta^)) -> inverse rows
 // ---------------------------------------------------------------------------
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2b_rowI(Tab2 tb, Work2 w, Brk2 b, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int cond,
          double2* __restrict__ direct_out) {
   if (!rhs_active(ctl, cond) || !brk_update(ctl, mode)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, Ny = tb.ny;
   const Pair P = row_pair(blockIdx.x, Ny);
   double2* out = rhs_out(rk, ctl, mode, direct_out);
@@ -216,11 +216,11 @@ k2b_rowI(Tab2 tb, Work2 w, Brk2 b, RK2 rk, const Ctl2* __restrict__ ctl, int mod
 
 // colI: inverse column FFT -> delphi (real part) and HilbEta (imaginary part) / N
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2b_colI(Tab2 tb, Brk2 b, const Ctl2* __restrict__ ctl, int mode, int cond) {
   if (!rhs_active(ctl, cond) || !brk_update(ctl, mode)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx;
   const int c = blockIdx.x;
   if (c == 0 && threadIdx.x == 0) b.st->npeaks = 0;
@@ -565,11 +565,11 @@ __global__ void k2b_flux(Tab2 tb, Work2 w, Brk2 b, const Ctl2* __restrict__ ctl,
 // sbcol: fun_gradient (periodic forward / backward differences, clipped), Sb = grad
 // Flux / (eta - bathy), Sb_x + i Sb_y -> forward column FFT
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2b_sbcol(Tab2 tb, Work2 w, Brk2 b, const Ctl2* __restrict__ ctl, int mode, int cond) {
   if (!rhs_active(ctl, cond) || !brk_update(ctl, mode) || b.st->sb_zero) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, Ny = tb.ny;
   const int c = blockIdx.x;
   const double* f = b.flux;
@@ -596,11 +596,11 @@ k2b_sbcol(Tab2 tb, Work2 w, Brk2 b, const Ctl2* __restrict__ ctl, int mode, int 
 // sbrow: forward row FFT and split -> Sb_xhat, Sb_yhat (on an update with B > 0),
 // then dt u^ += Sb_xhat aal, dt v^ += Sb_yhat aal whenever Sb is not zero
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2b_sbrow(Tab2 tb, Brk2 b, RK2 rk, const Ctl2* __restrict__ ctl, int mode, int cond, double2* __restrict__ direct_out) {
   if (!rhs_active(ctl, cond) || b.st->sb_zero) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, Ny = tb.ny;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, Ny);

@@ -76,7 +76,7 @@ void set_attrs() {
 template <int M>
 void launch_out(int which, int nblocks, cudaStream_t s, const Tab2& tb, const double2* z, double2* P, double* phys,
                 float* f32) {
-  const int blk = hw2d::thr2(M);
+  const int blk = hw2d::kThr2;
   if (which == 0) hw2d::k2o_row<M><<<nblocks, blk, smem_bytes<M>(4), s>>>(tb, z, P);
   else hw2d::k2o_col<M><<<nblocks, blk, smem_bytes<M>(4), s>>>(tb, P, phys, f32);
 }
@@ -94,7 +94,7 @@ void out_pass(int M, int which, int nb, cudaStream_t s, const Tab2& tb, const do
 // the flat bottom's wall round trip (row M = nx, column M = ny)
 template <int M>
 void launch_wall(int which, int nblocks, cudaStream_t s, const Tab2& tb, const Work2& w, const Ctl2* ctl, int cond) {
-  const int blk = hw2d::thr2(M);
+  const int blk = hw2d::kThr2;
   if (which == 0) hw2d::k2w_row1<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, ctl, cond);
   else if (which == 1) hw2d::k2w_col2<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, ctl, cond);
   else if (which == 2) hw2d::k2w_row3<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, ctl, cond);
@@ -116,14 +116,14 @@ void wall_pass(int M, int which, int nb, cudaStream_t s, const Tab2& tb, const W
 template <int M>
 void launch_brk_row(int which, int nblocks, cudaStream_t s, const Tab2& tb, const Work2& w, const hw2d::Brk2& b,
                     const RK2& rk, const Ctl2* ctl, int mode, int cond, double2* out) {
-  const int blk = hw2d::thr2(M);
+  const int blk = hw2d::kThr2;
   if (which == 0) hw2d::k2b_rowI<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, b, rk, ctl, mode, cond, out);
   else hw2d::k2b_sbrow<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, b, rk, ctl, mode, cond, out);
 }
 template <int M>
 void launch_brk_col(int which, int nblocks, cudaStream_t s, const Tab2& tb, const Work2& w, const hw2d::Brk2& b,
                     const Ctl2* ctl, int mode, int cond) {
-  const int blk = hw2d::thr2(M);
+  const int blk = hw2d::kThr2;
   if (which == 0) hw2d::k2b_colI<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, b, ctl, mode, cond);
   else hw2d::k2b_sbcol<M><<<nblocks, blk, smem_bytes<M>(2), s>>>(tb, w, b, ctl, mode, cond);
 }
@@ -166,7 +166,7 @@ template <int M>
 void launch_row(RowPass which, int cubic, const PassArgs& a) {
   const Tab2& tb = a.tb;
   const int nb = tb.ny / 2;
-  const int t2 = hw2d::thr2(M), t4 = hw2d::thr4(M);
+  const int t2 = hw2d::kThr2, t4 = hw2d::kThr4;
   switch (which) {
     case kRowA:
       hw2d::k2_rowA<M><<<dim3(nb, tb.model == 3 ? 3 : 2), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.ctl, a.mode, a.cond);
@@ -187,7 +187,7 @@ template <int M>
 void launch_col(ColPass which, int cubic, const PassArgs& a) {
   const Tab2& tb = a.tb;
   const int nb = tb.nx / 2;
-  const int t2 = hw2d::thr2(M), t4 = hw2d::thr4(M);
+  const int t2 = hw2d::kThr2, t4 = hw2d::kThr4;
   switch (which) {
     case kColB: hw2d::k2_colB<M><<<nb, t4, smem_bytes<M>(6), a.s>>>(tb, a.w, a.ctl, a.cond); break;
     case kColD: hw2d::k2_colD<M><<<dim3(nb, 3), t2, smem_bytes<M>(2), a.s>>>(tb, a.w, a.ctl, a.cond); break;
@@ -529,7 +529,6 @@ hw2d_ctx* hw2d_create(const hw2d_tables* t, const hw_opts* o) {
     g_err2d = "hw2d_create: HS1 runs no breaking process (rhs_AB1_2DF_uv, rhs_AB1_2DB_uv); pass breaking = 0";
     return nullptr;
   }
-  (void)var_tables;
   if (t->propagation < 0 || t->propagation > 2) {
     g_err2d = "hw2d_create: propagation must be 0 (Uni+), 1 (Uni-) or 2 (Bi)";
     return nullptr;

@@ -17,10 +17,10 @@
 namespace hw2d {
 
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2o_row(Tab2 tb, const double2* __restrict__ z, double2* __restrict__ P) {
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, Ny = tb.ny;
   const size_t n = (size_t)tb.n;
   const Pair pr = row_pair(blockIdx.x, Ny);
@@ -48,10 +48,10 @@ k2o_row(Tab2 tb, const double2* __restrict__ z, double2* __restrict__ P) {
 
 // phys: eta, u, v (3 n doubles); f32: the same as floats (nullptr: not kept)
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2o_col(Tab2 tb, const double2* __restrict__ P, double* __restrict__ phys, float* __restrict__ f32) {
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx;
   const size_t n = (size_t)tb.n;
   const int c = blockIdx.x;

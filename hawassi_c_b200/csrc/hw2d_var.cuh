@@ -29,11 +29,11 @@ namespace hw2d {
 
 // V1: one CTA per row pair and field (blockIdx.y): 0 (eta, u), 1 (v, -), 2 + j
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2v_row1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, Ctl2* ctlw, int mode, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = M, f = blockIdx.y;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, tb.ny);
@@ -70,11 +70,11 @@ k2v_row1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, Ctl2* ctlw, int mode, i
 // V2: slices 0, 1 the sum, 2..5 two references at a time.  Fields out: 0 the sum
 // (u in the real, v in the imaginary part), 1 + j (gam_j u, gam_j v).
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2v_col2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = tb.nx, c = blockIdx.x, K = tb.nk;
   const size_t n = (size_t)tb.n;
   const double invN = 1.0 / ((double)tb.n);
@@ -118,11 +118,11 @@ k2v_col2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 // at a time, 2, 3 the sum's kx part at the points that the symmetrisation keeps (columns up
 // to Nx / 2)
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2v_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = M, K = tb.nk;
   const size_t n = (size_t)tb.n;
   const bool hs3 = tb.model == 3;
@@ -198,11 +198,11 @@ __device__ __forceinline__ int products(const Tab2& tb, int cubic) { return cubi
 // 2 (eta^2 M0u, eta^2 M0v), the loss fields; q = eta L phi.  cubic = 1: L q, div(grad phi) in;
 // field 0 (p, h3); q = p.
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2v_col4(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = tb.nx, c = blockIdx.x, K = tb.nk, nd = cubic ? 0 : damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
   const bool hs3 = tb.model == 3;
@@ -256,11 +256,11 @@ k2v_col4(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
 // (delu + delv, deletaH, and 1/2 sum_j Omega_j F(gam_j q) / g), and Omega_j q^ goes to
 // physical space, two references to a field
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2v_row5(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = M, K = tb.nk, nd = cubic ? 0 : damp_fields(tb, w);
   const size_t n = (size_t)tb.n;
   const bool hs3 = tb.model == 3;
@@ -347,11 +347,11 @@ k2v_row5(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
 
 // V6: slices 0, 1 the sum of the weighted images (real), 2..5 four references at a time
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2v_col6(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = tb.nx, c = blockIdx.x, K = tb.nk;
   const size_t n = (size_t)tb.n;
   const double invN = 1.0 / ((double)tb.n);
@@ -380,11 +380,11 @@ k2v_col6(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 // operand's enters delu + delv with a minus, the cubic one's with a plus; under HS3 the
 // former, with div(grad phi), goes to physical space for the cubic products.
 template <int M>
-__global__ void __launch_bounds__(thr4(M), ctas(thr4(M)))
+__global__ void __launch_bounds__(kThr4, ctas(kThr4))
 k2v_row7(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond, int cubic) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr4(M);
+  constexpr int NT = kThr4;
   const int Nx = M;
   const size_t n = (size_t)tb.n;
   const bool more = tb.model == 3 && !cubic;

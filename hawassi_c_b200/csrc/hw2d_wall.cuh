@@ -23,11 +23,11 @@
 namespace hw2d {
 
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2w_row1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, Ny = tb.ny;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, Ny);
@@ -53,11 +53,11 @@ k2w_row1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 }
 
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2w_col2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx;
   const int c = blockIdx.x;
   const size_t n = (size_t)tb.n;
@@ -77,11 +77,11 @@ k2w_col2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 }
 
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2w_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, Ny = tb.ny;
   const Pair P = row_pair(blockIdx.x, Ny);
   row_load<M, NT>(sm, 0, 1, w.WP, P, (size_t)tb.n);
@@ -102,11 +102,11 @@ k2w_row3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 }
 
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2w_rowV1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, Ny = tb.ny;
   const size_t n = (size_t)tb.n;
   const Pair P = row_pair(blockIdx.x, Ny);
@@ -147,11 +147,11 @@ k2w_rowV1(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 }
 
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2w_colV2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx;
   const size_t n = (size_t)tb.n;
   const int c = blockIdx.x;
@@ -171,11 +171,11 @@ k2w_colV2(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
 }
 
 template <int M>
-__global__ void __launch_bounds__(thr2(M), ctas(thr2(M)))
+__global__ void __launch_bounds__(kThr2, ctas(kThr2))
 k2w_rowV3(Tab2 tb, Work2 w, const Ctl2* __restrict__ ctl, int cond) {
   if (!rhs_active(ctl, cond)) return;
   extern __shared__ double2 sm[];
-  constexpr int NT = thr2(M);
+  constexpr int NT = kThr2;
   const int Nx = tb.nx, Ny = tb.ny;
   const Pair P = row_pair(blockIdx.x, Ny);
   row_load<M, NT>(sm, 0, 1, w.WP, P, (size_t)tb.n);

@@ -10,7 +10,7 @@ namespace hwdev {
 
 constexpr double kG = 9.80665;       // gravity (1d/header.h:27)
 constexpr double kDelb = 1.2;        // breaking coefficient delta_b (1d/header.h:29)
-constexpr int kScratch = 12;         // N-point double2 scratch arrays per member
+constexpr int kScratch = 11;         // N-point double2 scratch arrays per member
 constexpr int kMaxRef = 16;          // reference depths of the varying-depth operator
 
 // status codes stored per member (mirrors GSL: 0 success)

@@ -1,9 +1,9 @@
 // hw_noalloc.cu -- one RHS evaluation that allocates no device memory.
 //
-// Its scratch (the stage input, the RHS output and the twelve intermediate
+// Its scratch (the stage input, the RHS output and the intermediate
 // fields of the RHS) lives in the file-scope array g_rhs_scratch below instead
 // of per-context cudaMalloc'd buffers.  Every GPU that loads this library holds
-// the array (1 MiB) until the process exits.  Host code cannot pass the array's
+// the array (960 KiB) until the process exits.  Host code cannot pass the array's
 // name to a kernel: the name is a host-side stand-in, not a device address.  The
 // device address is fetched once per device with cudaGetSymbolAddress (with that
 // device current) on the first call and reused.
@@ -24,7 +24,7 @@ namespace {
 using namespace hwdev;
 
 constexpr int kNoAllocMaxNx = 4096;   // largest grid the static scratch covers
-constexpr int kSlots = 16;            // 2N stage input + 2N output + 12 N fields, in N double2 units
+constexpr int kSlots = 4 + kScratch;  // 2N stage input + 2N output + the fields, in N double2 units
 static __device__ __align__(256) double2 g_rhs_scratch[size_t(kSlots) * kNoAllocMaxNx];
 
 constexpr int kMaxDevices = 128;
