@@ -89,6 +89,8 @@ def fp64_roofline(flops, ms, device, kernel, basis):
 
 
 T_START = time.time()
+# the kernels of one right-hand side of the 2D workload
+KERNELS_2D = "k2_stage, k2v_row1..k2v_row7, k2_colD, k2_rowE, k2b_*"
 
 
 def profile_traffic(workload, kernel=None):
@@ -488,16 +490,16 @@ def main_2d(args, rank, world, local):
     except OSError:
         pass
     peak = float(peaks.get("hbm_gbs", 6650.0))
-    per_pt, traffic_source = profile_traffic("2d")
+    per_pt, traffic_source = profile_traffic("2d", KERNELS_2D)
     traffic = per_pt * pts / max(1, args.steps) / (world or 1) if per_pt else None
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "traffic_source": traffic_source,
-            "kernel": "k2v_rowA..k2b_sbrow (one RHS = 9 fused FFT passes + the breaking kernels)",
+            "kernel": KERNELS_2D + " (one RHS = the stage input, 9 fused FFT passes, the breaking kernels)",
             "launch": f"one step = {STEP_2D} simulated s, {pts / max(1, args.steps):.3e} RHS grid points, "
                       f"{BYTES_PER_RHS_PT_2D:.1f} algorithmic B/point",
             "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if "hbm_gbs" in peaks else "fallback"}
     roof_fp64 = fp64_roofline(pts / max(1, world) * flops_per_rhs_pt(n, FFTS_PER_RHS_2D), ms, local,
-                              "k2v_rowA..k2b_sbrow",
+                              KERNELS_2D,
                               f"{FFTS_PER_RHS_2D} 2D c2c transforms x 5 log2(Nx Ny) + {POINTWISE_FLOPS:.0f} "
                               "pointwise flops per RHS point")
     # end to end through the public API: host state in (pinned), evolve, host state out
