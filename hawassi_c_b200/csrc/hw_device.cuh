@@ -10,7 +10,10 @@ namespace hwdev {
 
 constexpr double kG = 9.80665;       // gravity (1d/header.h:27)
 constexpr double kDelb = 1.2;        // breaking coefficient delta_b (1d/header.h:29)
-constexpr int kScratch = 11;         // N-point double2 scratch arrays per member
+// N-point double2 scratch arrays per member.  sc[9] is spare: with eleven arrays, and so another
+// layout of the descriptor and the member's arena, a 4096-point tank's run took 14.81 ms for
+// 14.66 and the 256-member ensemble's 60.2 for 59.6
+constexpr int kScratch = 12;
 constexpr int kMaxRef = 16;          // reference depths of the varying-depth operator
 
 // status codes stored per member (mirrors GSL: 0 success)

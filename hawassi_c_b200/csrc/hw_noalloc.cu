@@ -3,7 +3,7 @@
 // Its scratch (the stage input, the RHS output and the intermediate
 // fields of the RHS) lives in the file-scope array g_rhs_scratch below instead
 // of per-context cudaMalloc'd buffers.  Every GPU that loads this library holds
-// the array (960 KiB) until the process exits.  Host code cannot pass the array's
+// the array (1 MiB) until the process exits.  Host code cannot pass the array's
 // name to a kernel: the name is a host-side stand-in, not a device address.  The
 // device address is fetched once per device with cudaGetSymbolAddress (with that
 // device current) on the first call and reused.

@@ -414,7 +414,7 @@ __device__ __noinline__ void finish_rhs(Ctx<M> X, double2* __restrict__ dz, cons
   }
   // kinematic breaking: the eddy-viscosity force on the u-equation takes slice A, so
   // the adjusted terms move to global memory; the damping stays in slice B
-  double2 *AE = d.sc[2], *AU = d.sc[3], *RB = d.sc[10];
+  double2 *AE = d.sc[2], *AU = d.sc[3], *RB = d.sc[11];
   const PairBufs<M> pb(X);
 #pragma unroll 1
   for (int u = 0; u < kPts / 2; ++u) {

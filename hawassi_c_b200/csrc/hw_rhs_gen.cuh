@@ -383,7 +383,7 @@ __device__ __noinline__ void rest_spectral(Ctx<M> X, int it, int nout) {
   const int N = d.N, K = refs(X), at = rest_plan(K).at, last = it + 1 == rest_plan(K).nit;
   const bool hs3 = d.model == 3, brk = d.brk != 0, final_sweep = CUBIC || !hs3;
   const double invN = d.invN;
-  double2 *AE = d.sc[2], *AU = d.sc[3], *acc = d.sc[4], *Q = d.sc[9];
+  double2 *AE = d.sc[2], *AU = d.sc[3], *acc = d.sc[4], *Q = d.sc[10];
   const double2* ZE = d.zs;
   const double* __restrict__ kt = d.k;
   const double* __restrict__ c1t = d.c1;
@@ -498,7 +498,7 @@ __device__ __forceinline__ void rest_sweep(Ctx<M> X, double t) {
 
 // Scratch fields: sc[0] eta, u in physical space; sc[1] M0 u with H(eta) or d_x u; sc[2], sc[3]
 // spectral terms; sc[4] spectral and sc[5] physical sum of an HSS; sc[6] M0 u^; sc[7] L (eta M0 u)
-// with H(eta); sc[8] the breaking flux; sc[9] the operand's spectrum; sc[10] the breaking force.
+// with H(eta); sc[8] the breaking flux; sc[10] the operand's spectrum; sc[11] the breaking force.
 template <int M>
 __device__ __noinline__ void rhs_gen(Ctx<M> X, double t, double2* __restrict__ dz) {
   const int C = X.d.C;

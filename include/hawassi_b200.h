@@ -82,7 +82,7 @@ int hw_gsl_rhs(double t, const double* y, double* dydt, void* params);
  * under a device-memory budget managed by another framework's pool, or that must
  * not trigger allocations between set-up and tear-down).  y_dev and dydt_dev are
  * DEVICE pointers (4*Nx doubles, reference layout) owned by the caller; the call
- * allocates nothing: its scratch is a 960 KiB static device array held by every GPU
+ * allocates nothing: its scratch is a 1 MiB static device array held by every GPU
  * that loads the library, so Nx is limited to 4096 (larger grids are rejected with
  * an error).  The first call on a device looks up the array's device address (once
  * per device, under a lock); make that call before any stream capture.  All calls share the one array: calls that overlap on
